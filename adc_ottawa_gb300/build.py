@@ -32,6 +32,7 @@ SOURCES = [
     ("build_kernels.cu", ["--fmad=false"]),
     ("sigma.cu", []),
     ("sigma_umma.cu", []),
+    ("sigma_slices.cu", []),
     ("sigma_ab.cu", []),
     ("dense.cu", []),
     ("dense_umma.cu", []),

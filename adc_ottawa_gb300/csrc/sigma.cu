@@ -570,6 +570,121 @@ __global__ void __launch_bounds__(256) k_sigma_p3(GeomDev g, const int2* __restr
   }
 }
 
+// Segment A of the classes with a' < b' (W1 and W2 parts) beside the sliced
+// tensor-core pass: one warp per run of rows with equal a' in one slab, whose
+// rows (a', a'+1 .. nv-1) are consecutive.  Same lane groups as pass 2.
+template <typename T, typename TV, typename TA, int MC, int GS>
+__global__ void __launch_bounds__(256) k_sigma_sega(GeomDev g, const int2* __restrict__ items, int nitems,
+                                                    const TV* __restrict__ Bt, const T* __restrict__ V, int64_t ldv,
+                                                    T* __restrict__ W, int64_t ldw, TA* __restrict__ W1, int64_t ld1) {
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int no = g.no, nv = g.nv;
+  const int64_t n1 = g.n1;
+  const int nA = g.noP / 8;
+  const int slot = lane / GS, h = lane % GS;
+  constexpr int RPS = 32 / GS;
+  for (int it = warp; it < nitems; it += nwarps) {
+    const int2 item = items[it];
+    const int ap = item.y - 1;                       // items list b' = 1 .. nv-1
+    const Double r = decode_row(g, item.x);
+    const int cls = r.cls;
+    const int64_t L = g.len[cls], row0 = item.x + pair_index(ap, ap + 1, nv);
+    const int nrow = nv - 1 - ap;
+    const bool act = h < nA;
+    T xa[8][MC], ya[8][MC];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int c = 0; c < MC; ++c) {
+        const int kk = 8 * h + u;
+        xa[u][c] = (act && kk < no) ? V[(int64_t)c * ldv + (int64_t)ap * no + kk] : T(0);
+        ya[u][c] = T(0);
+      }
+    for (int b0 = 0; b0 < nrow; b0 += RPS) {
+      const int rr = b0 + slot;
+      const bool rv = rr < nrow;
+      T v[8], x2[MC], w2[MC];
+      int64_t d = 0;
+      if (rv) {
+        const int64_t row = row0 + rr;
+        const Double dd{ap, ap + 1 + rr, r.kp, r.lp, cls};
+        d = row_to_d(g, dd, row);
+        if (act) Load8<T, TV>::go(Bt + g.off[cls] + (row - g.start[cls]) * L + 8 * h, v);
+      }
+      if (!(rv && act)) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = T(0);
+      }
+#pragma unroll
+      for (int c = 0; c < MC; ++c) {
+        x2[c] = rv ? V[(int64_t)c * ldv + n1 + d] : T(0);
+        w2[c] = (rv && h == 0) ? W[(int64_t)c * ldw + n1 + d] : T(0);
+      }
+#pragma unroll
+      for (int c = 0; c < MC; ++c) {
+        T z = T(0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          ya[u][c] += v[u] * x2[c];
+          z += v[u] * xa[u][c];
+        }
+#pragma unroll
+        for (int o = 1; o < GS; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        if (rv && h == 0) W[(int64_t)c * ldw + n1 + d] = w2[c] + z;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int c = 0; c < MC; ++c) {
+        T y = ya[u][c];
+#pragma unroll
+        for (int o = GS; o < 32; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        ya[u][c] = y;
+      }
+    if (slot == 0 && act) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int kk = 8 * h + u;
+        if (kk >= no) continue;
+#pragma unroll
+        for (int c = 0; c < MC; ++c)
+          if (ya[u][c] != T(0)) atomicAdd(&W1[(int64_t)c * ld1 + (int64_t)ap * no + kk], (TA)ya[u][c]);
+      }
+    }
+  }
+}
+
+// Segment A of the classes with a' = b' (1 and 3), storage rows [row0, row1):
+// one warp per row, lanes over k.
+template <typename T, typename TV, typename TA>
+__global__ void __launch_bounds__(256) k_sigma_rows_a(GeomDev g, int64_t row0, int64_t row1,
+                                                      const TV* __restrict__ Bt, const T* __restrict__ V, int64_t ldv,
+                                                      int m, T* __restrict__ W, int64_t ldw, TA* __restrict__ W1,
+                                                      int64_t ld1) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t row = row0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5); row < row1; row += nw) {
+    const Double r = decode_row(g, row);
+    const TV* rp = Bt + g.off[r.cls] + (row - g.start[r.cls]) * g.len[r.cls];
+    for (int c = 0; c < m; ++c) {
+      const T x2 = V[(int64_t)c * ldv + g.n1 + row];
+      T z = T(0);
+      for (int k = lane; k < g.no; k += 32) {
+        const T a = (T)rp[k];
+        const int64_t s = (int64_t)r.ap * g.no + k;
+        z += a * V[(int64_t)c * ldv + s];
+        if (a != T(0)) atomicAdd(&W1[(int64_t)c * ld1 + s], (TA)(a * x2));
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+      if (lane == 0) W[(int64_t)c * ldw + g.n1 + row] += z;
+    }
+  }
+}
+
 // Arithmetic of the tiled pass 1.  Native: values, vectors and sums in T.
 // DF (FP64 inputs only): the C|D values and the vectors are held in shared
 // memory as double-float pairs and multiplied on the FP32 pipe (df.h), and so
@@ -1369,6 +1484,24 @@ int launch_p2(Ctx* c, const GeomDev& g, const SigmaPlan* plan, int mc, const TV*
   return ADCGPU_OK;
 }
 
+// segment A of FP64 values beside the sliced pass, for mc <= 4 columns
+int launch_sega(Ctx* c, const GeomDev& g, const SigmaPlan* plan, int mc, const double* Bt, const double* V,
+                int64_t ldv, double* W, int64_t ldw, double* W1, int64_t ld1) {
+  const int g2 = std::min(plan->nitems, c->nsm * 8 * 8) / 8 + 1;
+  const int gs = g.noP <= 8 ? 1 : (g.noP <= 16 ? 2 : 4);
+  cudaStream_t s = c->stream;
+#define SA(MC, GS)                                                                                                  \
+  k_sigma_sega<double, double, double, MC, GS><<<g2, 256, 0, s>>>(g, plan->d_items, plan->nitems, Bt, V, ldv, W, ldw, \
+                                                                  W1, ld1)
+  if (mc == 4) { if (gs == 1) SA(4, 1); else if (gs == 2) SA(4, 2); else SA(4, 4); }
+  else if (mc == 2) { if (gs == 1) SA(2, 1); else if (gs == 2) SA(2, 2); else SA(2, 4); }
+  else { if (gs == 1) SA(1, 1); else if (gs == 2) SA(1, 2); else SA(1, 4); }
+#undef SA
+  ADC_COUNT_LAUNCH();
+  ADC_CUDA(c, cudaGetLastError());
+  return ADCGPU_OK;
+}
+
 // pass 3 (segment A's W1 part, after the tensor-core pass) for mc <= 8 columns
 template <typename TV>
 int launch_p3(Ctx* c, const GeomDev& g, const int2* runs, int nruns, int mc, const TV* Bt, const float* V,
@@ -1425,9 +1558,37 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
   }
   // The coupling part over the work lists of P (the whole store, or the
   // rows of one chunk of the direct path) with the values at BtP.
-  bool umma_used = false;
-  auto coupling = [&](const SigmaPlan* P, const TV* BtP, bool allow_umma) -> int {
+  bool umma_used = false, oz_used = false;
+  auto coupling = [&](const SigmaPlan* P, const TV* BtP, bool allow_umma, int64_t row0, int64_t row1) -> int {
     int c0 = 0;
+    if constexpr (std::is_same<TV, double>::value) {
+      if (P->tiled == 1 && !P->umma_off) {
+        bool usable = false;
+        ST(oz_prepare(c, plan->oz, BtP, true, row0, row1, m, &usable));
+        if (usable) {
+          T* W1 = dW;
+          ST(oz_launch(c, plan->oz, diag, dV, ldv, m, dW, ldw, W1, ldw));
+          oz_used = true;
+          for (; P->nitems && c0 < m;) {
+            const int lb = m - c0, mc = lb >= 4 ? 4 : (lb >= 2 ? 2 : 1);
+            const T* Vb = dV + (int64_t)c0 * ldv;
+            T* Wb = dW + (int64_t)c0 * ldw;
+            ST(launch_sega(c, g, P, mc, BtP, Vb, ldv, Wb, ldw, Wb, ldw));
+            ST((launch_p2<T, TV, TAcc>(c, g, P, mc, BtP, Vb, ldv, Wb, ldw, reinterpret_cast<TAcc*>(Wb), ldw)));
+            c0 += mc;
+          }
+          for (int cls = 0; cls <= 2; cls += 2) {
+            const int64_t a = std::max(row0, G.start[cls]), b = std::min(row1, G.start[cls + 1]);
+            if (a >= b) continue;
+            k_sigma_rows_a<T, TV, T><<<(int)std::min<int64_t>((b - a + 7) / 8, c->nsm * 8), 256, 0, s>>>(
+                g, a, b, BtP, dV, ldv, m, dW, ldw, W1, ldw);
+            ADC_COUNT_LAUNCH();
+          }
+          ADC_CUDA(c, cudaGetLastError());
+          return ADCGPU_OK;
+        }
+      }
+    }
     // tiled pass 1 (k_sigma_tile) when its shared memory fits: widest column
     // group first; segment B still runs through pass 2 in groups of <= 4
     // FP32: 16 columns keep two blocks per SM (their loads overlap the other's
@@ -1594,13 +1755,13 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
         // shifting the base by the chunk's first value puts its rows in the buffer
         const TV* BtP = reinterpret_cast<const TV*>(reinterpret_cast<uintptr_t>(c->d_Bt) -
                                                     (uintptr_t)dc.vbase * sizeof(TV));
-        ST(coupling(&view, BtP, false));
+        ST(coupling(&view, BtP, false, dc.row0, dc.row1));
       }
     } else {
       return set_err(c, ADCGPU_UNSUPPORTED, "the direct path computes in FP64");
     }
   } else {
-    ST(coupling(plan, Bt, true));
+    ST(coupling(plan, Bt, true, 0, G.n2));
   }
   if (sizeof(T) == 4) {
     k_w1_finalize<<<(n1 * m + 255) / 256, 256, 0, s>>>(n1, m, reinterpret_cast<const double*>(W1base),
@@ -1608,6 +1769,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
   }
   ADC_CUDA(c, cudaEventRecord(c->st_ev1, s));
   if (umma_used) ST(umma_check(c, plan->umma));
+  if (oz_used) ST(oz_check(c, plan->oz));
   c->st_pending = true;
   c->st_pending_cols = m;
   c->st_pending_kind = std::is_same<TV, __nv_bfloat16>::value ? 0 : (std::is_same<TV, float>::value ? 1 : 2);
@@ -1709,6 +1871,7 @@ void free_sigma_plan(Ctx* c) {
   dfree(c, plan->d_acc);
   dfree(c, plan->d_sk);
   umma_free(c, plan->umma);
+  oz_free(c, plan->oz);
   ab_free(c, plan->ab);
   delete plan;
   c->sigma_plan = nullptr;

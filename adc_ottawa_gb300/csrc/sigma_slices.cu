@@ -1,0 +1,890 @@
+// FP64-accurate tensor-core pass of the sigma product: the C and D segments
+// (the singles (a, k') and (a, l') of a double (a', b', k', l'); layout in
+// internal.h) of FP64 values against FP64 vectors, or of FP32 values against
+// FP32 vectors.  Replaces the CUDA-core tile (k_sigma_tile) for hxvec_incore
+// (block_davidson.f90:844-883), hxq_incore (block_lanczos.f90:1325-1361) and
+// matxvec_treal_incore (tdselib.f90:352-437).
+//
+// Exact slicing (K. Ozaki, T. Ogita, S. Oishi, S. M. Rump, "Error-free
+// transformations of matrix multiplication by using fast routines of matrix
+// multiplication and its applications", Numer. Algorithms 59, 2012).  A row
+// of values is scaled by a power of two to |v| < 1 and written as S balanced
+// base-256 digits, v = sum_i d_i 2^(-7-8i), |d_i| <= 128; so are the vector
+// entries of a slab (one exponent per column) and of a row tile.  Every digit
+// is an exact BF16 number, a product of two digits has at most 14 bits, and
+// the FP32 accumulators in TMEM add whole numbers: up to 2^24 / 2^14 = 1024
+// products without rounding.  Products of equal weight (i + j = g) share an
+// accumulator; the groups g < S are kept (the dropped ones are below the last
+// digit's weight) and combined with 64-bit integer arithmetic, so one
+// rounding per tile replaces one per multiply-add.
+//   S = 7: 55 bits below the row / column maximum (FP64 values)
+//   S = 4: 31 bits (FP32 values and vectors)
+// W1 sums cover two tiles, 256 rows: g < 4 is exact whatever the digits are.
+// W2 sums cover K <= 512 values: g < 2 (K <= 341: g < 3) likewise.  The other
+// groups are exact while their partial sums stay below 2^24, which the
+// pseudo-random lower digits do by a factor of 50 (sum of n products: about
+// 2^12 sqrt(n)).
+//
+// What bounds it: the digit store is read once per 16 columns (S = 7), 14
+// bytes per value; the tensor cores need S (S + 1) / 2 = 28 slice products.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <string>
+#include <type_traits>
+#include <vector>
+
+#include "internal.h"
+#include "umma.h"
+
+namespace adcgpu {
+
+using namespace umma;
+
+namespace {
+
+constexpr int OZ_ROWS = 128;                       // rows per tile (MMA M)
+constexpr int OZ_BOX = 64;                         // values per box row (128 bytes)
+constexpr int OZ_SLOT_BYTES = 2 * OZ_ROWS * OZ_BOX * 2;
+constexpr int OZ_EPI = 512;                        // threads of the 16 epilogue warps
+constexpr int OZ_THREADS = 64 + OZ_EPI;            // and the producer and MMA issuer warps
+constexpr int OZ_MAXNR = 6;                        // ring slots
+constexpr int OZ_FLUSH = 2;                        // tiles per W1 accumulation in TMEM
+constexpr int OZ_NONFINITE = 1 << 20;              // exponent of a column that holds inf or NaN
+constexpr int OZ_ZERO = -(1 << 20);                // exponent of a zero
+constexpr int OZ_EMIN = -900;                      // smaller maxima are taken as this exponent
+
+__host__ __device__ constexpr int round16(int x) { return (x + 15) / 16 * 16; }
+// Vector operands: PAD zero rows, then slice j of column c at row PAD + j NP + c.
+// Value slice i multiplies the vector slices 0 .. S-1-i side by side into the
+// columns of the groups i .. S-1.  With 8-column slices every other slice
+// would start 8 columns off a 16-column boundary of TMEM: those start at the
+// zero rows instead, one slice earlier.
+template <int NP> __host__ __device__ constexpr int oz_pad() { return NP == 8 ? 8 : 0; }
+template <int NP> __host__ __device__ constexpr bool oz_early(int i) { return NP == 8 && (i & 1); }
+template <int S, int NP> __host__ __device__ constexpr int oz_n(int i) {   // MMA N
+  return round16(NP * (S - i + (oz_early<NP>(i) ? 1 : 0)));
+}
+template <int NP> __host__ __device__ constexpr int oz_col(int i) { return NP * (i - (oz_early<NP>(i) ? 1 : 0)); }
+template <int NP> __host__ __device__ constexpr int oz_brow(int i) { return oz_early<NP>(i) ? 0 : oz_pad<NP>(); }
+// rows of a vector operand (the widest MMA reads oz_n(0) rows from oz_brow(0))
+template <int S, int NP> __host__ __device__ constexpr int oz_xrows() { return oz_pad<NP>() + oz_n<S, NP>(0); }
+// TMEM columns of one accumulator region: those of slice 0
+template <int S, int NP> __host__ __device__ constexpr int oz_dw() { return oz_n<S, NP>(0); }
+
+// geometry and buffering of one launch
+struct OzShape {
+  int nslot;        // 128-value groups of the longest C|D row
+  int nb;           // buffers of D1 and of the V2 operand (1 or 2)
+  int nr;           // ring slots
+  uint32_t off_v2, off_ring, off_bar;   // shared-memory offsets
+};
+
+// --- digits --------------------------------------------------------------
+// x = (-1)^neg m 2^(e - MB), m < 2^MB; e = OZ_ZERO for zeros and subnormals,
+// OZ_NONFINITE for inf and NaN
+template <typename T> struct Parts;
+template <> struct Parts<double> {
+  static constexpr int MB = 53;
+  __device__ __forceinline__ static int exponent(double x) {
+    const int f = (int)((__double2hiint(x) >> 20) & 0x7ff);
+    return f == 0 ? OZ_ZERO : (f == 0x7ff ? OZ_NONFINITE : f - 1022);
+  }
+  __device__ __forceinline__ static unsigned long long mantissa(double x) {
+    return ((unsigned long long)__double_as_longlong(x) & 0xfffffffffffffull) | 0x10000000000000ull;
+  }
+  __device__ __forceinline__ static bool neg(double x) { return __double2hiint(x) < 0; }
+};
+template <> struct Parts<float> {
+  static constexpr int MB = 24;
+  __device__ __forceinline__ static int exponent(float x) {
+    const int f = (int)((__float_as_uint(x) >> 23) & 0xff);
+    return f == 0 ? OZ_ZERO : (f == 0xff ? OZ_NONFINITE : f - 126);
+  }
+  __device__ __forceinline__ static unsigned long long mantissa(float x) {
+    return (__float_as_uint(x) & 0x7fffffu) | 0x800000u;
+  }
+  __device__ __forceinline__ static bool neg(float x) { return (int)__float_as_uint(x) < 0; }
+};
+
+// round(x 2^(8S - 1 - h)) plus the digit bias, for x of exponent e <= h: byte
+// i from the top is digit i + 128
+template <int S, typename T>
+__device__ __forceinline__ unsigned long long oz_fixed(T x, int shift) {   // shift = 8S - 1 - h + (scale of x)
+  constexpr unsigned long long BIAS = S == 7 ? 0x80808080808080ull : 0x80808080ull;
+  const int e = Parts<T>::exponent(x);
+  if (e == OZ_ZERO || e == OZ_NONFINITE) return BIAS;
+  const unsigned long long m = Parts<T>::mantissa(x);
+  const int sh = e - Parts<T>::MB + shift;
+  unsigned long long q;
+  if (sh >= 0) q = m << sh;
+  else if (sh < -60) q = 0ull;
+  else q = (m + (1ull << (-sh - 1))) >> (-sh);
+  return Parts<T>::neg(x) ? BIAS - q : BIAS + q;
+}
+// digit i as an FP32 number; its upper half is the exact BF16 one (an
+// integer of at most 8 bits)
+template <int S>
+__device__ __forceinline__ uint32_t oz_digit(unsigned long long u, int i) {
+  const uint32_t f = i == 0 ? (uint32_t)(u >> (8 * (S - 1))) : (uint32_t)(u >> (8 * (S - 1 - i))) & 0xffu;
+  return __float_as_uint(__uint_as_float(0x4B000000u | f) - 8388736.0f);
+}
+// two digits as a BF16 pair (lo in the lower half)
+__device__ __forceinline__ uint32_t oz_pair(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
+// 2^e; NaN for a column that holds inf or NaN
+__device__ __forceinline__ double oz_pow2(int e) {
+  if (e > (OZ_NONFINITE >> 1)) return __longlong_as_double(0x7ff8000000000000ll);
+  if (e < -1022) return 0.0;
+  if (e > 1023) return __longlong_as_double(0x7ff0000000000000ll);
+  return __longlong_as_double((long long)(e + 1023) << 52);
+}
+
+// --- value digits of a range of storage rows ---------------------------------
+// The digit store holds every tile of 128 rows of a slab as the shared-memory
+// image the MMAs read: per 128-value group and slice two boxes of 128 rows x
+// 64 values (128-byte swizzle), 32 KB in a row, so a ring slot is one
+// contiguous bulk copy.  Rows past the slab's end and values past the
+// segment's are zero digits.
+struct OzDst {
+  int64_t base[5];      // first value of the class in the digit store
+  int64_t r0[5];        // first storage row of the class in the store (whole slabs)
+  int64_t slab[5];      // rows of a slab
+  int tps[5];           // tiles of a slab
+  int nbox[5];          // 64-value boxes of a row
+  int64_t tiles[6];     // tiles of the classes before this one
+  int64_t row0, row1;   // storage rows [row0, row1)
+};
+
+// values between the digits of consecutive tiles of a class
+template <int S> __host__ __device__ inline int64_t oz_tile_values(int nbox) { return (int64_t)S * nbox * OZ_ROWS * OZ_BOX; }
+
+// one warp per tile row: the exponent of the largest |C|D value|, then the
+// digits of 8 values per lane and step (16-byte stores, 128 bytes a box).
+// Bound by HBM: 8 (4) bytes read and 2 S written per value.
+template <typename TV, int S>
+__global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const TV* __restrict__ Bt,
+                                                   uint16_t* __restrict__ out, int16_t* __restrict__ rexp) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < dst.tiles[5] * OZ_ROWS; w += nw) {
+    const int64_t tile = w / OZ_ROWS;
+    const int r = (int)(w % OZ_ROWS);
+    int cls = 0;
+    while (cls < 4 && tile >= dst.tiles[cls + 1]) ++cls;
+    const int64_t tc = tile - dst.tiles[cls];              // tile of the class
+    const int64_t in_slab = tc % dst.tps[cls] * OZ_ROWS + r;
+    const bool valid = in_slab < dst.slab[cls];
+    const int64_t row = dst.r0[cls] + tc / dst.tps[cls] * dst.slab[cls] + in_slab;
+    const bool twoa = cls == 1 || cls >= 3;
+    const int nch = (cls >= 2 ? 2 : 1) * g.nvP / 8, nbox = dst.nbox[cls];
+    const TV* src = Bt + g.off[cls] + (row - g.start[cls]) * g.len[cls] + (twoa ? 2 * g.noP : g.noP);
+    TV v[2][8];
+    int mx = OZ_ZERO;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int q = lane + 32 * k;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[k][u] = TV(0);
+      if (valid && q < nch) {
+        const int4* p = reinterpret_cast<const int4*>(src + 8 * q);
+        int4* d = reinterpret_cast<int4*>(v[k]);
+#pragma unroll
+        for (int u = 0; u < (int)(8 * sizeof(TV) / 16); ++u) d[u] = __ldcs(p + u);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) mx = max(mx, Parts<TV>::exponent(v[k][u]));
+    }
+    mx = max(__reduce_max_sync(0xffffffffu, mx), OZ_EMIN);
+    // a row that holds inf or NaN (integrals that do): its W2 entries and the
+    // W1 sums of its tile become NaN
+    if (lane == 0 && valid) rexp[row - dst.row0] = (int16_t)min(mx, 32767);
+    uint16_t* o = out + dst.base[cls] + tc * oz_tile_values<S>(nbox);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int q = lane + 32 * k;
+      if (q >= 8 * nbox) continue;
+      unsigned long long u8[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) u8[u] = oz_fixed<S, TV>(v[k][u], 8 * S - 1 - mx);
+      // 128-value group q / 16: S slices of its (one or two) boxes
+      const int grp = q >> 4, bx = (q >> 3) & 1, two = 2 * grp + 1 < nbox ? 2 : 1;
+      uint16_t* og = o + ((int64_t)S * 2 * grp + bx) * (OZ_ROWS * OZ_BOX) + sw128_off(r, 8 * (q & 7)) / 2;
+#pragma unroll
+      for (int i = 0; i < S; ++i) {
+        uint4 w4;
+        w4.x = oz_pair(oz_digit<S>(u8[0], i), oz_digit<S>(u8[1], i));
+        w4.y = oz_pair(oz_digit<S>(u8[2], i), oz_digit<S>(u8[3], i));
+        w4.z = oz_pair(oz_digit<S>(u8[4], i), oz_digit<S>(u8[5], i));
+        w4.w = oz_pair(oz_digit<S>(u8[6], i), oz_digit<S>(u8[7], i));
+        __stcs(reinterpret_cast<uint4*>(og + (int64_t)i * two * (OZ_ROWS * OZ_BOX)), w4);
+      }
+    }
+  }
+}
+
+// exponent of the largest 2^rexp |V2| of each work item and column: the
+// scale of the V2 digits.  One block per item and 4 columns; reads V2 once
+// (the pass then finds most of it in L2).
+template <typename T>
+__global__ void __launch_bounds__(256) k_oz_vexp(GeomDev g, const int2* __restrict__ items, int64_t row0,
+                                                 const int16_t* __restrict__ rexp, const T* __restrict__ V, int64_t ldv,
+                                                 int m, int* __restrict__ vexp) {
+  __shared__ int s_mx[4];
+  const int2 item = items[blockIdx.x];
+  const int c0 = 4 * blockIdx.y;
+  if (threadIdx.x < 4) s_mx[threadIdx.x] = OZ_EMIN;
+  __syncthreads();
+  int mx[4] = {OZ_EMIN, OZ_EMIN, OZ_EMIN, OZ_EMIN};
+  const bool perm = item.x >= g.start[1] && item.x < g.start[2];
+  for (int row = item.x + threadIdx.x; row < item.y; row += 256) {
+    int64_t d = row;
+    if (perm) d = row_to_d(g, decode_row(g, row), row);
+    const int rx = rexp[row - row0];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (c0 + j >= m) break;
+      const int e = Parts<T>::exponent(__ldg(V + (int64_t)(c0 + j) * ldv + g.n1 + d));
+      if (e == OZ_NONFINITE || rx == 32767) mx[j] = OZ_NONFINITE;
+      else if (e != OZ_ZERO) mx[j] = max(mx[j], e + rx);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    mx[j] = __reduce_max_sync(0xffffffffu, mx[j]);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_mx[j], mx[j]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 4 && c0 + (int)threadIdx.x < m) vexp[(int64_t)blockIdx.x * m + c0 + threadIdx.x] = s_mx[threadIdx.x];
+}
+
+// --- the pass -----------------------------------------------------------------
+enum OzBar { O_XFULL = 0, O_V2FULL0, O_V2FULL1, O_D1FULL0, O_D1FULL1, O_D1EMPTY0, O_D1EMPTY1, O_D2FULL,
+             O_D2EMPTY = O_D2FULL + 4, O_EPI = O_D2EMPTY + 4, O_SLOT0 };
+
+__device__ __forceinline__ bool oz_failed(const int* err) { return *(const volatile int*)err != 0; }
+
+// 32 TMEM lanes x N columns; the caller waits (tcgen05.wait::ld)
+__device__ __forceinline__ void oz_tmem_ld(uint32_t taddr, float (&v)[2]) {
+  uint32_t r[2];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
+  v[0] = __uint_as_float(r[0]);
+  v[1] = __uint_as_float(r[1]);
+}
+__device__ __forceinline__ void oz_tmem_ld(uint32_t taddr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;\n" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+
+// the group sums of NH columns -> T 2^(-8 max(S-4, 0)), T = sum_g D_g 2^(8(S-1-g)):
+// whole numbers combined in 64-bit integers, then two FP64 additions (the
+// integers are placed in the mantissa of 1.5 2^52 and 1.5 2^28)
+template <int S, int NP, int NH>
+__device__ __forceinline__ void oz_combine(uint32_t taddr, double (&t)[NH]) {
+  float d[S][NH];
+#pragma unroll
+  for (int gI = 0; gI < S; ++gI) oz_tmem_ld(taddr + (uint32_t)(gI * NP), d[gI]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < NH; ++j) {
+    long long hi = (long long)__float2int_rn(d[3][j]);
+    hi = mad_wide(__float2int_rn(d[2][j]), 1 << 8, hi);
+    hi = mad_wide(__float2int_rn(d[1][j]), 1 << 16, hi);
+    hi = mad_wide(__float2int_rn(d[0][j]), 1 << 24, hi);
+    if constexpr (S == 4) {
+      t[j] = __longlong_as_double(0x4338000000000000ll + hi) - 6755399441055744.0;
+    } else {
+      long long lo = (long long)__float2int_rn(d[6][j]);
+      lo = mad_wide(__float2int_rn(d[5][j]), 1 << 8, lo);
+      lo = mad_wide(__float2int_rn(d[4][j]), 1 << 16, lo);
+      const double x = __longlong_as_double(0x4338000000000000ll + hi) - (6755399441055744.0 + 402653184.0);
+      t[j] = x + __longlong_as_double(0x41B8000000000000ll + lo);
+    }
+  }
+}
+
+// S digits, NP columns per pass, MS 128-value groups at most
+template <int S, int NP, int MS, typename T, typename TA>
+__global__ void __launch_bounds__(OZ_THREADS, 1)
+    k_sigma_oz(const __grid_constant__ GeomDev g, const int2* __restrict__ items, int nitems, int ngrp, OzShape sh,
+               const __grid_constant__ OzDst src, const uint16_t* __restrict__ dig, const int16_t* __restrict__ rexp,
+               const int* __restrict__ ivexp, const T* __restrict__ diag, const T* __restrict__ V, int64_t ldv, int m, T* __restrict__ W,
+               int64_t ldw, TA* __restrict__ W1, int64_t ld1, int* __restrict__ err) {
+  constexpr int DW = oz_dw<S, NP>();
+  constexpr int XR = oz_xrows<S, NP>();            // rows of the vector operands
+  constexpr int PAD = oz_pad<NP>();
+  constexpr int BOXB = XR * 128;
+  constexpr int V2B = 2 * BOXB;
+  constexpr int NH = NP / 4;                       // columns per epilogue thread
+  constexpr int FB = 8 * S - 1;                    // fraction bits of the digits
+  constexpr int TSH = -14 - 8 * (S - 1) + (S == 7 ? 24 : 0);   // weight of oz_combine4's unit
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sX = base;                        // 2 nslot boxes [XR rows x 64 k]
+  unsigned char* sV2 = base + sh.off_v2;           // nb x 2 boxes [XR rows x 64 tile rows]
+  unsigned char* sRing = base + sh.off_ring;       // nr x 32 KB
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + sh.off_bar);
+  uint64_t* slot_full = bars + O_SLOT0;
+  uint64_t* slot_empty = slot_full + OZ_MAXNR;
+  int* sXe = reinterpret_cast<int*>(slot_empty + OZ_MAXNR);    // [NP] exponents of X
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sXe + NP);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int no = g.no, nv = g.nv, nvP = g.nvP;
+  const int64_t n1 = g.n1;
+  const int nunits = nitems * ngrp;
+
+  if (tid == 0) {
+    for (int i = 0; i < O_SLOT0 + 2 * OZ_MAXNR; ++i) {
+      const bool epi = i == O_XFULL || i == O_V2FULL0 || i == O_V2FULL1 || i == O_D1EMPTY0 || i == O_D1EMPTY1 ||
+                       (i >= O_D2EMPTY && i <= O_EPI);
+      mbar_init(&bars[i], epi ? (uint32_t)OZ_EPI : 1u);
+    }
+  }
+  if (warp == 0) tmem_alloc(tmem_holder, 512);
+  // rows of the vector operands past S NP columns stay zero; so does, until a
+  // full group overwrites it, the second box of a slot (a group of one box
+  // leaves it as it is: its W1 lanes are not read)
+  for (uint32_t o = tid; o < sh.off_bar / 16; o += OZ_THREADS) reinterpret_cast<uint4*>(base)[o] = make_uint4(0, 0, 0, 0);
+  fence_proxy_async();
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tbase = *tmem_holder;
+  const uint32_t tD2 = tbase + (uint32_t)(sh.nb * DW);         // + s DW
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ producer
+    if (lane == 0) {
+      uint32_t use = 0;
+      bool ok = true;
+      for (int un = blockIdx.x; ok && un < nunits; un += gridDim.x) {
+        const int2 item = items[un / ngrp];
+        const int cls = decode_row(g, item.x).cls;
+        const int nbox = src.nbox[cls], nslot = (nbox + 1) / 2;
+        const int64_t rc = item.x - src.r0[cls], slab = rc / src.slab[cls];
+        const uint16_t* tp = dig + src.base[cls] +
+                             (slab * src.tps[cls] + (rc - slab * src.slab[cls]) / OZ_ROWS) * oz_tile_values<S>(nbox);
+        for (int row0 = item.x; ok && row0 < item.y; row0 += OZ_ROWS) {
+          for (int s = 0; ok && s < nslot; ++s) {
+            const uint32_t bytes = 2 * s + 1 < nbox ? OZ_SLOT_BYTES : OZ_SLOT_BYTES / 2;
+            for (int i = 0; i < S; ++i, ++use) {
+              const uint32_t ri = use % sh.nr;
+              ok = !oz_failed(err) && mbar_wait(&slot_empty[ri], ((use / sh.nr) & 1u) ^ 1u, err, 1);
+              if (!ok) break;
+              mbar_expect_tx(&slot_full[ri], bytes);
+              bulk_load(sRing + (size_t)ri * OZ_SLOT_BYTES, tp, bytes, &slot_full[ri]);
+              tp += bytes / 2;
+            }
+          }
+        }
+      }
+      // no copy may still be writing shared memory when the CTA exits
+      for (uint32_t k = 0; k < (uint32_t)sh.nr && k < use; ++k) {
+        const uint32_t u = use - 1 - k;
+        mbar_wait(&slot_full[u % sh.nr], (u / sh.nr) & 1u, err, 11);
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------- MMA issuer
+    // The whole warp walks the loops, so that descriptors and addresses stay
+    // in uniform registers; one elected lane issues.  (One lane walking them
+    // alone spent about 140 cycles an instruction and bound the pass.)
+    constexpr uint64_t KMAJ = sdesc(0, 16, 1024, LAYOUT_SW128), MNMAJ = sdesc(0, OZ_SLOT_BYTES / 2, 1024, LAYOUT_SW128);
+    const uint32_t sXa = smem_u32(sX), sVa = smem_u32(sV2), sRa = smem_u32(sRing);
+    uint32_t ri = 0, rph = 0, tile = 0, nun = 0;
+    uint32_t d2use[MS] = {};
+    bool ok = true;
+    for (int un = blockIdx.x; un < nunits && ok && !__any_sync(0xffffffffu, oz_failed(err)); un += gridDim.x, ++nun) {
+      const int2 item = items[un / ngrp];
+      const int cls = decode_row(g, item.x).cls;
+      const int K = (cls >= 2 ? 2 : 1) * nvP;
+      const int nbox = (K + OZ_BOX - 1) / OZ_BOX, nslot = (nbox + 1) / 2;
+      ok = mbar_wait_warp(&bars[O_XFULL], nun & 1u, err, 2);
+      for (int row0 = item.x; ok && row0 < item.y; row0 += OZ_ROWS, ++tile) {
+        const uint32_t b = sh.nb == 2 ? tile & 1u : 0u, ph = sh.nb == 2 ? (tile >> 1) & 1u : tile & 1u;
+        ok = mbar_wait_warp(&bars[O_D1EMPTY0 + b], ph ^ 1u, err, 4);
+        ok = ok && mbar_wait_warp(&bars[O_V2FULL0 + b], ph, err, 5);
+        fence_after_sync();
+        const uint32_t tD1 = tbase + b * DW;
+        const uint64_t vdesc = KMAJ + ((sVa + b * V2B) >> 4);
+        // the W1 sums run over OZ_FLUSH tiles of the item
+        const int pos = ((row0 - item.x) / OZ_ROWS) % OZ_FLUSH;
+        const bool d2first = pos == 0, d2last = pos == OZ_FLUSH - 1 || row0 + OZ_ROWS >= item.y;
+#pragma unroll
+        for (int s = 0; s < MS; ++s) {
+          if (!ok || s >= nslot) break;
+          if (d2first) {
+            ok = mbar_wait_warp(&bars[O_D2EMPTY + s], (d2use[s] & 1u) ^ 1u, err, 3);
+            ++d2use[s];
+            fence_after_sync();
+          }
+          const uint64_t xdesc = KMAJ + ((sXa + 2 * s * BOXB) >> 4);
+          const bool two = 2 * s + 1 < nbox;
+#pragma unroll
+          for (int i = 0; i < S; ++i) {
+            ok = ok && mbar_wait_warp(&slot_full[ri], rph, err, 6);
+            if (!ok) break;
+            fence_after_sync();
+            const uint32_t slot = sRa + ri * OZ_SLOT_BYTES;
+            const uint32_t idK = idesc_bf16(OZ_ROWS, oz_n<S, NP>(i), 0, 0);
+            const uint32_t idM = idesc_bf16(OZ_ROWS, oz_n<S, NP>(i), 1, 0);
+            const uint32_t d1 = tD1 + (uint32_t)oz_col<NP>(i), d2 = tD2 + (uint32_t)(s * DW + oz_col<NP>(i));
+            const uint64_t kd = KMAJ + (slot >> 4), md = MNMAJ + (slot >> 4);
+            const uint64_t xd = xdesc + oz_brow<NP>(i) * 8, vd = vdesc + oz_brow<NP>(i) * 8;
+            if (elect_one()) {
+              // W2 tile: the slot's boxes as K-major A, X slices 0 .. S-1-i as B
+              if (s == 0 && i == 0) mma_bf16_c<false>(d1, kd, xd, idK);
+              else mma_bf16_c<true>(d1, kd, xd, idK);
+#pragma unroll
+              for (int ks = 1; ks < 4; ++ks) mma_bf16_c<true>(d1, kd + 2 * ks, xd + 2 * ks, idK);
+              if (two) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                  mma_bf16_c<true>(d1, kd + OZ_SLOT_BYTES / 32 + 2 * ks, xd + BOXB / 16 + 2 * ks, idK);
+              }
+              // W1 part: the slot's 128 values of a as MN-major A, the tile's
+              // 128 rows as K, V2 slices 0 .. S-1-i as B
+              if (i == 0 && d2first) mma_bf16_c<false>(d2, md, vd, idM);
+              else mma_bf16_c<true>(d2, md, vd, idM);
+#pragma unroll
+              for (int ks = 1; ks < 8; ++ks)
+                mma_bf16_c<true>(d2, md + 128 * ks, vd + (ks >> 2) * (BOXB / 16) + 2 * (ks & 3), idM);
+              mma_commit(&slot_empty[ri]);
+              if (i == S - 1 && d2last) mma_commit(&bars[O_D2FULL + s]);
+            }
+            __syncwarp();
+            if (++ri == (uint32_t)sh.nr) { ri = 0; rph ^= 1u; }
+          }
+        }
+        if (elect_one()) mma_commit(&bars[O_D1FULL0 + b]);
+        __syncwarp();
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue
+    // thread = TMEM lane (tile row, or value index of a W1 group) and a
+    // quarter of the columns
+    const int ew = warp - 2;
+    const int q = warp & 3;
+    const int cbeg = (ew >> 2) * NH;
+    const int r = 32 * q + lane;
+    const uint32_t lane_off = (uint32_t)(32 * q) << 16;
+    uint32_t tile = 0;
+    uint32_t d2use[MS] = {};
+    bool ok = true;
+    int rx = 0;                 // exponent of the row of the tile being prepared
+    T v2[NH];
+    // V2 of a tile: this thread's row and columns
+    auto load_v2 = [&](int row, int row_end, int cls, int c0) {
+      const bool valid = row < row_end;
+      rx = 0;
+      int64_t d = 0;
+      if (valid) {
+        d = row;
+        if (cls == 1) {
+          const Double rr = decode_row(g, row);
+          d = row_to_d(g, rr, row);
+        }
+        rx = rexp[row - src.row0];
+      }
+#pragma unroll
+      for (int j = 0; j < NH; ++j) {
+        const int c = c0 + cbeg + j;
+        v2[j] = (valid && c < m) ? __ldg(V + (int64_t)c * ldv + n1 + d) : T(0);
+      }
+    };
+    // all epilogue threads (an mbarrier, so that the wait is bounded)
+    uint32_t nepi = 0;
+    auto epi_sync = [&]() {
+      mbar_arrive(&bars[O_EPI]);
+      ok = mbar_wait_warp(&bars[O_EPI], nepi & 1u, err, 12) && ok;
+      ++nepi;
+    };
+    int vexp[NH];               // exponents of the item's V2 columns
+    auto store_v2 = [&](uint32_t buf) {
+      unsigned char* bx = sV2 + buf * V2B + (r >> 6) * BOXB;
+#pragma unroll
+      for (int j = 0; j < NH; ++j) {
+        const unsigned long long u =
+            oz_fixed<S, T>(vexp[j] == OZ_NONFINITE ? T(0) : v2[j], FB - vexp[j] + rx);
+#pragma unroll
+        for (int i = 0; i < S; ++i)
+          *reinterpret_cast<uint16_t*>(bx + sw128_off(PAD + i * NP + cbeg + j, r & 63)) = (uint16_t)(oz_digit<S>(u, i) >> 16);
+      }
+      fence_proxy_async();
+      mbar_arrive(&bars[O_V2FULL0 + buf]);
+    };
+    for (int un = blockIdx.x; un < nunits && ok && !__any_sync(0xffffffffu, oz_failed(err)); un += gridDim.x) {
+      const int2 item = items[un / ngrp];
+      const int c0 = (un % ngrp) * NP;
+      const Double r0 = decode_row(g, item.x);
+      const int cls = r0.cls;
+      const int K = (cls >= 2 ? 2 : 1) * nvP;
+      const int nbox = (K + OZ_BOX - 1) / OZ_BOX, nslot = (nbox + 1) / 2;
+      const int kp = r0.kp, lp = r0.lp;
+      load_v2(item.x + r, item.y, cls, c0);
+#pragma unroll
+      for (int j = 0; j < NH; ++j)
+        vexp[j] = c0 + cbeg + j < m ? __ldg(ivexp + (int64_t)(un / ngrp) * m + c0 + cbeg + j) : OZ_EMIN;
+      // X of this item: the previous item's products have read the old one
+      // (its last D1 was waited for).  One warp per column
+#pragma unroll 1
+      for (int c = ew; c < NP; c += OZ_EPI / 32) {
+        T xv[4 * MS];
+        int mx = OZ_ZERO;
+#pragma unroll
+        for (int u = 0; u < 4 * MS; ++u) {
+          const int k = lane + 32 * u;
+          const int seg = k >= nvP ? 1 : 0, a = k - seg * nvP;
+          xv[u] = (c0 + c < m && k < K && a < nv) ? __ldg(V + (int64_t)(c0 + c) * ldv + (int64_t)a * no + (seg ? lp : kp)) : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4 * MS; ++u) mx = max(mx, Parts<T>::exponent(xv[u]));
+        mx = max(__reduce_max_sync(0xffffffffu, mx), OZ_EMIN);
+        if (lane == 0) sXe[c] = mx;
+#pragma unroll
+        for (int u = 0; u < 4 * MS; ++u) {
+          const int k = lane + 32 * u;
+          if (k >= nbox * OZ_BOX) continue;
+          const unsigned long long x = oz_fixed<S, T>(mx == OZ_NONFINITE ? T(0) : xv[u], FB - mx);
+          unsigned char* bx = sX + (k >> 6) * BOXB;
+#pragma unroll
+          for (int i = 0; i < S; ++i)
+            *reinterpret_cast<uint16_t*>(bx + sw128_off(PAD + i * NP + c, k & 63)) = (uint16_t)(oz_digit<S>(x, i) >> 16);
+        }
+      }
+      fence_proxy_async();
+      mbar_arrive(&bars[O_XFULL]);
+      double acc[MS][NH];
+#pragma unroll
+      for (int s = 0; s < MS; ++s)
+#pragma unroll
+        for (int j = 0; j < NH; ++j) acc[s][j] = 0.0;
+      epi_sync();               // sXe
+      if (!ok) break;
+      uint32_t buf = sh.nb == 2 ? tile & 1u : 0u;
+      store_v2(buf);
+      for (int row0 = item.x; ok && row0 < item.y; row0 += OZ_ROWS, ++tile) {
+        buf = sh.nb == 2 ? tile & 1u : 0u;
+        const uint32_t ph = sh.nb == 2 ? (tile >> 1) & 1u : tile & 1u;
+        const bool has_next = row0 + OZ_ROWS < item.y;
+        const int rx_t = rx;
+        const bool d2last = ((row0 - item.x) / OZ_ROWS) % OZ_FLUSH == OZ_FLUSH - 1 || !has_next;
+        if (has_next) load_v2(row0 + OZ_ROWS + r, item.y, cls, c0);
+        // W1 sums of one 128-value group
+        auto drain_d2 = [&](int s, double (&ac)[NH]) {
+          ok = ok && mbar_wait_warp(&bars[O_D2FULL + s], d2use[s] & 1u, err, 10);
+          if (!ok) return;
+          ++d2use[s];
+          fence_after_sync();
+          double t[NH];
+          oz_combine<S, NP, NH>(tD2 + (uint32_t)(s * DW) + lane_off + (uint32_t)cbeg, t);
+          fence_before_sync();
+          mbar_arrive(&bars[O_D2EMPTY + s]);
+#pragma unroll
+          for (int j = 0; j < NH; ++j) ac[j] += t[j];
+        };
+#pragma unroll
+        for (int s = 0; s + 1 < MS; ++s)
+          if (d2last && s + 1 < nslot) drain_d2(s, acc[s]);
+        // two buffers: the other one is free since the previous tile's end
+        if (has_next && sh.nb == 2) store_v2(buf ^ 1u);
+        ok = ok && mbar_wait_warp(&bars[O_D1FULL0 + buf], ph, err, 9);
+        if (!ok) break;
+        if (has_next && sh.nb == 1) store_v2(0);
+        fence_after_sync();
+        double t2[NH];
+        oz_combine<S, NP, NH>(tbase + buf * DW + lane_off + (uint32_t)cbeg, t2);
+        fence_before_sync();
+        mbar_arrive(&bars[O_D1EMPTY0 + buf]);
+        // the last group of the row (its sums end with the tile)
+#pragma unroll
+        for (int s = 0; s < MS; ++s)
+          if (d2last && s + 1 == nslot) drain_d2(s, acc[s]);
+        if (!ok) break;
+        const int row = row0 + r;
+        if (row < item.y) {
+          int64_t d = row;
+          if (cls == 1) {
+            const Double rr = decode_row(g, row);
+            d = row_to_d(g, rr, row);
+          }
+          const T dg = diag[n1 + d];
+          const int re = rx_t == 32767 ? OZ_NONFINITE : rx_t;
+#pragma unroll
+          for (int j = 0; j < NH; ++j) {
+            const int c = c0 + cbeg + j;
+            if (c >= m) continue;
+            const T x = V[(int64_t)c * ldv + n1 + d];
+            const double t = t2[j] * oz_pow2(sXe[cbeg + j] + re + TSH);
+            if constexpr (std::is_same<T, double>::value) W[(int64_t)c * ldw + n1 + d] = fma(dg, x, t);
+            else W[(int64_t)c * ldw + n1 + d] = fmaf(dg, x, (float)t);
+          }
+        }
+      }
+      if (!ok) break;
+      // every thread is past its reads of sXe before the next item's X
+      epi_sync();
+#pragma unroll
+      for (int s = 0; s < MS; ++s) {
+        if (s >= nslot) continue;
+        const int k = 128 * s + r;
+        const int seg = k >= nvP ? 1 : 0, a = k - seg * nvP;
+        if (k >= K || a >= nv) continue;
+        const int64_t single = (int64_t)a * no + (seg ? lp : kp);
+#pragma unroll
+        for (int j = 0; j < NH; ++j) {
+          const int c = c0 + cbeg + j;
+          const double w = acc[s][j] * oz_pow2(vexp[j] + TSH);
+          if (c < m && !(w == 0.0)) atomicAdd(&W1[(int64_t)c * ld1 + single], (TA)w);
+        }
+      }
+    }
+  }
+  // every role is done (or gave up): release TMEM
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  if (warp == 0) {
+    tmem_dealloc(tbase, 512);
+    tmem_relinquish();
+  }
+}
+
+}  // namespace
+
+// digit store of the rows [row0, row1) of B^T and the launch data of the pass
+struct OzPlan {
+  uint16_t* d_dig = nullptr;
+  int16_t* d_rexp = nullptr;
+  size_t dig_bytes = 0, rexp_rows = 0;
+  const void* values_for = nullptr;   // value store the digits were made of
+  int S = 0;
+  OzDst dst;
+  int2* d_items = nullptr;
+  int item_cap = 0, nitems = 0;
+  int64_t items_row0 = -1, items_row1 = -1;
+  int item_rows = 0;
+  int* d_vexp = nullptr;
+  int64_t vexp_cap = 0;
+  int* d_err = nullptr;
+  int* h_err = nullptr;
+};
+
+void oz_free(Ctx* c, void*& handle) {
+  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
+  if (!p) return;
+  dfree(c, p->d_dig);
+  dfree(c, p->d_rexp);
+  dfree(c, p->d_items);
+  dfree(c, p->d_vexp);
+  dfree(c, p->d_err);
+  if (p->h_err) cudaFreeHost(p->h_err);
+  delete p;
+  handle = nullptr;
+}
+
+void oz_invalidate(void* handle) {
+  if (OzPlan* p = reinterpret_cast<OzPlan*>(handle)) p->values_for = nullptr;
+}
+
+// C|D rows of up to 512 values (nvirt <= 256)
+bool oz_geometry_ok(const Geometry& G) { return G.no >= 2 && G.nv >= 2 && 2 * G.nvP <= 512; }
+
+namespace {
+
+size_t oz_digit_bytes(const Geometry& G, int64_t row0, int64_t row1, int S, OzDst* dst) {
+  int64_t n = 0, tiles = 0;
+  for (int cls = 0; cls < 5; ++cls) {
+    const int64_t a = std::max(row0, G.start[cls]), b = std::min(row1, G.start[cls + 1]), sl = G.slab_len(cls);
+    dst->base[cls] = n;
+    dst->r0[cls] = a;
+    dst->slab[cls] = sl;
+    dst->tps[cls] = (int)((sl + OZ_ROWS - 1) / OZ_ROWS);
+    dst->nbox[cls] = (int)(((cls >= 2 ? 2 : 1) * G.nvP + OZ_BOX - 1) / OZ_BOX);
+    dst->tiles[cls] = tiles;
+    const int64_t nt = a < b ? (b - a) / sl * dst->tps[cls] : 0;
+    tiles += nt;
+    n += nt * S * dst->nbox[cls] * OZ_ROWS * OZ_BOX;
+  }
+  dst->tiles[5] = tiles;
+  dst->row0 = row0;
+  dst->row1 = row1;
+  return (size_t)n * sizeof(uint16_t);
+}
+
+}  // namespace
+
+// Whether the pass may hold the digits of rows [row0, row1): they must fit a
+// third of the device memory that is free now (a matrix that nearly fills the
+// device keeps the CUDA-core tile).
+int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int m, bool* usable) {
+  *usable = false;
+  const Geometry& G = c->geom;
+  if (!oz_geometry_ok(G)) return ADCGPU_OK;
+  const int S = f64 ? 7 : 4;
+  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
+  if (!p) {
+    p = new OzPlan;
+    handle = p;
+  }
+  if (!p->d_err) {
+    ST(dmalloc(c, (void**)&p->d_err, sizeof(int)));
+    ADC_CUDA(c, cudaMallocHost((void**)&p->h_err, sizeof(int)));
+    ADC_CUDA(c, cudaMemsetAsync(p->d_err, 0, sizeof(int), c->stream));
+  }
+  OzDst dst;
+  const size_t bytes = oz_digit_bytes(G, row0, row1, S, &dst);
+  if (p->dig_bytes < bytes || p->rexp_rows < (size_t)(row1 - row0)) {
+    size_t free_b = 0, total_b = 0;
+    ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    if (bytes > (free_b + p->dig_bytes) / 3) return ADCGPU_OK;
+    dfree(c, p->d_dig);
+    dfree(c, p->d_rexp);
+    p->d_dig = nullptr;
+    p->d_rexp = nullptr;
+    p->dig_bytes = 0;
+    p->rexp_rows = 0;
+    p->values_for = nullptr;
+    ST(dmalloc(c, (void**)&p->d_dig, bytes));
+    p->dig_bytes = bytes;
+    ST(dmalloc(c, (void**)&p->d_rexp, sizeof(int16_t) * (size_t)(row1 - row0)));
+    p->rexp_rows = (size_t)(row1 - row0);
+  }
+  // the direct path rewrites one buffer chunk by chunk: values == nullptr
+  // never matches
+  if (!(p->values_for && p->values_for == values && p->S == S && p->dst.row0 == row0 && p->dst.row1 == row1)) {
+    p->dst = dst;
+    p->S = S;
+    const GeomDev g = to_dev(G);
+    const int grid = (int)std::min<int64_t>(dst.tiles[5] * OZ_ROWS / 8, (int64_t)c->nsm * 8);
+    if (f64) k_oz_values<double, 7><<<grid, 256, 0, c->stream>>>(g, dst, (const double*)values, p->d_dig, p->d_rexp);
+    else k_oz_values<float, 4><<<grid, 256, 0, c->stream>>>(g, dst, (const float*)values, p->d_dig, p->d_rexp);
+    ADC_COUNT_LAUNCH();
+    ADC_CUDA(c, cudaGetLastError());
+    p->values_for = c->direct ? nullptr : values;
+  }
+  // work items: pieces of one slab, about six per SM over the column
+  // groups, 4 to 32 tiles long
+  const int64_t ngrp = (m + 15) / 16;
+  int64_t want = (row1 - row0) * ngrp / ((int64_t)c->nsm * 6);
+  want = std::min<int64_t>(4096, std::max<int64_t>(512, (want + 127) / 128 * 128));
+  if (p->items_row0 != row0 || p->items_row1 != row1 || p->item_rows != (int)want) {
+    std::vector<int2> items;
+    for (int cls = 0; cls < 5; ++cls) {
+      const int64_t a = std::max(row0, G.start[cls]), b = std::min(row1, G.start[cls + 1]), sl = G.slab_len(cls);
+      for (int64_t s0 = a; s0 < b; s0 += sl) {
+        const int64_t npc = (sl + want - 1) / want, per = ((sl + npc - 1) / npc + 127) / 128 * 128;
+        for (int64_t x = s0; x < s0 + sl; x += per)
+          items.push_back(make_int2((int)x, (int)std::min<int64_t>(x + per, s0 + sl)));
+      }
+    }
+    if (p->item_cap < (int)items.size()) {
+      dfree(c, p->d_items);
+      p->d_items = nullptr;
+      p->item_cap = 0;
+      ST(dmalloc(c, (void**)&p->d_items, sizeof(int2) * items.size()));
+      p->item_cap = (int)items.size();
+    }
+    ADC_CUDA(c, h2d(c, p->d_items, items.data(), sizeof(int2) * items.size()));
+    p->nitems = (int)items.size();
+    p->items_row0 = row0;
+    p->items_row1 = row1;
+    p->item_rows = (int)want;
+  }
+  if (p->vexp_cap < (int64_t)p->nitems * m) {
+    dfree(c, p->d_vexp);
+    p->d_vexp = nullptr;
+    p->vexp_cap = 0;
+    ST(dmalloc(c, (void**)&p->d_vexp, sizeof(int) * (size_t)p->nitems * m));
+    p->vexp_cap = (int64_t)p->nitems * m;
+  }
+  *usable = true;
+  return ADCGPU_OK;
+}
+
+namespace {
+
+// shared memory of one launch; nb = 2 where TMEM and shared memory hold two
+// D1 / V2 buffers beside at least three ring slots; false when even one
+// buffer does not fit
+template <int S, int NP>
+bool oz_shape(const Geometry& G, int smax, OzShape* sh, size_t* bytes) {
+  constexpr int DW = oz_dw<S, NP>(), BOXB = oz_xrows<S, NP>() * 128, V2B = 2 * BOXB;
+  sh->nslot = (2 * G.nvP + 127) / 128;
+  const size_t tail = (size_t)(O_SLOT0 + 2 * OZ_MAXNR) * 8 + (size_t)NP * 4 + 16;
+  for (sh->nb = 2; sh->nb >= 1; --sh->nb) {
+    if ((sh->nb + sh->nslot) * DW > 512) continue;
+    sh->off_v2 = (uint32_t)(2 * sh->nslot) * BOXB;
+    sh->off_v2 = (sh->off_v2 + 1023) / 1024 * 1024;
+    sh->off_ring = sh->off_v2 + (uint32_t)sh->nb * V2B;
+    const int64_t room = (int64_t)smax - 1024 - (int64_t)tail - sh->off_ring;
+    sh->nr = (int)std::min<int64_t>(OZ_MAXNR, room / OZ_SLOT_BYTES);
+    if (sh->nr < (sh->nb == 2 ? 3 : 2)) continue;
+    sh->off_bar = sh->off_ring + (uint32_t)sh->nr * OZ_SLOT_BYTES;
+    *bytes = 1024 + sh->off_bar + tail;
+    return true;
+  }
+  return false;
+}
+
+template <int S, int NP, int MS, typename T, typename TA>
+int oz_go(Ctx* c, OzPlan* p, int smax, const OzShape& sh, size_t smem, const T* diag, const T* V, int64_t ldv, int m,
+          T* W, int64_t ldw, TA* W1, int64_t ld1) {
+  auto kern = k_sigma_oz<S, NP, MS, T, TA>;
+  ADC_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+  const int ngrp = (m + NP - 1) / NP;
+  const int grid = std::max(1, std::min(p->nitems * ngrp, c->nsm));
+  k_oz_vexp<T><<<dim3(p->nitems, (m + 3) / 4), 256, 0, c->stream>>>(to_dev(c->geom), p->d_items, p->dst.row0,
+                                                                    p->d_rexp, V, ldv, m, p->d_vexp);
+  ADC_COUNT_LAUNCH();
+  kern<<<grid, OZ_THREADS, smem, c->stream>>>(to_dev(c->geom), p->d_items, p->nitems, ngrp, sh, p->dst, p->d_dig,
+                                              p->d_rexp, p->d_vexp, diag, V, ldv, m, W, ldw, W1, ld1, p->d_err);
+  ADC_COUNT_LAUNCH();
+  ADC_CUDA(c, cudaGetLastError());
+  return ADCGPU_OK;
+}
+
+}  // namespace
+
+// The C|D products of m columns over the prepared rows: W2 rows are stored
+// with the diagonal term, W1 sums are added.
+int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t ldv, int m, double* W, int64_t ldw,
+              double* W1, int64_t ld1) {
+  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
+  const int smax = smem_optin_max(c);
+  OzShape sh;
+  size_t smem = 0;
+  // 16 columns per pass where their accumulators fit (rows of up to 384
+  // values); the column groups of an item run side by side, so the digits
+  // come from L2 for all but one of them
+  if (m > 8 && oz_shape<7, 16>(c->geom, smax, &sh, &smem))
+    return oz_go<7, 16, 3>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1);
+  if (!oz_shape<7, 8>(c->geom, smax, &sh, &smem)) return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
+  return oz_go<7, 8, 4>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1);
+}
+
+// Reads the kernel's error word (waits for the stream) and clears it.
+int oz_check(Ctx* c, void* handle) {
+  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
+  if (!p || !p->d_err) return ADCGPU_OK;
+  ADC_CUDA(c, cudaMemcpyAsync(p->h_err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  ADC_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (*p->h_err) {
+    const int code = *p->h_err;
+    ADC_CUDA(c, cudaMemsetAsync(p->d_err, 0, sizeof(int), c->stream));
+    return set_err(c, ADCGPU_DEVICE_TIMEOUT,
+                   "sliced sigma pass: a pipeline wait timed out (stage " + std::to_string(code) + ")");
+  }
+  return ADCGPU_OK;
+}
+
+}  // namespace adcgpu
