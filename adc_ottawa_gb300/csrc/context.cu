@@ -123,7 +123,8 @@ int adcgpu_ctx_create(int device, adcgpu_ctx** out) {
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && nsm > 0) c->nsm = nsm;
   else cudaGetLastError();
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
+      cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
+      cudaMallocHost((void**)&c->h_word, sizeof(int)) != cudaSuccess) {
     delete c;
     return ADCGPU_CUDA_ERROR;
   }
@@ -147,6 +148,7 @@ int adcgpu_ctx_destroy(adcgpu_ctx* h) {
   cudaEventDestroy(c->ev1);
   if (c->st_ev0) cudaEventDestroy(c->st_ev0);
   if (c->st_ev1) cudaEventDestroy(c->st_ev1);
+  cudaFreeHost(c->h_word);
   cudaStreamDestroy(c->stream);
   delete c;
   return ADCGPU_OK;

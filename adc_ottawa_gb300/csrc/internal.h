@@ -45,6 +45,7 @@
 #include <thread>
 #include <string>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "../../include/adcgpu.h"
@@ -247,6 +248,7 @@ struct Ctx {
   int nsm = 152;                  // streaming multiprocessors of the device (queried at creation)
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  int* h_word = nullptr;          // pinned word for device status reads
   std::string err;
   Geometry geom;
   bool have_orb = false, have_eri = false, have_matrix = false;
@@ -449,7 +451,9 @@ int umma3_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float
 
 // sigma_slices.cu : FP64-accurate tensor-core pass (exact digit slices)
 bool oz_geometry_ok(const Geometry& G);
-int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int m, bool* usable);
+std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, int64_t row1, int64_t* reserve);
+int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int64_t reserve, int m,
+               bool* usable);
 void oz_invalidate(void* handle);
 void oz_free(Ctx* c, void*& handle);
 int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t ldv, int m, double* W, int64_t ldw,

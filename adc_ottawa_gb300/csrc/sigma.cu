@@ -570,95 +570,8 @@ __global__ void __launch_bounds__(256) k_sigma_p3(GeomDev g, const int2* __restr
   }
 }
 
-// Segment A of the classes with a' < b' (W1 and W2 parts) beside the sliced
-// tensor-core pass: one warp per run of rows with equal a' in one slab, whose
-// rows (a', a'+1 .. nv-1) are consecutive.  Same lane groups as pass 2.
-template <typename T, typename TV, typename TA, int MC, int GS>
-__global__ void __launch_bounds__(256) k_sigma_sega(GeomDev g, const int2* __restrict__ items, int nitems,
-                                                    const TV* __restrict__ Bt, const T* __restrict__ V, int64_t ldv,
-                                                    T* __restrict__ W, int64_t ldw, TA* __restrict__ W1, int64_t ld1) {
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int no = g.no, nv = g.nv;
-  const int64_t n1 = g.n1;
-  const int nA = g.noP / 8;
-  const int slot = lane / GS, h = lane % GS;
-  constexpr int RPS = 32 / GS;
-  for (int it = warp; it < nitems; it += nwarps) {
-    const int2 item = items[it];
-    const int ap = item.y - 1;                       // items list b' = 1 .. nv-1
-    const Double r = decode_row(g, item.x);
-    const int cls = r.cls;
-    const int64_t L = g.len[cls], row0 = item.x + pair_index(ap, ap + 1, nv);
-    const int nrow = nv - 1 - ap;
-    const bool act = h < nA;
-    T xa[8][MC], ya[8][MC];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-#pragma unroll
-      for (int c = 0; c < MC; ++c) {
-        const int kk = 8 * h + u;
-        xa[u][c] = (act && kk < no) ? V[(int64_t)c * ldv + (int64_t)ap * no + kk] : T(0);
-        ya[u][c] = T(0);
-      }
-    for (int b0 = 0; b0 < nrow; b0 += RPS) {
-      const int rr = b0 + slot;
-      const bool rv = rr < nrow;
-      T v[8], x2[MC], w2[MC];
-      int64_t d = 0;
-      if (rv) {
-        const int64_t row = row0 + rr;
-        const Double dd{ap, ap + 1 + rr, r.kp, r.lp, cls};
-        d = row_to_d(g, dd, row);
-        if (act) Load8<T, TV>::go(Bt + g.off[cls] + (row - g.start[cls]) * L + 8 * h, v);
-      }
-      if (!(rv && act)) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = T(0);
-      }
-#pragma unroll
-      for (int c = 0; c < MC; ++c) {
-        x2[c] = rv ? V[(int64_t)c * ldv + n1 + d] : T(0);
-        w2[c] = (rv && h == 0) ? W[(int64_t)c * ldw + n1 + d] : T(0);
-      }
-#pragma unroll
-      for (int c = 0; c < MC; ++c) {
-        T z = T(0);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          ya[u][c] += v[u] * x2[c];
-          z += v[u] * xa[u][c];
-        }
-#pragma unroll
-        for (int o = 1; o < GS; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-        if (rv && h == 0) W[(int64_t)c * ldw + n1 + d] = w2[c] + z;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-#pragma unroll
-      for (int c = 0; c < MC; ++c) {
-        T y = ya[u][c];
-#pragma unroll
-        for (int o = GS; o < 32; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-        ya[u][c] = y;
-      }
-    if (slot == 0 && act) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int kk = 8 * h + u;
-        if (kk >= no) continue;
-#pragma unroll
-        for (int c = 0; c < MC; ++c)
-          if (ya[u][c] != T(0)) atomicAdd(&W1[(int64_t)c * ld1 + (int64_t)ap * no + kk], (TA)ya[u][c]);
-      }
-    }
-  }
-}
-
 // Segment A of the classes with a' = b' (1 and 3), storage rows [row0, row1):
-// one warp per row, lanes over k.
+// one warp per row and 4 columns, lanes over k.
 template <typename T, typename TV, typename TA>
 __global__ void __launch_bounds__(256) k_sigma_rows_a(GeomDev g, int64_t row0, int64_t row1,
                                                       const TV* __restrict__ Bt, const T* __restrict__ V, int64_t ldv,
@@ -669,7 +582,7 @@ __global__ void __launch_bounds__(256) k_sigma_rows_a(GeomDev g, int64_t row0, i
   for (int64_t row = row0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5); row < row1; row += nw) {
     const Double r = decode_row(g, row);
     const TV* rp = Bt + g.off[r.cls] + (row - g.start[r.cls]) * g.len[r.cls];
-    for (int c = 0; c < m; ++c) {
+    for (int c = 4 * blockIdx.y; c < min(m, 4 * (int)blockIdx.y + 4); ++c) {
       const T x2 = V[(int64_t)c * ldv + g.n1 + row];
       T z = T(0);
       for (int k = lane; k < g.no; k += 32) {
@@ -1368,23 +1281,24 @@ void launch_singles(Ctx* c, int m, const T* A, const T* diag, const T* V, int64_
   k_singles_gemm<T><<<grid, 128, 0, c->stream>>>(n1, A, diag, V, ldv, W, ldw, m); ADC_COUNT_LAUNCH();
 }
 
-// FP32 singles block with K split over about four blocks per SM: the
-// unsplit grid has only (n1/32) x (m/32) blocks, each walking all n1 values
-// of k, which leaves the product latency-bound.  The partials go to the
-// plan's scratch and are summed in a fixed order.
-int launch_singles_split(Ctx* c, int m, const float* A, const float* diag, const float* V, int64_t ldv, float* W,
-                         int64_t ldw) {
+// Singles block with K split over about four blocks per SM: the unsplit grid
+// has only (n1/32) x (m/32) blocks, each walking all n1 values of k, which
+// leaves the product latency-bound (FP64, nocc=10/nvirt=110, 10 columns:
+// 370 us).  The partials go to the plan's scratch and are summed in a fixed
+// order.
+template <typename T>
+int launch_singles_split(Ctx* c, int m, const T* A, const T* diag, const T* V, int64_t ldv, T* W, int64_t ldw) {
   const int n1 = (int)c->geom.n1;
   const int base = ((n1 + 31) / 32) * ((m + 31) / 32);
   const int ks = std::max(1, std::min(16, (4 * c->nsm + base - 1) / base));
   SigmaPlan* plan = reinterpret_cast<SigmaPlan*>(c->sigma_plan);
   if (ks == 1 || !plan) {
-    launch_singles<float>(c, m, A, diag, V, ldv, W, ldw);
+    launch_singles<T>(c, m, A, diag, V, ldv, W, ldw);
     return ADCGPU_OK;
   }
   const int kchunk = ((n1 + ks - 1) / ks + 31) / 32 * 32;
   const int ksu = (n1 + kchunk - 1) / kchunk;
-  const size_t need = sizeof(float) * (size_t)ksu * m * n1;
+  const size_t need = sizeof(T) * (size_t)ksu * m * n1;
   if (plan->sk_bytes < need) {
     dfree(c, plan->d_sk);
     plan->d_sk = nullptr;
@@ -1392,11 +1306,11 @@ int launch_singles_split(Ctx* c, int m, const float* A, const float* diag, const
     ST(dmalloc(c, &plan->d_sk, need));
     plan->sk_bytes = need;
   }
-  float* part = reinterpret_cast<float*>(plan->d_sk);
+  T* part = reinterpret_cast<T*>(plan->d_sk);
   dim3 grid((n1 + 31) / 32, (m + 31) / 32, ksu);
-  k_singles_gemm<float><<<grid, 128, 0, c->stream>>>(n1, A, diag, V, ldv, W, ldw, m, part, kchunk);
+  k_singles_gemm<T><<<grid, 128, 0, c->stream>>>(n1, A, diag, V, ldv, W, ldw, m, part, kchunk);
   ADC_COUNT_LAUNCH();
-  k_singles_reduce<float><<<std::min((n1 * m + 255) / 256, c->nsm * 8), 256, 0, c->stream>>>(n1, m, ksu, part, diag,
+  k_singles_reduce<T><<<std::min((n1 * m + 255) / 256, c->nsm * 8), 256, 0, c->stream>>>(n1, m, ksu, part, diag,
                                                                                           V, ldv, W, ldw);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
@@ -1484,24 +1398,6 @@ int launch_p2(Ctx* c, const GeomDev& g, const SigmaPlan* plan, int mc, const TV*
   return ADCGPU_OK;
 }
 
-// segment A of FP64 values beside the sliced pass, for mc <= 4 columns
-int launch_sega(Ctx* c, const GeomDev& g, const SigmaPlan* plan, int mc, const double* Bt, const double* V,
-                int64_t ldv, double* W, int64_t ldw, double* W1, int64_t ld1) {
-  const int g2 = std::min(plan->nitems, c->nsm * 8 * 8) / 8 + 1;
-  const int gs = g.noP <= 8 ? 1 : (g.noP <= 16 ? 2 : 4);
-  cudaStream_t s = c->stream;
-#define SA(MC, GS)                                                                                                  \
-  k_sigma_sega<double, double, double, MC, GS><<<g2, 256, 0, s>>>(g, plan->d_items, plan->nitems, Bt, V, ldv, W, ldw, \
-                                                                  W1, ld1)
-  if (mc == 4) { if (gs == 1) SA(4, 1); else if (gs == 2) SA(4, 2); else SA(4, 4); }
-  else if (mc == 2) { if (gs == 1) SA(2, 1); else if (gs == 2) SA(2, 2); else SA(2, 4); }
-  else { if (gs == 1) SA(1, 1); else if (gs == 2) SA(1, 2); else SA(1, 4); }
-#undef SA
-  ADC_COUNT_LAUNCH();
-  ADC_CUDA(c, cudaGetLastError());
-  return ADCGPU_OK;
-}
-
 // pass 3 (segment A's W1 part, after the tensor-core pass) for mc <= 8 columns
 template <typename TV>
 int launch_p3(Ctx* c, const GeomDev& g, const int2* runs, int nruns, int mc, const TV* Bt, const float* V,
@@ -1534,8 +1430,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
   ADC_CUDA(c, cudaEventRecord(c->st_ev0, s));
   GeomDev g = to_dev(G);
   // singles block first (plain stores), then the coupling adds atomically
-  if constexpr (sizeof(T) == 4) ST(launch_singles_split(c, m, A, diag, dV, ldv, dW, ldw));
-  else launch_singles<T>(c, m, A, diag, dV, ldv, dW, ldw);
+  ST(launch_singles_split<T>(c, m, A, diag, dV, ldv, dW, ldw));
   ADC_CUDA(c, cudaGetLastError());
   SigmaPlan* plan = reinterpret_cast<SigmaPlan*>(c->sigma_plan);
   if (!plan) return set_err(c, ADCGPU_NO_MATRIX, "sigma plan missing");
@@ -1563,24 +1458,22 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
     int c0 = 0;
     if constexpr (std::is_same<TV, double>::value) {
       if (P->tiled == 1 && !P->umma_off) {
-        bool usable = false;
-        ST(oz_prepare(c, plan->oz, BtP, true, row0, row1, m, &usable));
+        // the digits of a range are made and used before those of the next
+        int64_t reserve = 0;
+        bool usable = true;
+        for (const auto& rg : oz_ranges(c, row0, row1, &reserve)) {
+          ST(oz_prepare(c, plan->oz, BtP, true, rg.first, rg.second, reserve, m, &usable));
+          if (!usable) break;
+          ST(oz_launch(c, plan->oz, diag, dV, ldv, m, dW, ldw, dW, ldw));
+          oz_used = true;
+        }
         if (usable) {
           T* W1 = dW;
-          ST(oz_launch(c, plan->oz, diag, dV, ldv, m, dW, ldw, W1, ldw));
-          oz_used = true;
-          for (; P->nitems && c0 < m;) {
-            const int lb = m - c0, mc = lb >= 4 ? 4 : (lb >= 2 ? 2 : 1);
-            const T* Vb = dV + (int64_t)c0 * ldv;
-            T* Wb = dW + (int64_t)c0 * ldw;
-            ST(launch_sega(c, g, P, mc, BtP, Vb, ldv, Wb, ldw, Wb, ldw));
-            ST((launch_p2<T, TV, TAcc>(c, g, P, mc, BtP, Vb, ldv, Wb, ldw, reinterpret_cast<TAcc*>(Wb), ldw)));
-            c0 += mc;
-          }
+          // segment A of the classes with a' = b'
           for (int cls = 0; cls <= 2; cls += 2) {
             const int64_t a = std::max(row0, G.start[cls]), b = std::min(row1, G.start[cls + 1]);
             if (a >= b) continue;
-            k_sigma_rows_a<T, TV, T><<<(int)std::min<int64_t>((b - a + 7) / 8, c->nsm * 8), 256, 0, s>>>(
+            k_sigma_rows_a<T, TV, T><<<dim3((int)std::min<int64_t>((b - a + 7) / 8, c->nsm * 8), (m + 3) / 4), 256, 0, s>>>(
                 g, a, b, BtP, dV, ldv, m, dW, ldw, W1, ldw);
             ADC_COUNT_LAUNCH();
           }
@@ -2036,13 +1929,13 @@ int sigma_fp64(Ctx* c, int m, const double* dV, int64_t ldv, double* dW, int64_t
 // W = Hss V for the dense singles block alone (diag1 + A), m columns of n1
 // rows: the inner product of the folded preconditioner's MINRES solve.
 int singles_block_product(Ctx* c, int m, const double* V, int64_t ldv, double* W, int64_t ldw) {
-  launch_singles<double>(c, m, c->d_A, c->d_diag, V, ldv, W, ldw);
+  ST(launch_singles_split<double>(c, m, c->d_A, c->d_diag, V, ldv, W, ldw));
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
 }
 int singles_block_product(Ctx* c, int m, const float* V, int64_t ldv, float* W, int64_t ldw) {
   if (!c->d_A32 || !c->d_diag32) return set_err(c, ADCGPU_NO_MATRIX, "FP32 singles block missing");
-  ST(launch_singles_split(c, m, c->d_A32, c->d_diag32, V, ldv, W, ldw));
+  ST(launch_singles_split<float>(c, m, c->d_A32, c->d_diag32, V, ldv, W, ldw));
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
 }

@@ -283,9 +283,29 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
   return d;
 }
 
-// the group sums of NH columns -> T 2^(-8 max(S-4, 0)), T = sum_g D_g 2^(8(S-1-g)):
-// whole numbers combined in 64-bit integers, then two FP64 additions (the
-// integers are placed in the mantissa of 1.5 2^52 and 1.5 2^28)
+// group sums D_g (whole numbers) -> T 2^(-8 max(S-4, 0)), T = sum_g D_g 2^(8(S-1-g)):
+// combined in 64-bit integers, then two FP64 additions (the integers are
+// placed in the mantissa of 1.5 2^52 and 1.5 2^28)
+template <int S>
+__device__ __forceinline__ double oz_sum(const float (&d)[S]) {
+  long long hi = (long long)__float2int_rn(d[3]);
+  hi = mad_wide(__float2int_rn(d[2]), 1 << 8, hi);
+  hi = mad_wide(__float2int_rn(d[1]), 1 << 16, hi);
+  hi = mad_wide(__float2int_rn(d[0]), 1 << 24, hi);
+  if constexpr (S == 4) {
+    return __longlong_as_double(0x4338000000000000ll + hi) - 6755399441055744.0;
+  } else {
+    long long lo = (long long)__float2int_rn(d[6]);
+    lo = mad_wide(__float2int_rn(d[5]), 1 << 8, lo);
+    lo = mad_wide(__float2int_rn(d[4]), 1 << 16, lo);
+    const double x = __longlong_as_double(0x4338000000000000ll + hi) - (6755399441055744.0 + 402653184.0);
+    return x + __longlong_as_double(0x41B8000000000000ll + lo);
+  }
+}
+// weight exponent of oz_sum's unit against scaled operands |v| < 1
+template <int S> __host__ __device__ constexpr int oz_unit() { return -14 - 8 * (S - 1) + (S == 7 ? 24 : 0); }
+
+// the same of NH columns of a TMEM accumulator region
 template <int S, int NP, int NH>
 __device__ __forceinline__ void oz_combine(uint32_t taddr, double (&t)[NH]) {
   float d[S][NH];
@@ -294,19 +314,10 @@ __device__ __forceinline__ void oz_combine(uint32_t taddr, double (&t)[NH]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
   for (int j = 0; j < NH; ++j) {
-    long long hi = (long long)__float2int_rn(d[3][j]);
-    hi = mad_wide(__float2int_rn(d[2][j]), 1 << 8, hi);
-    hi = mad_wide(__float2int_rn(d[1][j]), 1 << 16, hi);
-    hi = mad_wide(__float2int_rn(d[0][j]), 1 << 24, hi);
-    if constexpr (S == 4) {
-      t[j] = __longlong_as_double(0x4338000000000000ll + hi) - 6755399441055744.0;
-    } else {
-      long long lo = (long long)__float2int_rn(d[6][j]);
-      lo = mad_wide(__float2int_rn(d[5][j]), 1 << 8, lo);
-      lo = mad_wide(__float2int_rn(d[4][j]), 1 << 16, lo);
-      const double x = __longlong_as_double(0x4338000000000000ll + hi) - (6755399441055744.0 + 402653184.0);
-      t[j] = x + __longlong_as_double(0x41B8000000000000ll + lo);
-    }
+    float x[S];
+#pragma unroll
+    for (int gI = 0; gI < S; ++gI) x[gI] = d[gI][j];
+    t[j] = oz_sum<S>(x);
   }
 }
 
@@ -324,7 +335,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   constexpr int V2B = 2 * BOXB;
   constexpr int NH = NP / 4;                       // columns per epilogue thread
   constexpr int FB = 8 * S - 1;                    // fraction bits of the digits
-  constexpr int TSH = -14 - 8 * (S - 1) + (S == 7 ? 24 : 0);   // weight of oz_combine4's unit
+  constexpr int TSH = oz_unit<S>();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sX = base;                        // 2 nslot boxes [XR rows x 64 k]
@@ -659,35 +670,307 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Segments A and B: singles (a', k) and (b', k) of the classes with a' < b'.
+//
+// A run is the rows of one slab with equal a' (segment A; consecutive rows)
+// or equal b' (segment B), coupled to the singles (f, k) of that fixed
+// virtual f.  With R the run's rows x nocc segment values the products are
+//   W2[r, c] += sum_k R[r, k] V[(f, k), c]
+//   W1[(f, k), c] += sum_r R[r, k] V2[r, c]
+// nocc is too short for a tcgen05 tile, so one warp takes a run and 16
+// columns with mma.sync m16n8k16 on the same digits: 16 rows a step, staged
+// by cp.async, their digits read by ldmatrix for W2 (K = k) and transposed
+// for W1 (K = rows); the vectors' digits are made in registers.
+// On the FP64 pipe the two segments took 34 of 50 ms (40 columns at
+// nocc=16/nvirt=180).
+// ---------------------------------------------------------------------------
+
+// digits of the segments: [row - row0][segment A, B][slice][kw], kw = nocc
+// rounded up to 16; one exponent per row over both segments
+template <typename TV, int S>
+__global__ void __launch_bounds__(256) k_oz_seg_values(GeomDev g, int64_t row0, int64_t row1, int kw,
+                                                       const TV* __restrict__ Bt, uint16_t* __restrict__ out,
+                                                       int16_t* __restrict__ sexp) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t row = row0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5); row < row1; row += nw) {
+    const int cls = row < g.start[1] ? 0 : row < g.start[2] ? 1 : row < g.start[3] ? 2 : row < g.start[4] ? 3 : 4;
+    if (!(cls == 1 || cls >= 3)) continue;
+    const TV* src = Bt + g.off[cls] + (row - g.start[cls]) * g.len[cls];
+    uint16_t* o = out + (row - row0) * 2 * S * kw;
+    int mx = OZ_ZERO;
+    for (int x = lane; x < 2 * kw; x += 32) {
+      const int seg = x >= kw ? 1 : 0, k = x - seg * kw;
+      if (k < g.no) mx = max(mx, Parts<TV>::exponent(src[seg * g.noP + k]));
+    }
+    mx = max(__reduce_max_sync(0xffffffffu, mx), OZ_EMIN);
+    if (lane == 0) sexp[row - row0] = (int16_t)min(mx, 32767);
+    for (int x = lane; x < 2 * kw; x += 32) {
+      const int seg = x >= kw ? 1 : 0, k = x - seg * kw;
+      const unsigned long long u = oz_fixed<S, TV>(k < g.no ? src[seg * g.noP + k] : TV(0), 8 * S - 1 - mx);
+#pragma unroll
+      for (int i = 0; i < S; ++i) o[(seg * S + i) * kw + k] = (uint16_t)(oz_digit<S>(u, i) >> 16);
+    }
+  }
+}
+
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_seg(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+constexpr int SEG_WARPS = 4;
+template <int S, int KT> __host__ __device__ constexpr int seg_pitch() { return S * KT * 32 + 16; }   // bytes of a staged row
+
+// exponent of a column over the four lanes that hold it
+__device__ __forceinline__ int quad_max(int e) {
+  e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+  return max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+}
+
+// digits of 8 vector values as A fragments of m16n8k16: columns c = lane / 4
+// and + 8, positions p = 2 (lane % 4), + 1, + 8, + 9; x[2 h + v] is position
+// v of column half h (v = 0..3 in that order), sc[v] its power-of-two scale
+template <int S, typename T>
+__device__ __forceinline__ void seg_fragments(const T (&x)[2][4], const int (&sc)[4], const int (&ex)[2],
+                                              uint32_t (&f)[S][4]) {
+  unsigned long long u[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      u[h][v] = oz_fixed<S, T>(ex[h] == OZ_NONFINITE ? T(0) : x[h][v], 8 * S - 1 - ex[h] + sc[v]);
+#pragma unroll
+  for (int i = 0; i < S; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      f[i][h] = oz_pair(oz_digit<S>(u[h][0], i), oz_digit<S>(u[h][1], i));
+      f[i][2 + h] = oz_pair(oz_digit<S>(u[h][2], i), oz_digit<S>(u[h][3], i));
+    }
+}
+
+// SEGB: runs of equal b' (segment B), else of equal a' (segment A)
+template <int S, int KT, bool SEGB, typename T, typename TA>
+__global__ void __launch_bounds__(32 * SEG_WARPS)
+    k_oz_seg(GeomDev g, const int2* __restrict__ slabs, int nslab, int ngrp, int64_t row_base,
+             const uint16_t* __restrict__ dig, const int16_t* __restrict__ sexp, const T* __restrict__ V, int64_t ldv,
+             int m, T* __restrict__ W, int64_t ldw, TA* __restrict__ W1, int64_t ld1) {
+  constexpr int PITCH = seg_pitch<S, KT>(), NPIECE = 16 * S * KT * 2, KW = 16 * KT, TSH = oz_unit<S>();
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int gid = lane >> 2, tig = lane & 3;
+  unsigned char* stage = smem + wid * 2 * 16 * PITCH;
+  const uint32_t sbase = smem_u32(stage);
+  const int no = g.no, nv = g.nv;
+  const int64_t n1 = g.n1;
+  const int64_t nrun = (int64_t)nslab * ngrp * (nv - 1);
+  for (int64_t run = blockIdx.x * (int64_t)SEG_WARPS + wid; run < nrun; run += (int64_t)gridDim.x * SEG_WARPS) {
+    const int fi = (int)(run % (nv - 1));
+    const int64_t sg = run / (nv - 1);
+    const int c0 = (int)(sg % ngrp) * 16;
+    const int2 sl = slabs[sg / ngrp];                   // first row, class
+    const int cls = sl.y;
+    const int f = SEGB ? fi + 1 : fi;
+    const int nrow = SEGB ? f : nv - 1 - f;
+    // slab-local pair of row t of the run; vector index of a pair
+    auto pair_of = [&](int t) -> int64_t { return SEGB ? pair_index(t, f, nv) : pair_index(f, f + 1 + t, nv); };
+    const int64_t kloc = cls == 1 ? (sl.x - g.start[1]) / g.npair_v : 0;
+    const int64_t dbase = n1 + (cls == 1 ? g.start[1] + kloc : (int64_t)sl.x);
+    const int dstr = cls == 1 ? no : 1;
+    const int64_t rloc = sl.x - row_base;
+    const int cc[2] = {c0 + gid, c0 + gid + 8};
+    auto issue = [&](int t0, int b) {
+      for (int p = lane; p < NPIECE; p += 32) {
+        const int rr = p / (S * KT * 2), w = p - rr * (S * KT * 2);
+        const bool ok = t0 + rr < nrow;
+        const uint16_t* src = dig + ((rloc + (ok ? pair_of(t0 + rr) : 0)) * 2 + (SEGB ? 1 : 0)) * (S * KW) + 8 * w;
+        const uint32_t dst = sbase + (uint32_t)((b * 16 + rr) * PITCH + 16 * w);
+        const int n = ok ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n));
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+    };
+    __syncwarp();
+    issue(0, 0);
+    // positions of this lane in a step of 16 rows
+    const int pos[4] = {2 * tig, 2 * tig + 1, 2 * tig + 8, 2 * tig + 9};
+    auto load_v2 = [&](int t0, T (&x)[2][4], int (&er)[4]) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int t = t0 + pos[v];
+        const bool ok = t < nrow;
+        const int64_t pr = ok ? pair_of(t) : 0;
+        er[v] = ok ? (int)sexp[rloc + pr] : OZ_EMIN;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          x[h][v] = (ok && cc[h] < m) ? __ldg(V + (int64_t)cc[h] * ldv + dbase + pr * dstr) : T(0);
+      }
+    };
+    // column exponents of the run's 2^er V2
+    int ev[2] = {OZ_EMIN, OZ_EMIN};
+    for (int t0 = 0; t0 < nrow; t0 += 16) {
+      T x[2][4];
+      int er[4];
+      load_v2(t0, x, er);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int e = Parts<T>::exponent(x[h][v]);
+          if (e == OZ_NONFINITE || er[v] == 32767) ev[h] = OZ_NONFINITE;
+          else if (e != OZ_ZERO) ev[h] = max(ev[h], e + er[v]);
+        }
+    }
+    ev[0] = quad_max(ev[0]);
+    ev[1] = quad_max(ev[1]);
+    // V of the singles (f, k)
+    uint32_t xf[KT][S][4];
+    int ex[2] = {OZ_EMIN, OZ_EMIN};
+    {
+      T x[KT][2][4];
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const int k = 16 * kt + pos[v];
+            x[kt][h][v] = (k < no && cc[h] < m) ? __ldg(V + (int64_t)cc[h] * ldv + (int64_t)f * no + k) : T(0);
+            ex[h] = max(ex[h], Parts<T>::exponent(x[kt][h][v]));
+          }
+      ex[0] = quad_max(ex[0]);
+      ex[1] = quad_max(ex[1]);
+      const int sc0[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt) seg_fragments<S, T>(x[kt], sc0, ex, xf[kt]);
+    }
+    float a1[2 * KT][S][4];
+#pragma unroll
+    for (int n = 0; n < 2 * KT; ++n)
+#pragma unroll
+      for (int i = 0; i < S; ++i) a1[n][i][0] = a1[n][i][1] = a1[n][i][2] = a1[n][i][3] = 0.f;
+    int b = 0;
+    for (int t0 = 0; t0 < nrow; t0 += 16, b ^= 1) {
+      __syncwarp();                                       // the other stage's readers are done
+      if (t0 + 16 < nrow) issue(t0 + 16, b ^ 1);
+      else asm volatile("cp.async.commit_group;\n" ::);
+      T x[2][4];
+      int er[4];
+      load_v2(t0, x, er);
+      uint32_t vf[S][4];
+      seg_fragments<S, T>(x, er, ev, vf);
+      asm volatile("cp.async.wait_group 1;\n" ::);
+      __syncwarp();
+      // 16 x 16 digits of slice i, k group kt: row lane % 16, half lane / 16
+      const uint32_t srow = sbase + (uint32_t)((b * 16 + (lane & 15)) * PITCH + (lane >> 4) * 16);
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+          uint32_t q[4];
+          ldsm_x4_t(q, srow + (i * KT + kt) * 32);        // (rows 0-7, 8-15) x k 0-7, then k 8-15
+#pragma unroll
+          for (int j = 0; j < S - i; ++j) {
+            mma_seg(a1[2 * kt][i + j], vf[j], q[0], q[1]);
+            mma_seg(a1[2 * kt + 1][i + j], vf[j], q[2], q[3]);
+          }
+        }
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {                    // rows t0 + 8 hr ..
+        float a2[S][4];
+#pragma unroll
+        for (int i = 0; i < S; ++i) a2[i][0] = a2[i][1] = a2[i][2] = a2[i][3] = 0.f;
+        // two slices at a time: (slice i, k 0-7), (i, k 8-15), (i + 1, ..)
+        const uint32_t srow2 = sbase + (uint32_t)((b * 16 + 8 * hr + (lane & 7)) * PITCH + ((lane >> 3) & 1) * 16);
+#pragma unroll
+        for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+          for (int i = 0; i < S; i += 2) {
+            uint32_t q[4];
+            const int i2 = i + 1 < S ? i + 1 : i;
+            ldsm_x4(q, srow2 + (uint32_t)(((lane >> 4) ? i2 : i) * KT + kt) * 32);
+#pragma unroll
+            for (int j = 0; j < S - i; ++j) mma_seg(a2[i + j], xf[kt][j], q[0], q[1]);
+            if (i + 1 < S) {
+#pragma unroll
+              for (int j = 0; j < S - i - 1; ++j) mma_seg(a2[i + 1 + j], xf[kt][j], q[2], q[3]);
+            }
+          }
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const int t = t0 + 8 * hr + pos[v];
+          if (t >= nrow) continue;
+          const int64_t d = dbase + pair_of(t) * dstr;
+          const int e = er[2 * hr + v] == 32767 ? OZ_NONFINITE : er[2 * hr + v];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (cc[h] >= m) continue;
+            float dsum[S];
+#pragma unroll
+            for (int i = 0; i < S; ++i) dsum[i] = a2[i][2 * h + v];
+            T* w = W + (int64_t)cc[h] * ldw + d;
+            *w = (T)fma(oz_sum<S>(dsum), oz_pow2(ex[h] + e + TSH), (double)*w);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2 * KT; ++n)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const int k = 8 * n + 2 * tig + v;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (k >= no || cc[h] >= m) continue;
+          float dsum[S];
+#pragma unroll
+          for (int i = 0; i < S; ++i) dsum[i] = a1[n][i][2 * h + v];
+          const double w = oz_sum<S>(dsum) * oz_pow2(ev[h] + TSH);
+          if (!(w == 0.0)) atomicAdd(&W1[(int64_t)cc[h] * ld1 + (int64_t)f * no + k], (TA)w);
+        }
+      }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+}
+
 }  // namespace
 
-// digit store of the rows [row0, row1) of B^T and the launch data of the pass
+// Digit store of the rows [row0, row1) of B^T and the work lists of the pass.
 struct OzPlan {
-  uint16_t* d_dig = nullptr;
-  int16_t* d_rexp = nullptr;
-  size_t dig_bytes = 0, rexp_rows = 0;
+  unsigned char* d_mem = nullptr;     // C|D digits, segment digits, their row exponents
+  size_t mem_bytes = 0;
+  uint16_t *dig = nullptr, *seg = nullptr;
+  int16_t *rexp = nullptr, *sexp = nullptr;
   const void* values_for = nullptr;   // value store the digits were made of
   int S = 0;
   OzDst dst;
-  int2* d_items = nullptr;
-  int item_cap = 0, nitems = 0;
-  int64_t items_row0 = -1, items_row1 = -1;
-  int item_rows = 0;
-  int* d_vexp = nullptr;
-  int64_t vexp_cap = 0;
-  int* d_err = nullptr;
-  int* h_err = nullptr;
+  unsigned char* d_lists = nullptr;   // error word, work items, slabs, item exponents
+  size_t list_bytes = 0;
+  int* err = nullptr;
+  int2 *items = nullptr, *slabs = nullptr;
+  int* vexp = nullptr;
+  std::vector<int2> h_items, h_slabs; // host copies: all rows, in storage order
+  int item0 = 0, nitems = 0;          // those of the prepared rows
+  int slab0 = 0, nslab = 0;
+  int item_rows = 0, lists_m = 0;
 };
 
 void oz_free(Ctx* c, void*& handle) {
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
   if (!p) return;
-  dfree(c, p->d_dig);
-  dfree(c, p->d_rexp);
-  dfree(c, p->d_items);
-  dfree(c, p->d_vexp);
-  dfree(c, p->d_err);
-  if (p->h_err) cudaFreeHost(p->h_err);
+  dfree(c, p->d_mem);
+  dfree(c, p->d_lists);
   delete p;
   handle = nullptr;
 }
@@ -696,10 +979,19 @@ void oz_invalidate(void* handle) {
   if (OzPlan* p = reinterpret_cast<OzPlan*>(handle)) p->values_for = nullptr;
 }
 
-// C|D rows of up to 512 values (nvirt <= 256)
-bool oz_geometry_ok(const Geometry& G) { return G.no >= 2 && G.nv >= 2 && 2 * G.nvP <= 512; }
+// C|D rows of up to 512 values (nvirt <= 256), segments of up to 32: every
+// system the library takes
+bool oz_geometry_ok(const Geometry& G) { return G.no <= 32 && G.nv >= 2 && 2 * G.nvP <= 512; }
 
 namespace {
+
+// rows of a typical range of the direct path: the digits of a range take about
+// as many bytes as the FP64 values of a chunk, three times those of its rows
+int64_t direct_range_rows(const Ctx* c) {
+  int64_t rows = 1;
+  for (const DirectChunk& d : c->dchunks) rows = std::max(rows, (d.row1 - d.row0) / 3);
+  return rows;
+}
 
 size_t oz_digit_bytes(const Geometry& G, int64_t row0, int64_t row1, int S, OzDst* dst) {
   int64_t n = 0, tiles = 0;
@@ -721,12 +1013,67 @@ size_t oz_digit_bytes(const Geometry& G, int64_t row0, int64_t row1, int S, OzDs
   return (size_t)n * sizeof(uint16_t);
 }
 
+size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+struct OzBytes { size_t dig, seg, exp, all; };
+OzBytes oz_bytes(const Geometry& G, int64_t row0, int64_t row1, int S, OzDst* dst) {
+  OzBytes b;
+  const int kw = (G.no + 15) / 16 * 16;
+  const size_t nrows = (size_t)(row1 - row0);
+  b.dig = align256(oz_digit_bytes(G, row0, row1, S, dst));
+  b.seg = align256(nrows * 2 * S * kw * sizeof(uint16_t));
+  b.exp = align256(nrows * sizeof(int16_t));
+  b.all = b.dig + b.seg + 2 * b.exp;
+  return b;
+}
+
 }  // namespace
 
-// Whether the pass may hold the digits of rows [row0, row1): they must fit a
-// third of the device memory that is free now (a matrix that nearly fills the
-// device keeps the CUDA-core tile).
-int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int m, bool* usable) {
+// The rows [row0, row1) as ranges of whole slabs whose digits are prepared
+// and used together: one range for a stored matrix; on the direct path, whose
+// point is a small footprint, ranges whose digits take no more than the chunk
+// buffer (never less than one slab).  *reserve: the most that any range of the
+// matrix takes.
+std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, int64_t row1, int64_t* reserve) {
+  const Geometry& G = c->geom;
+  std::vector<std::pair<int64_t, int64_t>> out;
+  *reserve = 0;
+  if (!c->direct) {
+    out.emplace_back(row0, row1);
+    return out;
+  }
+  const int64_t budget = direct_budget(G) * (int64_t)sizeof(double);
+  *reserve = budget;
+  for (int cls = 0; cls < 5; ++cls) {
+    OzDst d;
+    if (G.start[cls] < G.start[cls + 1])
+      *reserve = std::max<int64_t>(*reserve, oz_bytes(G, G.start[cls], G.start[cls] + G.slab_len(cls), 7, &d).all);
+  }
+  int64_t used = 0;
+  for (int cls = 0; cls < 5; ++cls) {
+    const int64_t a = std::max(row0, G.start[cls]), b = std::min(row1, G.start[cls + 1]), sl = G.slab_len(cls);
+    for (int64_t s0 = a; s0 < b; s0 += sl) {
+      OzDst d;
+      const int64_t n = (int64_t)oz_bytes(G, s0, s0 + sl, 7, &d).all;
+      if (out.empty() || used + n > budget) {
+        out.emplace_back(s0, s0);
+        used = 0;
+      }
+      out.back().second = s0 + sl;
+      used += n;
+    }
+  }
+  return out;
+}
+
+// Makes the digits of the rows [row0, row1) (kept until the values change;
+// the direct path's chunk buffer is rewritten for every chunk) and the work
+// lists of an m-column product.  reserve: bytes the digits of any range of
+// this matrix may take.  *usable stays false, and the CUDA-core tile takes the
+// product, for shapes the pass does not take and when the digits would fill
+// more than a third of the device memory that is free now.
+int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int64_t reserve, int m,
+               bool* usable) {
   *usable = false;
   const Geometry& G = c->geom;
   if (!oz_geometry_ok(G)) return ADCGPU_OK;
@@ -736,77 +1083,88 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
     p = new OzPlan;
     handle = p;
   }
-  if (!p->d_err) {
-    ST(dmalloc(c, (void**)&p->d_err, sizeof(int)));
-    ADC_CUDA(c, cudaMallocHost((void**)&p->h_err, sizeof(int)));
-    ADC_CUDA(c, cudaMemsetAsync(p->d_err, 0, sizeof(int), c->stream));
-  }
   OzDst dst;
-  const size_t bytes = oz_digit_bytes(G, row0, row1, S, &dst);
-  if (p->dig_bytes < bytes || p->rexp_rows < (size_t)(row1 - row0)) {
+  const int kw = (G.no + 15) / 16 * 16;
+  const OzBytes need = oz_bytes(G, row0, row1, S, &dst);
+  const size_t bytes = std::max(need.all, (size_t)reserve);
+  if (p->mem_bytes < bytes) {
     size_t free_b = 0, total_b = 0;
     ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
-    if (bytes > (free_b + p->dig_bytes) / 3) return ADCGPU_OK;
-    dfree(c, p->d_dig);
-    dfree(c, p->d_rexp);
-    p->d_dig = nullptr;
-    p->d_rexp = nullptr;
-    p->dig_bytes = 0;
-    p->rexp_rows = 0;
+    if (bytes > (free_b + p->mem_bytes) / 3) return ADCGPU_OK;
+    dfree(c, p->d_mem);
+    p->d_mem = nullptr;
+    p->mem_bytes = 0;
     p->values_for = nullptr;
-    ST(dmalloc(c, (void**)&p->d_dig, bytes));
-    p->dig_bytes = bytes;
-    ST(dmalloc(c, (void**)&p->d_rexp, sizeof(int16_t) * (size_t)(row1 - row0)));
-    p->rexp_rows = (size_t)(row1 - row0);
+    ST(dmalloc(c, (void**)&p->d_mem, bytes));
+    p->mem_bytes = bytes;
   }
-  // the direct path rewrites one buffer chunk by chunk: values == nullptr
-  // never matches
   if (!(p->values_for && p->values_for == values && p->S == S && p->dst.row0 == row0 && p->dst.row1 == row1)) {
     p->dst = dst;
     p->S = S;
+    p->dig = reinterpret_cast<uint16_t*>(p->d_mem);
+    p->seg = reinterpret_cast<uint16_t*>(p->d_mem + need.dig);
+    p->rexp = reinterpret_cast<int16_t*>(p->d_mem + need.dig + need.seg);
+    p->sexp = reinterpret_cast<int16_t*>(p->d_mem + need.dig + need.seg + need.exp);
     const GeomDev g = to_dev(G);
     const int grid = (int)std::min<int64_t>(dst.tiles[5] * OZ_ROWS / 8, (int64_t)c->nsm * 8);
-    if (f64) k_oz_values<double, 7><<<grid, 256, 0, c->stream>>>(g, dst, (const double*)values, p->d_dig, p->d_rexp);
-    else k_oz_values<float, 4><<<grid, 256, 0, c->stream>>>(g, dst, (const float*)values, p->d_dig, p->d_rexp);
-    ADC_COUNT_LAUNCH();
+    const int grid2 = (int)std::min<int64_t>((row1 - row0 + 7) / 8, (int64_t)c->nsm * 8);
+    auto make = [&](auto* v, auto s) {
+      using TV = typename std::remove_const<typename std::remove_pointer<decltype(v)>::type>::type;
+      k_oz_values<TV, decltype(s)::value><<<grid, 256, 0, c->stream>>>(g, dst, v, p->dig, p->rexp);
+      ADC_COUNT_LAUNCH();
+      k_oz_seg_values<TV, decltype(s)::value><<<grid2, 256, 0, c->stream>>>(g, row0, row1, kw, v, p->seg, p->sexp);
+      ADC_COUNT_LAUNCH();
+    };
+    if (f64) make((const double*)values, std::integral_constant<int, 7>());
+    else make((const float*)values, std::integral_constant<int, 4>());
     ADC_CUDA(c, cudaGetLastError());
     p->values_for = c->direct ? nullptr : values;
   }
-  // work items: pieces of one slab, about six per SM over the column
-  // groups, 4 to 32 tiles long
+  // work items: pieces of one slab, about six per SM over the column groups
+  // of the prepared rows, 1 to 32 tiles long (the vector operand of an item
+  // costs about a third of a tile)
   const int64_t ngrp = (m + 15) / 16;
-  int64_t want = (row1 - row0) * ngrp / ((int64_t)c->nsm * 6);
-  want = std::min<int64_t>(4096, std::max<int64_t>(512, (want + 127) / 128 * 128));
-  if (p->items_row0 != row0 || p->items_row1 != row1 || p->item_rows != (int)want) {
-    std::vector<int2> items;
+  int64_t want = (c->direct ? direct_range_rows(c) : row1 - row0) * ngrp / ((int64_t)c->nsm * 6);
+  want = std::min<int64_t>(4096, std::max<int64_t>(128, (want + 127) / 128 * 128));
+  if (p->item_rows != (int)want || p->lists_m < m) {
+    p->h_items.clear();
+    p->h_slabs.clear();
     for (int cls = 0; cls < 5; ++cls) {
-      const int64_t a = std::max(row0, G.start[cls]), b = std::min(row1, G.start[cls + 1]), sl = G.slab_len(cls);
-      for (int64_t s0 = a; s0 < b; s0 += sl) {
+      const int64_t sl = G.slab_len(cls);
+      for (int64_t s0 = G.start[cls]; s0 < G.start[cls + 1]; s0 += sl) {
         const int64_t npc = (sl + want - 1) / want, per = ((sl + npc - 1) / npc + 127) / 128 * 128;
         for (int64_t x = s0; x < s0 + sl; x += per)
-          items.push_back(make_int2((int)x, (int)std::min<int64_t>(x + per, s0 + sl)));
+          p->h_items.push_back(make_int2((int)x, (int)std::min<int64_t>(x + per, s0 + sl)));
+        if (cls == 1 || cls >= 3) p->h_slabs.push_back(make_int2((int)s0, cls));
       }
     }
-    if (p->item_cap < (int)items.size()) {
-      dfree(c, p->d_items);
-      p->d_items = nullptr;
-      p->item_cap = 0;
-      ST(dmalloc(c, (void**)&p->d_items, sizeof(int2) * items.size()));
-      p->item_cap = (int)items.size();
+    const size_t ni = p->h_items.size(), ns = p->h_slabs.size();
+    const size_t lb = align256(sizeof(int2) * (ni + ns)), lneed = 256 + lb + sizeof(int) * ni * m;
+    if (p->list_bytes < lneed) {
+      dfree(c, p->d_lists);
+      p->d_lists = nullptr;
+      p->list_bytes = 0;
+      ST(dmalloc(c, (void**)&p->d_lists, lneed));
+      p->list_bytes = lneed;
+      p->err = reinterpret_cast<int*>(p->d_lists);
+      ADC_CUDA(c, cudaMemsetAsync(p->err, 0, sizeof(int), c->stream));
     }
-    ADC_CUDA(c, h2d(c, p->d_items, items.data(), sizeof(int2) * items.size()));
-    p->nitems = (int)items.size();
-    p->items_row0 = row0;
-    p->items_row1 = row1;
+    p->items = reinterpret_cast<int2*>(p->d_lists + 256);
+    p->slabs = p->items + ni;
+    p->vexp = reinterpret_cast<int*>(p->d_lists + 256 + lb);
+    std::vector<int2> all(p->h_items);
+    all.insert(all.end(), p->h_slabs.begin(), p->h_slabs.end());
+    ADC_CUDA(c, h2d(c, p->items, all.data(), sizeof(int2) * all.size()));
     p->item_rows = (int)want;
+    p->lists_m = m;
   }
-  if (p->vexp_cap < (int64_t)p->nitems * m) {
-    dfree(c, p->d_vexp);
-    p->d_vexp = nullptr;
-    p->vexp_cap = 0;
-    ST(dmalloc(c, (void**)&p->d_vexp, sizeof(int) * (size_t)p->nitems * m));
-    p->vexp_cap = (int64_t)p->nitems * m;
-  }
+  auto first = [](const std::vector<int2>& v, int64_t row) {
+    return (int)(std::lower_bound(v.begin(), v.end(), row, [](const int2& a, int64_t r) { return a.x < r; }) - v.begin());
+  };
+  p->item0 = first(p->h_items, row0);
+  p->nitems = first(p->h_items, row1) - p->item0;
+  p->slab0 = first(p->h_slabs, row0);
+  p->nslab = first(p->h_slabs, row1) - p->slab0;
   *usable = true;
   return ADCGPU_OK;
 }
@@ -843,20 +1201,48 @@ int oz_go(Ctx* c, OzPlan* p, int smax, const OzShape& sh, size_t smem, const T* 
   ADC_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   const int ngrp = (m + NP - 1) / NP;
   const int grid = std::max(1, std::min(p->nitems * ngrp, c->nsm));
-  k_oz_vexp<T><<<dim3(p->nitems, (m + 3) / 4), 256, 0, c->stream>>>(to_dev(c->geom), p->d_items, p->dst.row0,
-                                                                    p->d_rexp, V, ldv, m, p->d_vexp);
+  k_oz_vexp<T><<<dim3(p->nitems, (m + 3) / 4), 256, 0, c->stream>>>(to_dev(c->geom), p->items + p->item0, p->dst.row0, p->rexp,
+                                                                    V, ldv, m, p->vexp);
   ADC_COUNT_LAUNCH();
-  kern<<<grid, OZ_THREADS, smem, c->stream>>>(to_dev(c->geom), p->d_items, p->nitems, ngrp, sh, p->dst, p->d_dig,
-                                              p->d_rexp, p->d_vexp, diag, V, ldv, m, W, ldw, W1, ld1, p->d_err);
+  kern<<<grid, OZ_THREADS, smem, c->stream>>>(to_dev(c->geom), p->items + p->item0, p->nitems, ngrp, sh, p->dst, p->dig, p->rexp,
+                                              p->vexp, diag, V, ldv, m, W, ldw, W1, ld1, p->err);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
 }
 
+// segments A and B of m columns: W2 rows and W1 sums are added to
+template <int S, int KT, bool SEGB, typename T, typename TA>
+int oz_seg_go(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t ldw, TA* W1, int64_t ld1) {
+  auto kern = k_oz_seg<S, KT, SEGB, T, TA>;
+  const size_t smem = (size_t)SEG_WARPS * 2 * 16 * seg_pitch<S, KT>();
+  ADC_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int ngrp = (m + 15) / 16;
+  const int64_t nrun = (int64_t)p->nslab * ngrp * (c->geom.nv - 1);
+  const int grid = (int)std::min<int64_t>((nrun + SEG_WARPS - 1) / SEG_WARPS, (int64_t)c->nsm * 16);
+  kern<<<grid, 32 * SEG_WARPS, smem, c->stream>>>(to_dev(c->geom), p->slabs + p->slab0, p->nslab, ngrp, p->dst.row0, p->seg,
+                                                  p->sexp, V, ldv, m, W, ldw, W1, ld1);
+  ADC_COUNT_LAUNCH();
+  ADC_CUDA(c, cudaGetLastError());
+  return ADCGPU_OK;
+}
+
+template <int S, typename T, typename TA>
+int oz_seg(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t ldw, TA* W1, int64_t ld1) {
+  if (p->nslab == 0) return ADCGPU_OK;
+  if (c->geom.no <= 16) {
+    ST((oz_seg_go<S, 1, false>(c, p, V, ldv, m, W, ldw, W1, ld1)));
+    return oz_seg_go<S, 1, true>(c, p, V, ldv, m, W, ldw, W1, ld1);
+  }
+  ST((oz_seg_go<S, 2, false>(c, p, V, ldv, m, W, ldw, W1, ld1)));
+  return oz_seg_go<S, 2, true>(c, p, V, ldv, m, W, ldw, W1, ld1);
+}
+
 }  // namespace
 
-// The C|D products of m columns over the prepared rows: W2 rows are stored
-// with the diagonal term, W1 sums are added.
+// The coupling products of m columns over the prepared rows, segment A of
+// the classes with a' = b' excepted: W2 rows are stored with the diagonal
+// term, W1 sums are added.
 int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t ldv, int m, double* W, int64_t ldw,
               double* W1, int64_t ld1) {
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
@@ -867,20 +1253,23 @@ int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t
   // values); the column groups of an item run side by side, so the digits
   // come from L2 for all but one of them
   if (m > 8 && oz_shape<7, 16>(c->geom, smax, &sh, &smem))
-    return oz_go<7, 16, 3>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1);
-  if (!oz_shape<7, 8>(c->geom, smax, &sh, &smem)) return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
-  return oz_go<7, 8, 4>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1);
+    ST((oz_go<7, 16, 3>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1)));
+  else if (oz_shape<7, 8>(c->geom, smax, &sh, &smem))
+    ST((oz_go<7, 8, 4>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1)));
+  else
+    return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
+  return oz_seg<7>(c, p, V, ldv, m, W, ldw, W1, ld1);
 }
 
 // Reads the kernel's error word (waits for the stream) and clears it.
 int oz_check(Ctx* c, void* handle) {
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
-  if (!p || !p->d_err) return ADCGPU_OK;
-  ADC_CUDA(c, cudaMemcpyAsync(p->h_err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if (!p || !p->err) return ADCGPU_OK;
+  ADC_CUDA(c, cudaMemcpyAsync(c->h_word, p->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (*p->h_err) {
-    const int code = *p->h_err;
-    ADC_CUDA(c, cudaMemsetAsync(p->d_err, 0, sizeof(int), c->stream));
+  if (*c->h_word) {
+    const int code = *c->h_word;
+    ADC_CUDA(c, cudaMemsetAsync(p->err, 0, sizeof(int), c->stream));
     return set_err(c, ADCGPU_DEVICE_TIMEOUT,
                    "sliced sigma pass: a pipeline wait timed out (stage " + std::to_string(code) + ")");
   }

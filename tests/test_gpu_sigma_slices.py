@@ -59,8 +59,9 @@ def _sigma(g, x, flag=0):
 
 
 @pytest.mark.parametrize("no,nv,m,pad", [
-    (2, 2, 1, 0), (3, 8, 8, 3), (3, 16, 9, 0), (4, 17, 16, 0), (2, 32, 17, 1), (5, 33, 3, 0), (3, 64, 33, 0),
-    (3, 65, 5, 0), (2, 96, 16, 0), (9, 40, 2, 0), (7, 53, 31, 0)])
+    (2, 2, 1, 0), (1, 20, 3, 0), (3, 8, 8, 3), (3, 16, 9, 0), (4, 17, 16, 0), (2, 32, 17, 1), (5, 33, 3, 0), (3, 64, 33, 0),
+    (3, 65, 5, 0), (2, 96, 16, 0), (9, 40, 2, 0), (7, 53, 31, 0), (16, 20, 18, 2), (17, 18, 5, 0),
+    (32, 7, 16, 0)])
 def test_sliced_product_matches_oracle(gpu, no, nv, m, pad):
     g, e, eri = _build(no, nv, 11 * no + nv)
     x = _vectors(g.ndim, m, g.ndim + pad, nv)
