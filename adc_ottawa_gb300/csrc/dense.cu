@@ -20,9 +20,6 @@ namespace adcgpu {
 
 namespace {
 
-constexpr int TN_ROWS = 32;     // rows staged per step
-constexpr int TN_P = 64, TN_Q = 32;   // output tile
-
 // Accumulator helpers: plain types add; df accumulates with two-sums.
 template <typename A> __device__ __forceinline__ A acc_zero() { return A(0); }
 template <> __device__ __forceinline__ df acc_zero<df>() { return df{0.f, 0.f}; }
@@ -38,141 +35,188 @@ template <> __device__ __forceinline__ float to_t<float, double>(double x) { ret
 __device__ __forceinline__ void sq_add(double& a, double v) { a += v * v; }
 __device__ __forceinline__ void sq_add(df& a, float v) { df_fma(a, df{v, 0.f}, df{v, 0.f}); }
 
-// Partial C tiles: part[(blk * ntile + tile) * TN_P * TN_Q + ...]
-// Block: a range of rows; output tile TN_P x TN_Q (64 x 32); thread -> 8
-// outputs (p = ti + 16 u, q = tj + 16 v), conflict-free shared-memory reads.
-// Products over one 32-row step are summed in T and added to TA accumulators
-// (FP64 for FP32 inputs: one FP64 add per 32 FP32 FMAs keeps the Rayleigh and
-// Gram matrices accurate to ~1e-7 over millions of rows).
-template <typename T, typename TA>
-__global__ void __launch_bounds__(256) k_gemm_tn_part(int64_t N, int p, int q, const T* __restrict__ A,
-                                                      int64_t lda, const T* __restrict__ B, int64_t ldb,
-                                                      TA* __restrict__ part, int64_t rows_per_blk) {
-  __shared__ T sA[TN_ROWS][TN_P + 1];
-  __shared__ T sB[TN_ROWS][TN_Q + 1];
-  const int ntq = (q + TN_Q - 1) / TN_Q;
-  const int tile = blockIdx.y;
-  const int tp = tile / ntq, tq = tile % ntq;
-  const int p0 = tp * TN_P, q0 = tq * TN_Q;
-  const int tid = threadIdx.x;
-  const int ti = tid & 15, tj = tid >> 4;
-  // FP32 inputs: the step sums go into double-float accumulators (FP32-pipe
-  // two-sums) instead of FP64 adds; FP64 inputs accumulate in FP64
-  typedef typename std::conditional<std::is_same<T, float>::value && std::is_same<TA, double>::value, df, TA>::type
-      TAcc;
-  TAcc acc[4][2];
+// Arithmetic of the FP64 products: FP64 multiply-adds, or double-float on the
+// FP32 pipe (df.h; the mixed ladder's refinement and adcgpu_set_fp64_arith).
+struct MulF64 {
+  typedef double S;
+  static constexpr int ROWS = 64;      // rows staged per step
+  __device__ __forceinline__ static S from(double x) { return x; }
+  __device__ __forceinline__ static void fma(S& s, S a, S b) { s = ::fma(a, b, s); }
+  __device__ __forceinline__ static void add(S& s, S a) { s += a; }
+  __device__ __forceinline__ static double value(S s) { return s; }
+};
+struct MulDf {
+  typedef df S;
+  static constexpr int ROWS = 32;
+  __device__ __forceinline__ static S from(double x) { return df_split(x); }
+  __device__ __forceinline__ static void fma(S& s, S a, S b) { df_fma(s, a, b); }
+  __device__ __forceinline__ static void add(S& s, S a) { s = df_add(s, a); }
+  __device__ __forceinline__ static double value(S s) { return df_value(s); }
+};
+template <typename AR> __device__ __forceinline__ typename AR::S mul_zero();
+template <> __device__ __forceinline__ double mul_zero<MulF64>() { return 0.0; }
+template <> __device__ __forceinline__ df mul_zero<MulDf>() { return df{0.f, 0.f}; }
+// two consecutive rows of a staged column
+__device__ __forceinline__ void ld_rows2(const double* p, double (&v)[2]) {
+  const double2 t = *reinterpret_cast<const double2*>(p);
+  v[0] = t.x; v[1] = t.y;
+}
+__device__ __forceinline__ void ld_rows2(const df* p, df (&v)[2]) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = df{t.x, t.y}; v[1] = df{t.z, t.w};
+}
+
+// Partial Gram tiles of FP64 inputs, C(p x q) = A(N x p)^T B(N x q).  Bound by
+// the multiply pipe (FP64: 2 multiply-adds per cycle and SM), so no lane may
+// work on padding: a block takes up to 32 columns of each side (p and q are
+// split evenly) and a range of rows; a thread owns 2 x 2 outputs, and where
+// the output has fewer than 256 such tiles the threads left form groups that
+// share the rows of a step.  (A fixed 64 x 32 tile took 2.1 ms for the 10 x 10
+// products of block Lanczos at nocc=10/nvirt=110; this takes 0.15 ms.)
+// part: [block][tile y][pb * qb], summed by k_tn64_reduce.
+constexpr int T64_C = 32;
+template <typename AR>
+__global__ void __launch_bounds__(256) k_tn64(int64_t N, int p, int q, int pb, int qb, const double* __restrict__ A,
+                                              int64_t lda, const double* __restrict__ B, int64_t ldb,
+                                              double* __restrict__ part, int64_t rows_per_blk) {
+  typedef typename AR::S S;
+  constexpr int RT = AR::ROWS, LD = RT + 2;
+  __shared__ __align__(16) S sA[T64_C * LD], sB[T64_C * LD];
+  __shared__ double red[256][4];
+  const int ntq = (q + qb - 1) / qb;
+  const int p0 = (blockIdx.y / ntq) * pb, q0 = (blockIdx.y % ntq) * qb;
+  const int pn = min(pb, p - p0), qn = min(qb, q - q0);
+  const int tp = (pn + 1) / 2, tq = (qn + 1) / 2, nt = tp * tq;
+  const int ngrp = min(256 / nt, RT / 2);
+  const int tid = threadIdx.x, tile = tid % nt, grp = tid / nt;
+  const bool act = grp < ngrp;
+  const S* a0 = sA + 2 * (tile / tq) * LD;
+  const S* b0 = sB + 2 * (tile % tq) * LD;
+  S acc[2][2];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) { acc[u][0] = acc_zero<TAcc>(); acc[u][1] = acc_zero<TAcc>(); }
-  const int64_t r_begin = blockIdx.x * rows_per_blk;
-  const int64_t r_end = min(N, r_begin + rows_per_blk);
-  for (int64_t r0 = r_begin; r0 < r_end; r0 += TN_ROWS) {
+  for (int u = 0; u < 2; ++u) acc[u][0] = acc[u][1] = mul_zero<AR>();
+  const int64_t r_begin = blockIdx.x * rows_per_blk, r_end = min(N, r_begin + rows_per_blk);
+  for (int64_t r0 = r_begin; r0 < r_end; r0 += RT) {
     __syncthreads();
-    for (int l = tid; l < TN_ROWS * TN_P; l += 256) {
-      int c = l / TN_ROWS, rr = l % TN_ROWS;
-      int64_t r = r0 + rr;
-      sA[rr][c] = (r < r_end && p0 + c < p) ? A[(int64_t)(p0 + c) * lda + r] : T(0);
-    }
-    for (int l = tid; l < TN_ROWS * TN_Q; l += 256) {
-      int c = l / TN_ROWS, rr = l % TN_ROWS;
-      int64_t r = r0 + rr;
-      sB[rr][c] = (r < r_end && q0 + c < q) ? B[(int64_t)(q0 + c) * ldb + r] : T(0);
+    // columns 0 .. 2 tp - 1 of A, then 0 .. 2 tq - 1 of B; rows fastest
+    for (int l = tid; l < 2 * (tp + tq) * RT; l += 256) {
+      const int c = l / RT, rr = l - c * RT;
+      const int64_t r = r0 + rr;
+      if (c < 2 * tp) sA[c * LD + rr] = AR::from(r < r_end && c < pn ? A[(int64_t)(p0 + c) * lda + r] : 0.0);
+      else sB[(c - 2 * tp) * LD + rr] =
+          AR::from(r < r_end && c - 2 * tp < qn ? B[(int64_t)(q0 + c - 2 * tp) * ldb + r] : 0.0);
     }
     __syncthreads();
-    T st[4][2];
+    if (act) {
+      S st[2][2];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) { st[u][0] = T(0); st[u][1] = T(0); }
-#pragma unroll 8
-    for (int rr = 0; rr < TN_ROWS; ++rr) {
-      T b0 = sB[rr][tj], b1 = sB[rr][tj + 16];
+      for (int u = 0; u < 2; ++u) st[u][0] = st[u][1] = mul_zero<AR>();
+      for (int r2 = grp; r2 < RT / 2; r2 += ngrp) {
+        S a[2][2], b[2][2];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        T a = sA[rr][ti + 16 * u];
-        st[u][0] += a * b0;
-        st[u][1] += a * b1;
+        for (int u = 0; u < 2; ++u) {
+          ld_rows2(a0 + u * LD + 2 * r2, a[u]);
+          ld_rows2(b0 + u * LD + 2 * r2, b[u]);
+        }
+#pragma unroll
+        for (int v = 0; v < 2; ++v)
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) AR::fma(st[i][j], a[i][v], b[j][v]);
       }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) AR::add(acc[i][j], st[i][j]);
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) { acc_add(acc[u][0], st[u][0]); acc_add(acc[u][1], st[u][1]); }
   }
-  TA* out = part + ((int64_t)blockIdx.x * gridDim.y + tile) * (TN_P * TN_Q);
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    out[(ti + 16 * u) * TN_Q + tj] = acc_value<TA>(acc[u][0]);
-    out[(ti + 16 * u) * TN_Q + tj + 16] = acc_value<TA>(acc[u][1]);
+  for (int i = 0; i < 4; ++i) red[tid][i] = AR::value(acc[i >> 1][i & 1]);
+  __syncthreads();
+  double* out = part + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * pb * qb;
+  for (int o = tid; o < pn * qn; o += 256) {
+    const int i = o / qn, j = o - i * qn;
+    double s = 0.0;
+    for (int g = 0; g < ngrp; ++g) s += red[g * nt + (i / 2) * tq + j / 2][2 * (i & 1) + (j & 1)];
+    out[i * qb + j] = s;
   }
 }
 
-// Threads walk the partial tiles in their stored order (jj fastest), so the
-// nblk reads of consecutive threads are contiguous.
-template <typename TA, typename TC>
-__global__ void k_gemm_tn_reduce(int p, int q, int nblk, int ntile, const TA* __restrict__ part,
-                                 TC* __restrict__ C, int ldc, TC alpha, TC beta) {
-  const int ntq = (q + TN_Q - 1) / TN_Q;
-  const int per_tile = TN_P * TN_Q;
-  for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < ntile * per_tile; o += gridDim.x * blockDim.x) {
-    const int tile = o / per_tile, w = o - tile * per_tile;
-    const int ii = w / TN_Q, jj = w - ii * TN_Q;
-    const int i = (tile / ntq) * TN_P + ii, j = (tile % ntq) * TN_Q + jj;
-    if (i >= p || j >= q) continue;
-    TA s = TA(0);
-    for (int b = 0; b < nblk; ++b) s += part[((int64_t)b * ntile + tile) * per_tile + w];
-    TC prev = beta == TC(0) ? TC(0) : beta * C[(int64_t)j * ldc + i];
-    C[(int64_t)j * ldc + i] = prev + alpha * (TC)s;
+// C = alpha * (partials summed in a fixed order) + beta C; one warp per output
+__global__ void __launch_bounds__(256) k_tn64_reduce(int p, int q, int pb, int qb, int nblk, int ny,
+                                                     const double* __restrict__ part, double* __restrict__ C, int ldc,
+                                                     double alpha, double beta) {
+  const int lane = threadIdx.x & 31;
+  const int ntq = (q + qb - 1) / qb;
+  for (int o = (blockIdx.x * 256 + threadIdx.x) >> 5; o < p * q; o += gridDim.x * 8) {
+    const int i = o / q, j = o - i * q;
+    const double* src = part + (int64_t)((i / pb) * ntq + j / qb) * pb * qb + (i % pb) * qb + j % qb;
+    double s = 0.0;
+    for (int b = lane; b < nblk; b += 32) s += src[(int64_t)b * ny * pb * qb];
+#pragma unroll
+    for (int t = 16; t; t >>= 1) s += __shfl_xor_sync(0xffffffffu, s, t);
+    if (lane == 0) {
+      const double prev = beta == 0.0 ? 0.0 : beta * C[(int64_t)j * ldc + i];
+      C[(int64_t)j * ldc + i] = prev + alpha * s;
+    }
   }
 }
 
-
-// k_gemm_tn_part for FP64 inputs: DF step sums added to DF accumulators.
-__global__ void __launch_bounds__(256) k_gemm_tn_part_df(int64_t N, int p, int q, const double* __restrict__ A,
-                                                         int64_t lda, const double* __restrict__ B, int64_t ldb,
-                                                         double* __restrict__ part, int64_t rows_per_blk) {
-  __shared__ df sA[TN_ROWS][TN_P + 1];
-  __shared__ df sB[TN_ROWS][TN_Q + 1];
-  const int ntq = (q + TN_Q - 1) / TN_Q;
-  const int tile = blockIdx.y;
-  const int tp = tile / ntq, tq = tile % ntq;
-  const int p0 = tp * TN_P, q0 = tq * TN_Q;
-  const int tid = threadIdx.x;
-  const int ti = tid & 15, tj = tid >> 4;
-  df acc[4][2];
+// C(N x q) = beta C + alpha A(N x p) B(p x q) for FP64 operands: a thread owns
+// one row and QT columns (q split evenly over blockIdx.y), B's columns in
+// shared memory (broadcast reads), eight values of A in flight.  Bound by the
+// multiply pipe like k_tn64; the 128 x 64 tile before it worked on padding for
+// q < 64 (10 x 10 at N = 606,650: 1.1 ms, now 0.15 ms).
+constexpr int NN64_K = 512;
+template <typename AR, int QT>
+__global__ void __launch_bounds__(256) k_nn64(int64_t N, int p, int q, int qb, double alpha,
+                                              const double* __restrict__ A, int64_t lda,
+                                              const double* __restrict__ B, int ldb, double beta,
+                                              double* __restrict__ C, int64_t ldc) {
+  typedef typename AR::S S;
+  extern __shared__ __align__(16) unsigned char nn_smem[];
+  S* sB = reinterpret_cast<S*>(nn_smem);                   // [k][QT]
+  const int q0 = blockIdx.y * qb, qn = min(qb, q - q0);
+  const int64_t row = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const bool ok = row < N;
+  const double* Ar = A + (ok ? row : 0);
+  S acc[QT];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) { acc[u][0] = df{0.f, 0.f}; acc[u][1] = df{0.f, 0.f}; }
-  const int64_t r_begin = blockIdx.x * rows_per_blk;
-  const int64_t r_end = min(N, r_begin + rows_per_blk);
-  for (int64_t r0 = r_begin; r0 < r_end; r0 += TN_ROWS) {
+  for (int j = 0; j < QT; ++j) acc[j] = mul_zero<AR>();
+  for (int kc = 0; kc < p; kc += NN64_K) {
+    const int kn = min(NN64_K, p - kc);
     __syncthreads();
-    for (int l = tid; l < TN_ROWS * TN_P; l += 256) {
-      int c = l / TN_ROWS, rr = l % TN_ROWS;
-      int64_t r = r0 + rr;
-      sA[rr][c] = df_split((r < r_end && p0 + c < p) ? A[(int64_t)(p0 + c) * lda + r] : 0.0);
-    }
-    for (int l = tid; l < TN_ROWS * TN_Q; l += 256) {
-      int c = l / TN_ROWS, rr = l % TN_ROWS;
-      int64_t r = r0 + rr;
-      sB[rr][c] = df_split((r < r_end && q0 + c < q) ? B[(int64_t)(q0 + c) * ldb + r] : 0.0);
+    for (int l = threadIdx.x; l < kn * QT; l += 256) {
+      const int k = l / QT, j = l - k * QT;
+      sB[l] = AR::from(j < qn ? B[(int64_t)(q0 + j) * ldb + kc + k] : 0.0);
     }
     __syncthreads();
-    df st[4][2];
+    int k = 0;
+    for (; k + 8 <= kn; k += 8) {
+      double a[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) { st[u][0] = df{0.f, 0.f}; st[u][1] = df{0.f, 0.f}; }
-#pragma unroll 4
-    for (int rr = 0; rr < TN_ROWS; ++rr) {
-      const df b0 = sB[rr][tj], b1 = sB[rr][tj + 16];
+      for (int u = 0; u < 8; ++u) a[u] = Ar[(int64_t)(kc + k + u) * lda];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const df a = sA[rr][ti + 16 * u];
-        df_fma(st[u][0], a, b0);
-        df_fma(st[u][1], a, b1);
+      for (int u = 0; u < 8; ++u) {
+        const S x = AR::from(a[u]);
+#pragma unroll
+        for (int j = 0; j < QT; ++j) AR::fma(acc[j], x, sB[(k + u) * QT + j]);
       }
     }
+    for (; k < kn; ++k) {
+      const S x = AR::from(Ar[(int64_t)(kc + k) * lda]);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) { acc[u][0] = df_add(acc[u][0], st[u][0]); acc[u][1] = df_add(acc[u][1], st[u][1]); }
+      for (int j = 0; j < QT; ++j) AR::fma(acc[j], x, sB[k * QT + j]);
+    }
   }
-  double* out = part + ((int64_t)blockIdx.x * gridDim.y + tile) * (TN_P * TN_Q);
+  if (!ok) return;
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    out[(ti + 16 * u) * TN_Q + tj] = df_value(acc[u][0]);
-    out[(ti + 16 * u) * TN_Q + tj + 16] = df_value(acc[u][1]);
+  for (int j = 0; j < QT; ++j) {
+    if (j >= qn) break;
+    double* cp = C + (int64_t)(q0 + j) * ldc + row;
+    const double prev = beta == 0.0 ? 0.0 : beta * *cp;
+    *cp = prev + alpha * AR::value(acc[j]);
   }
 }
 
@@ -229,62 +273,6 @@ __global__ void __launch_bounds__(256) k_gemm_nn(int64_t N, int p, int q, T alph
       if (r < N) {
         T prev = beta == T(0) ? T(0) : beta * C[(int64_t)col * ldc + r];
         C[(int64_t)col * ldc + r] = prev + alpha * acc[i][j];
-      }
-    }
-  }
-}
-
-// k_gemm_nn for FP64 operands with DF products and DF sums over all of K.
-__global__ void __launch_bounds__(256) k_gemm_nn_df(int64_t N, int p, int q, double alpha,
-                                                    const double* __restrict__ A, int64_t lda,
-                                                    const double* __restrict__ B, int ldb, double beta,
-                                                    double* __restrict__ C, int64_t ldc) {
-  __shared__ df sA[NN_K][NN_M];
-  __shared__ df sB[NN_K][NN_N];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int64_t m0 = (int64_t)blockIdx.x * NN_M;
-  const int n0 = blockIdx.y * NN_N;
-  df acc[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = df{0.f, 0.f};
-  for (int k0 = 0; k0 < p; k0 += NN_K) {
-    __syncthreads();
-    for (int l = tid; l < NN_K * NN_M; l += 256) {
-      const int kk = l / NN_M, rr = l % NN_M;
-      const int64_t r = m0 + rr;
-      sA[kk][rr] = df_split((r < N && k0 + kk < p) ? A[(int64_t)(k0 + kk) * lda + r] : 0.0);
-    }
-    for (int l = tid; l < NN_K * NN_N; l += 256) {
-      const int kk = l / NN_N, cc = l % NN_N;
-      sB[kk][cc] = df_split((k0 + kk < p && n0 + cc < q) ? B[(int64_t)(n0 + cc) * ldb + k0 + kk] : 0.0);
-    }
-    __syncthreads();
-#pragma unroll 2
-    for (int kk = 0; kk < NN_K; ++kk) {
-      df a[8], b[4];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = sA[kk][8 * ty + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = sB[kk][4 * tx + j];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) df_fma(acc[i][j], a[i], b[j]);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int col = n0 + 4 * tx + j;
-    if (col >= q) continue;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int64_t r = m0 + 8 * ty + i;
-      if (r < N) {
-        double prev = beta == 0.0 ? 0.0 : beta * C[(int64_t)col * ldc + r];
-        C[(int64_t)col * ldc + r] = prev + alpha * df_value(acc[i][j]);
       }
     }
   }
@@ -535,11 +523,15 @@ __global__ void k_resid(int64_t N, int nb, const T* __restrict__ X, const T* __r
 }
 
 __global__ void k_sum_parts(int nblk, int n, int stride, const double* __restrict__ part, double* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // one warp per sum, in a fixed order (one thread each took 35 us for 304 parts)
+  const int lane = threadIdx.x & 31;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= n) return;
   double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += part[(int64_t)b * stride + i];
-  out[i] = s;
+  for (int b = lane; b < nblk; b += 32) s += part[(int64_t)b * stride + i];
+#pragma unroll
+  for (int t = 16; t; t >>= 1) s += __shfl_xor_sync(0xffffffffu, s, t);
+  if (lane == 0) out[i] = s;
 }
 
 template <typename TS, typename TD>
@@ -579,27 +571,31 @@ template <typename T, typename TA, typename TC>
 int gemm_tn(Ctx* c, Workspace& ws, int64_t N, int p, int q, const T* A, int64_t lda, const T* B, int64_t ldb,
             TC* C, int ldc, TC alpha, TC beta) {
   if (p <= 0 || q <= 0) return ADCGPU_OK;
-  const int ntile = ((p + TN_P - 1) / TN_P) * ((q + TN_Q - 1) / TN_Q);
-  const int nblk = tn_blocks(c, N);
-  const int64_t rows = ((N + nblk - 1) / nblk + TN_ROWS - 1) / TN_ROWS * TN_ROWS;
-  size_t need = sizeof(TA) * (size_t)nblk * ntile * TN_P * TN_Q;
-  int st = ws.reserve(c, need);
-  if (st) return st;
-  if constexpr (std::is_same<T, double>::value && std::is_same<TA, double>::value) {
-    if (c->dense_df) {
-      k_gemm_tn_part_df<<<dim3(nblk, ntile), 256, 0, c->stream>>>(N, p, q, A, lda, B, ldb, (TA*)ws.p, rows); ADC_COUNT_LAUNCH();
-    } else {
-      k_gemm_tn_part<T, TA><<<dim3(nblk, ntile), 256, 0, c->stream>>>(N, p, q, A, lda, B, ldb, (TA*)ws.p, rows); ADC_COUNT_LAUNCH();
-    }
-  } else if constexpr (std::is_same<T, float>::value && std::is_same<TA, double>::value) {
-    if constexpr (std::is_same<TC, double>::value) {
-      // the tensor cores (three BF16 slices per value), q <= 48
-      if (gram_umma_usable(c, N, p, q)) return gram_umma(c, ws, N, p, q, A, lda, B, ldb, C, ldc, alpha, beta);
-    }
+  if constexpr (std::is_same<T, double>::value) {
+    const int np = (p + T64_C - 1) / T64_C, nq = (q + T64_C - 1) / T64_C;
+    const int pb = (p + np - 1) / np, qb = (q + nq - 1) / nq, ny = np * nq;
+    // about six blocks per SM (their loads overlap the others' arithmetic),
+    // at least 256 rows each
+    const int64_t want = std::max<int64_t>(1, (int64_t)c->nsm * 6 / ny);
+    const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(want, (N + 255) / 256));
+    const int64_t rows = ((N + nblk - 1) / nblk + 63) / 64 * 64;
+    int st = ws.reserve(c, sizeof(double) * (size_t)nblk * ny * pb * qb);
+    if (st) return st;
+    double* part = (double*)ws.p;
+    if (c->dense_df) k_tn64<MulDf><<<dim3(nblk, ny), 256, 0, c->stream>>>(N, p, q, pb, qb, A, lda, B, ldb, part, rows);
+    else k_tn64<MulF64><<<dim3(nblk, ny), 256, 0, c->stream>>>(N, p, q, pb, qb, A, lda, B, ldb, part, rows);
+    ADC_COUNT_LAUNCH();
+    k_tn64_reduce<<<std::min((p * q + 7) / 8, c->nsm * 8), 256, 0, c->stream>>>(p, q, pb, qb, nblk, ny, part, C, ldc,
+                                                                                alpha, beta);
+    ADC_COUNT_LAUNCH();
+  } else {
+    // the tensor cores (three BF16 slices per value), q <= 48
+    if (gram_umma_usable(c, N, p, q)) return gram_umma(c, ws, N, p, q, A, lda, B, ldb, C, ldc, alpha, beta);
     // FP32 inputs: 64 x 64 tiles with 4 x 4 float4 sub-tiles per thread
+    const int nblk = tn_blocks(c, N);
+    const int64_t rows = ((N + nblk - 1) / nblk + TF_ROWS - 1) / TF_ROWS * TF_ROWS;
     const int ntile2 = ((p + TF_T - 1) / TF_T) * ((q + TF_T - 1) / TF_T);
-    const size_t need2 = sizeof(double) * (size_t)nblk * ntile2 * TF_T * TF_T;
-    st = ws.reserve(c, need2);
+    int st = ws.reserve(c, sizeof(double) * (size_t)nblk * ntile2 * TF_T * TF_T);
     if (st) return st;
     k_gemm_tn_f32<<<dim3(nblk, ntile2), 256, 0, c->stream>>>(N, p, q, A, lda, B, ldb, (double*)ws.p, rows);
     ADC_COUNT_LAUNCH();
@@ -607,15 +603,7 @@ int gemm_tn(Ctx* c, Workspace& ws, int64_t N, int p, int q, const T* A, int64_t 
     k_gemm_tn_f32_reduce<TC><<<std::min((nout2 + 255) / 256, c->nsm * 8), 256, 0, c->stream>>>(
         p, q, nblk, ntile2, (const double*)ws.p, C, ldc, alpha, beta);
     ADC_COUNT_LAUNCH();
-    ADC_CUDA(c, cudaGetLastError());
-    return ADCGPU_OK;
-  } else {
-    k_gemm_tn_part<T, TA><<<dim3(nblk, ntile), 256, 0, c->stream>>>(N, p, q, A, lda, B, ldb, (TA*)ws.p, rows); ADC_COUNT_LAUNCH();
   }
-  const int nout = ntile * TN_P * TN_Q;
-  k_gemm_tn_reduce<TA, TC><<<std::min((nout + 255) / 256, c->nsm * 8), 256, 0, c->stream>>>(p, q, nblk, ntile,
-                                                                                         (TA*)ws.p, C, ldc, alpha,
-                                                                                         beta); ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
 }
@@ -631,15 +619,29 @@ int gemm_nn(Ctx* c, int64_t N, int p, int q, T alpha, const T* A, int64_t lda, c
     }
     return ADCGPU_OK;
   }
-  dim3 grid((unsigned)((N + NN_M - 1) / NN_M), (unsigned)((q + NN_N - 1) / NN_N));
-  if constexpr (std::is_same<T, double>::value && std::is_same<TB, double>::value) {
-    if (c->dense_df) {
-      k_gemm_nn_df<<<grid, 256, 0, c->stream>>>(N, p, q, alpha, A, lda, B, ldb, beta, C, ldc); ADC_COUNT_LAUNCH();
-      ADC_CUDA(c, cudaGetLastError());
-      return ADCGPU_OK;
+  if constexpr (std::is_same<T, double>::value) {
+    const int nq = (q + 7) / 8, qb = (q + nq - 1) / nq;
+    const dim3 g2((unsigned)((N + 255) / 256), (unsigned)nq);
+    const size_t smem = sizeof(double) * (size_t)std::min(p, NN64_K) * qb;
+    auto go = [&](auto qt) {
+      constexpr int QT = decltype(qt)::value;
+      if (c->dense_df) k_nn64<MulDf, QT><<<g2, 256, smem, c->stream>>>(N, p, q, qb, alpha, A, lda, B, ldb, beta, C, ldc);
+      else k_nn64<MulF64, QT><<<g2, 256, smem, c->stream>>>(N, p, q, qb, alpha, A, lda, B, ldb, beta, C, ldc);
+    };
+    switch (qb) {
+      case 1: go(std::integral_constant<int, 1>()); break;
+      case 2: go(std::integral_constant<int, 2>()); break;
+      case 3: go(std::integral_constant<int, 3>()); break;
+      case 4: go(std::integral_constant<int, 4>()); break;
+      case 5: go(std::integral_constant<int, 5>()); break;
+      case 6: go(std::integral_constant<int, 6>()); break;
+      case 7: go(std::integral_constant<int, 7>()); break;
+      default: go(std::integral_constant<int, 8>()); break;
     }
-  }
-  if constexpr (std::is_same<T, float>::value) {
+    ADC_COUNT_LAUNCH();
+    ADC_CUDA(c, cudaGetLastError());
+    return ADCGPU_OK;
+  } else {
     // FP32: B's column tile in shared memory, 2 rows x QT columns per thread
     const int QT = q <= 16 ? 16 : (q <= 32 ? 32 : (q <= 40 ? 40 : 48));
     const size_t smem = sizeof(float) * (size_t)p * QT;
@@ -674,10 +676,12 @@ int gemm_nn(Ctx* c, int64_t N, int p, int q, T alpha, const T* A, int64_t lda, c
       ADC_CUDA(c, cudaGetLastError());
       return ADCGPU_OK;
     }
-  }
+  // a B too large for shared memory
+  const dim3 grid((unsigned)((N + NN_M - 1) / NN_M), (unsigned)((q + NN_N - 1) / NN_N));
   k_gemm_nn<T, TB><<<grid, 256, 0, c->stream>>>(N, p, q, alpha, A, lda, B, ldb, beta, C, ldc); ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
+  }
 }
 
 template <typename T, typename TD>
@@ -697,7 +701,7 @@ int precond_olsen(Ctx* c, Workspace& ws, int64_t N, int nb, const T* X, const T*
   double* part = (double*)ws.p;
   double* sums = part + (size_t)nblk * nb * 2;
   k_olsen_dots<T, TD><<<nblk, 256, 0, c->stream>>>(N, nb, X, R, ld, d_lam, hii, part); ADC_COUNT_LAUNCH();
-  k_sum_parts<<<(2 * nb + 127) / 128, 128, 0, c->stream>>>(nblk, 2 * nb, 2 * nb, part, sums); ADC_COUNT_LAUNCH();
+  k_sum_parts<<<(2 * nb + 3) / 4, 128, 0, c->stream>>>(nblk, 2 * nb, 2 * nb, part, sums); ADC_COUNT_LAUNCH();
   std::vector<double> h(2 * nb), alpha(nb);
   ADC_CUDA(c, cudaMemcpyAsync(h.data(), sums, sizeof(double) * 2 * nb, cudaMemcpyDeviceToHost, c->stream));
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -720,7 +724,7 @@ int residuals(Ctx* c, Workspace& ws, int64_t N, int nb, const T* X, const T* WY,
   double* part = (double*)ws.p;
   double* sums = part + (size_t)nblk * nb;
   k_resid<T><<<nblk, 256, 0, c->stream>>>(N, nb, X, WY, ld, d_lam, Rout, part); ADC_COUNT_LAUNCH();
-  k_sum_parts<<<(nb + 127) / 128, 128, 0, c->stream>>>(nblk, nb, nb, part, sums); ADC_COUNT_LAUNCH();
+  k_sum_parts<<<(nb + 3) / 4, 128, 0, c->stream>>>(nblk, nb, nb, part, sums); ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   ADC_CUDA(c, cudaMemcpyAsync(h_norm2, sums, sizeof(double) * nb, cudaMemcpyDeviceToHost, c->stream));
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -737,8 +741,6 @@ int convert(Ctx* c, const TS* x, TD* y, int64_t n) {
 // explicit instantiations
 template int gemm_tn<double, double, double>(Ctx*, Workspace&, int64_t, int, int, const double*, int64_t,
                                              const double*, int64_t, double*, int, double, double);
-template int gemm_tn<float, float, double>(Ctx*, Workspace&, int64_t, int, int, const float*, int64_t, const float*,
-                                           int64_t, double*, int, double, double);
 template int gemm_tn<float, double, double>(Ctx*, Workspace&, int64_t, int, int, const float*, int64_t, const float*,
                                             int64_t, double*, int, double, double);
 template int gemm_nn<double, double>(Ctx*, int64_t, int, int, double, const double*, int64_t, const double*, int,
