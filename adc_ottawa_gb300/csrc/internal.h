@@ -422,7 +422,7 @@ struct SigmaPlan {
   void* ab = nullptr;         // compact segment-A/B tables (sigma_ab.cu), built on first use
   int ab_off = 0;             // 1: segments A/B through pass 2 / pass 3 instead
   int umma3_on = 0;           // 1: FP32 values on the two tcgen05 passes (BF16 slices)
-  void* oz = nullptr;         // digit store of the FP64-accurate tensor-core pass (sigma_slices.cu)
+  void* oz[2] = {nullptr, nullptr};   // digit stores of the sliced tensor-core pass: FP64, FP32 values
   std::vector<DirectChunk> dchunks;   // direct path: chunks with their work-list ranges
 };
 int prepare_desc(Ctx* c);
@@ -449,7 +449,7 @@ bool umma3_supported(const Ctx* c);
 int umma3_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float* W, int64_t ldw, double* W1,
                  int64_t ld1);
 
-// sigma_slices.cu : FP64-accurate tensor-core pass (exact digit slices)
+// sigma_slices.cu : tensor-core pass by exact digit slices (FP64 and FP32 values)
 bool oz_geometry_ok(const Geometry& G);
 std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, int64_t row1, int64_t* reserve);
 int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int64_t reserve, int m,
@@ -457,6 +457,8 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
 void oz_invalidate(void* handle);
 void oz_free(Ctx* c, void*& handle);
 int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t ldv, int m, double* W, int64_t ldw,
+              double* W1, int64_t ld1);
+int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t ldv, int m, float* W, int64_t ldw,
               double* W1, int64_t ld1);
 int oz_check(Ctx* c, void* handle);
 

@@ -1456,25 +1456,28 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
   bool umma_used = false, oz_used = false;
   auto coupling = [&](const SigmaPlan* P, const TV* BtP, bool allow_umma, int64_t row0, int64_t row1) -> int {
     int c0 = 0;
-    if constexpr (std::is_same<TV, double>::value) {
-      if (P->tiled == 1 && !P->umma_off) {
+    if constexpr (!std::is_same<TV, __nv_bfloat16>::value) {
+      // FP64 and FP32 values on the tensor cores by exact digit slices
+      if (P->tiled == 1 && !P->umma_off && !(sizeof(T) == 4 && (P->umma3_on || P->ab_off))) {
+        void*& oz = plan->oz[sizeof(T) == 8 ? 0 : 1];
         // the digits of a range are made and used before those of the next
         int64_t reserve = 0;
         bool usable = true;
+        TAcc* W1 = sizeof(T) == 8 ? reinterpret_cast<TAcc*>(dW) : W1base;
+        const int64_t ld1 = sizeof(T) == 8 ? ldw : (int64_t)n1;
         for (const auto& rg : oz_ranges(c, row0, row1, &reserve)) {
-          ST(oz_prepare(c, plan->oz, BtP, true, rg.first, rg.second, reserve, m, &usable));
+          ST(oz_prepare(c, oz, BtP, sizeof(T) == 8, rg.first, rg.second, reserve, m, &usable));
           if (!usable) break;
-          ST(oz_launch(c, plan->oz, diag, dV, ldv, m, dW, ldw, dW, ldw));
+          ST(oz_launch(c, oz, diag, dV, ldv, m, dW, ldw, W1, ld1));
           oz_used = true;
         }
         if (usable) {
-          T* W1 = dW;
           // segment A of the classes with a' = b'
           for (int cls = 0; cls <= 2; cls += 2) {
             const int64_t a = std::max(row0, G.start[cls]), b = std::min(row1, G.start[cls + 1]);
             if (a >= b) continue;
-            k_sigma_rows_a<T, TV, T><<<dim3((int)std::min<int64_t>((b - a + 7) / 8, c->nsm * 8), (m + 3) / 4), 256, 0, s>>>(
-                g, a, b, BtP, dV, ldv, m, dW, ldw, W1, ldw);
+            k_sigma_rows_a<T, TV, TAcc><<<dim3((int)std::min<int64_t>((b - a + 7) / 8, c->nsm * 8), (m + 3) / 4), 256, 0, s>>>(
+                g, a, b, BtP, dV, ldv, m, dW, ldw, W1, ld1);
             ADC_COUNT_LAUNCH();
           }
           ADC_CUDA(c, cudaGetLastError());
@@ -1662,7 +1665,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
   }
   ADC_CUDA(c, cudaEventRecord(c->st_ev1, s));
   if (umma_used) ST(umma_check(c, plan->umma));
-  if (oz_used) ST(oz_check(c, plan->oz));
+  if (oz_used) ST(oz_check(c, plan->oz[sizeof(T) == 8 ? 0 : 1]));
   c->st_pending = true;
   c->st_pending_cols = m;
   c->st_pending_kind = std::is_same<TV, __nv_bfloat16>::value ? 0 : (std::is_same<TV, float>::value ? 1 : 2);
@@ -1764,7 +1767,8 @@ void free_sigma_plan(Ctx* c) {
   dfree(c, plan->d_acc);
   dfree(c, plan->d_sk);
   umma_free(c, plan->umma);
-  oz_free(c, plan->oz);
+  oz_free(c, plan->oz[0]);
+  oz_free(c, plan->oz[1]);
   ab_free(c, plan->ab);
   delete plan;
   c->sigma_plan = nullptr;
@@ -1794,7 +1798,10 @@ int prepare_mixed(Ctx* c) {
     ADC_CUDA(c, cudaGetLastError());
   }
   // the value stores were rewritten: the compact segment-A/B tables follow
-  if (SigmaPlan* plan = reinterpret_cast<SigmaPlan*>(c->sigma_plan)) ab_invalidate(plan->ab);
+  if (SigmaPlan* plan = reinterpret_cast<SigmaPlan*>(c->sigma_plan)) {
+    ab_invalidate(plan->ab);
+    oz_invalidate(plan->oz[1]);
+  }
   return ADCGPU_OK;
 }
 

@@ -302,12 +302,34 @@ __device__ __forceinline__ double oz_sum(const float (&d)[S]) {
     return x + __longlong_as_double(0x41B8000000000000ll + lo);
   }
 }
+// the same rounded to the vectors' type (FP32: without the FP64 pipe), and
+// powers of two of that type (those below its range are 0)
+template <int S, typename T> __device__ __forceinline__ T oz_round(const float (&d)[S]) {
+  if constexpr (std::is_same<T, double>::value) {
+    return oz_sum<S>(d);
+  } else {
+    static_assert(S == 4, "FP32 results come from four digits");
+    long long hi = (long long)__float2int_rn(d[3]);
+    hi = mad_wide(__float2int_rn(d[2]), 1 << 8, hi);
+    hi = mad_wide(__float2int_rn(d[1]), 1 << 16, hi);
+    hi = mad_wide(__float2int_rn(d[0]), 1 << 24, hi);
+    return __ll2float_rn(hi);
+  }
+}
+template <typename T> __device__ __forceinline__ T oz_scale(int e);
+template <> __device__ __forceinline__ double oz_scale<double>(int e) { return oz_pow2(e); }
+template <> __device__ __forceinline__ float oz_scale<float>(int e) {
+  if (e > (OZ_NONFINITE >> 1)) return __int_as_float(0x7fc00000);
+  if (e < -126) return 0.f;
+  if (e > 127) return __int_as_float(0x7f800000);
+  return __int_as_float((e + 127) << 23);
+}
 // weight exponent of oz_sum's unit against scaled operands |v| < 1
 template <int S> __host__ __device__ constexpr int oz_unit() { return -14 - 8 * (S - 1) + (S == 7 ? 24 : 0); }
 
 // the same of NH columns of a TMEM accumulator region
-template <int S, int NP, int NH>
-__device__ __forceinline__ void oz_combine(uint32_t taddr, double (&t)[NH]) {
+template <int S, int NP, int NH, typename TR>
+__device__ __forceinline__ void oz_combine(uint32_t taddr, TR (&t)[NH]) {
   float d[S][NH];
 #pragma unroll
   for (int gI = 0; gI < S; ++gI) oz_tmem_ld(taddr + (uint32_t)(gI * NP), d[gI]);
@@ -317,7 +339,7 @@ __device__ __forceinline__ void oz_combine(uint32_t taddr, double (&t)[NH]) {
     float x[S];
 #pragma unroll
     for (int gI = 0; gI < S; ++gI) x[gI] = d[gI][j];
-    t[j] = oz_sum<S>(x);
+    t[j] = oz_round<S, TR>(x);
   }
 }
 
@@ -597,7 +619,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           ++d2use[s];
           fence_after_sync();
           double t[NH];
-          oz_combine<S, NP, NH>(tD2 + (uint32_t)(s * DW) + lane_off + (uint32_t)cbeg, t);
+          oz_combine<S, NP, NH, double>(tD2 + (uint32_t)(s * DW) + lane_off + (uint32_t)cbeg, t);
           fence_before_sync();
           mbar_arrive(&bars[O_D2EMPTY + s]);
 #pragma unroll
@@ -612,8 +634,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         if (!ok) break;
         if (has_next && sh.nb == 1) store_v2(0);
         fence_after_sync();
-        double t2[NH];
-        oz_combine<S, NP, NH>(tbase + buf * DW + lane_off + (uint32_t)cbeg, t2);
+        T t2[NH];
+        oz_combine<S, NP, NH, T>(tbase + buf * DW + lane_off + (uint32_t)cbeg, t2);
         fence_before_sync();
         mbar_arrive(&bars[O_D1EMPTY0 + buf]);
         // the last group of the row (its sums end with the tile)
@@ -635,9 +657,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const int c = c0 + cbeg + j;
             if (c >= m) continue;
             const T x = V[(int64_t)c * ldv + n1 + d];
-            const double t = t2[j] * oz_pow2(sXe[cbeg + j] + re + TSH);
-            if constexpr (std::is_same<T, double>::value) W[(int64_t)c * ldw + n1 + d] = fma(dg, x, t);
-            else W[(int64_t)c * ldw + n1 + d] = fmaf(dg, x, (float)t);
+            const T t = t2[j] * oz_scale<T>(sXe[cbeg + j] + re + TSH);
+            W[(int64_t)c * ldw + n1 + d] = dg * x + t;
           }
         }
       }
@@ -920,7 +941,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
 #pragma unroll
             for (int i = 0; i < S; ++i) dsum[i] = a2[i][2 * h + v];
             T* w = W + (int64_t)cc[h] * ldw + d;
-            *w = (T)fma(oz_sum<S>(dsum), oz_pow2(ex[h] + e + TSH), (double)*w);
+            *w += oz_round<S, T>(dsum) * oz_scale<T>(ex[h] + e + TSH);
           }
         }
       }
@@ -1043,7 +1064,7 @@ std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, i
     return out;
   }
   const int64_t budget = direct_budget(G) * (int64_t)sizeof(double);
-  *reserve = budget;
+  *reserve = budget;   // (the direct path computes in FP64: seven digits)
   for (int cls = 0; cls < 5; ++cls) {
     OzDst d;
     if (G.start[cls] < G.start[cls + 1])
@@ -1259,6 +1280,18 @@ int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t
   else
     return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
   return oz_seg<7>(c, p, V, ldv, m, W, ldw, W1, ld1);
+}
+
+// FP32 values and vectors (four digits), FP64 W1 accumulators
+int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t ldv, int m, float* W, int64_t ldw,
+              double* W1, int64_t ld1) {
+  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
+  const int smax = smem_optin_max(c);
+  OzShape sh;
+  size_t smem = 0;
+  if (!oz_shape<4, 16>(c->geom, smax, &sh, &smem)) return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
+  ST((oz_go<4, 16, 4>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1)));
+  return oz_seg<4>(c, p, V, ldv, m, W, ldw, W1, ld1);
 }
 
 // Reads the kernel's error word (waits for the stream) and clears it.

@@ -93,3 +93,40 @@ def test_nonfinite_column_stays_in_its_column(gpu):
             assert np.abs(w[c] - clean[c]).max() <= TOL * np.abs(clean[c]).max()
         # wherever the multiply-add product is not finite, so is the sliced one
         assert not np.isfinite(w[2][~np.isfinite(ref[2])]).any()
+
+
+@pytest.mark.parametrize("no,nv,m,pad", [
+    (2, 2, 1, 0), (1, 20, 3, 0), (4, 17, 16, 1), (2, 32, 17, 0), (5, 33, 3, 2), (3, 64, 33, 0), (3, 65, 20, 0),
+    (16, 20, 18, 0), (17, 18, 5, 0), (2, 200, 7, 0)])
+def test_sliced_fp32_values_match_oracle(gpu, no, nv, m, pad):
+    """FP32 values and vectors (shape flag 256: the ladder's FP32 store).  The
+    result is rounded to FP32 and the values were: 2^-24 of |W| and of
+    sum |h| |x|, which stays below 8 max|W| for these vectors: 5e-7, 1e-6 with
+    the accumulation."""
+    import torch
+
+    from adc_ottawa_gb300 import ADCGPU_MIXED, AdcGpu
+    from adc_ottawa_gb300._native import lib
+
+    e, eri = system(no, nv, 7 * no + nv)
+    g = AdcGpu(0)
+    g.set_orbitals(no, nv, e)
+    g.set_eri_packed(eri)
+    g.write_fspace_adc2_1(None, precision=ADCGPU_MIXED)
+    x = _vectors(g.ndim, m, g.ndim + pad, nv).astype(np.float32)
+    v = torch.from_numpy(x).cuda()
+    w = {}
+    for flag in (0, 32):
+        assert lib().adcgpu_sigma_set_shape(g._h, 64, 2 | 8, 4 | 8 | 256 | flag) == 0
+        o = torch.full_like(v, 3.0)
+        torch.cuda.synchronize()
+        st = lib().adcgpu_sigma_device(g._h, m, C.c_void_p(v.data_ptr()), C.c_void_p(o.data_ptr()), x.shape[1])
+        assert st == 0, lib().adcgpu_last_error(g._h)
+        assert (o.cpu().numpy()[:, g.ndim:] == 3.0).all()
+        w[flag] = o.cpu().numpy()[:, :g.ndim].astype(np.float64)
+    if nv <= 100:
+        ref = oracle.Matrix.build(no, nv, e, eri).matvec(np.asfortranarray(x[:, :g.ndim].T.astype(np.float64))).T
+    else:
+        ref = w[32]     # the CUDA-core tile
+    for c in range(m):
+        assert np.abs(w[0][c] - ref[c]).max() <= 1e-6 * np.abs(ref[c]).max()
