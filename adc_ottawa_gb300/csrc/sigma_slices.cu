@@ -222,39 +222,51 @@ __global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const T
   }
 }
 
-// exponent of the largest 2^rexp |V2| of each work item and column: the
-// scale of the V2 digits.  One block per item and 4 columns; reads V2 once
-// (the pass then finds most of it in L2).
+// exponents of the largest 2^rexp |V2| and 2^sexp |V2| of each work item and
+// column: the scales of the V2 digits for the C|D segments (vexp) and for
+// segments A and B (sexp of the classes with a' < b'; the runs of a slab take
+// the maximum over its items).  One block per item and 4 columns; reads V2
+// once (the pass then finds most of it in L2).
 template <typename T>
 __global__ void __launch_bounds__(256) k_oz_vexp(GeomDev g, const int2* __restrict__ items, int64_t row0,
-                                                 const int16_t* __restrict__ rexp, const T* __restrict__ V, int64_t ldv,
-                                                 int m, int* __restrict__ vexp) {
-  __shared__ int s_mx[4];
+                                                 const int16_t* __restrict__ rexp, const int16_t* __restrict__ sexp,
+                                                 const T* __restrict__ V, int64_t ldv, int m, int* __restrict__ vexp,
+                                                 int* __restrict__ vsexp) {
+  __shared__ int s_mx[8];
   const int2 item = items[blockIdx.x];
   const int c0 = 4 * blockIdx.y;
-  if (threadIdx.x < 4) s_mx[threadIdx.x] = OZ_EMIN;
+  if (threadIdx.x < 8) s_mx[threadIdx.x] = OZ_EMIN;
   __syncthreads();
-  int mx[4] = {OZ_EMIN, OZ_EMIN, OZ_EMIN, OZ_EMIN};
+  int mx[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) mx[j] = OZ_EMIN;
   const bool perm = item.x >= g.start[1] && item.x < g.start[2];
+  const bool pairs = perm || item.x >= g.start[3];
   for (int row = item.x + threadIdx.x; row < item.y; row += 256) {
     int64_t d = row;
     if (perm) d = row_to_d(g, decode_row(g, row), row);
-    const int rx = rexp[row - row0];
+    const int rx = rexp[row - row0], sx = pairs ? (int)sexp[row - row0] : OZ_EMIN;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (c0 + j >= m) break;
       const int e = Parts<T>::exponent(__ldg(V + (int64_t)(c0 + j) * ldv + g.n1 + d));
-      if (e == OZ_NONFINITE || rx == 32767) mx[j] = OZ_NONFINITE;
-      else if (e != OZ_ZERO) mx[j] = max(mx[j], e + rx);
+      if (e == OZ_NONFINITE || rx == 32767 || sx == 32767) mx[j] = mx[4 + j] = OZ_NONFINITE;
+      else if (e != OZ_ZERO) {
+        mx[j] = max(mx[j], e + rx);
+        mx[4 + j] = max(mx[4 + j], e + sx);
+      }
     }
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 8; ++j) {
     mx[j] = __reduce_max_sync(0xffffffffu, mx[j]);
     if ((threadIdx.x & 31) == 0) atomicMax(&s_mx[j], mx[j]);
   }
   __syncthreads();
-  if (threadIdx.x < 4 && c0 + (int)threadIdx.x < m) vexp[(int64_t)blockIdx.x * m + c0 + threadIdx.x] = s_mx[threadIdx.x];
+  if (threadIdx.x < 4 && c0 + (int)threadIdx.x < m) {
+    vexp[(int64_t)blockIdx.x * m + c0 + threadIdx.x] = s_mx[threadIdx.x];
+    vsexp[(int64_t)blockIdx.x * m + c0 + threadIdx.x] = s_mx[4 + threadIdx.x];
+  }
 }
 
 // --- the pass -----------------------------------------------------------------
@@ -784,8 +796,8 @@ __device__ __forceinline__ void seg_fragments(const T (&x)[2][4], const int (&sc
 // SEGB: runs of equal b' (segment B), else of equal a' (segment A)
 template <int S, int KT, bool SEGB, typename T, typename TA>
 __global__ void __launch_bounds__(32 * SEG_WARPS)
-    k_oz_seg(GeomDev g, const int2* __restrict__ slabs, int nslab, int ngrp, int64_t row_base,
-             const uint16_t* __restrict__ dig, const int16_t* __restrict__ sexp, const T* __restrict__ V, int64_t ldv,
+    k_oz_seg(GeomDev g, const int4* __restrict__ slabs, int nslab, int ngrp, int64_t row_base, int item0,
+             const uint16_t* __restrict__ dig, const int16_t* __restrict__ sexp, const int* __restrict__ vsexp, const T* __restrict__ V, int64_t ldv,
              int m, T* __restrict__ W, int64_t ldw, TA* __restrict__ W1, int64_t ld1) {
   constexpr int PITCH = seg_pitch<S, KT>(), NPIECE = 16 * S * KT * 2, KW = 16 * KT, TSH = oz_unit<S>();
   extern __shared__ __align__(16) unsigned char smem[];
@@ -800,7 +812,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
     const int fi = (int)(run % (nv - 1));
     const int64_t sg = run / (nv - 1);
     const int c0 = (int)(sg % ngrp) * 16;
-    const int2 sl = slabs[sg / ngrp];                   // first row, class
+    const int4 sl = slabs[sg / ngrp];                   // first row, class, first item, items
     const int cls = sl.y;
     const int f = SEGB ? fi + 1 : fi;
     const int nrow = SEGB ? f : nv - 1 - f;
@@ -838,23 +850,15 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
           x[h][v] = (ok && cc[h] < m) ? __ldg(V + (int64_t)cc[h] * ldv + dbase + pr * dstr) : T(0);
       }
     };
-    // column exponents of the run's 2^er V2
-    int ev[2] = {OZ_EMIN, OZ_EMIN};
-    for (int t0 = 0; t0 < nrow; t0 += 16) {
-      T x[2][4];
-      int er[4];
-      load_v2(t0, x, er);
+    // column exponents of the slab's 2^er V2
+    int ev[2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int e = Parts<T>::exponent(x[h][v]);
-          if (e == OZ_NONFINITE || er[v] == 32767) ev[h] = OZ_NONFINITE;
-          else if (e != OZ_ZERO) ev[h] = max(ev[h], e + er[v]);
-        }
+    for (int h = 0; h < 2; ++h) {
+      int e = OZ_EMIN;
+      if (cc[h] < m)
+        for (int i = 0; i < sl.w; ++i) e = max(e, __ldg(vsexp + (int64_t)(sl.z - item0 + i) * m + cc[h]));
+      ev[h] = e;
     }
-    ev[0] = quad_max(ev[0]);
-    ev[1] = quad_max(ev[1]);
     // V of the singles (f, k)
     uint32_t xf[KT][S][4];
     int ex[2] = {OZ_EMIN, OZ_EMIN};
@@ -882,15 +886,27 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
 #pragma unroll
       for (int i = 0; i < S; ++i) a1[n][i][0] = a1[n][i][1] = a1[n][i][2] = a1[n][i][3] = 0.f;
     int b = 0;
+    T x[2][4];
+    int er[4];
+    load_v2(0, x, er);
     for (int t0 = 0; t0 < nrow; t0 += 16, b ^= 1) {
       __syncwarp();                                       // the other stage's readers are done
       if (t0 + 16 < nrow) issue(t0 + 16, b ^ 1);
       else asm volatile("cp.async.commit_group;\n" ::);
-      T x[2][4];
-      int er[4];
-      load_v2(t0, x, er);
       uint32_t vf[S][4];
       seg_fragments<S, T>(x, er, ev, vf);
+      // this step's W2 rows and the next step's V2, ahead of their use
+      int ee[4];
+      T wv[2][4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        ee[v] = er[v] == 32767 ? OZ_NONFINITE : er[v];
+        const int t = t0 + pos[v];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          wv[h][v] = (t < nrow && cc[h] < m) ? W[(int64_t)cc[h] * ldw + dbase + pair_of(t) * dstr] : T(0);
+      }
+      if (t0 + 16 < nrow) load_v2(t0 + 16, x, er);
       asm volatile("cp.async.wait_group 1;\n" ::);
       __syncwarp();
       // 16 x 16 digits of slice i, k group kt: row lane % 16, half lane / 16
@@ -933,15 +949,14 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
           const int t = t0 + 8 * hr + pos[v];
           if (t >= nrow) continue;
           const int64_t d = dbase + pair_of(t) * dstr;
-          const int e = er[2 * hr + v] == 32767 ? OZ_NONFINITE : er[2 * hr + v];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (cc[h] >= m) continue;
             float dsum[S];
 #pragma unroll
             for (int i = 0; i < S; ++i) dsum[i] = a2[i][2 * h + v];
-            T* w = W + (int64_t)cc[h] * ldw + d;
-            *w += oz_round<S, T>(dsum) * oz_scale<T>(ex[h] + e + TSH);
+            W[(int64_t)cc[h] * ldw + d] =
+                wv[h][2 * hr + v] + oz_round<S, T>(dsum) * oz_scale<T>(ex[h] + ee[2 * hr + v] + TSH);
           }
         }
       }
@@ -979,9 +994,11 @@ struct OzPlan {
   unsigned char* d_lists = nullptr;   // error word, work items, slabs, item exponents
   size_t list_bytes = 0;
   int* err = nullptr;
-  int2 *items = nullptr, *slabs = nullptr;
-  int* vexp = nullptr;
-  std::vector<int2> h_items, h_slabs; // host copies: all rows, in storage order
+  int2* items = nullptr;
+  int4* slabs = nullptr;
+  int *vexp = nullptr, *vsexp = nullptr;
+  std::vector<int2> h_items;          // host copies: all rows, in storage order
+  std::vector<int4> h_slabs;          // first row, class, first item, items
   int item0 = 0, nitems = 0;          // those of the prepared rows
   int slab0 = 0, nslab = 0;
   int item_rows = 0, lists_m = 0;
@@ -1154,13 +1171,15 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
       const int64_t sl = G.slab_len(cls);
       for (int64_t s0 = G.start[cls]; s0 < G.start[cls + 1]; s0 += sl) {
         const int64_t npc = (sl + want - 1) / want, per = ((sl + npc - 1) / npc + 127) / 128 * 128;
+        const int i0 = (int)p->h_items.size();
         for (int64_t x = s0; x < s0 + sl; x += per)
           p->h_items.push_back(make_int2((int)x, (int)std::min<int64_t>(x + per, s0 + sl)));
-        if (cls == 1 || cls >= 3) p->h_slabs.push_back(make_int2((int)s0, cls));
+        if (cls == 1 || cls >= 3) p->h_slabs.push_back(make_int4((int)s0, cls, i0, (int)p->h_items.size() - i0));
       }
     }
     const size_t ni = p->h_items.size(), ns = p->h_slabs.size();
-    const size_t lb = align256(sizeof(int2) * (ni + ns)), lneed = 256 + lb + sizeof(int) * ni * m;
+    const size_t ib = align256(sizeof(int2) * ni), lb = ib + align256(sizeof(int4) * ns);
+    const size_t lneed = 256 + lb + 2 * sizeof(int) * ni * m;
     if (p->list_bytes < lneed) {
       dfree(c, p->d_lists);
       p->d_lists = nullptr;
@@ -1171,16 +1190,18 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
       ADC_CUDA(c, cudaMemsetAsync(p->err, 0, sizeof(int), c->stream));
     }
     p->items = reinterpret_cast<int2*>(p->d_lists + 256);
-    p->slabs = p->items + ni;
+    p->slabs = reinterpret_cast<int4*>(p->d_lists + 256 + ib);
     p->vexp = reinterpret_cast<int*>(p->d_lists + 256 + lb);
-    std::vector<int2> all(p->h_items);
-    all.insert(all.end(), p->h_slabs.begin(), p->h_slabs.end());
-    ADC_CUDA(c, h2d(c, p->items, all.data(), sizeof(int2) * all.size()));
+    p->vsexp = p->vexp + ni * m;
+    std::vector<unsigned char> all(lb);
+    std::copy_n(reinterpret_cast<const unsigned char*>(p->h_items.data()), sizeof(int2) * ni, all.data());
+    std::copy_n(reinterpret_cast<const unsigned char*>(p->h_slabs.data()), sizeof(int4) * ns, all.data() + ib);
+    ADC_CUDA(c, h2d(c, p->items, all.data(), lb));
     p->item_rows = (int)want;
     p->lists_m = m;
   }
-  auto first = [](const std::vector<int2>& v, int64_t row) {
-    return (int)(std::lower_bound(v.begin(), v.end(), row, [](const int2& a, int64_t r) { return a.x < r; }) - v.begin());
+  auto first = [](const auto& v, int64_t row) {
+    return (int)(std::lower_bound(v.begin(), v.end(), row, [](const auto& a, int64_t r) { return a.x < r; }) - v.begin());
   };
   p->item0 = first(p->h_items, row0);
   p->nitems = first(p->h_items, row1) - p->item0;
@@ -1223,7 +1244,7 @@ int oz_go(Ctx* c, OzPlan* p, int smax, const OzShape& sh, size_t smem, const T* 
   const int ngrp = (m + NP - 1) / NP;
   const int grid = std::max(1, std::min(p->nitems * ngrp, c->nsm));
   k_oz_vexp<T><<<dim3(p->nitems, (m + 3) / 4), 256, 0, c->stream>>>(to_dev(c->geom), p->items + p->item0, p->dst.row0, p->rexp,
-                                                                    V, ldv, m, p->vexp);
+                                                                    p->sexp, V, ldv, m, p->vexp, p->vsexp);
   ADC_COUNT_LAUNCH();
   kern<<<grid, OZ_THREADS, smem, c->stream>>>(to_dev(c->geom), p->items + p->item0, p->nitems, ngrp, sh, p->dst, p->dig, p->rexp,
                                               p->vexp, diag, V, ldv, m, W, ldw, W1, ld1, p->err);
@@ -1241,8 +1262,8 @@ int oz_seg_go(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t l
   const int ngrp = (m + 15) / 16;
   const int64_t nrun = (int64_t)p->nslab * ngrp * (c->geom.nv - 1);
   const int grid = (int)std::min<int64_t>((nrun + SEG_WARPS - 1) / SEG_WARPS, (int64_t)c->nsm * 16);
-  kern<<<grid, 32 * SEG_WARPS, smem, c->stream>>>(to_dev(c->geom), p->slabs + p->slab0, p->nslab, ngrp, p->dst.row0, p->seg,
-                                                  p->sexp, V, ldv, m, W, ldw, W1, ld1);
+  kern<<<grid, 32 * SEG_WARPS, smem, c->stream>>>(to_dev(c->geom), p->slabs + p->slab0, p->nslab, ngrp, p->dst.row0, p->item0, p->seg,
+                                                  p->sexp, p->vsexp, V, ldv, m, W, ldw, W1, ld1);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
