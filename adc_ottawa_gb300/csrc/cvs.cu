@@ -21,17 +21,21 @@
 namespace adcgpu {
 namespace {
 
-// W1(i,q) = sum_j Ac(i,j) V1(j,q), one thread per (i, q)
+// W1(i,q) = sum_j Ac(i,j) V1(j,q), one warp per (i, q) (one thread per output
+// walked a row alone: 78 us at 321 singles, 7 columns)
 __global__ void k_cvs_singles(int cn1, int m, const double* __restrict__ Ac, const double* __restrict__ V,
                               int64_t ldv, double* __restrict__ W, int64_t ldw) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)cn1 * m;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(t % cn1), q = (int)(t / cn1);
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < (int64_t)cn1 * m; t += nw) {
+    const int i = (int)(t / m), q = (int)(t % m);
     const double* a = Ac + (int64_t)i * cn1;
     const double* v = V + q * ldv;
     double acc = 0.0;
-    for (int j = 0; j < cn1; ++j) acc = fma(a[j], v[j], acc);
-    W[i + q * ldw] = acc;
+    for (int j = lane; j < cn1; j += 32) acc = fma(a[j], v[j], acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) W[i + q * ldw] = acc;
   }
 }
 
@@ -89,12 +93,12 @@ __global__ void __launch_bounds__(256) k_cvs_rows(int64_t n2, int cn1, int q0, c
 }
 
 template <int MG>
-int launch_rows(Ctx* c, int q0, const double* dV, int64_t ldv, double* dW, int64_t ldw) {
+int launch_rows(Ctx* c, int64_t n2, int q0, const double* dV, int64_t ldv, double* dW, int64_t ldw) {
   const size_t smem = sizeof(double) * 2 * (size_t)c->cvs_n1 * MG;
   if (smem > 48 * 1024)
     ADC_CUDA(c, cudaFuncSetAttribute(k_cvs_rows<MG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t n2 = c->cvs_N - c->cvs_n1;
-  k_cvs_rows<MG><<<c->nsm * 2, 256, smem, c->stream>>>(n2, (int)c->cvs_n1, q0, c->d_crow, c->d_ccol, c->d_cval,
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n2 + 7) / 8, c->nsm * 2));
+  k_cvs_rows<MG><<<grid, 256, smem, c->stream>>>(n2, (int)c->cvs_n1, q0, c->d_crow, c->d_ccol, c->d_cval,
                                                          c->d_diag, dV, ldv, dW, ldw);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
@@ -137,10 +141,22 @@ __global__ void k_cvs_export_coupling(int64_t n2, int cn1, int64_t base, const i
 
 int sigma_cvs(Ctx* c, int m, const double* dV, int64_t ldv, double* dW, int64_t ldw) {
   const int cn1 = (int)c->cvs_n1;
-  k_cvs_singles<<<std::max(1, std::min(c->nsm * 8, (cn1 * m + 255) / 256)), 256, 0, c->stream>>>(cn1, m, c->d_Ac, dV,
+  k_cvs_singles<<<std::max(1, std::min(c->nsm * 8, (cn1 * m + 7) / 8)), 256, 0, c->stream>>>(cn1, m, c->d_Ac, dV,
                                                                                                   ldv, dW, ldw);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
+  // the pair rows (all but the first npp nvirt) on the tensor cores by exact
+  // digit slices; the compressed-row kernel (FP64 multiply-adds and shared
+  // atomics: 1.85 ms for 7 columns at nocc=9, nvirt=107, 3 core orbitals)
+  // takes the rows with a' = b', and all rows when the digits do not fit
+  bool usable = false;
+  ST(oz_prepare_cvs(c, c->cvs_oz, m, &usable));
+  int64_t n2 = c->cvs_N - cn1;
+  if (usable) {
+    ST(oz_launch(c, c->cvs_oz, c->d_diag, dV, ldv, m, dW, ldw, dW, ldw));
+    const int64_t nc = cn1 / c->geom.nv;
+    n2 = nc * (c->geom.no - nc) * c->geom.nv;
+  }
   // columns per pass: both shared arrays within 200 KiB
   const int64_t cap = (int64_t)200 * 1024 / (2 * (int64_t)sizeof(double) * cn1);
   for (int q0 = 0; q0 < m;) {
@@ -149,15 +165,15 @@ int sigma_cvs(Ctx* c, int m, const double* dV, int64_t ldv, double* dW, int64_t 
     for (int t : {16, 8, 4, 2})
       if (t <= left && t <= cap) { mg = t; break; }
     switch (mg) {
-      case 16: ST(launch_rows<16>(c, q0, dV, ldv, dW, ldw)); break;
-      case 8: ST(launch_rows<8>(c, q0, dV, ldv, dW, ldw)); break;
-      case 4: ST(launch_rows<4>(c, q0, dV, ldv, dW, ldw)); break;
-      case 2: ST(launch_rows<2>(c, q0, dV, ldv, dW, ldw)); break;
-      default: ST(launch_rows<1>(c, q0, dV, ldv, dW, ldw)); break;
+      case 16: ST(launch_rows<16>(c, n2, q0, dV, ldv, dW, ldw)); break;
+      case 8: ST(launch_rows<8>(c, n2, q0, dV, ldv, dW, ldw)); break;
+      case 4: ST(launch_rows<4>(c, n2, q0, dV, ldv, dW, ldw)); break;
+      case 2: ST(launch_rows<2>(c, n2, q0, dV, ldv, dW, ldw)); break;
+      default: ST(launch_rows<1>(c, n2, q0, dV, ldv, dW, ldw)); break;
     }
     q0 += mg;
   }
-  return ADCGPU_OK;
+  return usable ? oz_check(c, c->cvs_oz) : ADCGPU_OK;
 }
 
 int export_coo_cvs(Ctx* c, double* d_h, int32_t* d_oi, int32_t* d_oj) {
@@ -194,6 +210,7 @@ void free_cvs(Ctx* c) {
   dfree(c, c->d_crow); c->d_crow = nullptr;
   dfree(c, c->d_ccol); c->d_ccol = nullptr;
   dfree(c, c->d_cval); c->d_cval = nullptr;
+  oz_free(c, c->cvs_oz);
   c->cvs = 0;
   c->cvs_n1 = c->cvs_N = c->cvs_nnz = 0;
   c->cvs_kpq.clear();

@@ -316,6 +316,7 @@ struct Ctx {
   int64_t* d_crow = nullptr;      // row offsets, n2 + 1
   int32_t* d_ccol = nullptr;
   double* d_cval = nullptr;
+  void* cvs_oz = nullptr;         // digit store of its pair rows (sigma_slices.cu)
   // SIL persistent state for adcgpu_silstep (device Krylov vectors)
   double* d_sil = nullptr;
   int64_t sil_cap = 0;
@@ -454,6 +455,7 @@ bool oz_geometry_ok(const Geometry& G);
 std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, int64_t row1, int64_t* reserve);
 int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int64_t reserve, int m,
                bool* usable);
+int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable);
 void oz_invalidate(void* handle);
 void oz_free(Ctx* c, void*& handle);
 int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t ldv, int m, double* W, int64_t ldw,

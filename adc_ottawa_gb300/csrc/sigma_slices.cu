@@ -80,6 +80,27 @@ struct OzShape {
   uint32_t off_v2, off_ring, off_bar;   // shared-memory offsets
 };
 
+// the space the kernels work in: the stored matrix, or the CVS space (core
+// holes only)
+struct OzGeom {
+  int no, nv, nvP;      // holes of the singles, virtuals (padded)
+  int64_t n1, row0;     // singles; storage row of the first row exponent
+};
+// rows [row0, row1) of one slab: row r is vector element n1 + dbase + (r - row0) dstr
+struct OzItem {
+  int row0, row1;
+  int tile;             // its first tile in the digit store, in boxes of all slices
+  int holes;            // k' | l' << 8 | OZ_TWO: C and D segments | OZ_PAIRS: classes with a' < b'
+  int dbase, dstr;
+  int pad0, pad1;
+};
+constexpr int OZ_TWO = 1 << 16, OZ_PAIRS = 1 << 17;
+struct OzSlab {         // pair rows (a' < b') of one slab
+  int row0, dbase, dstr;
+  int item0, nitem;     // its work items
+  int pad0, pad1, pad2;
+};
+
 // --- digits --------------------------------------------------------------
 // x = (-1)^neg m 2^(e - MB), m < 2^MB; e = OZ_ZERO for zeros and subnormals,
 // OZ_NONFINITE for inf and NaN
@@ -222,30 +243,106 @@ __global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const T
   }
 }
 
+// Digits of the CVS matrix's pair rows (spins I, II) from its compressed
+// rows: one warp per tile row spreads the kept entries over the index-free
+// segments (C: (a, core hole of the slab), A: (a', k), B: (b', k)) in shared
+// memory, then writes the digits of both stores as k_oz_values and
+// k_oz_seg_values do.  rows: 2 npp npair (hole pair major, spin I first),
+// compressed row crow0 + row.
+template <int S>
+__global__ void __launch_bounds__(128) k_oz_cvs_values(OzGeom g, int npp, int64_t crow0,
+                                                       const int64_t* __restrict__ rowptr,
+                                                       const int32_t* __restrict__ col, const double* __restrict__ val,
+                                                       int kw, uint16_t* __restrict__ out, uint16_t* __restrict__ seg,
+                                                       int16_t* __restrict__ rexp, int16_t* __restrict__ sexp) {
+  extern __shared__ double cvs_sh[];
+  const int lane = threadIdx.x & 31;
+  double* row_c = cvs_sh + (threadIdx.x >> 5) * (g.nvP + 2 * kw);
+  double* row_ab = row_c + g.nvP;
+  const int nbox = (g.nvP + OZ_BOX - 1) / OZ_BOX;
+  const int64_t npair = (int64_t)g.nv * (g.nv - 1) / 2, tps = (npair + OZ_ROWS - 1) / OZ_ROWS;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5), ntot = 2 * npp * tps * OZ_ROWS;
+  for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < ntot; w += nw) {
+    const int64_t tile = w / OZ_ROWS, slab = tile / tps;
+    const int r = (int)(w % OZ_ROWS);
+    const int64_t p = tile % tps * OZ_ROWS + r;
+    const bool valid = p < npair;
+    const int64_t row = slab * npair + p;
+    __syncwarp();
+    for (int x = lane; x < g.nvP + 2 * kw; x += 32) row_c[x] = 0.0;
+    __syncwarp();
+    int mc = OZ_EMIN, ms = OZ_EMIN;
+    if (valid) {
+      int ap, bp;
+      pair_decode(p, g.nv, ap, bp);
+      for (int64_t e = rowptr[crow0 + row] + lane; e < rowptr[crow0 + row + 1]; e += 32) {
+        const int j = col[e], a = j / g.no, k = j - a * g.no;
+        const double x = val[e];
+        if (a == ap || a == bp) {
+          row_ab[(a == bp ? kw : 0) + k] = x;
+          ms = max(ms, Parts<double>::exponent(x));
+        } else {
+          row_c[a] = x;      // k is the slab's core hole: the row's only other couplings
+          mc = max(mc, Parts<double>::exponent(x));
+        }
+      }
+    }
+    mc = __reduce_max_sync(0xffffffffu, mc);
+    ms = __reduce_max_sync(0xffffffffu, ms);
+    __syncwarp();
+    if (lane == 0 && valid) {
+      rexp[row] = (int16_t)min(mc, 32767);
+      sexp[row] = (int16_t)min(ms, 32767);
+    }
+    uint16_t* o = out + tile * oz_tile_values<S>(nbox);
+    for (int q = lane; q < 8 * nbox; q += 32) {
+      unsigned long long u8[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) u8[u] = oz_fixed<S, double>(8 * q < g.nvP ? row_c[8 * q + u] : 0.0, 8 * S - 1 - mc);
+      const int grp = q >> 4, bx = (q >> 3) & 1, two = 2 * grp + 1 < nbox ? 2 : 1;
+      uint16_t* og = o + ((int64_t)S * 2 * grp + bx) * (OZ_ROWS * OZ_BOX) + sw128_off(r, 8 * (q & 7)) / 2;
+#pragma unroll
+      for (int i = 0; i < S; ++i)
+        *reinterpret_cast<uint4*>(og + (int64_t)i * two * (OZ_ROWS * OZ_BOX)) =
+            make_uint4(oz_pair(oz_digit<S>(u8[0], i), oz_digit<S>(u8[1], i)),
+                       oz_pair(oz_digit<S>(u8[2], i), oz_digit<S>(u8[3], i)),
+                       oz_pair(oz_digit<S>(u8[4], i), oz_digit<S>(u8[5], i)),
+                       oz_pair(oz_digit<S>(u8[6], i), oz_digit<S>(u8[7], i)));
+    }
+    if (valid) {
+      uint16_t* os = seg + row * 2 * S * kw;
+      for (int x = lane; x < 2 * kw; x += 32) {
+        const int sg = x >= kw ? 1 : 0, k = x - sg * kw;
+        const unsigned long long u = oz_fixed<S, double>(row_ab[x], 8 * S - 1 - ms);
+#pragma unroll
+        for (int i = 0; i < S; ++i) os[(sg * S + i) * kw + k] = (uint16_t)(oz_digit<S>(u, i) >> 16);
+      }
+    }
+  }
+}
+
 // exponents of the largest 2^rexp |V2| and 2^sexp |V2| of each work item and
 // column: the scales of the V2 digits for the C|D segments (vexp) and for
 // segments A and B (sexp of the classes with a' < b'; the runs of a slab take
 // the maximum over its items).  One block per item and 4 columns; reads V2
 // once (the pass then finds most of it in L2).
 template <typename T>
-__global__ void __launch_bounds__(256) k_oz_vexp(GeomDev g, const int2* __restrict__ items, int64_t row0,
+__global__ void __launch_bounds__(256) k_oz_vexp(OzGeom g, const OzItem* __restrict__ items,
                                                  const int16_t* __restrict__ rexp, const int16_t* __restrict__ sexp,
                                                  const T* __restrict__ V, int64_t ldv, int m, int* __restrict__ vexp,
                                                  int* __restrict__ vsexp) {
   __shared__ int s_mx[8];
-  const int2 item = items[blockIdx.x];
+  const OzItem item = items[blockIdx.x];
   const int c0 = 4 * blockIdx.y;
   if (threadIdx.x < 8) s_mx[threadIdx.x] = OZ_EMIN;
   __syncthreads();
   int mx[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) mx[j] = OZ_EMIN;
-  const bool perm = item.x >= g.start[1] && item.x < g.start[2];
-  const bool pairs = perm || item.x >= g.start[3];
-  for (int row = item.x + threadIdx.x; row < item.y; row += 256) {
-    int64_t d = row;
-    if (perm) d = row_to_d(g, decode_row(g, row), row);
-    const int rx = rexp[row - row0], sx = pairs ? (int)sexp[row - row0] : OZ_EMIN;
+  const bool pairs = item.holes & OZ_PAIRS;
+  for (int row = item.row0 + threadIdx.x; row < item.row1; row += 256) {
+    const int64_t d = item.dbase + (int64_t)(row - item.row0) * item.dstr;
+    const int rx = rexp[row - g.row0], sx = pairs ? (int)sexp[row - g.row0] : OZ_EMIN;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (c0 + j >= m) break;
@@ -358,8 +455,7 @@ __device__ __forceinline__ void oz_combine(uint32_t taddr, TR (&t)[NH]) {
 // S digits, NP columns per pass, MS 128-value groups at most
 template <int S, int NP, int MS, typename T, typename TA>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
-    k_sigma_oz(const __grid_constant__ GeomDev g, const int2* __restrict__ items, int nitems, int ngrp, OzShape sh,
-               const __grid_constant__ OzDst src, const uint16_t* __restrict__ dig, const int16_t* __restrict__ rexp,
+    k_sigma_oz(OzGeom g, const OzItem* __restrict__ items, int nitems, int ngrp, OzShape sh, const uint16_t* __restrict__ dig, const int16_t* __restrict__ rexp,
                const int* __restrict__ ivexp, const T* __restrict__ diag, const T* __restrict__ V, int64_t ldv, int m, T* __restrict__ W,
                int64_t ldw, TA* __restrict__ W1, int64_t ld1, int* __restrict__ err) {
   constexpr int DW = oz_dw<S, NP>();
@@ -411,13 +507,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       uint32_t use = 0;
       bool ok = true;
       for (int un = blockIdx.x; ok && un < nunits; un += gridDim.x) {
-        const int2 item = items[un / ngrp];
-        const int cls = decode_row(g, item.x).cls;
-        const int nbox = src.nbox[cls], nslot = (nbox + 1) / 2;
-        const int64_t rc = item.x - src.r0[cls], slab = rc / src.slab[cls];
-        const uint16_t* tp = dig + src.base[cls] +
-                             (slab * src.tps[cls] + (rc - slab * src.slab[cls]) / OZ_ROWS) * oz_tile_values<S>(nbox);
-        for (int row0 = item.x; ok && row0 < item.y; row0 += OZ_ROWS) {
+        const OzItem item = items[un / ngrp];
+        const int nbox = ((item.holes & OZ_TWO ? 2 : 1) * nvP + OZ_BOX - 1) / OZ_BOX, nslot = (nbox + 1) / 2;
+        const uint16_t* tp = dig + (int64_t)item.tile * (S * OZ_ROWS * OZ_BOX);
+        for (int row0 = item.row0; ok && row0 < item.row1; row0 += OZ_ROWS) {
           for (int s = 0; ok && s < nslot; ++s) {
             const uint32_t bytes = 2 * s + 1 < nbox ? OZ_SLOT_BYTES : OZ_SLOT_BYTES / 2;
             for (int i = 0; i < S; ++i, ++use) {
@@ -448,12 +541,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint32_t d2use[MS] = {};
     bool ok = true;
     for (int un = blockIdx.x; un < nunits && ok && !__any_sync(0xffffffffu, oz_failed(err)); un += gridDim.x, ++nun) {
-      const int2 item = items[un / ngrp];
-      const int cls = decode_row(g, item.x).cls;
-      const int K = (cls >= 2 ? 2 : 1) * nvP;
+      const OzItem item = items[un / ngrp];
+      const int K = (item.holes & OZ_TWO ? 2 : 1) * nvP;
       const int nbox = (K + OZ_BOX - 1) / OZ_BOX, nslot = (nbox + 1) / 2;
       ok = mbar_wait_warp(&bars[O_XFULL], nun & 1u, err, 2);
-      for (int row0 = item.x; ok && row0 < item.y; row0 += OZ_ROWS, ++tile) {
+      for (int row0 = item.row0; ok && row0 < item.row1; row0 += OZ_ROWS, ++tile) {
         const uint32_t b = sh.nb == 2 ? tile & 1u : 0u, ph = sh.nb == 2 ? (tile >> 1) & 1u : tile & 1u;
         ok = mbar_wait_warp(&bars[O_D1EMPTY0 + b], ph ^ 1u, err, 4);
         ok = ok && mbar_wait_warp(&bars[O_V2FULL0 + b], ph, err, 5);
@@ -461,8 +553,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const uint32_t tD1 = tbase + b * DW;
         const uint64_t vdesc = KMAJ + ((sVa + b * V2B) >> 4);
         // the W1 sums run over OZ_FLUSH tiles of the item
-        const int pos = ((row0 - item.x) / OZ_ROWS) % OZ_FLUSH;
-        const bool d2first = pos == 0, d2last = pos == OZ_FLUSH - 1 || row0 + OZ_ROWS >= item.y;
+        const int pos = ((row0 - item.row0) / OZ_ROWS) % OZ_FLUSH;
+        const bool d2first = pos == 0, d2last = pos == OZ_FLUSH - 1 || row0 + OZ_ROWS >= item.row1;
 #pragma unroll
         for (int s = 0; s < MS; ++s) {
           if (!ok || s >= nslot) break;
@@ -528,18 +620,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     int rx = 0;                 // exponent of the row of the tile being prepared
     T v2[NH];
     // V2 of a tile: this thread's row and columns
-    auto load_v2 = [&](int row, int row_end, int cls, int c0) {
-      const bool valid = row < row_end;
-      rx = 0;
-      int64_t d = 0;
-      if (valid) {
-        d = row;
-        if (cls == 1) {
-          const Double rr = decode_row(g, row);
-          d = row_to_d(g, rr, row);
-        }
-        rx = rexp[row - src.row0];
-      }
+    auto load_v2 = [&](const OzItem& item, int row, int c0) {
+      const bool valid = row < item.row1;
+      const int64_t d = valid ? item.dbase + (int64_t)(row - item.row0) * item.dstr : 0;
+      rx = valid ? (int)rexp[row - g.row0] : 0;
 #pragma unroll
       for (int j = 0; j < NH; ++j) {
         const int c = c0 + cbeg + j;
@@ -568,14 +652,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       mbar_arrive(&bars[O_V2FULL0 + buf]);
     };
     for (int un = blockIdx.x; un < nunits && ok && !__any_sync(0xffffffffu, oz_failed(err)); un += gridDim.x) {
-      const int2 item = items[un / ngrp];
+      const OzItem item = items[un / ngrp];
       const int c0 = (un % ngrp) * NP;
-      const Double r0 = decode_row(g, item.x);
-      const int cls = r0.cls;
-      const int K = (cls >= 2 ? 2 : 1) * nvP;
+      const int K = (item.holes & OZ_TWO ? 2 : 1) * nvP;
       const int nbox = (K + OZ_BOX - 1) / OZ_BOX, nslot = (nbox + 1) / 2;
-      const int kp = r0.kp, lp = r0.lp;
-      load_v2(item.x + r, item.y, cls, c0);
+      const int kp = item.holes & 255, lp = (item.holes >> 8) & 255;
+      load_v2(item, item.row0 + r, c0);
 #pragma unroll
       for (int j = 0; j < NH; ++j)
         vexp[j] = c0 + cbeg + j < m ? __ldg(ivexp + (int64_t)(un / ngrp) * m + c0 + cbeg + j) : OZ_EMIN;
@@ -617,13 +699,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       if (!ok) break;
       uint32_t buf = sh.nb == 2 ? tile & 1u : 0u;
       store_v2(buf);
-      for (int row0 = item.x; ok && row0 < item.y; row0 += OZ_ROWS, ++tile) {
+      for (int row0 = item.row0; ok && row0 < item.row1; row0 += OZ_ROWS, ++tile) {
         buf = sh.nb == 2 ? tile & 1u : 0u;
         const uint32_t ph = sh.nb == 2 ? (tile >> 1) & 1u : tile & 1u;
-        const bool has_next = row0 + OZ_ROWS < item.y;
+        const bool has_next = row0 + OZ_ROWS < item.row1;
         const int rx_t = rx;
-        const bool d2last = ((row0 - item.x) / OZ_ROWS) % OZ_FLUSH == OZ_FLUSH - 1 || !has_next;
-        if (has_next) load_v2(row0 + OZ_ROWS + r, item.y, cls, c0);
+        const bool d2last = ((row0 - item.row0) / OZ_ROWS) % OZ_FLUSH == OZ_FLUSH - 1 || !has_next;
+        if (has_next) load_v2(item, row0 + OZ_ROWS + r, c0);
         // W1 sums of one 128-value group
         auto drain_d2 = [&](int s, double (&ac)[NH]) {
           ok = ok && mbar_wait_warp(&bars[O_D2FULL + s], d2use[s] & 1u, err, 10);
@@ -656,12 +738,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           if (d2last && s + 1 == nslot) drain_d2(s, acc[s]);
         if (!ok) break;
         const int row = row0 + r;
-        if (row < item.y) {
-          int64_t d = row;
-          if (cls == 1) {
-            const Double rr = decode_row(g, row);
-            d = row_to_d(g, rr, row);
-          }
+        if (row < item.row1) {
+          const int64_t d = item.dbase + (int64_t)(row - item.row0) * item.dstr;
           const T dg = diag[n1 + d];
           const int re = rx_t == 32767 ? OZ_NONFINITE : rx_t;
 #pragma unroll
@@ -796,7 +874,7 @@ __device__ __forceinline__ void seg_fragments(const T (&x)[2][4], const int (&sc
 // SEGB: runs of equal b' (segment B), else of equal a' (segment A)
 template <int S, int KT, bool SEGB, typename T, typename TA>
 __global__ void __launch_bounds__(32 * SEG_WARPS)
-    k_oz_seg(GeomDev g, const int4* __restrict__ slabs, int nslab, int ngrp, int64_t row_base, int item0,
+    k_oz_seg(OzGeom g, const OzSlab* __restrict__ slabs, int nslab, int ngrp, int item0,
              const uint16_t* __restrict__ dig, const int16_t* __restrict__ sexp, const int* __restrict__ vsexp, const T* __restrict__ V, int64_t ldv,
              int m, T* __restrict__ W, int64_t ldw, TA* __restrict__ W1, int64_t ld1) {
   constexpr int PITCH = seg_pitch<S, KT>(), NPIECE = 16 * S * KT * 2, KW = 16 * KT, TSH = oz_unit<S>();
@@ -812,16 +890,14 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
     const int fi = (int)(run % (nv - 1));
     const int64_t sg = run / (nv - 1);
     const int c0 = (int)(sg % ngrp) * 16;
-    const int4 sl = slabs[sg / ngrp];                   // first row, class, first item, items
-    const int cls = sl.y;
+    const OzSlab sl = slabs[sg / ngrp];
     const int f = SEGB ? fi + 1 : fi;
     const int nrow = SEGB ? f : nv - 1 - f;
     // slab-local pair of row t of the run; vector index of a pair
     auto pair_of = [&](int t) -> int64_t { return SEGB ? pair_index(t, f, nv) : pair_index(f, f + 1 + t, nv); };
-    const int64_t kloc = cls == 1 ? (sl.x - g.start[1]) / g.npair_v : 0;
-    const int64_t dbase = n1 + (cls == 1 ? g.start[1] + kloc : (int64_t)sl.x);
-    const int dstr = cls == 1 ? no : 1;
-    const int64_t rloc = sl.x - row_base;
+    const int64_t dbase = n1 + sl.dbase;
+    const int dstr = sl.dstr;
+    const int64_t rloc = sl.row0 - g.row0;
     const int cc[2] = {c0 + gid, c0 + gid + 8};
     auto issue = [&](int t0, int b) {
       for (int p = lane; p < NPIECE; p += 32) {
@@ -856,7 +932,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
     for (int h = 0; h < 2; ++h) {
       int e = OZ_EMIN;
       if (cc[h] < m)
-        for (int i = 0; i < sl.w; ++i) e = max(e, __ldg(vsexp + (int64_t)(sl.z - item0 + i) * m + cc[h]));
+        for (int i = 0; i < sl.nitem; ++i) e = max(e, __ldg(vsexp + (int64_t)(sl.item0 - item0 + i) * m + cc[h]));
       ev[h] = e;
     }
     // V of the singles (f, k)
@@ -991,14 +1067,15 @@ struct OzPlan {
   const void* values_for = nullptr;   // value store the digits were made of
   int S = 0;
   OzDst dst;
+  OzGeom geom;
   unsigned char* d_lists = nullptr;   // error word, work items, slabs, item exponents
   size_t list_bytes = 0;
   int* err = nullptr;
-  int2* items = nullptr;
-  int4* slabs = nullptr;
+  OzItem* items = nullptr;
+  OzSlab* slabs = nullptr;
   int *vexp = nullptr, *vsexp = nullptr;
-  std::vector<int2> h_items;          // host copies: all rows, in storage order
-  std::vector<int4> h_slabs;          // first row, class, first item, items
+  std::vector<OzItem> h_items;        // host copies: all rows, in storage order
+  std::vector<OzSlab> h_slabs;
   int item0 = 0, nitems = 0;          // those of the prepared rows
   int slab0 = 0, nslab = 0;
   int item_rows = 0, lists_m = 0;
@@ -1104,6 +1181,56 @@ std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, i
   return out;
 }
 
+namespace {
+
+// rows per work item: about six items per SM over the column groups of the
+// prepared rows, 1 to 32 tiles (the vector operand of an item costs about a
+// third of a tile)
+int oz_item_rows(const Ctx* c, int64_t rows, int m) {
+  const int64_t want = rows * ((m + 15) / 16) / ((int64_t)c->nsm * 6);
+  return (int)std::min<int64_t>(4096, std::max<int64_t>(128, (want + 127) / 128 * 128));
+}
+
+// the work items of one slab, in equal pieces of whole tiles
+void oz_add_slab(OzPlan* p, int64_t s0, int64_t len, int item_rows, int holes, bool pairs, int64_t dbase, int dstr) {
+  const int64_t npc = (len + item_rows - 1) / item_rows;
+  const int64_t per = ((len + npc - 1) / npc + OZ_ROWS - 1) / OZ_ROWS * OZ_ROWS;
+  const int i0 = (int)p->h_items.size();
+  for (int64_t x = 0; x < len; x += per)
+    p->h_items.push_back(OzItem{(int)(s0 + x), (int)(s0 + std::min(x + per, len)), -1,
+                                holes | (pairs ? OZ_PAIRS : 0), (int)(dbase + x * dstr), dstr, 0, 0});
+  if (pairs)
+    p->h_slabs.push_back(OzSlab{(int)s0, (int)dbase, dstr, i0, (int)p->h_items.size() - i0, 0, 0, 0});
+}
+
+int oz_upload_lists(Ctx* c, OzPlan* p, int item_rows, int m) {
+  const size_t ni = p->h_items.size(), ns = p->h_slabs.size();
+  const size_t ib = align256(sizeof(OzItem) * ni), lb = ib + align256(sizeof(OzSlab) * ns);
+  const size_t need = 256 + lb + 2 * sizeof(int) * ni * m;
+  if (p->list_bytes < need) {
+    dfree(c, p->d_lists);
+    p->d_lists = nullptr;
+    p->list_bytes = 0;
+    ST(dmalloc(c, (void**)&p->d_lists, need));
+    p->list_bytes = need;
+    p->err = reinterpret_cast<int*>(p->d_lists);
+    ADC_CUDA(c, cudaMemsetAsync(p->err, 0, sizeof(int), c->stream));
+  }
+  p->items = reinterpret_cast<OzItem*>(p->d_lists + 256);
+  p->slabs = reinterpret_cast<OzSlab*>(p->d_lists + 256 + ib);
+  p->vexp = reinterpret_cast<int*>(p->d_lists + 256 + lb);
+  p->vsexp = p->vexp + ni * m;
+  std::vector<unsigned char> all(lb);
+  std::copy_n(reinterpret_cast<const unsigned char*>(p->h_items.data()), sizeof(OzItem) * ni, all.data());
+  std::copy_n(reinterpret_cast<const unsigned char*>(p->h_slabs.data()), sizeof(OzSlab) * ns, all.data() + ib);
+  ADC_CUDA(c, h2d(c, p->items, all.data(), lb));
+  p->item_rows = item_rows;
+  p->lists_m = m;
+  return ADCGPU_OK;
+}
+
+}  // namespace
+
 // Makes the digits of the rows [row0, row1) (kept until the values change;
 // the direct path's chunk buffer is rewritten for every chunk) and the work
 // lists of an m-column product.  reserve: bytes the digits of any range of
@@ -1158,68 +1285,127 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
     ADC_CUDA(c, cudaGetLastError());
     p->values_for = c->direct ? nullptr : values;
   }
-  // work items: pieces of one slab, about six per SM over the column groups
-  // of the prepared rows, 1 to 32 tiles long (the vector operand of an item
-  // costs about a third of a tile)
-  const int64_t ngrp = (m + 15) / 16;
-  int64_t want = (c->direct ? direct_range_rows(c) : row1 - row0) * ngrp / ((int64_t)c->nsm * 6);
-  want = std::min<int64_t>(4096, std::max<int64_t>(128, (want + 127) / 128 * 128));
-  if (p->item_rows != (int)want || p->lists_m < m) {
+  // an item's place in the digit store of the prepared rows
+  auto set_tile = [&](OzItem& it) {
+    int cls = 0;
+    while (cls < 4 && it.row0 >= G.start[cls + 1]) ++cls;
+    const int64_t rc = it.row0 - dst.r0[cls], slab = rc / dst.slab[cls];
+    it.tile = (int)(dst.base[cls] / ((int64_t)S * OZ_ROWS * OZ_BOX) +
+                    (slab * dst.tps[cls] + (rc - slab * dst.slab[cls]) / OZ_ROWS) * dst.nbox[cls]);
+  };
+  const int item_rows = oz_item_rows(c, c->direct ? direct_range_rows(c) : row1 - row0, m);
+  if (p->item_rows != item_rows || p->lists_m < m) {
     p->h_items.clear();
     p->h_slabs.clear();
     for (int cls = 0; cls < 5; ++cls) {
       const int64_t sl = G.slab_len(cls);
-      for (int64_t s0 = G.start[cls]; s0 < G.start[cls + 1]; s0 += sl) {
-        const int64_t npc = (sl + want - 1) / want, per = ((sl + npc - 1) / npc + 127) / 128 * 128;
-        const int i0 = (int)p->h_items.size();
-        for (int64_t x = s0; x < s0 + sl; x += per)
-          p->h_items.push_back(make_int2((int)x, (int)std::min<int64_t>(x + per, s0 + sl)));
-        if (cls == 1 || cls >= 3) p->h_slabs.push_back(make_int4((int)s0, cls, i0, (int)p->h_items.size() - i0));
+      for (int64_t s0 = G.start[cls], k = 0; s0 < G.start[cls + 1]; s0 += sl, ++k) {
+        int kp = (int)k, lp = (int)k;
+        if (cls >= 2) pair_decode(k, G.no, kp, lp);
+        // class 2 (stored hole outer) is hole inner in the vectors
+        oz_add_slab(p, s0, sl, item_rows, kp | lp << 8 | (cls >= 2 ? OZ_TWO : 0), cls == 1 || cls >= 3,
+                    cls == 1 ? G.start[1] + k : s0, cls == 1 ? G.no : 1);
       }
     }
-    const size_t ni = p->h_items.size(), ns = p->h_slabs.size();
-    const size_t ib = align256(sizeof(int2) * ni), lb = ib + align256(sizeof(int4) * ns);
-    const size_t lneed = 256 + lb + 2 * sizeof(int) * ni * m;
-    if (p->list_bytes < lneed) {
-      dfree(c, p->d_lists);
-      p->d_lists = nullptr;
-      p->list_bytes = 0;
-      ST(dmalloc(c, (void**)&p->d_lists, lneed));
-      p->list_bytes = lneed;
-      p->err = reinterpret_cast<int*>(p->d_lists);
-      ADC_CUDA(c, cudaMemsetAsync(p->err, 0, sizeof(int), c->stream));
-    }
-    p->items = reinterpret_cast<int2*>(p->d_lists + 256);
-    p->slabs = reinterpret_cast<int4*>(p->d_lists + 256 + ib);
-    p->vexp = reinterpret_cast<int*>(p->d_lists + 256 + lb);
-    p->vsexp = p->vexp + ni * m;
-    std::vector<unsigned char> all(lb);
-    std::copy_n(reinterpret_cast<const unsigned char*>(p->h_items.data()), sizeof(int2) * ni, all.data());
-    std::copy_n(reinterpret_cast<const unsigned char*>(p->h_slabs.data()), sizeof(int4) * ns, all.data() + ib);
-    ADC_CUDA(c, h2d(c, p->items, all.data(), lb));
-    p->item_rows = (int)want;
-    p->lists_m = m;
+    if (!c->direct)
+      for (OzItem& it : p->h_items) set_tile(it);
+    ST(oz_upload_lists(c, p, item_rows, m));
   }
+  // the prepared rows' items
   auto first = [](const auto& v, int64_t row) {
-    return (int)(std::lower_bound(v.begin(), v.end(), row, [](const auto& a, int64_t r) { return a.x < r; }) - v.begin());
+    return (int)(std::lower_bound(v.begin(), v.end(), row, [](const auto& a, int64_t r) { return a.row0 < r; }) - v.begin());
   };
   p->item0 = first(p->h_items, row0);
   p->nitems = first(p->h_items, row1) - p->item0;
   p->slab0 = first(p->h_slabs, row0);
   p->nslab = first(p->h_slabs, row1) - p->slab0;
+  // a range of the direct path: its tiles, counted from the range's first
+  // (the same in every product)
+  if (c->direct && p->nitems && p->h_items[p->item0].tile < 0) {
+    for (int i = p->item0; i < p->item0 + p->nitems; ++i) set_tile(p->h_items[i]);
+    ADC_CUDA(c, h2d(c, p->items + p->item0, p->h_items.data() + p->item0, sizeof(OzItem) * (size_t)p->nitems));
+  }
+  p->geom = OzGeom{G.no, G.nv, G.nvP, G.n1, row0};
+  *usable = true;
+  return ADCGPU_OK;
+}
+
+// Digits and work lists of the CVS matrix's pair rows (spins I and II); the
+// rows with a' = b' stay with the compressed-row kernel.
+int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable) {
+  *usable = false;
+  const Geometry& G = c->geom;
+  constexpr int S = 7;
+  const int nc = (int)(c->cvs_n1 / G.nv), kw = 16 * ((nc + 15) / 16);
+  std::vector<char> core(G.no, 0);
+  for (int k = 0; k < nc; ++k) core[c->cvs_kpq[7 * (1 + k) + 2] - 1] = 1;   // holes of the first virtual's singles
+  std::vector<int> index(G.no, -1), hole;                                   // hole pairs with one core orbital
+  for (int i = 0, n = 0; i < G.no; ++i) if (core[i]) index[i] = n++;
+  for (int i = 0; i < G.no; ++i)
+    for (int j = i + 1; j < G.no; ++j)
+      if (core[i] + core[j] == 1) hole.push_back(core[i] ? index[i] : index[j]);
+  const int npp = (int)hole.size();
+  const int64_t npair = G.npair_v, nrows = 2 * npp * npair, c3 = (int64_t)npp * G.nv;
+  const int nbox = (G.nvP + OZ_BOX - 1) / OZ_BOX;
+  const int64_t tps = (npair + OZ_ROWS - 1) / OZ_ROWS;
+  if (nrows == 0 || c->cvs_N != c->cvs_n1 + c3 + nrows) return ADCGPU_OK;
+  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
+  if (!p) {
+    p = new OzPlan;
+    handle = p;
+  }
+  const size_t dig_b = align256(sizeof(uint16_t) * (size_t)(2 * npp * tps) * S * nbox * OZ_ROWS * OZ_BOX);
+  const size_t seg_b = align256(sizeof(uint16_t) * (size_t)nrows * 2 * S * kw), exp_b = align256(sizeof(int16_t) * (size_t)nrows);
+  if (!p->d_mem) {
+    const size_t bytes = dig_b + seg_b + 2 * exp_b;
+    size_t free_b = 0, total_b = 0;
+    ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    if (bytes > free_b / 3) return ADCGPU_OK;
+    ST(dmalloc(c, (void**)&p->d_mem, bytes));
+    p->mem_bytes = bytes;
+  }
+  p->geom = OzGeom{nc, G.nv, G.nvP, c->cvs_n1, 0};
+  if (p->values_for != c->d_cval) {
+    p->S = S;
+    p->dig = reinterpret_cast<uint16_t*>(p->d_mem);
+    p->seg = reinterpret_cast<uint16_t*>(p->d_mem + dig_b);
+    p->rexp = reinterpret_cast<int16_t*>(p->d_mem + dig_b + seg_b);
+    p->sexp = reinterpret_cast<int16_t*>(p->d_mem + dig_b + seg_b + exp_b);
+    const int grid = (int)std::min<int64_t>(2 * npp * tps * OZ_ROWS / 4, (int64_t)c->nsm * 16);
+    k_oz_cvs_values<S><<<grid, 128, sizeof(double) * 4 * (size_t)(G.nvP + 2 * kw), c->stream>>>(
+        p->geom, npp, c3, c->d_crow, c->d_ccol, c->d_cval, kw, p->dig, p->seg, p->rexp, p->sexp);
+    ADC_COUNT_LAUNCH();
+    ADC_CUDA(c, cudaGetLastError());
+    p->values_for = c->d_cval;
+  }
+  const int item_rows = oz_item_rows(c, nrows, m);
+  if (p->item_rows != item_rows || p->lists_m < m) {
+    p->h_items.clear();
+    p->h_slabs.clear();
+    for (int s = 0; s < 2 * npp; ++s) {
+      const int first = (int)p->h_items.size();
+      oz_add_slab(p, s * npair, npair, item_rows, hole[s % npp], true, c3 + s * npair, 1);
+      for (int i = first; i < (int)p->h_items.size(); ++i)
+        p->h_items[i].tile = (int)((s * tps + (p->h_items[i].row0 - s * npair) / OZ_ROWS) * nbox);
+    }
+    ST(oz_upload_lists(c, p, item_rows, m));
+  }
+  p->item0 = p->slab0 = 0;
+  p->nitems = (int)p->h_items.size();
+  p->nslab = (int)p->h_slabs.size();
   *usable = true;
   return ADCGPU_OK;
 }
 
 namespace {
 
-// shared memory of one launch; nb = 2 where TMEM and shared memory hold two
+// shared memory of one launch over rows of up to 'values' C|D values; nb = 2 where TMEM and shared memory hold two
 // D1 / V2 buffers beside at least three ring slots; false when even one
 // buffer does not fit
 template <int S, int NP>
-bool oz_shape(const Geometry& G, int smax, OzShape* sh, size_t* bytes) {
+bool oz_shape(int values, int smax, OzShape* sh, size_t* bytes) {
   constexpr int DW = oz_dw<S, NP>(), BOXB = oz_xrows<S, NP>() * 128, V2B = 2 * BOXB;
-  sh->nslot = (2 * G.nvP + 127) / 128;
+  sh->nslot = (values + 127) / 128;
   const size_t tail = (size_t)(O_SLOT0 + 2 * OZ_MAXNR) * 8 + (size_t)NP * 4 + 16;
   for (sh->nb = 2; sh->nb >= 1; --sh->nb) {
     if ((sh->nb + sh->nslot) * DW > 512) continue;
@@ -1243,10 +1429,10 @@ int oz_go(Ctx* c, OzPlan* p, int smax, const OzShape& sh, size_t smem, const T* 
   ADC_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
   const int ngrp = (m + NP - 1) / NP;
   const int grid = std::max(1, std::min(p->nitems * ngrp, c->nsm));
-  k_oz_vexp<T><<<dim3(p->nitems, (m + 3) / 4), 256, 0, c->stream>>>(to_dev(c->geom), p->items + p->item0, p->dst.row0, p->rexp,
-                                                                    p->sexp, V, ldv, m, p->vexp, p->vsexp);
+  k_oz_vexp<T><<<dim3(p->nitems, (m + 3) / 4), 256, 0, c->stream>>>(p->geom, p->items + p->item0, p->rexp, p->sexp, V,
+                                                                    ldv, m, p->vexp, p->vsexp);
   ADC_COUNT_LAUNCH();
-  kern<<<grid, OZ_THREADS, smem, c->stream>>>(to_dev(c->geom), p->items + p->item0, p->nitems, ngrp, sh, p->dst, p->dig, p->rexp,
+  kern<<<grid, OZ_THREADS, smem, c->stream>>>(p->geom, p->items + p->item0, p->nitems, ngrp, sh, p->dig, p->rexp,
                                               p->vexp, diag, V, ldv, m, W, ldw, W1, ld1, p->err);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
@@ -1260,10 +1446,10 @@ int oz_seg_go(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t l
   const size_t smem = (size_t)SEG_WARPS * 2 * 16 * seg_pitch<S, KT>();
   ADC_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int ngrp = (m + 15) / 16;
-  const int64_t nrun = (int64_t)p->nslab * ngrp * (c->geom.nv - 1);
+  const int64_t nrun = (int64_t)p->nslab * ngrp * (p->geom.nv - 1);
   const int grid = (int)std::min<int64_t>((nrun + SEG_WARPS - 1) / SEG_WARPS, (int64_t)c->nsm * 16);
-  kern<<<grid, 32 * SEG_WARPS, smem, c->stream>>>(to_dev(c->geom), p->slabs + p->slab0, p->nslab, ngrp, p->dst.row0, p->item0, p->seg,
-                                                  p->sexp, p->vsexp, V, ldv, m, W, ldw, W1, ld1);
+  kern<<<grid, 32 * SEG_WARPS, smem, c->stream>>>(p->geom, p->slabs + p->slab0, p->nslab, ngrp, p->item0, p->seg, p->sexp,
+                                                  p->vsexp, V, ldv, m, W, ldw, W1, ld1);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
@@ -1272,7 +1458,7 @@ int oz_seg_go(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t l
 template <int S, typename T, typename TA>
 int oz_seg(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t ldw, TA* W1, int64_t ld1) {
   if (p->nslab == 0) return ADCGPU_OK;
-  if (c->geom.no <= 16) {
+  if (p->geom.no <= 16) {
     ST((oz_seg_go<S, 1, false>(c, p, V, ldv, m, W, ldw, W1, ld1)));
     return oz_seg_go<S, 1, true>(c, p, V, ldv, m, W, ldw, W1, ld1);
   }
@@ -1288,15 +1474,15 @@ int oz_seg(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t ldw,
 int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t ldv, int m, double* W, int64_t ldw,
               double* W1, int64_t ld1) {
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
-  const int smax = smem_optin_max(c);
+  const int smax = smem_optin_max(c), values = (c->cvs ? 1 : 2) * p->geom.nvP;   // of the longest C|D row
   OzShape sh;
   size_t smem = 0;
   // 16 columns per pass where their accumulators fit (rows of up to 384
   // values); the column groups of an item run side by side, so the digits
   // come from L2 for all but one of them
-  if (m > 8 && oz_shape<7, 16>(c->geom, smax, &sh, &smem))
+  if (m > 8 && oz_shape<7, 16>(values, smax, &sh, &smem))
     ST((oz_go<7, 16, 3>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1)));
-  else if (oz_shape<7, 8>(c->geom, smax, &sh, &smem))
+  else if (oz_shape<7, 8>(values, smax, &sh, &smem))
     ST((oz_go<7, 8, 4>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1)));
   else
     return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
@@ -1307,10 +1493,10 @@ int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t
 int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t ldv, int m, float* W, int64_t ldw,
               double* W1, int64_t ld1) {
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
-  const int smax = smem_optin_max(c);
+  const int smax = smem_optin_max(c), values = (c->cvs ? 1 : 2) * p->geom.nvP;   // of the longest C|D row
   OzShape sh;
   size_t smem = 0;
-  if (!oz_shape<4, 16>(c->geom, smax, &sh, &smem)) return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
+  if (!oz_shape<4, 16>(values, smax, &sh, &smem)) return set_err(c, ADCGPU_UNSUPPORTED, "sliced sigma pass: shape");
   ST((oz_go<4, 16, 4>(c, p, smax, sh, smem, diag, V, ldv, m, W, ldw, W1, ld1)));
   return oz_seg<4>(c, p, V, ldv, m, W, ldw, W1, ld1);
 }

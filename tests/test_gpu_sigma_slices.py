@@ -130,3 +130,20 @@ def test_sliced_fp32_values_match_oracle(gpu, no, nv, m, pad):
         ref = w[32]     # the CUDA-core tile
     for c in range(m):
         assert np.abs(w[0][c] - ref[c]).max() <= 1e-6 * np.abs(ref[c]).max()
+
+
+@pytest.mark.parametrize("no,nv,core,m", [(3, 9, [2], 1), (5, 33, [1, 4], 17), (19, 6, list(range(1, 18)), 9)])
+def test_sliced_cvs_rows_match_oracle(gpu, no, nv, core, m):
+    """The CVS pair rows (one to seventeen core holes per segment)."""
+    from adc_ottawa_gb300 import AdcGpu
+
+    e, eri = system(no, nv, no + nv)
+    g = AdcGpu(0)
+    g.set_orbitals(no, nv, e)
+    g.set_eri_packed(eri)
+    g.write_fspace_adc2_1_cvs(core)
+    x = _vectors(g.ndim, m, g.ndim, 3)
+    ref = oracle.Matrix.build_cvs(no, nv, e, eri, core).matvec(np.asfortranarray(x.T)).T
+    w = g.sigma(np.asfortranarray(x.T)).T
+    for c in range(m):
+        assert np.abs(w[c] - ref[c]).max() <= TOL * np.abs(ref[c]).max()
