@@ -32,8 +32,9 @@ struct Eri {
   __device__ double OOOV(int i, int j, int k, int a) const {
     return ooov[(((int64_t)i * no + j) * no + k) * nv + a];
   }
+  // (a b|i c) with a innermost: the coupling kernel's lanes run over a
   __device__ double VVOV(int a, int b, int i, int c) const {
-    return vvov[(((int64_t)a * nv + b) * no + i) * nv + c];
+    return vvov[(((int64_t)b * no + i) * nv + c) * nv + a];
   }
 };
 
@@ -79,37 +80,64 @@ __global__ void k_gather_block(const double* __restrict__ packed, double* __rest
   }
 }
 
-// CA_ph_ph(a,a1), adc_ph.f90:769-812, for a <= a1 (0-based virtuals).
-__global__ void k_ca(Eri E, const double* __restrict__ e, double* __restrict__ ca) {
-  const int no = E.no, nv = E.nv;
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= (int64_t)nv * nv) return;
-  int a = (int)(t / nv), a1 = (int)(t % nv);
-  if (a > a1) return;
-  const double ea = e[no + a], ea1 = e[no + a1];
-  double acc = 0.0;
-  for (int r = 0; r < nv; ++r)
-    for (int u = 0; u < no; ++u)
-      for (int v = 0; v < no; ++v) {
-        double eijc = e[u] + e[v] - e[no + r];
-        double DA = (eijc - 0.5 * (ea + ea1)) / ((eijc - ea) * (eijc - ea1));
-        double term = 0.0;
-        term = term + E.VOVO(a, u, r, v) * (2.0 * E.VOVO(a1, u, r, v) - E.VOVO(r, u, a1, v));
-        term = term + E.VOVO(a, v, r, u) * (2.0 * E.VOVO(r, u, a1, v) - E.VOVO(a1, u, r, v));
-        term = DA * term;
-        acc = acc + term;
-      }
-  double x = -0.5 * acc;
-  ca[(int64_t)a * nv + a1] = x;
-  ca[(int64_t)a1 * nv + a] = x;
+// (a b|i c) from [a][b][i][c] to the stored [b][i][c][a]: per b a transposition
+// of nv x (no nv) through 32 x 32 tiles.
+__global__ void __launch_bounds__(256) k_vvov_layout(const double* __restrict__ in, double* __restrict__ out, int no,
+                                                     int nv) {
+  __shared__ double t[32][33];
+  const int64_t w = (int64_t)no * nv;
+  const int b = blockIdx.z, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int y = ty; y < 32; y += 8) {
+    const int a = blockIdx.y * 32 + y;
+    const int64_t x = blockIdx.x * 32ll + tx;
+    if (a < nv && x < w) t[y][tx] = in[((int64_t)a * nv + b) * w + x];
+  }
+  __syncthreads();
+  for (int y = ty; y < 32; y += 8) {
+    const int64_t x = blockIdx.x * 32ll + y;
+    const int a = blockIdx.y * 32 + tx;
+    if (a < nv && x < w) out[((int64_t)b * w + x) * nv + a] = t[tx][y];
+  }
 }
 
-// CB_ph_ph(k,k1), adc_ph.f90:819-912 ("dumbed down" branch), k <= k1, in two
-// passes: every term of the (r, s, u) sum of one pair evaluated in parallel
-// (the reference's expression, operation by operation), then the terms summed
-// in the reference's loop order by one thread per pair.  The result is bit
-// for bit that of the serial loop while the divisions run on all SMs.
-// terms: [pair][(r*nv + s)*no + u], pairs k <= k1 enumerated row by row.
+// The second-order intermediates CA(a,a1), a <= a1, and CB(k,k1), k <= k1, are
+// serial sums in the reference (over (r,u,v) and (r,s,u)), which fixes every
+// bit of the result.  Their terms are evaluated in parallel, with the
+// reference's expression operation by operation, into [sum][term]; then
+// k_ordered_sum adds the terms of each sum in the reference's loop order.
+//
+// CA_ph_ph (adc_ph.f90:769-812) and, DIRECT, Ca1_ph_ph (:98-152).
+template <bool DIRECT>
+__global__ void k_ca_terms(Eri E, const double* __restrict__ e, const int2* __restrict__ pairs, int npairs,
+                           double* __restrict__ terms) {
+  const int no = E.no, nv = E.nv;
+  const int64_t nt = (int64_t)nv * no * no;
+  for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < npairs * nt;
+       x += (int64_t)gridDim.x * blockDim.x) {
+    const int pi = (int)(x / nt);
+    const int t = (int)(x - pi * nt);
+    const int v = t % no, u = (t / no) % no, r = t / (no * no);
+    const int a = pairs[pi].x, a1 = pairs[pi].y;
+    const double ea = e[no + a], ea1 = e[no + a1], er = e[no + r];
+    double DA, term = 0.0;
+    if (DIRECT) {
+      const double eija = er + ea - e[u] - e[v], eijc = er + ea1 - e[u] - e[v];
+      DA = 1.0 / (eija * eijc);
+      term = term + eijc * E.VOVO(a1, u, r, v) * (2.0 * E.VOVO(a, u, r, v) - E.VOVO(r, u, a, v));
+      term = term + eija * E.VOVO(a, v, r, u) * (2.0 * E.VOVO(r, u, a1, v) - E.VOVO(a1, u, r, v));
+    } else {
+      const double eijc = e[u] + e[v] - er;
+      DA = (eijc - 0.5 * (ea + ea1)) / ((eijc - ea) * (eijc - ea1));
+      term = term + E.VOVO(a, u, r, v) * (2.0 * E.VOVO(a1, u, r, v) - E.VOVO(r, u, a1, v));
+      term = term + E.VOVO(a, v, r, u) * (2.0 * E.VOVO(r, u, a1, v) - E.VOVO(a1, u, r, v));
+    }
+    terms[x] = DA * term;
+  }
+}
+
+// CB_ph_ph (adc_ph.f90:819-912, "dumbed down" branch) and, DIRECT, Cb1_ph_ph
+// (:158-211); term (r nv + s) no + u.
+template <bool DIRECT>
 __global__ void k_cb_terms(Eri E, const double* __restrict__ e, const int2* __restrict__ pairs, int npairs,
                            double* __restrict__ terms) {
   const int no = E.no, nv = E.nv;
@@ -117,85 +145,72 @@ __global__ void k_cb_terms(Eri E, const double* __restrict__ e, const int2* __re
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < npairs * nt;
        x += (int64_t)gridDim.x * blockDim.x) {
     const int pi = (int)(x / nt);
-    const int64_t t = x % nt;
+    const int64_t t = x - pi * nt;
     const int u = (int)(t % no), s = (int)((t / no) % nv), r = (int)(t / ((int64_t)no * nv));
     const int k = pairs[pi].x, k1 = pairs[pi].y;
     const double ek = e[k], ek1 = e[k1];
-    double eicd = e[u] - e[no + r] - e[no + s];
-    double DB = (eicd + 0.5 * (ek + ek1)) / ((eicd + ek) * (eicd + ek1));
-    double term = 0.0;
-    term = term + E.VOVO(r, k, s, u) * (2.0 * E.VOVO(r, k1, s, u) - E.VOVO(s, k1, r, u));
-    term = term + E.VOVO(r, u, s, k) * (2.0 * E.VOVO(s, k1, r, u) - E.VOVO(r, k1, s, u));
+    double DB, term = 0.0;
+    if (DIRECT) {
+      const double er = e[no + r], es = e[no + s];
+      const double eicd = er + es - e[u] - ek, ejcd = er + es - e[u] - ek1;
+      DB = 1.0 / (eicd * ejcd);
+      term = term + ejcd * E.VOVO(r, k1, s, u) * (2.0 * E.VOVO(r, k, s, u) - E.VOVO(s, k, r, u));
+      term = term + eicd * E.VOVO(r, u, s, k) * (2.0 * E.VOVO(s, k1, r, u) - E.VOVO(r, k1, s, u));
+    } else {
+      const double eicd = e[u] - e[no + r] - e[no + s];
+      DB = (eicd + 0.5 * (ek + ek1)) / ((eicd + ek) * (eicd + ek1));
+      term = term + E.VOVO(r, k, s, u) * (2.0 * E.VOVO(r, k1, s, u) - E.VOVO(s, k1, r, u));
+      term = term + E.VOVO(r, u, s, k) * (2.0 * E.VOVO(s, k1, r, u) - E.VOVO(r, k1, s, u));
+    }
     terms[x] = DB * term;
   }
 }
 
-__global__ void k_cb_sum(const double* __restrict__ terms, const int2* __restrict__ pairs, int npairs, int64_t nt,
-                         int no, double* __restrict__ cb) {
-  const int pi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pi >= npairs) return;
-  const double* tp = terms + (int64_t)pi * nt;
+// out(x, y) = out(y, x) = factor * (0 + t_0 + t_1 + ..), added one by one.  A
+// block takes 32 sums: its warps stage 64 terms of each in shared memory
+// (coalesced, the next stage's loads in flight), lane i of the first warp adds
+// those of sum i.  Bound by the latency of the addition chain; one thread
+// reading its sum alone took 99 ns a term.
+constexpr int OS_T = 64;
+__global__ void __launch_bounds__(128) k_ordered_sum(const double* __restrict__ terms, const int2* __restrict__ pairs,
+                                                     int nsum, int64_t nt, int dim, double factor,
+                                                     double* __restrict__ out) {
+  __shared__ double st[2][32][OS_T + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int s0 = blockIdx.x * 32;
+  double v[16];
+  auto load = [&](int64_t t0) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int s = s0 + 8 * warp + (j >> 1);
+      const int64_t t = t0 + 32 * (j & 1) + lane;
+      v[j] = s < nsum && t < nt ? __ldcs(terms + s * nt + t) : 0.0;
+    }
+  };
+  load(0);
   double acc = 0.0;
-  for (int64_t t = 0; t < nt; ++t) acc = acc + tp[t];
-  const double x = -0.5 * acc;
-  const int k = pairs[pi].x, k1 = pairs[pi].y;
-  cb[k * no + k1] = x;
-  cb[k1 * no + k] = x;
-}
-
-// The direct path's intermediates (get_interm_adc2_save, get_matrix.f90
-// :625-701): Ca1_ph_ph(a,a1) (adc_ph.f90:98-152) for a <= a1 and
-// Cb1_ph_ph(k,k1) (:158-211) for k <= k1, in the reference's operation order.
-__global__ void k_ca1(Eri E, const double* __restrict__ e, double* __restrict__ ca) {
-  const int no = E.no, nv = E.nv;
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= (int64_t)nv * nv) return;
-  int a = (int)(t / nv), a1 = (int)(t % nv);
-  if (a > a1) return;
-  const double ea = e[no + a], ea1 = e[no + a1];
-  double acc = 0.0;
-  for (int r = 0; r < nv; ++r)
-    for (int u = 0; u < no; ++u)
-      for (int v = 0; v < no; ++v) {
-        const double er = e[no + r];
-        double eija = er + ea - e[u] - e[v];
-        double eijc = er + ea1 - e[u] - e[v];
-        double DA = 1.0 / ((er + ea - e[u] - e[v]) * (er + ea1 - e[u] - e[v]));
-        double term = 0.0;
-        term = term + eijc * E.VOVO(a1, u, r, v) * (2.0 * E.VOVO(a, u, r, v) - E.VOVO(r, u, a, v));
-        term = term + eija * E.VOVO(a, v, r, u) * (2.0 * E.VOVO(r, u, a1, v) - E.VOVO(a1, u, r, v));
-        term = DA * term;
-        acc = acc + term;
+  int b = 0;
+  for (int64_t t0 = 0; t0 < nt; t0 += OS_T, b ^= 1) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) st[b][8 * warp + (j >> 1)][32 * (j & 1) + lane] = v[j];
+    __syncthreads();   // also: the first warp is past the stage before last
+    if (t0 + OS_T < nt) load(t0 + OS_T);
+    if (warp == 0) {
+      const int n = (int)min((int64_t)OS_T, nt - t0);
+      if (n == OS_T) {
+#pragma unroll 16
+        for (int t = 0; t < OS_T; ++t) acc = acc + st[b][lane][t];
+      } else {
+        for (int t = 0; t < n; ++t) acc = acc + st[b][lane][t];
       }
-  double x = 0.5 * acc;
-  ca[(int64_t)a * nv + a1] = x;
-  ca[(int64_t)a1 * nv + a] = x;
-}
-
-__global__ void k_cb1(Eri E, const double* __restrict__ e, double* __restrict__ cb) {
-  const int no = E.no, nv = E.nv;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= no * no) return;
-  int k = t / no, k1 = t % no;
-  if (k > k1) return;
-  const double ek = e[k], ek1 = e[k1];
-  double acc = 0.0;
-  for (int r = 0; r < nv; ++r)
-    for (int s = 0; s < nv; ++s)
-      for (int u = 0; u < no; ++u) {
-        const double er = e[no + r], es = e[no + s];
-        double eicd = er + es - e[u] - ek;
-        double ejcd = er + es - e[u] - ek1;
-        double DB = 1.0 / ((er + es - e[u] - ek) * (er + es - e[u] - ek1));
-        double term = 0.0;
-        term = term + ejcd * E.VOVO(r, k1, s, u) * (2.0 * E.VOVO(r, k, s, u) - E.VOVO(s, k, r, u));
-        term = term + eicd * E.VOVO(r, u, s, k) * (2.0 * E.VOVO(s, k1, r, u) - E.VOVO(r, k1, s, u));
-        term = DB * term;
-        acc = acc + term;
-      }
-  double x = 0.5 * acc;
-  cb[k * no + k1] = x;
-  cb[k1 * no + k] = x;
+    }
+  }
+  if (warp == 0 && s0 + lane < nsum) {
+    const int2 p = pairs[s0 + lane];
+    const double x = factor * acc;
+    out[(int64_t)p.x * dim + p.y] = x;
+    out[(int64_t)p.y * dim + p.x] = x;
+  }
 }
 
 // Per (single, (c,i)) tables for CC_ph_ph (adc_ph.f90:918-957):
@@ -344,6 +359,19 @@ __global__ void k_diag2(GeomDev g, const double* __restrict__ e, double* __restr
   }
 }
 
+// x / sqrt(2.0), correctly rounded, in two operations instead of a division:
+// x (zh + zl) with zh + zl = 1 / sqrt(2.0) to 106 bits and one final rounding
+// (N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans.
+// Computers 53, 2004).  Its error before the rounding is below 2^-105
+// relative, so only dividends whose quotient lies that close to a midpoint
+// could round differently; for this divisor those were enumerated (remainders
+// up to 64 units) and all round as the division does
+// (tests/test_build_division.py).
+__device__ __forceinline__ double div_sqrt2(double x) {
+  return __fma_rn(x, 0x1.6a09e667f3bccp-1, __dmul_rn(x, 0x1.08b2fb1366eaap-56));
+}
+
 // ph-2p2h coupling value of single (a,k) with double r (adc_ph.f90:974-1073),
 // in the argument mapping of get_matrix.f90:900,931,964,997,1030.
 __device__ inline double coupling(const Eri& E, int a, int k, const Double& r) {
@@ -369,42 +397,68 @@ __device__ inline double coupling(const Eri& E, int a, int k, const Double& r) {
       if (a == bp) f = f - (E.OOOV(kp, k, lp, ap) + E.OOOV(lp, k, kp, ap));
       if (k == kp) f = f + (E.VVOV(a, ap, lp, bp) + E.VVOV(a, bp, lp, ap));
       if (k == lp) f = f + (E.VVOV(a, ap, kp, bp) + E.VVOV(a, bp, kp, ap));
-      return f / sqrt(2.0);
+      return div_sqrt2(f);
     default:  // C2_ph_2p2h(a,k,a',b',k',l')
       if (a == ap) f = f - (E.OOOV(kp, k, lp, bp) - E.OOOV(lp, k, kp, bp));
       if (a == bp) f = f + (E.OOOV(kp, k, lp, ap) - E.OOOV(lp, k, kp, ap));
       if (k == kp) f = f + (E.VVOV(a, ap, lp, bp) - E.VVOV(a, bp, lp, ap));
       if (k == lp) f = f - (E.VVOV(a, ap, kp, bp) - E.VVOV(a, bp, kp, ap));
-      return sqrt(3.0) * f / sqrt(2.0);
+      return div_sqrt2(sqrt(3.0) * f);
   }
 }
 
 // One warp per stored row of B^T: evaluates its structural entries, applies
 // the minc threshold (get_matrix.f90:904 etc.), zeroes the padding and counts
-// the kept entries.
+// the kept entries.  The C and D entries (a outside {a', b'}, one coincidence)
+// are the terms of coupling() that remain, operation by operation, with the
+// lanes along the innermost index of the integrals; the few A and B entries go
+// through coupling().  (Every entry through coupling() with gathered integrals
+// and FP64 divisions: 3.4 ms at nocc=10/nvirt=110.)
 // Rows [row_begin, row_end) of the store; Bt holds the values from the
 // value offset vbase on (the whole store: vbase = 0; one chunk of the direct
 // path: vbase = the chunk's first value).  rowcount may be null.
-__global__ void k_coupling(Eri E, GeomDev g, double* __restrict__ Bt, int64_t vbase, int64_t row_begin,
-                           int64_t row_end, int64_t* __restrict__ rowcount) {
+__global__ void __launch_bounds__(256) k_coupling(Eri E, GeomDev g, double* __restrict__ Bt, int64_t vbase,
+                                                  int64_t row_begin, int64_t row_end, int64_t* __restrict__ rowcount) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int no = g.no, nv = g.nv, noP = g.noP, nvP = g.nvP;
+  const long long minc = __double_as_longlong(MINC);
   for (int64_t row_i = row_begin + warp; row_i < row_end; row_i += nwarps) {
-    Double r = decode_row(g, row_i);
-    const int64_t L = g.len[r.cls];
-    double* row = Bt + (g.off[r.cls] + (row_i - g.start[r.cls]) * L - vbase);
+    const Double r = decode_row(g, row_i);
+    const bool twoa = r.cls == 1 || r.cls >= 3, two = r.cls >= 2;
+    double* row = Bt + (g.off[r.cls] + (row_i - g.start[r.cls]) * g.len[r.cls] - vbase);
     int cnt = 0;
-    for (int e = lane; e < L; e += 32) {
-      int64_t s = entry_single(g, r, e);
-      double x = 0.0;
-      if (s >= 0) {
-        int a = (int)(s / g.no), k = (int)(s % g.no);
-        x = coupling(E, a, k, r);
-      }
-      bool keep = s >= 0 && fabs(x) > MINC;
-      row[e] = keep ? x : 0.0;
+    auto put = [&](double* at, double x) {
+      const long long ax = __double_as_longlong(x) & 0x7fffffffffffffffll;
+      const bool keep = ax > minc && ax <= 0x7ff0000000000000ll;   // fabs(x) > minc (false for NaN)
+      *at = keep ? x : 0.0;
       cnt += keep;
+    };
+    for (int e = lane; e < (twoa ? 2 : 1) * noP; e += 32) {
+      const int seg = e >= noP ? 1 : 0, k = e - seg * noP;
+      put(row + e, k < no ? coupling(E, seg ? r.bp : r.ap, k, r) : 0.0);
+    }
+    double* rc = row + (twoa ? 2 : 1) * noP;
+    for (int seg = 0; seg < (two ? 2 : 1); ++seg, rc += nvP) {
+      const int h = two && seg == 0 ? r.lp : r.kp;         // the hole that is not the single's
+      // (a a'|h b') and (a b'|h a') along a
+      const double* v1 = E.vvov + (((int64_t)r.ap * no + h) * nv + r.bp) * nv;
+      const double* v2 = E.vvov + (((int64_t)r.bp * no + h) * nv + r.ap) * nv;
+      for (int a = lane; a < nvP; a += 32) {
+        double x = 0.0;
+        if (a < nv && a != r.ap && a != r.bp) {
+          const double p = v1[a], q = twoa ? v2[a] : 0.0;
+          switch (r.cls) {
+            case 0: x = sqrt(2.0) * -p; break;
+            case 1: x = -(p + q); break;
+            case 2: x = p; break;
+            case 3: x = div_sqrt2(p + q); break;
+            default: x = div_sqrt2(sqrt(3.0) * (seg ? -(p - q) : p - q)); break;
+          }
+        }
+        put(rc + a, x);
+      }
     }
     for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0 && rowcount) rowcount[row_i] = cnt;
@@ -614,8 +668,18 @@ int build_eri_blocks_from_packed(Ctx* c, const double* d_packed) {
     if (*dst[k]) { dfree(c, *dst[k], 0); *dst[k] = nullptr; }
     int st = dmalloc(c, (void**)dst[k], sizeof(double) * sz[k]);
     if (st) return st;
-    k_gather_block<<<grid_for(c, sz[k], 256), 256, 0, c->stream>>>(d_packed, *dst[k], k, no, nv, sz[k]); ADC_COUNT_LAUNCH();
+    // (vv|ov): gathered as [a][b][i][c], then brought into the stored order
+    double* to = *dst[k];
+    if (k == 3 && (st = dmalloc(c, (void**)&to, sizeof(double) * sz[k]))) return st;
+    k_gather_block<<<grid_for(c, sz[k], 256), 256, 0, c->stream>>>(d_packed, to, k, no, nv, sz[k]); ADC_COUNT_LAUNCH();
     ADC_CUDA(c, cudaGetLastError());
+    if (k == 3) {
+      k_vvov_layout<<<dim3((no * nv + 31) / 32, (nv + 31) / 32, nv), 256, 0, c->stream>>>(to, *dst[k], no, nv);
+      ADC_COUNT_LAUNCH();
+      ADC_CUDA(c, cudaGetLastError());
+      ADC_CUDA(c, cudaStreamSynchronize(c->stream));
+      dfree(c, to);
+    }
   }
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
   return ADCGPU_OK;
@@ -637,35 +701,84 @@ int coupling_values(Ctx* c, double* buf, int64_t vbase, int64_t row0, int64_t ro
   return ADCGPU_OK;
 }
 
-// CB_ph_ph for all k <= k1 (two passes: k_cb_terms + k_cb_sum; pairs in
-// batches that keep the term buffer near 1 GiB)
-static int compute_cb(Ctx* c, const Eri& E, double* d_cb) {
-  const int no = E.no, nv = E.nv;
-  const int64_t nt = (int64_t)nv * nv * no;
-  std::vector<int2> pairs;
-  for (int k = 0; k < no; ++k)
-    for (int k1 = k; k1 < no; ++k1) pairs.push_back(make_int2(k, k1));
-  const int np = (int)pairs.size();
-  const int batch = (int)std::max<int64_t>(1, std::min<int64_t>(np, ((int64_t)1 << 27) / nt));
+namespace {
+
+// CA and CB on two streams: CB's few long sums (nvirt^2 nocc terms each) are
+// bound by their addition chains on a couple of SMs, so they run beside CA
+// and whatever the caller queues on the context's stream before join().
+struct SecondOrder {
+  Ctx* c;
+  double *d_terms_a = nullptr, *d_terms_b = nullptr;
   int2* d_pairs = nullptr;
-  double* d_terms = nullptr;
-  int st = dmalloc(c, (void**)&d_pairs, sizeof(int2) * np);
-  if (!st) st = dmalloc(c, (void**)&d_terms, sizeof(double) * (size_t)batch * nt);
-  if (!st && cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(int2) * np, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
-    st = set_err(c, ADCGPU_CUDA_ERROR, "CB pairs");
-  for (int p0 = 0; !st && p0 < np; p0 += batch) {
-    const int nb = std::min(batch, np - p0);
-    k_cb_terms<<<grid_for(c, (int64_t)nb * nt, 256), 256, 0, c->stream>>>(E, c->d_e, d_pairs + p0, nb, d_terms);
-    ADC_COUNT_LAUNCH();
-    k_cb_sum<<<(nb + 31) / 32, 32, 0, c->stream>>>(d_terms, d_pairs + p0, nb, nt, no, d_cb);
-    ADC_COUNT_LAUNCH();
-    if (cudaGetLastError() != cudaSuccess) st = set_err(c, ADCGPU_CUDA_ERROR, "CB kernels");
+  cudaStream_t side = nullptr;
+  cudaEvent_t ready = nullptr, done = nullptr;
+  explicit SecondOrder(Ctx* c_) : c(c_) {}
+  ~SecondOrder() {
+    if (side) {
+      cudaStreamSynchronize(side);   // the buffers' last readers
+      cudaStreamSynchronize(c->stream);
+      cudaStreamDestroy(side);
+    }
+    if (ready) cudaEventDestroy(ready);
+    if (done) cudaEventDestroy(done);
+    dfree(c, d_terms_a);
+    dfree(c, d_terms_b);
+    dfree(c, d_pairs);
   }
-  if (!st && cudaStreamSynchronize(c->stream) != cudaSuccess) st = set_err(c, ADCGPU_CUDA_ERROR, "CB kernels");
-  dfree(c, d_terms);
-  dfree(c, d_pairs);
-  return st;
-}
+  // d_ca (nv x nv) is complete on the context's stream, d_cb (no x no) after join()
+  int launch(const Eri& E, double* d_ca, double* d_cb) {
+    const int no = E.no, nv = E.nv;
+    const int64_t nta = (int64_t)nv * no * no, ntb = (int64_t)nv * nv * no;
+    std::vector<int2> pairs;
+    for (int a = 0; a < nv; ++a)
+      for (int a1 = a; a1 < nv; ++a1) pairs.push_back(make_int2(a, a1));
+    const int na = (int)pairs.size();
+    for (int k = 0; k < no; ++k)
+      for (int k1 = k; k1 < no; ++k1) pairs.push_back(make_int2(k, k1));
+    const int nb = (int)pairs.size() - na;
+    // batches of sums: term buffers near 1 GiB (a quarter on the direct path)
+    const int64_t budget = (int64_t)1 << (c->direct ? 25 : 27);
+    const int ba = (int)std::max<int64_t>(1, std::min<int64_t>(na, budget / nta));
+    const int bb = (int)std::max<int64_t>(1, std::min<int64_t>(nb, budget / ntb));
+    ST(dmalloc(c, (void**)&d_pairs, sizeof(int2) * pairs.size()));
+    ST(dmalloc(c, (void**)&d_terms_a, sizeof(double) * (size_t)ba * nta));
+    ST(dmalloc(c, (void**)&d_terms_b, sizeof(double) * (size_t)bb * ntb));
+    ADC_CUDA(c, cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    ADC_CUDA(c, cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+    ADC_CUDA(c, cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    ADC_CUDA(c, h2d(c, d_pairs, pairs.data(), sizeof(int2) * pairs.size()));
+    ADC_CUDA(c, cudaEventRecord(ready, c->stream));
+    ADC_CUDA(c, cudaStreamWaitEvent(side, ready, 0));
+    const double factor = c->direct ? 0.5 : -0.5;
+    for (int p0 = 0; p0 < nb; p0 += bb) {
+      const int n = std::min(bb, nb - p0);
+      const int2* pp = d_pairs + na + p0;
+      if (c->direct) k_cb_terms<true><<<grid_for(c, n * ntb, 256), 256, 0, side>>>(E, c->d_e, pp, n, d_terms_b);
+      else k_cb_terms<false><<<grid_for(c, n * ntb, 256), 256, 0, side>>>(E, c->d_e, pp, n, d_terms_b);
+      ADC_COUNT_LAUNCH();
+      k_ordered_sum<<<(n + 31) / 32, 128, 0, side>>>(d_terms_b, pp, n, ntb, no, factor, d_cb);
+      ADC_COUNT_LAUNCH();
+    }
+    for (int p0 = 0; p0 < na; p0 += ba) {
+      const int n = std::min(ba, na - p0);
+      const int2* pp = d_pairs + p0;
+      if (c->direct) k_ca_terms<true><<<grid_for(c, n * nta, 256), 256, 0, c->stream>>>(E, c->d_e, pp, n, d_terms_a);
+      else k_ca_terms<false><<<grid_for(c, n * nta, 256), 256, 0, c->stream>>>(E, c->d_e, pp, n, d_terms_a);
+      ADC_COUNT_LAUNCH();
+      k_ordered_sum<<<(n + 31) / 32, 128, 0, c->stream>>>(d_terms_a, pp, n, nta, nv, factor, d_ca);
+      ADC_COUNT_LAUNCH();
+    }
+    ADC_CUDA(c, cudaGetLastError());
+    ADC_CUDA(c, cudaEventRecord(done, side));
+    return ADCGPU_OK;
+  }
+  int join() {
+    ADC_CUDA(c, cudaStreamWaitEvent(c->stream, done, 0));
+    return ADCGPU_OK;
+  }
+};
+
+}  // namespace
 
 int build_matrix(Ctx* c) {
   const Geometry& G = c->geom;
@@ -696,25 +809,15 @@ int build_matrix(Ctx* c) {
   if (!c->d_rowcount && (st = dmalloc(c, (void**)&c->d_rowcount, sizeof(int64_t) * (G.n2 + n1 + 1))))
     return st;
 
-  dim3 tiles((unsigned)((n1 + PT - 1) / PT), (unsigned)((n1 + PT - 1) / PT));
-  if (c->direct) {
-    // the direct path's formulas (get_interm_adc2_save, hiivec, get_matvec_adc2s_omp)
-    k_ca1<<<(int)((nv * (int64_t)nv + 127) / 128), 128, 0, s>>>(E, c->d_e, d_ca); ADC_COUNT_LAUNCH();
-    k_cb1<<<(no * no + 63) / 64, 64, 0, s>>>(E, c->d_e, d_cb); ADC_COUNT_LAUNCH();
-    k_cc_tables<true><<<grid_for(c, n1 * n1, 256), 256, 0, s>>>(E, c->d_e, d_X, d_D1); ADC_COUNT_LAUNCH();
-    ADC_CUDA(c, cudaGetLastError());
-    k_phph<true><<<tiles, dim3(PT, PT), 0, s>>>(E, c->d_e, d_X, d_D1, d_ca, d_cb, c->d_A, c->d_diag, d_kept);
-    ADC_COUNT_LAUNCH();
-  } else {
-    k_ca<<<(int)((nv * (int64_t)nv + 127) / 128), 128, 0, s>>>(E, c->d_e, d_ca); ADC_COUNT_LAUNCH();
-    ST(compute_cb(c, E, d_cb));
-    k_cc_tables<false><<<grid_for(c, n1 * n1, 256), 256, 0, s>>>(E, c->d_e, d_X, d_D1); ADC_COUNT_LAUNCH();
-    ADC_CUDA(c, cudaGetLastError());
-    k_phph<false><<<tiles, dim3(PT, PT), 0, s>>>(E, c->d_e, d_X, d_D1, d_ca, d_cb, c->d_A, c->d_diag, d_kept);
-    ADC_COUNT_LAUNCH();
-  }
-  ADC_CUDA(c, cudaGetLastError());
+  const dim3 tiles((unsigned)((n1 + PT - 1) / PT), (unsigned)((n1 + PT - 1) / PT));
+  SecondOrder so(c);
+  ST(so.launch(E, d_ca, d_cb));
+  // what does not need CB, while its sums run
+  if (c->direct) k_cc_tables<true><<<grid_for(c, n1 * n1, 256), 256, 0, s>>>(E, c->d_e, d_X, d_D1);
+  else k_cc_tables<false><<<grid_for(c, n1 * n1, 256), 256, 0, s>>>(E, c->d_e, d_X, d_D1);
+  ADC_COUNT_LAUNCH();
   k_diag2<<<grid_for(c, G.n2, 256), 256, 0, s>>>(g, c->d_e, c->d_diag); ADC_COUNT_LAUNCH();
+  ADC_CUDA(c, cudaGetLastError());
   if (c->direct) {
     // the kept count (noffd) from one pass over the chunks; no values stay
     for (const DirectChunk& dc : c->dchunks)
@@ -722,6 +825,11 @@ int build_matrix(Ctx* c) {
   } else {
     ST(coupling_values(c, c->d_Bt, 0, 0, G.n2, c->d_rowcount + n1));
   }
+  ST(so.join());
+  // the direct path's formulas: get_interm_adc2_save, hiivec, get_matvec_adc2s_omp
+  if (c->direct) k_phph<true><<<tiles, dim3(PT, PT), 0, s>>>(E, c->d_e, d_X, d_D1, d_ca, d_cb, c->d_A, c->d_diag, d_kept);
+  else k_phph<false><<<tiles, dim3(PT, PT), 0, s>>>(E, c->d_e, d_X, d_D1, d_ca, d_cb, c->d_A, c->d_diag, d_kept);
+  ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   unsigned long long kept_ph = 0;
   ADC_CUDA(c, cudaMemcpyAsync(&kept_ph, d_kept, sizeof(kept_ph), cudaMemcpyDeviceToHost, s));
@@ -828,9 +936,10 @@ int build_matrix_cvs(Ctx* c, const int32_t* kpq, int64_t ndim, int ncore, const 
     ADC_CUDA(c, cudaMemcpyAsync(d_coreorb, coreorb.data(), sizeof(int) * ncore, cudaMemcpyHostToDevice, s));
     if (n2 > 0)
       ADC_CUDA(c, cudaMemcpyAsync(d_cols, kpq + 7 * (cn1 + 1), sizeof(int32_t) * 7 * n2, cudaMemcpyHostToDevice, s));
-    k_ca<<<(int)((nv * (int64_t)nv + 127) / 128), 128, 0, s>>>(E, c->d_e, d_ca); ADC_COUNT_LAUNCH();
-    ST(compute_cb(c, E, d_cb));
+    SecondOrder so(c);
+    ST(so.launch(E, d_ca, d_cb));
     k_cc_tables<false><<<grid_for(c, n1 * n1, 256), 256, 0, s>>>(E, c->d_e, d_X, d_D1); ADC_COUNT_LAUNCH();
+    ST(so.join());
     k_phph_cvs<<<grid_for(c, (int64_t)cn1 * cn1, 128), 128, 0, s>>>(E, c->d_e, d_X, d_D1, d_ca, d_cb, d_sidx, cn1,
                                                                      c->d_Ac, c->d_diag, d_kept);
     ADC_COUNT_LAUNCH();

@@ -68,7 +68,9 @@ const std::vector<int64_t>& diag_order(Ctx* c) {
 }
 
 static void free_matrix(Ctx* c) {
+  c->diag_order_stop = true;
   join_diag_order(c);
+  c->diag_order_stop = false;
   c->diag_order.clear();
   void** ps[] = {(void**)&c->d_diag, (void**)&c->d_A, (void**)&c->d_Bt, (void**)&c->d_A32, (void**)&c->d_Bt16,
                  (void**)&c->d_Bt32, (void**)&c->d_diag32, (void**)&c->d_rowcount, &c->d_ws,
@@ -242,7 +244,7 @@ int adcgpu_set_eri_mo_complex(adcgpu_ctx* h, const double* buf) {
                   p = no + a; q = no + b; r = i; s = j; } break;
         case 2: { int64_t a = x % nv; x /= nv; int64_t kk = x % no; x /= no; int64_t j = x % no; int64_t i = x / no;
                   p = i; q = j; r = kk; s = no + a; } break;
-        default: { int64_t cc = x % nv; x /= nv; int64_t i = x % no; x /= no; int64_t b = x % nv; int64_t a = x / nv;
+        default: { int64_t a = x % nv; x /= nv; int64_t cc = x % nv; x /= nv; int64_t i = x % no; int64_t b = x / no;
                    p = no + a; q = no + b; r = i; s = no + cc; } break;
       }
       hb[t] = V(p, q, r, s);
@@ -290,7 +292,7 @@ int adcgpu_build_adc2s(adcgpu_ctx* h, int ndim, const int32_t* kpq, int64_t* nof
     ADC_CUDA(c, d2h(c, ah.data(), c->d_diag, sizeof(double) * ah.size()));
     c->diag_order_thread = std::thread([c, ah = std::move(ah)]() mutable {
       for (double& x : ah) x = std::fabs(x);
-      host_heapsort_index((int64_t)ah.size(), ah.data(), c->diag_order);
+      host_heapsort_index((int64_t)ah.size(), ah.data(), c->diag_order, &c->diag_order_stop);
     });
   }
   c->flag = flag;
@@ -372,7 +374,7 @@ int adcgpu_build_adc2s_cvs(adcgpu_ctx* h, int ndim, const int32_t* kpq, int ncor
     ADC_CUDA(c, d2h(c, ah.data(), c->d_diag, sizeof(double) * ah.size()));
     c->diag_order_thread = std::thread([c, ah = std::move(ah)]() mutable {
       for (double& x : ah) x = std::fabs(x);
-      host_heapsort_index((int64_t)ah.size(), ah.data(), c->diag_order);
+      host_heapsort_index((int64_t)ah.size(), ah.data(), c->diag_order, &c->diag_order_stop);
     });
   }
   c->flag = flag;

@@ -320,10 +320,10 @@ __global__ void __launch_bounds__(256) k_fv_tau_vo(int mode, int no, int nv, con
     double g;
     const double* arow;
     if (mode == 0) {
-      g = 2.0 * vvov[(((int64_t)v * nv + c) * no + l) * nv + b] - vvov[(((int64_t)v * nv + b) * no + l) * nv + c];
+      g = 2.0 * vvov[(((int64_t)v * no + l) * nv + b) * nv + c] - vvov[(((int64_t)v * no + l) * nv + c) * nv + b];
       arow = A1 + ((int64_t)b * no + l) * n1 + (int64_t)c * no;
     } else {
-      g = 2.0 * vvov[(((int64_t)v * nv + b) * no + l) * nv + c] - vvov[(((int64_t)v * nv + c) * no + l) * nv + b];
+      g = 2.0 * vvov[(((int64_t)v * no + l) * nv + c) * nv + b] - vvov[(((int64_t)v * no + l) * nv + b) * nv + c];
       arow = A1 + ((int64_t)c * no + l) * n1 + (int64_t)b * no;
     }
 #pragma unroll

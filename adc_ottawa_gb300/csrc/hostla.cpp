@@ -259,7 +259,7 @@ void host_triu_inverse(int n, const double* R, double* Ri) {
 // Numerical Recipes heapsort of an index array, ascending (dsortindxa1 'A').
 // The order of equal keys is that of the heap construction, as in the
 // reference, because the Davidson guess vectors are taken from it.
-void host_heapsort_index(int64_t n, const double* arrin, std::vector<int64_t>& indx) {
+void host_heapsort_index(int64_t n, const double* arrin, std::vector<int64_t>& indx, const std::atomic<bool>* stop) {
   // The keys travel with their indices (one array of pairs), so a sift step
   // reads one location instead of an index and then its key; comparisons and
   // moves are those of the index-array formulation, so the permutation, and
@@ -273,6 +273,7 @@ void host_heapsort_index(int64_t n, const double* arrin, std::vector<int64_t>& i
   int64_t l = n / 2 + 1, ir = n, i, j;
   KI t;
   for (;;) {
+    if (stop && ((l + ir) & 1023) == 0 && stop->load(std::memory_order_relaxed)) { indx.clear(); return; }
     if (l > 1) {
       l = l - 1;
       t = h[l - 1];
@@ -291,6 +292,10 @@ void host_heapsort_index(int64_t n, const double* arrin, std::vector<int64_t>& i
     h[i - 1] = t;
   }
   for (int64_t k = 0; k < n; ++k) indx[k] = h[k].idx;
+}
+
+void host_heapsort_index(int64_t n, const double* arr, std::vector<int64_t>& indx) {
+  host_heapsort_index(n, arr, indx, nullptr);
 }
 
 }  // namespace adcgpu

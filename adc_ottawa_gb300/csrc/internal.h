@@ -262,7 +262,7 @@ struct Ctx {
   double* d_vovo = nullptr;       // (a i|b j) [nv][no][nv][no]
   double* d_vvoo = nullptr;       // (a b|i j) [nv][nv][no][no]
   double* d_ooov = nullptr;       // (i j|k a) [no][no][no][nv]
-  double* d_vvov = nullptr;       // (a b|i c) [nv][nv][no][nv]
+  double* d_vvov = nullptr;       // (a b|i c) [b][i][c][a]
   double* d_oooo = nullptr;       // (i j|k l) [no][no][no][no]
   double* d_vvvv = nullptr;       // (a c|b d) over virtual pairs: [tri(pair(a,c), pair(b,d))]
   double* d_dpl = nullptr;        // dipole matrix dpl(p,q) [nbas][nbas] (q-major), adcgpu_set_dipole
@@ -283,6 +283,7 @@ struct Ctx {
   // end of the matrix build, joined by the first solve that needs it
   std::vector<int64_t> diag_order;
   std::thread diag_order_thread;
+  std::atomic<bool> diag_order_stop{false};   // the matrix goes before a solve needed the order
   int64_t nnz_kept = 0;           // reference noffd
   int64_t nnz_ph = 0;             // kept ph-ph entries
   int64_t* d_rowcount = nullptr;  // kept entries per double row (for COO export)
@@ -485,5 +486,8 @@ int host_cholesky_upper(int n, const double* G, double* R, double rel_tol);
 void host_triu_inverse(int n, const double* R, double* Rinv);
 // NR heapsort index (dsortindxa1 'A', misc.f90:492+); indx 1-based.
 void host_heapsort_index(int64_t n, const double* arr, std::vector<int64_t>& indx);
+// stop (may be null): another thread sets it when the result is not wanted
+// any more; the sort then ends early with an empty indx.
+void host_heapsort_index(int64_t n, const double* arr, std::vector<int64_t>& indx, const std::atomic<bool>* stop);
 
 }  // namespace adcgpu
