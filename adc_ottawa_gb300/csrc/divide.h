@@ -2,12 +2,12 @@
 // per cycle and SM, and a division is about nine of them).
 //
 // Schoolbook: a quotient estimate from single-precision arithmetic (within a
-// few hundred units of the last place), its exact remainder from 64-bit
-// integers, a small integer correction, round to nearest even from the
-// remainder.  Every step after the estimate is exact, so the result does not
-// depend on the accuracy of the reciprocal (an estimate within 1.5 2^-23
-// relative keeps the remainder in 63 bits; rcp.approx is documented to 2^-23); tests/test_divide.py
-// compares it with the host's division.
+// hundred units of the last place), its exact remainder from 64-bit integers, a
+// small integer correction, round to nearest even from the remainder.  Every
+// step after the estimate is exact, so the result does not depend on the
+// accuracy of the hardware's reciprocal: any within 2^-21 relative keeps the
+// remainder inside 63 bits (rcp.approx is documented to 2^-23).
+// tests/test_divide.py compares it with the host's division.
 #pragma once
 
 #include <math.h>
@@ -76,7 +76,8 @@ ADC_DIV_FN double div_rn(double n, double d, float host_error = 0.0f) {
   float nl = (float)(int32_t)((uint32_t)mn & 0x1fffffffu) * 0x1p-52f;
   const int lt = mn < md;               // quotient of the mantissas into [1, 2)
   if (lt) { mn <<= 1; nh += nh; nl += nl; }
-  const float y = div_rcp(dh, host_error);
+  float y = div_rcp(dh, host_error);
+  y = fmaf(y, fmaf(-dl, y, fmaf(-dh, y, 1.0f)), y);   // of d, to about 2^-23
   const float q1 = nh * y;
   const float r1 = fmaf(-q1, dh, nh) + fmaf(-q1, dl, nl);
   const float q2 = r1 * y;

@@ -1,6 +1,6 @@
 // Compares adc_ottawa_gb300/csrc/divide.h with the host's division (compiled
 // and run by tests/test_divide.py): argv[1] random operand pairs of several
-// kinds, each with a reciprocal estimate off by up to +-1.5 2^-23.  Prints the
+// kinds, each with a reciprocal estimate off by up to +-2^-21.  Prints the
 // number of differing bit patterns.
 #include <cstdint>
 #include <cstdio>
@@ -36,12 +36,12 @@ int main(int argc, char** argv) {
       const double q = adcgpu::div_double((1023ull << 52) | (next() & frac));
       const long double m = (long double)q + 0x1p-53L;
       const double xx = (double)(m * (long double)y);
-      const double e = ((float)(int)(next() % 3) - 1.0f) * 0x1.8p-23f;
+      const double e = ((float)(int)(next() % 3) - 1.0f) * 0x1p-21f;
       const double z = xx / y, w = adcgpu::div_rn(xx, y, (float)e);
       bad += adcgpu::div_bits(z) != adcgpu::div_bits(w);
       continue;
     }
-    const float err = ((float)(next() % 2001) - 1000.0f) * (0x1.8p-23f / 1000.0f);
+    const float err = ((float)(next() % 2001) - 1000.0f) * (0x1p-21f / 1000.0f);
     const double z = x / y, w = adcgpu::div_rn(x, y, err);
     if (z != z) { bad += w == w; continue; }
     bad += adcgpu::div_bits(z) != adcgpu::div_bits(w);
