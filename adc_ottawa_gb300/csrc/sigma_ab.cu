@@ -1,6 +1,7 @@
 // Segments A and B of the coupling block (the singles (a', k) and (b', k) of
-// a double (a', b', k', l'); layout in internal.h) in compact form, for the
-// mixed-precision sigma product.  Replaces the per-(slab, b') pass 2 and the
+// a double (a', b', k', l'); layout in internal.h) for the mixed-precision
+// sigma product: BF16 values by mma.sync runs (k_seg_bf16), FP32 values beside
+// the CUDA-core tile or the two-pass tcgen05 product in compact form.  Replaces the per-(slab, b') pass 2 and the
 // per-run pass 3 of sigma.cu on the BF16 tensor-core path and the FP32-value
 // tiled path; the product is that of hxvec_incore (block_davidson.f90:
 // 844-883) restricted to these entries.
@@ -284,16 +285,228 @@ __global__ void __launch_bounds__(256) k_ab_pairs(GeomDev g, const float* __rest
   }
 }
 
+// ---------------------------------------------------------------------------
+// BF16 values: the pair-class rows' segments on mma.sync.  A run (the rows of
+// one slab with equal a', segment A, or equal b', segment B) couples to the
+// singles (f, k) of its fixed virtual f:
+//   W2[r, c] += sum_k R[r, k] V[(f, k), c],   W1[(f, k), c] += sum_r R[r, k] V2[r, c]
+// A block takes eight consecutive f (one warp and run each) and 16 columns, 16
+// rows of every run a step: their V2 and W2 entries, contiguous along a' or b'
+// for the block but not for one run, move through shared memory (with a warp
+// on its own, each 4-byte access of segment B was a sector of its own: 2.4 ms
+// instead of 1.0).  The values come by cp.async, the next V2 and this step's
+// W2 are loaded a step ahead.  The values are BF16 already; a vector entry is
+// three BF16 slices, which hold its 24 bits, so the products are those of the
+// FP32 vectors.  A step's sums (48 products an entry) come from one FP32
+// accumulator chain, lowest slice first, and are added to the run's in FP32.
+// Bound by the latency of its loads: 0.93 ms (A) and 0.96 ms (B) for 40 columns
+// at nocc=16/nvirt=180, where the per-thread compact kernel above took 3.06 ms.
+// ---------------------------------------------------------------------------
+// segments of the pair-class rows, packed: [pair row][A, B][kw]
+__global__ void k_seg_pack(GeomDev g, const __nv_bfloat16* __restrict__ Bt, int kw, __nv_bfloat16* __restrict__ out) {
+  const int64_t c2 = g.start[2] - g.start[1], n = (c2 + (g.start[5] - g.start[3])) * 2 * kw;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = i / (2 * kw);
+    const int x = (int)(i - t * (2 * kw)), seg = x >= kw ? 1 : 0, k = x - seg * kw;
+    const int64_t row = t < c2 ? g.start[1] + t : g.start[3] + (t - c2);
+    const int cls = t < c2 ? 1 : (row < g.start[4] ? 3 : 4);
+    out[i] = k < g.no ? Bt[g.off[cls] + (row - g.start[cls]) * g.len[cls] + seg * g.noP + k] : __float2bfloat16(0.f);
+  }
+}
+
+__device__ __forceinline__ void seg_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// three BF16 slices of a pair of FP32 values (x = s0 + s1 + s2 to 24 bits)
+__device__ __forceinline__ void seg_split(float x, float y, uint32_t (&s)[3]) {
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    s[t] = *reinterpret_cast<const uint32_t*>(&h);
+    x -= __low2float(h);
+    y -= __high2float(h);
+  }
+}
+// A fragments of m16n8k16: rows (columns c) lane / 4 and + 8, positions
+// 2 (lane % 4), + 1, + 8, + 9
+__device__ __forceinline__ void seg_frag(const float (&x)[2][4], uint32_t (&f)[3][4]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      uint32_t s[3];
+      seg_split(x[h][2 * v], x[h][2 * v + 1], s);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) f[t][2 * v + h] = s[t];
+    }
+}
+
+constexpr int SEG_F = 8;
+template <int KT, bool SEGB>
+__global__ void __launch_bounds__(32 * SEG_F)
+    k_seg_bf16(GeomDev g, int nslab, int ngrp, const __nv_bfloat16* __restrict__ seg, const float* __restrict__ V,
+                 int64_t ldv, int m, float* __restrict__ W, int64_t ldw, double* __restrict__ W1, int64_t ld1) {
+  constexpr int PITCH = KT * 32 + 16, KW = 16 * KT, NPIECE = 32 * KT;
+  constexpr int PA = SEG_F + 1, PC = 16 * PA + 1;        // pitches of a' and c in the tiles
+  __shared__ __align__(16) unsigned char smem_seg[SEG_F * 2 * 16 * PITCH];
+  __shared__ float sV[16 * PC], sW[16 * PC];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int gid = lane >> 2, tig = lane & 3;
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem_seg + wid * 2 * 16 * PITCH);
+  const int no = g.no, nv = g.nv;
+  const int64_t n1 = g.n1;
+  const int pos[4] = {2 * tig, 2 * tig + 1, 2 * tig + 8, 2 * tig + 9};
+  // this thread's part of a tile: fixed virtual f0 + tb, the other o0 + ta,
+  // columns tc + 2 j; consecutive threads along b'
+  const int tb = SEGB ? tid & 7 : (tid >> 4) & 7, ta = SEGB ? (tid >> 3) & 15 : tid & 15, tc = tid >> 7;
+  const int nfb = (nv - 1 + SEG_F - 1) / SEG_F;
+  const int64_t nblk = (int64_t)nslab * ngrp * nfb;
+  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+    const int f0 = (SEGB ? 1 : 0) + SEG_F * (int)(blk % nfb);
+    const int64_t sg = blk / nfb;
+    const int c0 = (int)(sg % ngrp) * 16;
+    const PairSlab ps = pair_slab(g, (int)(sg / ngrp));
+    // this warp's run: f with every a' < f (SEGB), or every b' > f
+    const int f = f0 + wid;
+    const int obeg = SEGB ? 0 : f0 + 1, oend = SEGB ? min(f0 + SEG_F - 1, nv - 1) : nv;
+    auto valid = [&](int fx, int o) { return SEGB ? fx < nv && o < fx : fx < nv - 1 && o > fx && o < nv; };
+    auto pair_of = [&](int fx, int o) -> int64_t { return SEGB ? pair_index(o, fx, nv) : pair_index(fx, o, nv); };
+    const int dstr = ps.cls == 1 ? no : 1;
+    const int64_t dbase = n1 + (ps.cls == 1 ? g.start[1] + ps.kp : ps.row0);
+    const __nv_bfloat16* sv = seg + (pair_row_index(g, ps.cls, ps.row0) * 2 + (SEGB ? 1 : 0)) * KW;
+    auto issue = [&](int o0, int b) {
+      for (int p = lane; p < NPIECE; p += 32) {
+        const int rr = p / (2 * KT), w = p - rr * (2 * KT);
+        const bool ok = valid(f, o0 + rr);
+        const __nv_bfloat16* src = sv + (ok ? pair_of(f, o0 + rr) : 0) * 2 * KW + 8 * w;
+        const int n = ok ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sbase + (uint32_t)((b * 16 + rr) * PITCH + 16 * w)),
+                     "l"(src), "r"(n));
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+    };
+    issue(obeg, 0);
+    float v[8], w[8];
+    auto load_v = [&](int o0) {
+      const bool ok = valid(f0 + tb, o0 + ta);
+      const int64_t d = dbase + (ok ? pair_of(f0 + tb, o0 + ta) : 0) * dstr;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c = c0 + tc + 2 * j;
+        v[j] = ok && c < m ? __ldg(V + (int64_t)c * ldv + d) : 0.f;
+      }
+    };
+    load_v(obeg);
+    uint32_t xf[KT][3][4];
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt) {
+      float xk[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int k = 16 * kt + pos[u], c = c0 + gid + 8 * h;
+          xk[h][u] = (f < nv && k < no && c < m) ? __ldg(V + (int64_t)c * ldv + (int64_t)f * no + k) : 0.f;
+        }
+      seg_frag(xk, xf[kt]);
+    }
+    float a1[2 * KT][4];
+#pragma unroll
+    for (int n = 0; n < 2 * KT; ++n) a1[n][0] = a1[n][1] = a1[n][2] = a1[n][3] = 0.f;
+    int b = 0;
+    for (int o0 = obeg; o0 < oend; o0 += 16, b ^= 1) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sV[(tc + 2 * j) * PC + ta * PA + tb] = v[j];
+      if (o0 + 16 < oend) issue(o0 + 16, b ^ 1);
+      else asm volatile("cp.async.commit_group;\n" ::);
+      __syncthreads();
+      // this step's W2 and the next step's V2, ahead of their use
+      const bool wok = valid(f0 + tb, o0 + ta);
+      const int64_t wd = dbase + (wok ? pair_of(f0 + tb, o0 + ta) : 0) * dstr;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c = c0 + tc + 2 * j;
+        w[j] = wok && c < m ? W[(int64_t)c * ldw + wd] : 0.f;
+      }
+      if (o0 + 16 < oend) load_v(o0 + 16);
+      float x[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[h][u] = sV[(gid + 8 * h) * PC + pos[u] * PA + wid];
+      uint32_t vf[3][4];
+      seg_frag(x, vf);
+      asm volatile("cp.async.wait_group 1;\n" ::);
+      __syncwarp();
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt) {
+        uint32_t q[4];
+        const uint32_t at = sbase + (uint32_t)((b * 16 + (lane & 15)) * PITCH + (lane >> 4) * 16 + kt * 32);
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(at));
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int t = 2; t >= 0; --t) seg_mma(s, vf[t], q[2 * n], q[2 * n + 1]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a1[2 * kt + n][i] += s[i];
+        }
+      }
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t q[2 * KT];
+#pragma unroll
+        for (int kt = 0; kt < KT; ++kt) {
+          const uint32_t at = sbase + (uint32_t)((b * 16 + 8 * hr + (lane & 7)) * PITCH + ((lane >> 3) & 1) * 16 + kt * 32);
+          asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
+                       : "=r"(q[2 * kt]), "=r"(q[2 * kt + 1]) : "r"(at));
+        }
+#pragma unroll
+        for (int t = 2; t >= 0; --t)
+#pragma unroll
+          for (int kt = 0; kt < KT; ++kt) seg_mma(s, xf[kt][t], q[2 * kt], q[2 * kt + 1]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) sW[(gid + 8 * h) * PC + (8 * hr + pos[u]) * PA + wid] = s[2 * h + u];
+      }
+      __syncthreads();   // sW complete; sV and this stage of the values read
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c = c0 + tc + 2 * j;
+        if (wok && c < m) W[(int64_t)c * ldw + wd] = w[j] + sW[(tc + 2 * j) * PC + ta * PA + tb];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2 * KT; ++n)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = 8 * n + 2 * tig + u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c = c0 + gid + 8 * h;
+          if (f < nv && k < no && c < m && a1[n][2 * h + u] != 0.f)
+            atomicAdd(&W1[(int64_t)c * ld1 + (int64_t)f * no + k], (double)a1[n][2 * h + u]);
+        }
+      }
+    __syncthreads();     // sW's readers, before the next block's tile
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+}
+
 // Segment A of the rows with a' = b' (classes 1 and 3: one row per virtual a
-// in each slab).  Thread <-> (a, 4 columns) over a group of AB_DIAG_SLABS slabs
+// in each slab).  Thread <-> (a, 4 columns) over a group of per slabs
 // (class-1 slabs k' = 0..no-1, then the class-3 hole pairs): V1[(a, k)] of its
 // columns in registers, W2 of each row updated, the W1 sums of single (a, k)
 // accumulated over the group.
-constexpr int AB_DIAG_SLABS = 8;
-
 template <typename TV, int NOP>
 __global__ void __launch_bounds__(256) k_ab_diag(GeomDev g, const TV* __restrict__ Bt, const float* __restrict__ V,
-                                                 int64_t ldv, int m, float* __restrict__ W, int64_t ldw,
+                                                 int64_t ldv, int m, int per, float* __restrict__ W, int64_t ldw,
                                                  double* __restrict__ W1, int64_t ld1) {
   const int nv = g.nv, no = g.no;
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -301,7 +514,7 @@ __global__ void __launch_bounds__(256) k_ab_diag(GeomDev g, const TV* __restrict
   const int ncol = min(4, m - c0);
   if (a >= nv) return;
   const int nslab = no + (int)g.npair_o;
-  const int q0 = blockIdx.z * AB_DIAG_SLABS, q1 = min(nslab, q0 + AB_DIAG_SLABS);
+  const int q0 = blockIdx.z * per, q1 = min(nslab, q0 + per);
   const int64_t n1 = g.n1;
   float x1[NOP][4], acc[NOP][4];
 #pragma unroll
@@ -353,6 +566,7 @@ struct AbTables {
   float* Y = nullptr;                // [nslab][nv][noP]
   float* Z = nullptr;
   float4* coin = nullptr;            // [pair-class rows]
+  __nv_bfloat16* seg = nullptr;      // BF16 store: [pair-class rows][A, B][kw]
 };
 
 struct AbPlan {
@@ -379,6 +593,7 @@ void ab_free(Ctx* c, void*& handle) {
     dfree(c, t.Y);
     dfree(c, t.Z);
     dfree(c, t.coin);
+    dfree(c, t.seg);
   }
   delete p;
   handle = nullptr;
@@ -387,21 +602,26 @@ void ab_free(Ctx* c, void*& handle) {
 static int ab_tables(Ctx* c, void*& handle, int which, const void* Bt) {
   if (!handle) handle = new AbPlan;
   AbTables& t = reinterpret_cast<AbPlan*>(handle)->t[which];
-  if (t.made_from == Bt && t.Y) return ADCGPU_OK;
+  if (t.made_from == Bt && (t.Y || t.seg)) return ADCGPU_OK;
   const Geometry& G = c->geom;
   const GeomDev g = to_dev(G);
   const int nslab = G.no + 2 * (int)G.npair_o;
   const size_t ntab = (size_t)nslab * G.nv * G.noP;
   const size_t nrow = (size_t)((G.start[2] - G.start[1]) + (G.start[5] - G.start[3]));
   int st;
+  if (which == 0) {
+    const int kw = (G.no + 15) / 16 * 16;
+    if (!t.seg && (st = dmalloc(c, (void**)&t.seg, sizeof(uint16_t) * std::max<size_t>(nrow, 1) * 2 * kw))) return st;
+    k_seg_pack<<<c->nsm * 8, 256, 0, c->stream>>>(g, (const __nv_bfloat16*)Bt, kw, t.seg);
+    ADC_COUNT_LAUNCH();
+    ADC_CUDA(c, cudaGetLastError());
+    t.made_from = Bt;
+    return ADCGPU_OK;
+  }
   if (!t.Y && (st = dmalloc(c, (void**)&t.Y, sizeof(float) * ntab))) return st;
   if (!t.Z && (st = dmalloc(c, (void**)&t.Z, sizeof(float) * ntab))) return st;
   if (!t.coin && (st = dmalloc(c, (void**)&t.coin, sizeof(float4) * std::max<size_t>(nrow, 1)))) return st;
-  if (which == 0)
-    k_ab_extract<__nv_bfloat16><<<c->nsm * 8, 256, 0, c->stream>>>(g, (const __nv_bfloat16*)Bt, nslab, t.Y, t.Z,
-                                                                   t.coin);
-  else
-    k_ab_extract<float><<<c->nsm * 8, 256, 0, c->stream>>>(g, (const float*)Bt, nslab, t.Y, t.Z, t.coin);
+  k_ab_extract<float><<<c->nsm * 8, 256, 0, c->stream>>>(g, (const float*)Bt, nslab, t.Y, t.Z, t.coin);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   t.made_from = Bt;
@@ -434,7 +654,21 @@ int ab_launch(Ctx* c, void*& handle, const TV* Bt, bool do_a, const float* V, in
     ADC_CUDA(c, cudaGetLastError());
     return ADCGPU_OK;
   };
-  if (nslab > 0) {
+  if constexpr (std::is_same<TV, __nv_bfloat16>::value) {
+    const int ngrp = (m + 15) / 16;
+    const int64_t nblk = (int64_t)nslab * ngrp * ((G.nv - 1 + SEG_F - 1) / SEG_F);
+    const int grid = (int)std::min<int64_t>(nblk, (int64_t)c->nsm * 16);
+    auto seg = [&](auto kern) -> int {
+      if (nblk == 0) return ADCGPU_OK;
+      kern<<<grid, 32 * SEG_F, 0, c->stream>>>(g, nslab, ngrp, t.seg, V, ldv, m, W, ldw, W1, ld1);
+      ADC_COUNT_LAUNCH();
+      ADC_CUDA(c, cudaGetLastError());
+      return ADCGPU_OK;
+    };
+    // BF16 values are stored for nocc <= 16 only (umma_supported): one k tile
+    if (do_a) ST(seg(k_seg_bf16<1, false>));
+    ST(seg(k_seg_bf16<1, true>));
+  } else if (nslab > 0) {
     switch (G.noP) {
       case 8: ST(do_a ? pairs(k_ab_pairs<8, true>) : pairs(k_ab_pairs<8, false>)); break;
       case 16: ST(do_a ? pairs(k_ab_pairs<16, true>) : pairs(k_ab_pairs<16, false>)); break;
@@ -444,12 +678,15 @@ int ab_launch(Ctx* c, void*& handle, const TV* Bt, bool do_a, const float* V, in
   }
   if (do_a) {
     const int nq = G.no + (int)G.npair_o;
-    const dim3 grid((G.nv + 127) / 128, ncb, (nq + AB_DIAG_SLABS - 1) / AB_DIAG_SLABS);
+    // up to eight slabs a group (fewer atomics), fewer where that leaves SMs
+    // idle (9/101, 5 columns: 12 blocks of eight slabs took 27 us)
+    const int per = std::max(1, std::min(8, (G.nv + 127) / 128 * ncb * nq / (2 * c->nsm)));
+    const dim3 grid((G.nv + 127) / 128, ncb, (nq + per - 1) / per);
     switch (G.noP) {
-      case 8: k_ab_diag<TV, 8><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, W, ldw, W1, ld1); break;
-      case 16: k_ab_diag<TV, 16><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, W, ldw, W1, ld1); break;
-      case 24: k_ab_diag<TV, 24><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, W, ldw, W1, ld1); break;
-      default: k_ab_diag<TV, 32><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, W, ldw, W1, ld1); break;
+      case 8: k_ab_diag<TV, 8><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, per, W, ldw, W1, ld1); break;
+      case 16: k_ab_diag<TV, 16><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, per, W, ldw, W1, ld1); break;
+      case 24: k_ab_diag<TV, 24><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, per, W, ldw, W1, ld1); break;
+      default: k_ab_diag<TV, 32><<<grid, 128, 0, c->stream>>>(g, Bt, V, ldv, m, per, W, ldw, W1, ld1); break;
     }
     ADC_COUNT_LAUNCH();
     ADC_CUDA(c, cudaGetLastError());

@@ -20,7 +20,7 @@
 //   warp 0, one thread : TMA producer.  Each tile of 128 rows is loaded as
 //                        slots of two 64-column boxes (128-byte swizzle) into
 //                        a ring of NSLOT slots.
-//   warp 1, one thread : MMA issuer.  Per slot: W2 tile (M = 128 rows,
+//   warp 1             : MMA issuer (one elected lane).  Per slot: W2 tile (M = 128 rows,
 //                        N = 2 NP, K = 128) into a double-buffered TMEM
 //                        accumulator D1; W1 part (M = 128 values of a,
 //                        N = 2 NP, K = 128 rows) into D2[slot], summed over
@@ -177,62 +177,77 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t idK = idesc_bf16(UMMA_ROWS, N2, 0, 0);     // W2: A K-major
-      const uint32_t idM = idesc_bf16(UMMA_ROWS, N2, 1, 0);     // W1: A MN-major
-      const uint32_t sXa = smem_u32(sX), sVa = smem_u32(sV2), sRa = smem_u32(sRing);
-      uint32_t use = 0, tile = 0, nitem = 0;
-      bool ok = true;
-      for (int it = blockIdx.x; it < nitems && ok && !failed(err); it += gridDim.x, ++nitem) {
-        const int2 item = items[it];
-        const Double r0 = decode_row(g, item.x);
-        const int cls = r0.cls;
-        const int K = (cls >= 2 ? 2 : 1) * nvP;
-        const int nbox = (K + UMMA_BOX - 1) / UMMA_BOX;
-        const int nslot = (nbox + 1) / 2;
-        ok = mbar_wait(&bars[B_XFULL], nitem & 1u, err, 2);          // X of this item built
-        ok = ok && mbar_wait(&bars[B_D2EMPTY], (nitem & 1u) ^ 1u, err, 3);   // D2 of the last item read
+    // The whole warp walks the loops, so that descriptors and addresses stay
+    // in uniform registers; one elected lane issues (one lane walking them
+    // alone took about 200 cycles an instruction).
+    constexpr uint64_t KMAJ = sdesc(0, 16, 1024, LAYOUT_SW128), MNMAJ = sdesc(0, UMMA_SLOT_BYTES / 2, 1024, LAYOUT_SW128);
+    const uint32_t idK = idesc_bf16(UMMA_ROWS, N2, 0, 0);     // W2: A K-major
+    const uint32_t idM = idesc_bf16(UMMA_ROWS, N2, 1, 0);     // W1: A MN-major
+    const uint64_t xdesc = KMAJ + (smem_u32(sX) >> 4), vdesc = KMAJ + (smem_u32(sV2) >> 4);
+    const uint32_t sRa = smem_u32(sRing);
+    uint32_t use = 0, tile = 0, nitem = 0;
+    bool ok = true;
+    for (int it = blockIdx.x; it < nitems && ok && !__any_sync(0xffffffffu, failed(err)); it += gridDim.x, ++nitem) {
+      const int2 item = items[it];
+      const Double r0 = decode_row(g, item.x);
+      const int cls = r0.cls;
+      const int K = (cls >= 2 ? 2 : 1) * nvP;
+      const int nbox = (K + UMMA_BOX - 1) / UMMA_BOX;
+      const int nslot = (nbox + 1) / 2;
+      ok = mbar_wait_warp(&bars[B_XFULL], nitem & 1u, err, 2);          // X of this item built
+      ok = ok && mbar_wait_warp(&bars[B_D2EMPTY], (nitem & 1u) ^ 1u, err, 3);   // D2 of the last item read
+      fence_after_sync();
+      bool first_tile = true;
+      for (int row0 = item.x; ok && row0 < item.y; row0 += UMMA_ROWS, ++tile) {
+        const int db = tile & 1;
+        ok = mbar_wait_warp(&bars[B_D1EMPTY0 + db], ((tile >> 1) & 1u) ^ 1u, err, 4);
+        ok = ok && mbar_wait_warp(&bars[B_V2FULL], tile & 1u, err, 5);
         fence_after_sync();
-        bool first_tile = true;
-        for (int row0 = item.x; ok && row0 < item.y; row0 += UMMA_ROWS, ++tile) {
-          const int db = tile & 1;
-          ok = mbar_wait(&bars[B_D1EMPTY0 + db], ((tile >> 1) & 1u) ^ 1u, err, 4);
-          ok = ok && mbar_wait(&bars[B_V2FULL], tile & 1u, err, 5);
-          fence_after_sync();
-          for (int vs = 0; vs < VS && ok; ++vs)
+        for (int vs = 0; vs < VS && ok; ++vs)
           for (int s = 0; ok && s < nslot; ++s, ++use) {
             const int ri = (int)(use % NSLOT);
             const uint32_t ph = (use / NSLOT) & 1u;
-            ok = mbar_wait(&slot_full[ri], ph, err, 6);
+            ok = mbar_wait_warp(&slot_full[ri], ph, err, 6);
             if (!ok) break;
             fence_after_sync();
             const uint32_t slot = sRa + (uint32_t)ri * UMMA_SLOT_BYTES;
-            // W2 tile: the slot's boxes as K-major A, X boxes 2s, 2s+1 as B
-            for (int b = 0; b < 2; ++b) {
-              const int box = 2 * s + b;
-              if (box >= nbox) break;
-              for (int ks = 0; ks < 4; ++ks) {
-                const uint64_t ad = sdesc(slot + b * (UMMA_SLOT_BYTES / 2) + ks * 32, 16, 1024, LAYOUT_SW128);
-                const uint64_t bd = sdesc(sXa + box * BOXB + ks * 32, 16, 1024, LAYOUT_SW128);
-                mma_bf16(tD1[db], ad, bd, idK, (vs | box | ks) ? 1u : 0u);
+            const uint64_t kd = KMAJ + (slot >> 4), md = MNMAJ + (slot >> 4);
+            const uint64_t xd = xdesc + (uint64_t)(2 * s) * (BOXB / 16);
+            const bool two = 2 * s + 1 < nbox;
+            const uint32_t acc1 = (vs | s) ? 1u : 0u, acc2 = (first_tile && vs == 0) ? 0u : 1u;
+            const uint32_t d2 = tD2 + (uint32_t)s * N2;
+            if (elect_one()) {
+              // W2 tile: the slot's boxes as K-major A, X boxes 2s, 2s+1 as B
+              mma_bf16(tD1[db], kd, xd, idK, acc1);
+#pragma unroll
+              for (int ks = 1; ks < 4; ++ks) mma_bf16_c<true>(tD1[db], kd + 2 * ks, xd + 2 * ks, idK);
+              if (two) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                  mma_bf16_c<true>(tD1[db], kd + UMMA_SLOT_BYTES / 32 + 2 * ks, xd + BOXB / 16 + 2 * ks, idK);
               }
+              // W1 part: the slot's 128 values of a as MN-major A (two 64-wide
+              // groups 16 KB apart), the tile's 128 rows as K; V2 as B
+              mma_bf16(d2, md, vdesc, idM, acc2);
+#pragma unroll
+              for (int ks = 1; ks < 8; ++ks)
+                mma_bf16_c<true>(d2, md + 128 * ks, vdesc + (ks >> 2) * (BOXB / 16) + 2 * (ks & 3), idM);
+              mma_commit(&slot_empty[ri]);
             }
-            // W1 part: the slot's 128 values of a as MN-major A (two 64-wide
-            // groups 16 KB apart), the tile's 128 rows as K; V2 as B
-            for (int ks = 0; ks < 8; ++ks) {
-              const uint64_t ad = sdesc(slot + ks * 2048, UMMA_SLOT_BYTES / 2, 1024, LAYOUT_SW128);
-              const uint64_t bd = sdesc(sVa + (ks >> 2) * BOXB + (ks & 3) * 32, 16, 1024, LAYOUT_SW128);
-              mma_bf16(tD2 + (uint32_t)s * N2, ad, bd, idM, (first_tile && vs == 0 && ks == 0) ? 0u : 1u);
-            }
-            mma_commit(&slot_empty[ri]);
+            __syncwarp();
           }
+        if (elect_one()) {
           mma_commit(&bars[B_D1FULL0 + db]);
           mma_commit(&bars[B_V2EMPTY]);
-          first_tile = false;
         }
+        __syncwarp();
+        first_tile = false;
+      }
+      if (elect_one()) {
         mma_commit(&bars[B_D2FULL]);
         mma_commit(&bars[B_XEMPTY]);
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ epilogue
