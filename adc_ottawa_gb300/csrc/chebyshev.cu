@@ -342,7 +342,7 @@ extern "C" int adcgpu_chebyshev_auto(adcgpu_ctx* h, int nvec, const double* q0, 
     }
   }
   if (order_out) *order_out = ord;
-  return ADCGPU_OK;
+  return sigma_status(c);
 }
 
 extern "C" int adcgpu_chebyshev_project(adcgpu_ctx* h, int nvec, double* q0, const double* bounds, int chebyord,
@@ -381,7 +381,7 @@ extern "C" int adcgpu_chebyshev_project(adcgpu_ctx* h, int nvec, double* q0, con
   ST(G.expand(a, b, &coef, 0, df));
   ADC_CUDA(c, cudaMemcpyAsync(q0, G.acc, G.blk_bytes, cudaMemcpyDeviceToHost, c->stream));
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
-  return ADCGPU_OK;
+  return sigma_status(c);
 }
 
 extern "C" int adcgpu_spectral_bounds(adcgpu_ctx* h, const adcgpu_dav_params* fp, double* bounds) {
@@ -426,5 +426,5 @@ extern "C" int adcgpu_spectral_bounds(adcgpu_ctx* h, const adcgpu_dav_params* fp
   ST(adcgpu_block_lanczos(h, 2, 100, 1, q0.data(), nullptr, ev.data(), nullptr));
   bounds[0] = lower;
   bounds[1] = ev[199];
-  return ADCGPU_OK;
+  return sigma_status(c);
 }

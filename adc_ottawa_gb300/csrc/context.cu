@@ -126,7 +126,9 @@ int adcgpu_ctx_create(int device, adcgpu_ctx** out) {
   else cudaGetLastError();
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
-      cudaMallocHost((void**)&c->h_word, sizeof(int)) != cudaSuccess) {
+      cudaMallocHost((void**)&c->h_word, sizeof(int)) != cudaSuccess ||
+      cudaMalloc((void**)&c->d_word, sizeof(int)) != cudaSuccess ||
+      cudaMemsetAsync(c->d_word, 0, sizeof(int), c->stream) != cudaSuccess) {
     delete c;
     return ADCGPU_CUDA_ERROR;
   }
@@ -151,6 +153,7 @@ int adcgpu_ctx_destroy(adcgpu_ctx* h) {
   if (c->st_ev0) cudaEventDestroy(c->st_ev0);
   if (c->st_ev1) cudaEventDestroy(c->st_ev1);
   cudaFreeHost(c->h_word);
+  cudaFree(c->d_word);
   cudaStreamDestroy(c->stream);
   delete c;
   return ADCGPU_OK;
@@ -498,7 +501,7 @@ int adcgpu_sigma_device(adcgpu_ctx* h, int m, const void* dv, void* dw, int64_t 
   float ms = 0.f;
   cudaEventElapsedTime(&ms, c->ev0, c->ev1);
   c->last_sigma_ms = ms;
-  return ADCGPU_OK;
+  return sigma_status(c);
 }
 
 int adcgpu_sigma(adcgpu_ctx* h, int m, const double* v, double* w) {

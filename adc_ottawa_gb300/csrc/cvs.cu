@@ -173,7 +173,7 @@ int sigma_cvs(Ctx* c, int m, const double* dV, int64_t ldv, double* dW, int64_t 
     }
     q0 += mg;
   }
-  return usable ? oz_check(c, c->cvs_oz) : ADCGPU_OK;
+  return usable ? sigma_queue_status(c) : ADCGPU_OK;
 }
 
 int export_coo_cvs(Ctx* c, double* d_h, int32_t* d_oi, int32_t* d_oj) {

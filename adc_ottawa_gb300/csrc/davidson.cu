@@ -648,7 +648,8 @@ extern "C" int adcgpu_davidson(adcgpu_ctx* h, const adcgpu_dav_params* p, double
   if (!c || !p || !evals) return ADCGPU_BAD_INPUT;
   cudaSetDevice(c->device);
   if (!c->have_matrix) return set_err(c, ADCGPU_NO_MATRIX, "build the matrix first");
-  return davidson_solve(c, p, evals, evecs, info, nullptr);
+  const int st = davidson_solve(c, p, evals, evecs, info, nullptr), status = sigma_status(c);
+  return status ? status : st;
 }
 
 extern "C" int adcgpu_davidson_trace(adcgpu_ctx* h, const adcgpu_dav_params* p, int every, int max_records,
@@ -684,7 +685,8 @@ extern "C" int adcgpu_davidson_trace(adcgpu_ctx* h, const adcgpu_dav_params* p, 
   if (nrec) *nrec = D.tr_n;
   D.release();
   dfree(c, out, 0);
-  return st;
+  const int status = sigma_status(c);
+  return status ? status : st;
 }
 
 extern "C" int adcgpu_write_davidson_file(const char* path, int ndim, int nstates, const double* evals,

@@ -248,7 +248,11 @@ struct Ctx {
   int nsm = 152;                  // streaming multiprocessors of the device (queried at creation)
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  int* h_word = nullptr;          // pinned word for device status reads
+  // status of the bounded waits in the tensor-core sigma kernels: they write
+  // d_word, every product queues a copy to the pinned h_word, sigma_status()
+  // reads it once the copy is done
+  int *d_word = nullptr, *h_word = nullptr;
+  bool word_pending = false;
   std::string err;
   Geometry geom;
   bool have_orb = false, have_eri = false, have_matrix = false;
@@ -419,7 +423,6 @@ struct SigmaPlan {
   void* d_sk = nullptr;       // split-K partials of the FP32 singles block
   size_t sk_bytes = 0;
   void* umma = nullptr;       // tensor-core pass plan (sigma_umma.cu), built on first use
-  int umma_item_rows = 4096;  // rows per tensor-core work item (autotuned)
   int umma_off = 0;           // 1: the tensor-core pass is not used
   void* ab = nullptr;         // compact segment-A/B tables (sigma_ab.cu), built on first use
   int ab_off = 0;             // 1: segments A/B through pass 2 / pass 3 instead
@@ -445,8 +448,8 @@ void umma_free(Ctx* c, void*& handle);
 int umma_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float* W, int64_t ldw, double* W1,
                 int64_t ld1, int seg_a);
 int umma_runs(void* handle, const int2** runs, int* nruns);
-int umma_check(Ctx* c, void* handle);
 bool umma_geometry_ok(const Geometry& G);
+int umma_item_rows(const Ctx* c);
 bool umma3_supported(const Ctx* c);
 int umma3_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float* W, int64_t ldw, double* W1,
                  int64_t ld1);
@@ -463,7 +466,11 @@ int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t
               double* W1, int64_t ld1);
 int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t ldv, int m, float* W, int64_t ldw,
               double* W1, int64_t ld1);
-int oz_check(Ctx* c, void* handle);
+int sigma_queue_status(Ctx* c);
+// Waits for the products queued so far and returns ADCGPU_DEVICE_TIMEOUT when
+// a pipeline wait gave up.  Called before the next product and before results
+// leave the library, not after every product.
+int sigma_status(Ctx* c);
 
 // sigma_ab.cu : segments A and B of the mixed-precision sigma product in
 // compact form (tables copied from the BF16 or FP32 value store on first use)

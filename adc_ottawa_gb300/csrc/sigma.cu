@@ -1427,6 +1427,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
     ADC_CUDA(c, cudaEventCreate(&c->st_ev1));
   }
   sigma_stats_flush(c);
+  if (c->word_pending && *c->h_word) ST(sigma_status(c));   // copied before the stop event just waited for
   ADC_CUDA(c, cudaEventRecord(c->st_ev0, s));
   GeomDev g = to_dev(G);
   // singles block first (plain stores), then the coupling adds atomically
@@ -1502,7 +1503,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
       // W2 part of segment A, then segment B (pass 2) and the W1 part of
       // segment A (pass 3), up to 48 columns per matrix pass
       if (allow_umma && P->tiled == 1 && !P->umma_off && umma_supported(c)) {
-        ST(umma_prepare(c, plan->umma, plan->umma_item_rows));
+        ST(umma_prepare(c, plan->umma, umma_item_rows(c)));
         const int2* runs = nullptr;
         int nruns = 0;
         ST(umma_runs(plan->umma, &runs, &nruns));
@@ -1541,7 +1542,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
       // FP32 store, up to 32 columns per matrix pass
       if (allow_umma && P->umma3_on && P->tiled == 1 && !P->umma_off && !P->ab_off && !c->direct &&
           umma3_supported(c) && ab_supported(c)) {
-        ST(umma_prepare(c, plan->umma, plan->umma_item_rows));
+        ST(umma_prepare(c, plan->umma, umma_item_rows(c)));
         for (; c0 < m;) {
           const int nc = std::min(m - c0, 32);
           const T* V = dV + (int64_t)c0 * ldv;
@@ -1663,9 +1664,8 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
     k_w1_finalize<<<(n1 * m + 255) / 256, 256, 0, s>>>(n1, m, reinterpret_cast<const double*>(W1base),
                                                        reinterpret_cast<float*>(dW), ldw); ADC_COUNT_LAUNCH();
   }
+  if (umma_used || oz_used) ST(sigma_queue_status(c));
   ADC_CUDA(c, cudaEventRecord(c->st_ev1, s));
-  if (umma_used) ST(umma_check(c, plan->umma));
-  if (oz_used) ST(oz_check(c, plan->oz[sizeof(T) == 8 ? 0 : 1]));
   c->st_pending = true;
   c->st_pending_cols = m;
   c->st_pending_kind = std::is_same<TV, __nv_bfloat16>::value ? 0 : (std::is_same<TV, float>::value ? 1 : 2);
@@ -1883,6 +1883,7 @@ extern "C" int adcgpu_sigma_autotune(adcgpu_ctx* h, int m, int* best_chunk, int*
       if (t < best) { best = t; bc = ch; bm = mc; bs = stg; bt = 0; }
     }
   }
+  if (!st) st = sigma_status(c);
   sigma_stats_flush(c);
   c->st_calls = 0; c->st_cols = 0; c->st_ms = 0.0; c->st_bytes = 0.0;
   for (auto& b : c->st_by) for (double& x : b) x = 0.0;

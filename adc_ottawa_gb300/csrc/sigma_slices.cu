@@ -1068,9 +1068,8 @@ struct OzPlan {
   int S = 0;
   OzDst dst;
   OzGeom geom;
-  unsigned char* d_lists = nullptr;   // error word, work items, slabs, item exponents
+  unsigned char* d_lists = nullptr;   // work items, slabs, item exponents
   size_t list_bytes = 0;
-  int* err = nullptr;
   OzItem* items = nullptr;
   OzSlab* slabs = nullptr;
   int *vexp = nullptr, *vsexp = nullptr;
@@ -1206,19 +1205,17 @@ void oz_add_slab(OzPlan* p, int64_t s0, int64_t len, int item_rows, int holes, b
 int oz_upload_lists(Ctx* c, OzPlan* p, int item_rows, int m) {
   const size_t ni = p->h_items.size(), ns = p->h_slabs.size();
   const size_t ib = align256(sizeof(OzItem) * ni), lb = ib + align256(sizeof(OzSlab) * ns);
-  const size_t need = 256 + lb + 2 * sizeof(int) * ni * m;
+  const size_t need = lb + 2 * sizeof(int) * ni * m;
   if (p->list_bytes < need) {
     dfree(c, p->d_lists);
     p->d_lists = nullptr;
     p->list_bytes = 0;
     ST(dmalloc(c, (void**)&p->d_lists, need));
     p->list_bytes = need;
-    p->err = reinterpret_cast<int*>(p->d_lists);
-    ADC_CUDA(c, cudaMemsetAsync(p->err, 0, sizeof(int), c->stream));
   }
-  p->items = reinterpret_cast<OzItem*>(p->d_lists + 256);
-  p->slabs = reinterpret_cast<OzSlab*>(p->d_lists + 256 + ib);
-  p->vexp = reinterpret_cast<int*>(p->d_lists + 256 + lb);
+  p->items = reinterpret_cast<OzItem*>(p->d_lists);
+  p->slabs = reinterpret_cast<OzSlab*>(p->d_lists + ib);
+  p->vexp = reinterpret_cast<int*>(p->d_lists + lb);
   p->vsexp = p->vexp + ni * m;
   std::vector<unsigned char> all(lb);
   std::copy_n(reinterpret_cast<const unsigned char*>(p->h_items.data()), sizeof(OzItem) * ni, all.data());
@@ -1433,7 +1430,7 @@ int oz_go(Ctx* c, OzPlan* p, int smax, const OzShape& sh, size_t smem, const T* 
                                                                     ldv, m, p->vexp, p->vsexp);
   ADC_COUNT_LAUNCH();
   kern<<<grid, OZ_THREADS, smem, c->stream>>>(p->geom, p->items + p->item0, p->nitems, ngrp, sh, p->dig, p->rexp,
-                                              p->vexp, diag, V, ldv, m, W, ldw, W1, ld1, p->err);
+                                              p->vexp, diag, V, ldv, m, W, ldw, W1, ld1, c->d_word);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   return ADCGPU_OK;
@@ -1501,19 +1498,21 @@ int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t l
   return oz_seg<4>(c, p, V, ldv, m, W, ldw, W1, ld1);
 }
 
-// Reads the kernel's error word (waits for the stream) and clears it.
-int oz_check(Ctx* c, void* handle) {
-  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
-  if (!p || !p->err) return ADCGPU_OK;
-  ADC_CUDA(c, cudaMemcpyAsync(c->h_word, p->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  ADC_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (*c->h_word) {
-    const int code = *c->h_word;
-    ADC_CUDA(c, cudaMemsetAsync(p->err, 0, sizeof(int), c->stream));
-    return set_err(c, ADCGPU_DEVICE_TIMEOUT,
-                   "sliced sigma pass: a pipeline wait timed out (stage " + std::to_string(code) + ")");
-  }
+int sigma_queue_status(Ctx* c) {
+  ADC_CUDA(c, cudaMemcpyAsync(c->h_word, c->d_word, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  c->word_pending = true;
   return ADCGPU_OK;
+}
+
+int sigma_status(Ctx* c) {
+  if (!c->word_pending) return ADCGPU_OK;
+  ADC_CUDA(c, cudaStreamSynchronize(c->stream));
+  c->word_pending = false;
+  if (!*c->h_word) return ADCGPU_OK;
+  const int code = *c->h_word;
+  ADC_CUDA(c, cudaMemsetAsync(c->d_word, 0, sizeof(int), c->stream));
+  return set_err(c, ADCGPU_DEVICE_TIMEOUT,
+                 "tensor-core sigma pass: a pipeline wait timed out (stage " + std::to_string(code) + ")");
 }
 
 }  // namespace adcgpu

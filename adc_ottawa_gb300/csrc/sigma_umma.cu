@@ -15,7 +15,7 @@
 // [0, NP) hi, [NP, 2 NP) lo), so one MMA gives both products and the
 // epilogue adds them (x = hi + lo to ~2^-17 relative).
 //
-// One CTA per SM, persistent over work items (up to UMMA_ITEM_ROWS rows of
+// One CTA per SM, persistent over work items (up to UMMA_ITEM_ROWS_MAX rows of
 // one slab), warp-specialised:
 //   warp 0, one thread : TMA producer.  Each tile of 128 rows is loaded as
 //                        slots of two 64-column boxes (128-byte swizzle) into
@@ -60,7 +60,7 @@ constexpr int UMMA_SLOT_BYTES = 2 * UMMA_ROWS * UMMA_BOX * 2;   // two boxes
 constexpr int UMMA_MAX_BOXES = 6;           // K <= 384
 constexpr int UMMA_THREADS = 320;             // producer, MMA issuer, 8 epilogue warps
 constexpr int UMMA_NOP = 16;                  // segment A lengths (noP) up to 16 (nocc <= 16)
-constexpr int UMMA_ITEM_ROWS_DEFAULT = 4096;  // rows per work item (a piece of one slab)
+constexpr int UMMA_ITEM_ROWS_MAX = 4096;      // rows per work item (a piece of one slab)
 // rows per work item of the FP32-value main pass: the W1 sums of an item run
 // in one TMEM chain (8 MMA steps per 128-row tile), and shorter chains keep
 // the tensor cores' truncating FP32 accumulation near FP32 rounding
@@ -508,9 +508,7 @@ struct UmmaPlan {
   int nitems_s = 0;
   int2* d_runs = nullptr;           // pass-3 runs: (first row, rows) of equal a' in one slab
   int nruns = 0;
-  int* d_err = nullptr;             // device error word of the kernel's bounded waits
-  int* h_err = nullptr;             // pinned host copy
-  int item_rows = UMMA_ITEM_ROWS_DEFAULT;
+  int item_rows = 0;
 };
 
 namespace {
@@ -554,7 +552,7 @@ int launch_umma_np(Ctx* c, UmmaPlan* u, const float* V, int64_t ldv, int m, floa
     ADC_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
     kern<<<grid, UMMA_THREADS, smem, c->stream>>>(g, items, nitems, u->maps,
                                                   (const __nv_bfloat16*)c->d_Bt16, c->d_diag32, V, ldv, m, W, ldw, W1,
-                                                  ld1, seg_a, vbase, w2_add, u->d_err);
+                                                  ld1, seg_a, vbase, w2_add, c->d_word);
     ADC_COUNT_LAUNCH();
     ADC_CUDA(c, cudaGetLastError());
     return ADCGPU_OK;
@@ -593,6 +591,14 @@ bool umma_geometry_ok(const Geometry& G) {
   return G.noP <= UMMA_NOP && 2 * G.nvP <= UMMA_MAX_BOXES * UMMA_BOX && G.no >= 2 && G.nv >= 2;
 }
 
+// Rows per work item: about six items per SM (4,096 rows whatever the size
+// left 1.3 rounds of items at nocc=9/nvirt=101), 512 to 4,096 (an item's X
+// operand and W1 atomics cost about a tile).
+int umma_item_rows(const Ctx* c) {
+  const int64_t want = (c->geom.n2 / ((int64_t)c->nsm * 6) + 127) / 128 * 128;
+  return (int)std::min<int64_t>(UMMA_ITEM_ROWS_MAX, std::max<int64_t>(512, want));
+}
+
 bool umma3_supported(const Ctx* c) {
   return umma_supported(c) && c->d_Bt16s[0] != nullptr && c->d_Bt16s[1] != nullptr;
 }
@@ -603,8 +609,6 @@ void umma_free(Ctx* c, void*& handle) {
   dfree(c, u->d_items);
   dfree(c, u->d_items_s);
   dfree(c, u->d_runs);
-  dfree(c, u->d_err);
-  if (u->h_err) cudaFreeHost(u->h_err);
   delete u;
   handle = nullptr;
 }
@@ -645,11 +649,8 @@ int umma_prepare(Ctx* c, void*& handle, int item_rows) {
   ADC_CUDA(c, h2d(c, u->d_items_s, items_s.data(), sizeof(int2) * items_s.size()));
   u->nitems_s = (int)items_s.size();
   if ((st = dmalloc(c, (void**)&u->d_runs, sizeof(int2) * runs.size()))) return st;
-  if ((st = dmalloc(c, (void**)&u->d_err, sizeof(int)))) return st;
-  ADC_CUDA(c, cudaMallocHost((void**)&u->h_err, sizeof(int)));
   ADC_CUDA(c, h2d(c, u->d_items, items.data(), sizeof(int2) * items.size()));
   ADC_CUDA(c, h2d(c, u->d_runs, runs.data(), sizeof(int2) * runs.size()));
-  ADC_CUDA(c, cudaMemsetAsync(u->d_err, 0, sizeof(int), c->stream));
   u->nitems = (int)items.size();
   u->nruns = (int)runs.size();
   PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
@@ -718,21 +719,6 @@ int umma3_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float
   }
   ST((launch_umma_np<32, 1, 3>(c, u, V, ldv, m, W, ldw, W1, ld1, 0, 0, 0, true)));
   return launch_umma_np<32, 2, 2>(c, u, V, ldv, m, W, ldw, W1, ld1, 0, 1, 1, false);
-}
-
-// Reads the kernel's error word (waits for the stream) and clears it.
-int umma_check(Ctx* c, void* handle) {
-  UmmaPlan* u = reinterpret_cast<UmmaPlan*>(handle);
-  if (!u) return ADCGPU_OK;
-  ADC_CUDA(c, cudaMemcpyAsync(u->h_err, u->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  ADC_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (*u->h_err) {
-    const int code = *u->h_err;
-    ADC_CUDA(c, cudaMemsetAsync(u->d_err, 0, sizeof(int), c->stream));
-    return set_err(c, ADCGPU_DEVICE_TIMEOUT, "tensor-core sigma pass: a pipeline wait timed out (stage " +
-                                          std::to_string(code) + ")");
-  }
-  return ADCGPU_OK;
 }
 
 }  // namespace adcgpu

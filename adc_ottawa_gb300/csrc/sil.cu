@@ -482,7 +482,7 @@ extern "C" int adcgpu_autocorr(adcgpu_ctx* h, int nwp, const double* f, double t
   }
   if (ntimes_out) *ntimes_out = ntimes;
   if (nmult_out) *nmult_out = E.nmult / std::max(1, nwp);
-  return ADCGPU_OK;
+  return sigma_status(c);
 }
 
 extern "C" int adcgpu_silstep(adcgpu_ctx* h, double* psi, double* dtpsi, int psidim, double intperiod, int intorder,
@@ -518,5 +518,5 @@ extern "C" int adcgpu_silstep(adcgpu_ctx* h, double* psi, double* dtpsi, int psi
   if (stepsize_out) *stepsize_out = pk[0].Stepsize;
   if (trueorder_out) *trueorder_out = pk[0].TrueOrder;
   if (st) *st = pk[0].save;
-  return ADCGPU_OK;
+  return sigma_status(c);
 }
