@@ -841,8 +841,12 @@ __device__ __forceinline__ void mma_seg(float (&c)[4], const uint32_t (&a)[4], u
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-constexpr int SEG_WARPS = 4;
+constexpr int SEG_WARPS = 4;   // two a run
 template <int S, int KT> __host__ __device__ constexpr int seg_pitch() { return S * KT * 32 + 16; }   // bytes of a staged row
+
+// resident blocks the register budget is set for: 128 registers a thread where
+// the slices of one k tile fit
+template <int KT> __host__ __device__ constexpr int seg_blocks() { return KT == 1 ? 4 : 2; }
 
 // exponent of a column over the four lanes that hold it
 __device__ __forceinline__ int quad_max(int e) {
@@ -871,9 +875,16 @@ __device__ __forceinline__ void seg_fragments(const T (&x)[2][4], const int (&sc
     }
 }
 
-// SEGB: runs of equal b' (segment B), else of equal a' (segment A)
+// SEGB: runs of equal b' (segment B), else of equal a' (segment A).  Two warps
+// a run: the even one takes its W1 sums, the odd one its W2 rows, each with
+// its own stage of the digits (the second read comes from L2).  One warp for
+// both held 250 registers, eight warps an SM that spent 2.6 of their 5 stall
+// cycles on fixed-latency results: 30 columns at nocc=13/nvirt=131 in 6.85 ms
+// for the whole product, 5.82 with two warps.  Staging V2 and W2 of eight
+// neighbouring runs through shared memory made segment B 7% faster and A 20%
+// slower.
 template <int S, int KT, bool SEGB, typename T, typename TA>
-__global__ void __launch_bounds__(32 * SEG_WARPS)
+__global__ void __launch_bounds__(32 * SEG_WARPS, seg_blocks<KT>())
     k_oz_seg(OzGeom g, const OzSlab* __restrict__ slabs, int nslab, int ngrp, int item0,
              const uint16_t* __restrict__ dig, const int16_t* __restrict__ sexp, const int* __restrict__ vsexp, const T* __restrict__ V, int64_t ldv,
              int m, T* __restrict__ W, int64_t ldw, TA* __restrict__ W1, int64_t ld1) {
@@ -881,12 +892,14 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int gid = lane >> 2, tig = lane & 3;
-  unsigned char* stage = smem + wid * 2 * 16 * PITCH;
-  const uint32_t sbase = smem_u32(stage);
+  const uint32_t sbase = smem_u32(smem + wid * 2 * 16 * PITCH);
   const int no = g.no, nv = g.nv;
   const int64_t n1 = g.n1;
   const int64_t nrun = (int64_t)nslab * ngrp * (nv - 1);
-  for (int64_t run = blockIdx.x * (int64_t)SEG_WARPS + wid; run < nrun; run += (int64_t)gridDim.x * SEG_WARPS) {
+  // positions of this lane in a step of 16 rows (or singles)
+  const int pos[4] = {2 * tig, 2 * tig + 1, 2 * tig + 8, 2 * tig + 9};
+  for (int64_t run = blockIdx.x * (int64_t)(SEG_WARPS / 2) + (wid >> 1); run < nrun;
+       run += (int64_t)gridDim.x * (SEG_WARPS / 2)) {
     const int fi = (int)(run % (nv - 1));
     const int64_t sg = run / (nv - 1);
     const int c0 = (int)(sg % ngrp) * 16;
@@ -912,146 +925,153 @@ __global__ void __launch_bounds__(32 * SEG_WARPS)
     };
     __syncwarp();
     issue(0, 0);
-    // positions of this lane in a step of 16 rows
-    const int pos[4] = {2 * tig, 2 * tig + 1, 2 * tig + 8, 2 * tig + 9};
-    auto load_v2 = [&](int t0, T (&x)[2][4], int (&er)[4]) {
+    if (!(wid & 1)) {
+      // ---- W1[(f, k), c] += sum_t R[t, k] V2[t, c]
+      // column exponents of the slab's 2^er V2
+      int ev[2];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int t = t0 + pos[v];
-        const bool ok = t < nrow;
-        const int64_t pr = ok ? pair_of(t) : 0;
-        er[v] = ok ? (int)sexp[rloc + pr] : OZ_EMIN;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          x[h][v] = (ok && cc[h] < m) ? __ldg(V + (int64_t)cc[h] * ldv + dbase + pr * dstr) : T(0);
+      for (int h = 0; h < 2; ++h) {
+        int e = OZ_EMIN;
+        if (cc[h] < m)
+          for (int i = 0; i < sl.nitem; ++i) e = max(e, __ldg(vsexp + (int64_t)(sl.item0 - item0 + i) * m + cc[h]));
+        ev[h] = e;
       }
-    };
-    // column exponents of the slab's 2^er V2
-    int ev[2];
+      float a1[2 * KT][S][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      int e = OZ_EMIN;
-      if (cc[h] < m)
-        for (int i = 0; i < sl.nitem; ++i) e = max(e, __ldg(vsexp + (int64_t)(sl.item0 - item0 + i) * m + cc[h]));
-      ev[h] = e;
-    }
-    // V of the singles (f, k)
-    uint32_t xf[KT][S][4];
-    int ex[2] = {OZ_EMIN, OZ_EMIN};
-    {
-      T x[KT][2][4];
+      for (int n = 0; n < 2 * KT; ++n)
 #pragma unroll
-      for (int kt = 0; kt < KT; ++kt)
+        for (int i = 0; i < S; ++i) a1[n][i][0] = a1[n][i][1] = a1[n][i][2] = a1[n][i][3] = 0.f;
+      for (int t0 = 0, b = 0; t0 < nrow; t0 += 16, b ^= 1) {
+        __syncwarp();                                     // the other stage's readers are done
+        if (t0 + 16 < nrow) issue(t0 + 16, b ^ 1);
+        else asm volatile("cp.async.commit_group;\n" ::);
+        T x[2][4];
+        int er[4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int v = 0; v < 4; ++v) {
+          const int t = t0 + pos[v];
+          const bool ok = t < nrow;
+          const int64_t pr = ok ? pair_of(t) : 0;
+          er[v] = ok ? (int)sexp[rloc + pr] : OZ_EMIN;
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int k = 16 * kt + pos[v];
-            x[kt][h][v] = (k < no && cc[h] < m) ? __ldg(V + (int64_t)cc[h] * ldv + (int64_t)f * no + k) : T(0);
-            ex[h] = max(ex[h], Parts<T>::exponent(x[kt][h][v]));
-          }
-      ex[0] = quad_max(ex[0]);
-      ex[1] = quad_max(ex[1]);
-      const int sc0[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int kt = 0; kt < KT; ++kt) seg_fragments<S, T>(x[kt], sc0, ex, xf[kt]);
-    }
-    float a1[2 * KT][S][4];
-#pragma unroll
-    for (int n = 0; n < 2 * KT; ++n)
-#pragma unroll
-      for (int i = 0; i < S; ++i) a1[n][i][0] = a1[n][i][1] = a1[n][i][2] = a1[n][i][3] = 0.f;
-    int b = 0;
-    T x[2][4];
-    int er[4];
-    load_v2(0, x, er);
-    for (int t0 = 0; t0 < nrow; t0 += 16, b ^= 1) {
-      __syncwarp();                                       // the other stage's readers are done
-      if (t0 + 16 < nrow) issue(t0 + 16, b ^ 1);
-      else asm volatile("cp.async.commit_group;\n" ::);
-      uint32_t vf[S][4];
-      seg_fragments<S, T>(x, er, ev, vf);
-      // this step's W2 rows and the next step's V2, ahead of their use
-      int ee[4];
-      T wv[2][4];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        ee[v] = er[v] == 32767 ? OZ_NONFINITE : er[v];
-        const int t = t0 + pos[v];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          wv[h][v] = (t < nrow && cc[h] < m) ? W[(int64_t)cc[h] * ldw + dbase + pair_of(t) * dstr] : T(0);
-      }
-      if (t0 + 16 < nrow) load_v2(t0 + 16, x, er);
-      asm volatile("cp.async.wait_group 1;\n" ::);
-      __syncwarp();
-      // 16 x 16 digits of slice i, k group kt: row lane % 16, half lane / 16
-      const uint32_t srow = sbase + (uint32_t)((b * 16 + (lane & 15)) * PITCH + (lane >> 4) * 16);
-#pragma unroll
-      for (int kt = 0; kt < KT; ++kt)
-#pragma unroll
-        for (int i = 0; i < S; ++i) {
-          uint32_t q[4];
-          ldsm_x4_t(q, srow + (i * KT + kt) * 32);        // (rows 0-7, 8-15) x k 0-7, then k 8-15
-#pragma unroll
-          for (int j = 0; j < S - i; ++j) {
-            mma_seg(a1[2 * kt][i + j], vf[j], q[0], q[1]);
-            mma_seg(a1[2 * kt + 1][i + j], vf[j], q[2], q[3]);
-          }
+          for (int h = 0; h < 2; ++h)
+            x[h][v] = (ok && cc[h] < m) ? __ldg(V + (int64_t)cc[h] * ldv + dbase + pr * dstr) : T(0);
         }
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {                    // rows t0 + 8 hr ..
-        float a2[S][4];
-#pragma unroll
-        for (int i = 0; i < S; ++i) a2[i][0] = a2[i][1] = a2[i][2] = a2[i][3] = 0.f;
-        // two slices at a time: (slice i, k 0-7), (i, k 8-15), (i + 1, ..)
-        const uint32_t srow2 = sbase + (uint32_t)((b * 16 + 8 * hr + (lane & 7)) * PITCH + ((lane >> 3) & 1) * 16);
+        uint32_t vf[S][4];
+        seg_fragments<S, T>(x, er, ev, vf);
+        asm volatile("cp.async.wait_group 1;\n" ::);
+        __syncwarp();
+        // 16 x 16 digits of slice i, k group kt: row lane % 16, half lane / 16
+        const uint32_t srow = sbase + (uint32_t)((b * 16 + (lane & 15)) * PITCH + (lane >> 4) * 16);
 #pragma unroll
         for (int kt = 0; kt < KT; ++kt)
 #pragma unroll
-          for (int i = 0; i < S; i += 2) {
+          for (int i = 0; i < S; ++i) {
             uint32_t q[4];
-            const int i2 = i + 1 < S ? i + 1 : i;
-            ldsm_x4(q, srow2 + (uint32_t)(((lane >> 4) ? i2 : i) * KT + kt) * 32);
+            ldsm_x4_t(q, srow + (i * KT + kt) * 32);      // (rows 0-7, 8-15) x k 0-7, then k 8-15
 #pragma unroll
-            for (int j = 0; j < S - i; ++j) mma_seg(a2[i + j], xf[kt][j], q[0], q[1]);
-            if (i + 1 < S) {
-#pragma unroll
-              for (int j = 0; j < S - i - 1; ++j) mma_seg(a2[i + 1 + j], xf[kt][j], q[2], q[3]);
+            for (int j = 0; j < S - i; ++j) {
+              mma_seg(a1[2 * kt][i + j], vf[j], q[0], q[1]);
+              mma_seg(a1[2 * kt + 1][i + j], vf[j], q[2], q[3]);
             }
           }
+      }
+#pragma unroll
+      for (int n = 0; n < 2 * KT; ++n)
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
-          const int t = t0 + 8 * hr + pos[v];
-          if (t >= nrow) continue;
-          const int64_t d = dbase + pair_of(t) * dstr;
+          const int k = 8 * n + 2 * tig + v;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            if (cc[h] >= m) continue;
+            if (k >= no || cc[h] >= m) continue;
             float dsum[S];
 #pragma unroll
-            for (int i = 0; i < S; ++i) dsum[i] = a2[i][2 * h + v];
-            W[(int64_t)cc[h] * ldw + d] =
-                wv[h][2 * hr + v] + oz_round<S, T>(dsum) * oz_scale<T>(ex[h] + ee[2 * hr + v] + TSH);
+            for (int i = 0; i < S; ++i) dsum[i] = a1[n][i][2 * h + v];
+            const double w = oz_sum<S>(dsum) * oz_pow2(ev[h] + TSH);
+            if (!(w == 0.0)) atomicAdd(&W1[(int64_t)cc[h] * ld1 + (int64_t)f * no + k], (TA)w);
+          }
+        }
+    } else {
+      // ---- W2[t, c] += sum_k R[t, k] V[(f, k), c]
+      uint32_t xf[KT][S][4];
+      int ex[2] = {OZ_EMIN, OZ_EMIN};
+      {
+        T x[KT][2][4];
+#pragma unroll
+        for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int k = 16 * kt + pos[v];
+              x[kt][h][v] = (k < no && cc[h] < m) ? __ldg(V + (int64_t)cc[h] * ldv + (int64_t)f * no + k) : T(0);
+              ex[h] = max(ex[h], Parts<T>::exponent(x[kt][h][v]));
+            }
+        ex[0] = quad_max(ex[0]);
+        ex[1] = quad_max(ex[1]);
+        const int sc0[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int kt = 0; kt < KT; ++kt) seg_fragments<S, T>(x[kt], sc0, ex, xf[kt]);
+      }
+      for (int t0 = 0, b = 0; t0 < nrow; t0 += 16, b ^= 1) {
+        __syncwarp();
+        if (t0 + 16 < nrow) issue(t0 + 16, b ^ 1);
+        else asm volatile("cp.async.commit_group;\n" ::);
+        // this step's W2 rows, ahead of their use
+        int ee[4];
+        T wv[2][4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int t = t0 + pos[v];
+          const bool ok = t < nrow;
+          const int64_t pr = ok ? pair_of(t) : 0;
+          const int er = ok ? (int)sexp[rloc + pr] : OZ_EMIN;
+          ee[v] = er == 32767 ? OZ_NONFINITE : er;
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            wv[h][v] = (ok && cc[h] < m) ? W[(int64_t)cc[h] * ldw + dbase + pr * dstr] : T(0);
+        }
+        asm volatile("cp.async.wait_group 1;\n" ::);
+        __syncwarp();
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {                  // rows t0 + 8 hr ..
+          float a2[S][4];
+#pragma unroll
+          for (int i = 0; i < S; ++i) a2[i][0] = a2[i][1] = a2[i][2] = a2[i][3] = 0.f;
+          // two slices at a time: (slice i, k 0-7), (i, k 8-15), (i + 1, ..)
+          const uint32_t srow2 = sbase + (uint32_t)((b * 16 + 8 * hr + (lane & 7)) * PITCH + ((lane >> 3) & 1) * 16);
+#pragma unroll
+          for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+            for (int i = 0; i < S; i += 2) {
+              uint32_t q[4];
+              const int i2 = i + 1 < S ? i + 1 : i;
+              ldsm_x4(q, srow2 + (uint32_t)(((lane >> 4) ? i2 : i) * KT + kt) * 32);
+#pragma unroll
+              for (int j = 0; j < S - i; ++j) mma_seg(a2[i + j], xf[kt][j], q[0], q[1]);
+              if (i + 1 < S) {
+#pragma unroll
+                for (int j = 0; j < S - i - 1; ++j) mma_seg(a2[i + 1 + j], xf[kt][j], q[2], q[3]);
+              }
+            }
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            const int t = t0 + 8 * hr + pos[v];
+            if (t >= nrow) continue;
+            const int64_t d = dbase + pair_of(t) * dstr;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (cc[h] >= m) continue;
+              float dsum[S];
+#pragma unroll
+              for (int i = 0; i < S; ++i) dsum[i] = a2[i][2 * h + v];
+              W[(int64_t)cc[h] * ldw + d] =
+                  wv[h][2 * hr + v] + oz_round<S, T>(dsum) * oz_scale<T>(ex[h] + ee[2 * hr + v] + TSH);
+            }
           }
         }
       }
     }
-#pragma unroll
-    for (int n = 0; n < 2 * KT; ++n)
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const int k = 8 * n + 2 * tig + v;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (k >= no || cc[h] >= m) continue;
-          float dsum[S];
-#pragma unroll
-          for (int i = 0; i < S; ++i) dsum[i] = a1[n][i][2 * h + v];
-          const double w = oz_sum<S>(dsum) * oz_pow2(ev[h] + TSH);
-          if (!(w == 0.0)) atomicAdd(&W1[(int64_t)cc[h] * ld1 + (int64_t)f * no + k], (TA)w);
-        }
-      }
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
 }
@@ -1220,7 +1240,8 @@ int oz_upload_lists(Ctx* c, OzPlan* p, int item_rows, int m) {
   std::vector<unsigned char> all(lb);
   std::copy_n(reinterpret_cast<const unsigned char*>(p->h_items.data()), sizeof(OzItem) * ni, all.data());
   std::copy_n(reinterpret_cast<const unsigned char*>(p->h_slabs.data()), sizeof(OzSlab) * ns, all.data() + ib);
-  ADC_CUDA(c, h2d(c, p->items, all.data(), lb));
+  // pageable source: staged before the call returns, no need to wait
+  ADC_CUDA(c, cudaMemcpyAsync(p->items, all.data(), lb, cudaMemcpyHostToDevice, c->stream));
   p->item_rows = item_rows;
   p->lists_m = m;
   return ADCGPU_OK;
@@ -1250,14 +1271,19 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
   const OzBytes need = oz_bytes(G, row0, row1, S, &dst);
   const size_t bytes = std::max(need.all, (size_t)reserve);
   if (p->mem_bytes < bytes) {
-    size_t free_b = 0, total_b = 0;
-    ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
-    if (bytes > (free_b + p->mem_bytes) / 3) return ADCGPU_OK;
+    // below 64 MB the question costs more than the answer is worth (40 us)
+    if (bytes > (64u << 20)) {
+      size_t free_b = 0, total_b = 0;
+      ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+      if (bytes > (free_b + p->mem_bytes) / 3) return ADCGPU_OK;
+    }
     dfree(c, p->d_mem);
     p->d_mem = nullptr;
     p->mem_bytes = 0;
     p->values_for = nullptr;
-    ST(dmalloc(c, (void**)&p->d_mem, bytes));
+    const int st = dmalloc(c, (void**)&p->d_mem, bytes);
+    if (st == ADCGPU_OUT_OF_MEMORY) return ADCGPU_OK;
+    ST(st);
     p->mem_bytes = bytes;
   }
   if (!(p->values_for && p->values_for == values && p->S == S && p->dst.row0 == row0 && p->dst.row1 == row1)) {
@@ -1443,8 +1469,8 @@ int oz_seg_go(Ctx* c, OzPlan* p, const T* V, int64_t ldv, int m, T* W, int64_t l
   const size_t smem = (size_t)SEG_WARPS * 2 * 16 * seg_pitch<S, KT>();
   ADC_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int ngrp = (m + 15) / 16;
-  const int64_t nrun = (int64_t)p->nslab * ngrp * (p->geom.nv - 1);
-  const int grid = (int)std::min<int64_t>((nrun + SEG_WARPS - 1) / SEG_WARPS, (int64_t)c->nsm * 16);
+  const int64_t nblk = ((int64_t)p->nslab * ngrp * (p->geom.nv - 1) + SEG_WARPS / 2 - 1) / (SEG_WARPS / 2);
+  const int grid = (int)std::min<int64_t>(nblk, (int64_t)c->nsm * 16);
   kern<<<grid, 32 * SEG_WARPS, smem, c->stream>>>(p->geom, p->slabs + p->slab0, p->nslab, ngrp, p->item0, p->seg, p->sexp,
                                                   p->vsexp, V, ldv, m, W, ldw, W1, ld1);
   ADC_COUNT_LAUNCH();
