@@ -17,8 +17,11 @@
 // One CTA per (row block, 128-column tile of A), 256 threads: all threads
 // load the next 64 rows of their columns into registers while the tensor
 // cores work on the current ones, split them and store the slices into a
-// 3-stage ring of 128-byte-swizzled K-major operand tiles; thread 0 issues
-// the MMAs (24 per 64 rows) and commits them to mbarriers; threads 0-127
+// 3-stage ring of 128-byte-swizzled K-major operand tiles; one elected lane of
+// warp 0 issues the MMAs (24 per 64 rows; the warp takes the branch together,
+// which keeps descriptors in uniform registers: thread 0 alone took about 200
+// cycles an instruction, 165 us for any p <= 128 at N = 610,000) and commits
+// them to mbarriers; threads 0-127
 // (the 128 TMEM lanes) drain the accumulator every 128 rows.  TMEM holds two
 // accumulators, so the MMAs of the next 128 rows run while one is drained.
 // Every wait is bounded; a wait that gives up sets the error word and the
@@ -102,12 +105,16 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
 
   // this thread's columns: A columns m0 + warp + 8u (u < 16), B columns
   // warp + 8u (u < NB); rows r0 + 2 lane, r0 + 2 lane + 1 of each stage
+  // (only the A columns below p: the other rows of the operand tile, whatever
+  // they hold, feed output rows that nothing reads)
+  const int nu = min(GU_M / 8, (p - m0 + 7) / 8);
   float2 pa[GU_M / 8], pb[NB];
   auto fetch = [&](int i) {
     const int64_t r = r_begin + (int64_t)i * GU_K + 2 * lane;
     const bool ok0 = r < r_end, ok1 = r + 1 < r_end;
 #pragma unroll
     for (int u = 0; u < GU_M / 8; ++u) {
+      if (u >= nu) break;
       const int m = m0 + warp + 8 * u;
       const float* col = A + (int64_t)m * lda;
       pa[u].x = (m < p && ok0) ? __ldg(col + r) : 0.f;
@@ -126,6 +133,7 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
     unsigned char* sb = sa + 3 * GU_A_SLICE;
 #pragma unroll
     for (int u = 0; u < GU_M / 8; ++u) {
+      if (u >= nu) break;
       const uint32_t off = sw128_off(warp + 8 * u, 2 * lane);
       __nv_bfloat162 s0, s1, s2;
       split3(pa[u].x, pa[u].y, s0, s1, s2);
@@ -167,6 +175,8 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
     return true;
   };
 
+  constexpr uint64_t KMAJ = sdesc(0, 16, 1024, LAYOUT_SW128);
+  constexpr uint32_t idesc = idesc_bf16(GU_M, NQ, 0, 0);
   const int ngrp = (nch + GU_F - 1) / GU_F;
   int drained = 0, issued = 0;
   bool ok = true;
@@ -186,25 +196,23 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
       ok = false;
       break;
     }
-    if (tid == 0) {
+    if (warp == 0) {
       fence_after_sync();
       const int grp = i / GU_F;
-      const uint32_t idesc = idesc_bf16(GU_M, NQ, 0, 0);
-      const uint32_t sa = smem_u32(base + (size_t)s * SB), sb = sa + 3 * GU_A_SLICE;
+      const uint64_t ad = KMAJ + (smem_u32(base + (size_t)s * SB) >> 4), bd = ad + 3 * GU_A_SLICE / 16;
       const uint32_t d = tacc + (uint32_t)((grp & 1) * NQ);
       constexpr int PA[6] = {0, 0, 1, 0, 1, 2}, PB[6] = {0, 1, 0, 2, 1, 0};
-      uint32_t accum = (i % GU_F) ? 1u : 0u;
+      if (elect_one()) {
+        mma_bf16(d, ad, bd, idesc, (i % GU_F) ? 1u : 0u);
 #pragma unroll
-      for (int pr = 0; pr < 6; ++pr)
+        for (int pr = 0; pr < 6; ++pr)
 #pragma unroll
-        for (int ks = 0; ks < GU_K / 16; ++ks) {
-          const uint64_t ad = sdesc(sa + PA[pr] * GU_A_SLICE + ks * 32, 16, 1024, LAYOUT_SW128);
-          const uint64_t bd = sdesc(sb + PB[pr] * B_SLICE + ks * 32, 16, 1024, LAYOUT_SW128);
-          mma_bf16(d, ad, bd, idesc, accum);
-          accum = 1u;
-        }
-      mma_commit(&mma_done[s]);
-      if (i % GU_F == GU_F - 1 || i == nch - 1) mma_commit(&acc_full[grp & 1]);
+          for (int ks = pr == 0 ? 1 : 0; ks < GU_K / 16; ++ks)
+            mma_bf16_c<true>(d, ad + PA[pr] * (GU_A_SLICE / 16) + 2 * ks, bd + PB[pr] * (B_SLICE / 16) + 2 * ks, idesc);
+        mma_commit(&mma_done[s]);
+        if (i % GU_F == GU_F - 1 || i == nch - 1) mma_commit(&acc_full[grp & 1]);
+      }
+      __syncwarp();
       issued = i + 1;
     }
     // the previous accumulator is complete once the first stage of the next
