@@ -14,16 +14,14 @@
 // double-float registers (df.h), and the per-block partials are summed in
 // FP64 in a fixed order, as the CUDA-core kernel of dense.cu does.
 //
-// One CTA per (row block, 128-column tile of A), 256 threads: all threads
-// load the next 64 rows of their columns into registers while the tensor
-// cores work on the current ones, split them and store the slices into a
-// 3-stage ring of 128-byte-swizzled K-major operand tiles; one elected lane of
-// warp 0 issues the MMAs (24 per 64 rows; the warp takes the branch together,
-// which keeps descriptors in uniform registers: thread 0 alone took about 200
-// cycles an instruction, 165 us for any p <= 128 at N = 610,000) and commits
-// them to mbarriers; threads 0-127
-// (the 128 TMEM lanes) drain the accumulator every 128 rows.  TMEM holds two
-// accumulators, so the MMAs of the next 128 rows run while one is drained.
+// One CTA per (row block, 128-column tile of A), warp-specialised: 16 producer
+// warps hold the next two 64-row stages of their columns in registers, split
+// them and store the slices into a 3-stage ring of 128-byte-swizzled K-major
+// operand tiles; one warp issues the MMAs (24 per stage, by an elected lane:
+// one thread walking them alone took about 200 cycles each, 165 us a product
+// of any p <= 128 at N = 610,000); eight warps drain the accumulator every 128
+// rows.  TMEM holds two accumulators, so the MMAs of the next 128 rows run
+// while one is drained.
 // Every wait is bounded; a wait that gives up sets the error word and the
 // call returns ADCGPU_DEVICE_TIMEOUT.
 #include <cuda_bf16.h>
@@ -41,7 +39,8 @@ using namespace umma;
 
 namespace {
 
-constexpr int GU_THREADS = 256;
+constexpr int GU_WARPS = 16;   // producer warps
+constexpr int GU_THREADS = 32 * (GU_WARPS + 8 + 1);   // and 8 drain warps, 1 MMA issuer
 constexpr int GU_M = 128;      // A columns per CTA (MMA M)
 constexpr int GU_K = 64;       // rows per stage: one 128-byte swizzled row of 64 BF16 values
 constexpr int GU_NS = 3;       // ring stages
@@ -56,10 +55,8 @@ __host__ __device__ constexpr uint32_t gu_tmem_cols() { return 2 * NQ <= 32 ? 32
 
 template <int NQ>
 __host__ __device__ constexpr size_t gu_smem_bytes() {
-  return 1024 + (size_t)GU_NS * gu_stage_bytes<NQ>() + 8 * (GU_NS + 2) + 16;
+  return 1024 + (size_t)GU_NS * gu_stage_bytes<NQ>() + 8 * (2 * GU_NS + 4) + 16;
 }
-
-__device__ __forceinline__ bool gu_failed(const int* err) { return *(const volatile int*)err != 0; }
 
 // three BF16 slices of a pair of FP32 values (stored as bf16x2 words)
 __device__ __forceinline__ void split3(float x, float y, __nv_bfloat162& s0, __nv_bfloat162& s1,
@@ -79,14 +76,17 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
                 int64_t ldb, int64_t rows_per_blk, double* __restrict__ part, int* __restrict__ err) {
   constexpr int SB = gu_stage_bytes<NQ>();
   constexpr int B_SLICE = NQ * 128;
-  constexpr int NB = NQ / 8;          // B columns per warp
+  constexpr int NA = GU_M / GU_WARPS, NB = NQ / GU_WARPS;   // A and B columns per warp
+  constexpr int NH = NQ / 2;          // C columns per drain warp
   constexpr uint32_t TCOLS = gu_tmem_cols<NQ>();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + (size_t)GU_NS * SB);
-  uint64_t* mma_done = bars;                 // [GU_NS]
-  uint64_t* acc_full = bars + GU_NS;         // [2]
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + GU_NS + 2);
+  uint64_t* full = bars;                     // [GU_NS] operands of a stage stored
+  uint64_t* mma_done = bars + GU_NS;         // [GU_NS] and read
+  uint64_t* acc_full = bars + 2 * GU_NS;     // [2]
+  uint64_t* acc_empty = acc_full + 2;        // [2]
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * GU_M;
@@ -95,7 +95,14 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
   const int nch = r_begin < r_end ? (int)((r_end - r_begin + GU_K - 1) / GU_K) : 0;
 
   if (tid == 0) {
-    for (int i = 0; i < GU_NS + 2; ++i) mbar_init(&bars[i], 1u);
+    for (int i = 0; i < GU_NS; ++i) {
+      mbar_init(&full[i], GU_WARPS);
+      mbar_init(&mma_done[i], 1u);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc_full[i], 1u);
+      mbar_init(&acc_empty[i], 8u);
+    }
   }
   if (warp == 0) tmem_alloc(tmem_holder, TCOLS);
   fence_before_sync();
@@ -103,105 +110,121 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
   fence_after_sync();
   const uint32_t tacc = *tmem_holder;
 
-  // this thread's columns: A columns m0 + warp + 8u (u < 16), B columns
-  // warp + 8u (u < NB); rows r0 + 2 lane, r0 + 2 lane + 1 of each stage
-  // (only the A columns below p: the other rows of the operand tile, whatever
-  // they hold, feed output rows that nothing reads)
-  const int nu = min(GU_M / 8, (p - m0 + 7) / 8);
-  float2 pa[GU_M / 8], pb[NB];
-  auto fetch = [&](int i) {
-    const int64_t r = r_begin + (int64_t)i * GU_K + 2 * lane;
-    const bool ok0 = r < r_end, ok1 = r + 1 < r_end;
-#pragma unroll
-    for (int u = 0; u < GU_M / 8; ++u) {
-      if (u >= nu) break;
-      const int m = m0 + warp + 8 * u;
-      const float* col = A + (int64_t)m * lda;
-      pa[u].x = (m < p && ok0) ? __ldg(col + r) : 0.f;
-      pa[u].y = (m < p && ok1) ? __ldg(col + r + 1) : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      const int n = warp + 8 * u;
-      const float* col = B + (int64_t)n * ldb;
-      pb[u].x = (n < q && ok0) ? __ldg(col + r) : 0.f;
-      pb[u].y = (n < q && ok1) ? __ldg(col + r + 1) : 0.f;
-    }
-  };
-  auto store = [&](int s) {
-    unsigned char* sa = base + (size_t)s * SB;
-    unsigned char* sb = sa + 3 * GU_A_SLICE;
-#pragma unroll
-    for (int u = 0; u < GU_M / 8; ++u) {
-      if (u >= nu) break;
-      const uint32_t off = sw128_off(warp + 8 * u, 2 * lane);
-      __nv_bfloat162 s0, s1, s2;
-      split3(pa[u].x, pa[u].y, s0, s1, s2);
-      *reinterpret_cast<__nv_bfloat162*>(sa + off) = s0;
-      *reinterpret_cast<__nv_bfloat162*>(sa + GU_A_SLICE + off) = s1;
-      *reinterpret_cast<__nv_bfloat162*>(sa + 2 * GU_A_SLICE + off) = s2;
-    }
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-      const uint32_t off = sw128_off(warp + 8 * u, 2 * lane);
-      __nv_bfloat162 s0, s1, s2;
-      split3(pb[u].x, pb[u].y, s0, s1, s2);
-      *reinterpret_cast<__nv_bfloat162*>(sb + off) = s0;
-      *reinterpret_cast<__nv_bfloat162*>(sb + B_SLICE + off) = s1;
-      *reinterpret_cast<__nv_bfloat162*>(sb + 2 * B_SLICE + off) = s2;
-    }
-  };
-  // double-float sums of this thread's row (TMEM lane = tid < 128) of C
-  df acc[NQ];
-#pragma unroll
-  for (int j = 0; j < NQ; ++j) acc[j] = df{0.f, 0.f};
-  const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
-  auto drain = [&](int grp) -> bool {
-    // threads 0-127 read accumulator grp & 1 once its MMAs are complete
-    if (tid < GU_M) {
-      // tcgen05.ld is warp-aligned: the warp leaves together if any lane's
-      // wait gave up
-      const bool w = mbar_wait(&acc_full[grp & 1], (uint32_t)(grp >> 1) & 1u, err, 3);
-      if (!__all_sync(0xffffffffu, w)) return false;
-      fence_after_sync();
-#pragma unroll
-      for (int j0 = 0; j0 < NQ; j0 += 8) {
-        float v[8];
-        tmem_ld8(tacc + (uint32_t)((grp & 1) * NQ + j0) + lane_off, v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j0 + j] = df_add(acc[j0 + j], df{v[j], 0.f});
-      }
-    }
-    return true;
-  };
-
-  constexpr uint64_t KMAJ = sdesc(0, 16, 1024, LAYOUT_SW128);
-  constexpr uint32_t idesc = idesc_bf16(GU_M, NQ, 0, 0);
   const int ngrp = (nch + GU_F - 1) / GU_F;
-  int drained = 0, issued = 0;
-  bool ok = true;
-  if (nch > 0) fetch(0);
-  for (int i = 0; i < nch; ++i) {
-    const int s = i % GU_NS;
-    // the stage's previous MMAs (chunk i - GU_NS) have read it
-    if (ok && i >= GU_NS) ok = mbar_wait(&mma_done[s], (uint32_t)((i - GU_NS) / GU_NS) & 1u, err, 1);
-    if (ok) {
-      store(s);
+  if (warp < GU_WARPS) {
+    // ------------------------------------------------------------ producers
+    // this thread's columns: A columns m0 + warp + 16u, B columns warp + 16u;
+    // rows r0 + 2 lane, r0 + 2 lane + 1 of each stage
+    // (only the A columns below p: the other rows of the operand tile, whatever
+    // they hold, feed output rows that nothing reads)
+    const int nu = min(NA, (p - m0 - warp + GU_WARPS - 1) / GU_WARPS);
+    const float* const colA = A + (int64_t)(m0 + warp) * lda + r_begin + 2 * lane;
+    const float* const colB = B + (int64_t)warp * ldb + r_begin + 2 * lane;
+    const int64_t nrow = r_end - r_begin;
+    // 8-byte loads where every column allows them (r_begin is a multiple of 64)
+    const bool pairs = ((lda | ldb) & 1) == 0 && (((uintptr_t)A | (uintptr_t)B) & 7) == 0;
+    struct Stage {
+      float2 a[NA], b[NB];
+    };
+    auto fetch = [&](int i, Stage& x) {
+      const int64_t o = (int64_t)i * GU_K;
+      const float* pa = colA + o;
+      const float* pb = colB + o;
+      const bool ok0 = o + 2 * lane < nrow, ok1 = o + 2 * lane + 1 < nrow;
+#pragma unroll
+      for (int u = 0; u < NA; ++u, pa += GU_WARPS * lda) {
+        if (u >= nu) break;
+        if (pairs && ok1) {
+          x.a[u] = __ldg(reinterpret_cast<const float2*>(pa));
+        } else {
+          x.a[u].x = ok0 ? __ldg(pa) : 0.f;
+          x.a[u].y = ok1 ? __ldg(pa + 1) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < NB; ++u, pb += GU_WARPS * ldb) {
+        const bool in = warp + GU_WARPS * u < q;
+        if (pairs && ok1 && in) {
+          x.b[u] = __ldg(reinterpret_cast<const float2*>(pb));
+        } else {
+          x.b[u].x = in && ok0 ? __ldg(pb) : 0.f;
+          x.b[u].y = in && ok1 ? __ldg(pb + 1) : 0.f;
+        }
+      }
+    };
+    auto put = [&](unsigned char* at, int slice, const float2& x) {
+      __nv_bfloat162 s0, s1, s2;
+      split3(x.x, x.y, s0, s1, s2);
+      *reinterpret_cast<__nv_bfloat162*>(at) = s0;
+      *reinterpret_cast<__nv_bfloat162*>(at + slice) = s1;
+      *reinterpret_cast<__nv_bfloat162*>(at + 2 * slice) = s2;
+    };
+    // one stage: P holds its values, and those two stages on afterwards
+    auto step = [&](int i, Stage& P) -> bool {
+      const int s = i % GU_NS;
+      if (!mbar_wait_warp(&mma_done[s], ((uint32_t)(i / GU_NS) & 1u) ^ 1u, err, 1)) return false;
+      unsigned char* sa = base + (size_t)s * SB;
+#pragma unroll
+      for (int u = 0; u < NA; ++u) {
+        if (u >= nu) break;
+        put(sa + sw128_off(warp + GU_WARPS * u, 2 * lane), GU_A_SLICE, P.a[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < NB; ++u)
+        put(sa + 3 * GU_A_SLICE + sw128_off(warp + GU_WARPS * u, 2 * lane), B_SLICE, P.b[u]);
       fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[s]);
+      if (i + 2 < nch) fetch(i + 2, P);
+      return true;
+    };
+    Stage even, odd;
+    if (nch > 0) fetch(0, even);
+    if (nch > 1) fetch(1, odd);
+    for (int i = 0; i < nch; i += 2) {
+      if (!step(i, even)) break;
+      if (i + 1 < nch && !step(i + 1, odd)) break;
     }
-    if (i + 1 < nch) fetch(i + 1);
-    // every thread takes the same branch: a failed wait anywhere ends the loop
-    // for the whole CTA, so no thread is left at a barrier
-    if (!__syncthreads_and(ok && !gu_failed(err))) {
-      ok = false;
-      break;
-    }
-    if (warp == 0) {
+  } else if (warp < GU_WARPS + 8) {
+    // --------------------------------------------------------------- drains
+    // double-float sums of row 32 (warp & 3) + lane (its TMEM lane) of C
+    const int half = (warp - GU_WARPS) >> 2;
+    df acc[NH];
+#pragma unroll
+    for (int j = 0; j < NH; ++j) acc[j] = df{0.f, 0.f};
+    const uint32_t at = tacc + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(half * NH);
+    for (int grp = 0; grp < ngrp; ++grp) {
+      const int ab = grp & 1;
+      if (!mbar_wait_warp(&acc_full[ab], (uint32_t)(grp >> 1) & 1u, err, 3)) break;
       fence_after_sync();
-      const int grp = i / GU_F;
+      float v[NH];
+#pragma unroll
+      for (int j0 = 0; j0 < NH; j0 += 8) tmem_ld8(at + (uint32_t)(ab * NQ + j0), *reinterpret_cast<float(*)[8]>(v + j0));
+      fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[ab]);
+#pragma unroll
+      for (int j = 0; j < NH; ++j) acc[j] = df_add(acc[j], df{v[j], 0.f});
+    }
+    double* out = part + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (GU_M * NQ) +
+                  (int64_t)(32 * (warp & 3) + lane) * NQ + half * NH;
+#pragma unroll
+    for (int j = 0; j < NH; ++j) out[j] = df_value(acc[j]);
+  } else {
+    // ----------------------------------------------------------- MMA issuer
+    constexpr uint64_t KMAJ = sdesc(0, 16, 1024, LAYOUT_SW128);
+    constexpr uint32_t idesc = idesc_bf16(GU_M, NQ, 0, 0);
+    constexpr int PA[6] = {0, 0, 1, 0, 1, 2}, PB[6] = {0, 1, 0, 2, 1, 0};
+    int issued = 0;
+    for (int i = 0; i < nch; ++i) {
+      const int s = i % GU_NS, grp = i / GU_F, ab = grp & 1;
+      bool ok = true;
+      if (i % GU_F == 0) ok = mbar_wait_warp(&acc_empty[ab], ((uint32_t)(grp >> 1) & 1u) ^ 1u, err, 2);
+      ok = ok && mbar_wait_warp(&full[s], (uint32_t)(i / GU_NS) & 1u, err, 5);
+      if (!ok) break;
+      fence_after_sync();
       const uint64_t ad = KMAJ + (smem_u32(base + (size_t)s * SB) >> 4), bd = ad + 3 * GU_A_SLICE / 16;
-      const uint32_t d = tacc + (uint32_t)((grp & 1) * NQ);
-      constexpr int PA[6] = {0, 0, 1, 0, 1, 2}, PB[6] = {0, 1, 0, 2, 1, 0};
+      const uint32_t d = tacc + (uint32_t)(ab * NQ);
       if (elect_one()) {
         mma_bf16(d, ad, bd, idesc, (i % GU_F) ? 1u : 0u);
 #pragma unroll
@@ -210,30 +233,16 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
           for (int ks = pr == 0 ? 1 : 0; ks < GU_K / 16; ++ks)
             mma_bf16_c<true>(d, ad + PA[pr] * (GU_A_SLICE / 16) + 2 * ks, bd + PB[pr] * (B_SLICE / 16) + 2 * ks, idesc);
         mma_commit(&mma_done[s]);
-        if (i % GU_F == GU_F - 1 || i == nch - 1) mma_commit(&acc_full[grp & 1]);
+        if (i % GU_F == GU_F - 1 || i == nch - 1) mma_commit(&acc_full[ab]);
       }
       __syncwarp();
       issued = i + 1;
     }
-    // the previous accumulator is complete once the first stage of the next
-    // one is issued: drain it while the tensor cores work (its result joins
-    // the next iteration's vote)
-    if (i % GU_F == 0 && i > 0) {
-      if (!drain(drained)) ok = false;
-      ++drained;
-      fence_before_sync();
-    }
-  }
-  while (ok && drained < ngrp) {
-    if (!drain(drained)) ok = false;
-    ++drained;
-  }
-  // no MMA may still be running when TMEM is released: wait (bounded) for the
-  // last commit of every stage
-  if (tid == 0) {
+    // no MMA may still be running when TMEM is released: wait (bounded) for
+    // the last commit of every stage
     for (int k = 0; k < GU_NS && k < issued; ++k) {
       const int i = issued - 1 - k;
-      mbar_wait(&mma_done[i % GU_NS], (uint32_t)(i / GU_NS) & 1u, err, 4);
+      mbar_wait_warp(&mma_done[i % GU_NS], (uint32_t)(i / GU_NS) & 1u, err, 4);
     }
   }
   fence_before_sync();
@@ -242,11 +251,6 @@ __global__ void __launch_bounds__(GU_THREADS, 1)
   if (warp == 0) {
     tmem_dealloc(tacc, TCOLS);
     tmem_relinquish();
-  }
-  if (tid < GU_M) {
-    double* out = part + ((int64_t)blockIdx.x * gridDim.y + blockIdx.y) * (GU_M * NQ) + (int64_t)tid * NQ;
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) out[j] = df_value(acc[j]);
   }
 }
 
@@ -315,9 +319,9 @@ int gram_umma(Ctx* c, Workspace& ws, int64_t N, int p, int q, const float* A, in
   }
   const int nq = q <= 16 ? 16 : (q <= 32 ? 32 : 48);
   const int ntile = (p + GU_M - 1) / GU_M;
-  // at most two blocks per SM over all column tiles (one CTA fits an SM, so
-  // that is two full waves), each row block a multiple of the stage height
-  const int64_t want = std::max<int64_t>(1, ((int64_t)c->nsm * 2) / ntile);
+  // one block per SM over all column tiles (one fits an SM), each row block a
+  // multiple of the stage height
+  const int64_t want = std::max<int64_t>(1, (int64_t)c->nsm / ntile);
   const int64_t rows = std::max<int64_t>(GU_K, ((N + want - 1) / want + GU_K - 1) / GU_K * GU_K);
   const int nblk = (int)((N + rows - 1) / rows);
   ST(ws.reserve(c, sizeof(double) * (size_t)nblk * ntile * GU_M * nq));
