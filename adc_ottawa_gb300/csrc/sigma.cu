@@ -1207,36 +1207,49 @@ __global__ void __launch_bounds__(256) k_singles(int n1, const T* __restrict__ A
   if (r < n1 && c < m) W[(int64_t)c * ldw + r] = diag[r] * V[(int64_t)c * ldv + r] + acc;
 }
 
-// W1 = diag1 . V1 + A V1 as a register-tiled GEMM: block tile 32 rows x 32
-// columns, K staged 32 at a time, 128 threads with 4 x 2 outputs each.
+// W1 = diag1 . V1 + A V1 as a register-tiled GEMM: 128 threads with 4 x 2
+// outputs each, 2 txn columns and 4 (128 / txn) rows a block, K staged 32 at a
+// time.  In FP64 the pipe bounds it and the tile follows the column count (a
+// fixed 32 columns took 77 us for 10 at n1 = 1,100; 41 us more than now).  Small blocks and
+// FP32 are bound by latency and keep 32 columns, whose shorter tiles make more
+// blocks (n1 = 95, 1 column: 2 us less; FP32, n1 = 909, 5 columns: 4 us less).
 // Used by the sigma product and by the folded preconditioner's MINRES.
+constexpr int SG_MINTX = 4, SG_ROWS = 4 * (128 / SG_MINTX);
+// column pairs of a block tile: the columns in equal parts of at most 32
+template <typename T>
+inline int singles_txn(int n1, int m) {
+  if (sizeof(T) < 8 || n1 < 512) return 16;
+  const int ng = (m + 31) / 32;
+  return std::max(SG_MINTX, ((m + ng - 1) / ng + 1) / 2);
+}
 template <typename T>
 __global__ void __launch_bounds__(128) k_singles_gemm(int n1, const T* __restrict__ A, const T* __restrict__ diag,
                                                       const T* __restrict__ V, int64_t ldv, T* __restrict__ W,
-                                                      int64_t ldw, int m, T* __restrict__ part = nullptr,
+                                                      int64_t ldw, int m, int txn, T* __restrict__ part = nullptr,
                                                       int kchunk = 0) {
-  __shared__ __align__(16) T sA[32][36];   // sA[k][r]
-  __shared__ T sV[32][33];                 // sV[k][c]
+  __shared__ __align__(16) T sA[32][SG_ROWS + 4];   // sA[k][r]
+  __shared__ T sV[32][33];                          // sV[k][c]
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;   // columns 2tx, 2tx+1; rows 4ty..4ty+3
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  const int tx = tid % txn, ty = tid / txn;   // columns 2tx, 2tx+1; rows 4ty..4ty+3
+  const int rows = 4 * (128 / txn), cols = 2 * txn;
+  const bool act = 4 * ty < rows;
+  const int r0 = blockIdx.x * rows, c0 = blockIdx.y * cols;
   T acc[4][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i) { acc[i][0] = T(0); acc[i][1] = T(0); }
   // split K (part != null): this block sums k in [kbeg, kend) into part
   const int kbeg = part ? blockIdx.z * kchunk : 0;
   const int kend = part ? min(n1, kbeg + kchunk) : n1;
+  const int kk0 = tid & 31, rr0 = tid >> 5;
   for (int k0 = kbeg; k0 < kend; k0 += 32) {
+    const int k = k0 + kk0;
     __syncthreads();
-#pragma unroll
-    for (int l = tid; l < 32 * 32; l += 128) {
-      const int kk = l & 31, rr = l >> 5;
-      const int r = r0 + rr, k = k0 + kk;
-      sA[kk][rr] = (r < n1 && k < kend) ? A[(int64_t)r * n1 + k] : T(0);
-      const int c = c0 + rr;
-      sV[kk][rr] = (c < m && k < kend) ? V[(int64_t)c * ldv + k] : T(0);
-    }
+#pragma unroll 8
+    for (int rr = rr0; rr < rows; rr += 4) sA[kk0][rr] = (r0 + rr < n1 && k < kend) ? A[(int64_t)(r0 + rr) * n1 + k] : T(0);
+#pragma unroll 4
+    for (int cc = rr0; cc < cols; cc += 4) sV[kk0][cc] = (c0 + cc < m && k < kend) ? V[(int64_t)(c0 + cc) * ldv + k] : T(0);
     __syncthreads();
+    if (!act) continue;
 #pragma unroll 8
     for (int kk = 0; kk < 32; ++kk) {
       T a[4];
@@ -1247,6 +1260,7 @@ __global__ void __launch_bounds__(128) k_singles_gemm(int n1, const T* __restric
       for (int i = 0; i < 4; ++i) { acc[i][0] += a[i] * b0; acc[i][1] += a[i] * b1; }
     }
   }
+  if (!act) return;
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int c = c0 + 2 * tx + j;
@@ -1277,8 +1291,9 @@ __global__ void k_singles_reduce(int n1, int m, int ks, const T* __restrict__ pa
 template <typename T>
 void launch_singles(Ctx* c, int m, const T* A, const T* diag, const T* V, int64_t ldv, T* W, int64_t ldw) {
   const int n1 = (int)c->geom.n1;
-  dim3 grid((n1 + 31) / 32, (m + 31) / 32);
-  k_singles_gemm<T><<<grid, 128, 0, c->stream>>>(n1, A, diag, V, ldv, W, ldw, m); ADC_COUNT_LAUNCH();
+  const int txn = singles_txn<T>(n1, m), rows = 4 * (128 / txn);
+  dim3 grid((n1 + rows - 1) / rows, (m + 2 * txn - 1) / (2 * txn));
+  k_singles_gemm<T><<<grid, 128, 0, c->stream>>>(n1, A, diag, V, ldv, W, ldw, m, txn); ADC_COUNT_LAUNCH();
 }
 
 // Singles block with K split over about four blocks per SM: the unsplit grid
@@ -1289,8 +1304,9 @@ void launch_singles(Ctx* c, int m, const T* A, const T* diag, const T* V, int64_
 template <typename T>
 int launch_singles_split(Ctx* c, int m, const T* A, const T* diag, const T* V, int64_t ldv, T* W, int64_t ldw) {
   const int n1 = (int)c->geom.n1;
-  const int base = ((n1 + 31) / 32) * ((m + 31) / 32);
-  const int ks = std::max(1, std::min(16, (4 * c->nsm + base - 1) / base));
+  const int txn = singles_txn<T>(n1, m), rows = 4 * (128 / txn);
+  const int base = ((n1 + rows - 1) / rows) * ((m + 2 * txn - 1) / (2 * txn));
+  const int ks = std::max(1, std::min(32, (4 * c->nsm + base - 1) / base));
   SigmaPlan* plan = reinterpret_cast<SigmaPlan*>(c->sigma_plan);
   if (ks == 1 || !plan) {
     launch_singles<T>(c, m, A, diag, V, ldv, W, ldw);
@@ -1307,8 +1323,8 @@ int launch_singles_split(Ctx* c, int m, const T* A, const T* diag, const T* V, i
     plan->sk_bytes = need;
   }
   T* part = reinterpret_cast<T*>(plan->d_sk);
-  dim3 grid((n1 + 31) / 32, (m + 31) / 32, ksu);
-  k_singles_gemm<T><<<grid, 128, 0, c->stream>>>(n1, A, diag, V, ldv, W, ldw, m, part, kchunk);
+  dim3 grid((n1 + rows - 1) / rows, (m + 2 * txn - 1) / (2 * txn), ksu);
+  k_singles_gemm<T><<<grid, 128, 0, c->stream>>>(n1, A, diag, V, ldv, W, ldw, m, txn, part, kchunk);
   ADC_COUNT_LAUNCH();
   k_singles_reduce<T><<<std::min((n1 * m + 255) / 256, c->nsm * 8), 256, 0, c->stream>>>(n1, m, ksu, part, diag,
                                                                                           V, ldv, W, ldw);
