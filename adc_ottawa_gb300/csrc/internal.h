@@ -443,13 +443,17 @@ int gram_set_off(Ctx* c, int off);
 
 // sigma_umma.cu : the tensor-core (tcgen05) pass of the BF16 sigma product
 bool umma_supported(const Ctx* c);
-int umma_prepare(Ctx* c, void*& handle, int item_rows);
+int umma_prepare(Ctx* c, void*& handle);
 void umma_free(Ctx* c, void*& handle);
 int umma_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float* W, int64_t ldw, double* W1,
                 int64_t ld1, int seg_a);
 int umma_runs(void* handle, const int2** runs, int* nruns);
 bool umma_geometry_ok(const Geometry& G);
-int umma_item_rows(const Ctx* c);
+// Rows (whole 128-row tiles, at most 32) of the work items that nslab slabs of
+// len rows are cut into, for kernels with one persistent block per SM that
+// take the items in turn: the size that makes the fullest rounds, an item
+// costing its tiles plus 'overhead' tiles (operand of the singles, W1 atomics).
+int item_rows_for(const Ctx* c, int64_t nslab, int64_t len, int groups, double overhead);
 bool umma3_supported(const Ctx* c);
 int umma3_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float* W, int64_t ldw, double* W1,
                  int64_t ld1);

@@ -1519,7 +1519,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
       // W2 part of segment A, then segment B (pass 2) and the W1 part of
       // segment A (pass 3), up to 48 columns per matrix pass
       if (allow_umma && P->tiled == 1 && !P->umma_off && umma_supported(c)) {
-        ST(umma_prepare(c, plan->umma, umma_item_rows(c)));
+        ST(umma_prepare(c, plan->umma));
         const int2* runs = nullptr;
         int nruns = 0;
         ST(umma_runs(plan->umma, &runs, &nruns));
@@ -1558,7 +1558,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
       // FP32 store, up to 32 columns per matrix pass
       if (allow_umma && P->umma3_on && P->tiled == 1 && !P->umma_off && !P->ab_off && !c->direct &&
           umma3_supported(c) && ab_supported(c)) {
-        ST(umma_prepare(c, plan->umma, umma_item_rows(c)));
+        ST(umma_prepare(c, plan->umma));
         for (; c0 < m;) {
           const int nc = std::min(m - c0, 32);
           const T* V = dV + (int64_t)c0 * ldv;

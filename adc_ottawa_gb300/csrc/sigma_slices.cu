@@ -1202,13 +1202,8 @@ std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, i
 
 namespace {
 
-// rows per work item: about six items per SM over the column groups of the
-// prepared rows, 1 to 32 tiles (the vector operand of an item costs about a
-// third of a tile)
-int oz_item_rows(const Ctx* c, int64_t rows, int m) {
-  const int64_t want = rows * ((m + 15) / 16) / ((int64_t)c->nsm * 6);
-  return (int)std::min<int64_t>(4096, std::max<int64_t>(128, (want + 127) / 128 * 128));
-}
+// an item's vector operand in tiles (about a third) and its last drains
+constexpr double OZ_ITEM_OVERHEAD = 0.5;
 
 // the work items of one slab, in equal pieces of whole tiles
 void oz_add_slab(OzPlan* p, int64_t s0, int64_t len, int item_rows, int holes, bool pairs, int64_t dbase, int dstr) {
@@ -1316,7 +1311,11 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
     it.tile = (int)(dst.base[cls] / ((int64_t)S * OZ_ROWS * OZ_BOX) +
                     (slab * dst.tps[cls] + (rc - slab * dst.slab[cls]) / OZ_ROWS) * dst.nbox[cls]);
   };
-  const int item_rows = oz_item_rows(c, c->direct ? direct_range_rows(c) : row1 - row0, m);
+  // slabs of pairs: classes 1, 4I and 4II (of the whole matrix, or as many as
+  // a typical range of the direct path holds)
+  const int64_t nslab = c->direct ? std::max<int64_t>(1, direct_range_rows(c) / std::max<int64_t>(1, G.npair_v))
+                                  : G.no + 2 * G.npair_o;
+  const int item_rows = item_rows_for(c, nslab, G.npair_v, (m + 15) / 16, OZ_ITEM_OVERHEAD);
   if (p->item_rows != item_rows || p->lists_m < m) {
     p->h_items.clear();
     p->h_slabs.clear();
@@ -1401,7 +1400,7 @@ int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable) {
     ADC_CUDA(c, cudaGetLastError());
     p->values_for = c->d_cval;
   }
-  const int item_rows = oz_item_rows(c, nrows, m);
+  const int item_rows = item_rows_for(c, 2 * npp, npair, (m + 15) / 16, OZ_ITEM_OVERHEAD);
   if (p->item_rows != item_rows || p->lists_m < m) {
     p->h_items.clear();
     p->h_slabs.clear();

@@ -15,7 +15,7 @@
 // [0, NP) hi, [NP, 2 NP) lo), so one MMA gives both products and the
 // epilogue adds them (x = hi + lo to ~2^-17 relative).
 //
-// One CTA per SM, persistent over work items (up to UMMA_ITEM_ROWS_MAX rows of
+// One CTA per SM, persistent over work items (up to 4,096 rows of
 // one slab), warp-specialised:
 //   warp 0, one thread : TMA producer.  Each tile of 128 rows is loaded as
 //                        slots of two 64-column boxes (128-byte swizzle) into
@@ -60,7 +60,10 @@ constexpr int UMMA_SLOT_BYTES = 2 * UMMA_ROWS * UMMA_BOX * 2;   // two boxes
 constexpr int UMMA_MAX_BOXES = 6;           // K <= 384
 constexpr int UMMA_THREADS = 320;             // producer, MMA issuer, 8 epilogue warps
 constexpr int UMMA_NOP = 16;                  // segment A lengths (noP) up to 16 (nocc <= 16)
-constexpr int UMMA_ITEM_ROWS_MAX = 4096;      // rows per work item (a piece of one slab)
+// an item's X operand and W1 atomics in tiles (nocc=9/nvirt=101, 5 columns:
+// 4,096 rows make two rounds, 86 us for the pass, 512 rows six rounds, 81 us;
+// the rule's choice takes 70 us)
+constexpr double UMMA_ITEM_OVERHEAD = 5.0;
 // rows per work item of the FP32-value main pass: the W1 sums of an item run
 // in one TMEM chain (8 MMA steps per 128-row tile), and shorter chains keep
 // the tensor cores' truncating FP32 accumulation near FP32 rounding
@@ -591,12 +594,20 @@ bool umma_geometry_ok(const Geometry& G) {
   return G.noP <= UMMA_NOP && 2 * G.nvP <= UMMA_MAX_BOXES * UMMA_BOX && G.no >= 2 && G.nv >= 2;
 }
 
-// Rows per work item: about six items per SM (4,096 rows whatever the size
-// left 1.3 rounds of items at nocc=9/nvirt=101), 512 to 4,096 (an item's X
-// operand and W1 atomics cost about a tile).
-int umma_item_rows(const Ctx* c) {
-  const int64_t want = (c->geom.n2 / ((int64_t)c->nsm * 6) + 127) / 128 * 128;
-  return (int)std::min<int64_t>(UMMA_ITEM_ROWS_MAX, std::max<int64_t>(512, want));
+int item_rows_for(const Ctx* c, int64_t nslab, int64_t len, int groups, double overhead) {
+  int best = 1;
+  double best_cost = 0.0;
+  for (int t = 1; t <= 32; ++t) {
+    const int64_t npc = std::max<int64_t>(1, (len + 128 * t - 1) / (128 * t));
+    const int64_t tiles = ((len + npc - 1) / npc + 127) / 128;
+    const int64_t rounds = (nslab * npc * groups + c->nsm - 1) / c->nsm;
+    const double cost = (double)rounds * ((double)tiles + overhead);
+    if (t == 1 || cost <= best_cost) {
+      best = t;
+      best_cost = cost;
+    }
+  }
+  return best * 128;
 }
 
 bool umma3_supported(const Ctx* c) {
@@ -614,7 +625,9 @@ void umma_free(Ctx* c, void*& handle) {
 }
 
 // Work items, pass-3 runs and the tensor maps of the BF16 B^T values.
-int umma_prepare(Ctx* c, void*& handle, int item_rows) {
+int umma_prepare(Ctx* c, void*& handle) {
+  // slabs of pairs: classes 1, 4I and 4II
+  const int item_rows = item_rows_for(c, c->geom.no + 2 * c->geom.npair_o, c->geom.npair_v, 1, UMMA_ITEM_OVERHEAD);
   if (handle && reinterpret_cast<UmmaPlan*>(handle)->maps_for == c->d_Bt16 &&
       reinterpret_cast<UmmaPlan*>(handle)->slices_for == c->d_Bt16s[0] &&
       reinterpret_cast<UmmaPlan*>(handle)->item_rows == item_rows)
