@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm_nn_f32(int64_t N, int p, int q,
 // sums a range of rows for one 64 x 64 output tile; a thread owns a 4 x 4
 // sub-tile read as float4 from row-major staged rows (32 rows per step).
 // The products of one step are summed in FP32 and added to double-float
-// accumulators, as in k_gemm_tn_part.  part: [blk][tile][64 x 64] doubles.
+// accumulators.  part: [blk][tile][64 x 64] doubles.
 constexpr int TF_T = 64, TF_ROWS = 32, TF_LD = TF_T + 4;
 __global__ void __launch_bounds__(256) k_gemm_tn_f32(int64_t N, int p, int q, const float* __restrict__ A,
                                                      int64_t lda, const float* __restrict__ B, int64_t ldb,

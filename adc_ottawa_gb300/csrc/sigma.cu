@@ -8,12 +8,14 @@
 //   W1 = diag1 . V1 + A V1 + B V2       (A dense n1 x n1, B index-free)
 //   W2 = diag2 . V2 + B^T V1
 //
-// k_doubles: one warp per row of B^T (a double).  Lanes stride over the
-// row's entries (coalesced value loads); W2[d] is a warp reduction of
-// val * V1[s]; the B V2 contributions val * V2[d] go to a per-CTA partial of W1
-// in shared memory, flushed to global memory once per CTA.  V1 (n1 x m) is
-// tiny and stays in L1/L2.
-// k_singles: W1 = diag1 . V1 + A V1 as a tiled dense product (n1 <= ~5000).
+// k_singles_gemm: W1 = diag1 . V1 + A V1 as a tiled dense product.  The
+// coupling, by value type and shape (sigma_impl):
+//   FP64 and FP32 values: exact digit slices on the tensor cores
+//     (sigma_slices.cu), segment A of the rows with a' = b' by k_sigma_rows_a
+//   BF16 values: sigma_umma.cu, segments in sigma_ab.cu
+//   otherwise (no room for the digits, nocc > 32 or nvirt > 256, or a launch
+//     shape that asks for it): the tiles k_sigma_tile / k_sigma_tile_mma from
+//     16 columns, the per-warp pass 1 below, segment B in k_sigma_p2
 #include <cuda_bf16.h>
 
 #include <mutex>

@@ -40,15 +40,15 @@ METRIC = "time-to-converge 20 roots (mixed+learned vs FP64 GPU) at 1e-6 Ha; matv
 # DRAM bytes moved by the kernels of one sigma call per algorithmic byte,
 # by value store, from one-kernel ncu captures (dram__bytes_read.sum +
 # dram__bytes_write.sum, --clock-control none) at nocc=10/nvirt=110 summed
-# over the kernels of a call (profiles/): BF16 values, 48 columns: tcgen05
-# pass 0.485 GB + compact segments 0.266 GB against 1.03 GB algorithmic;
-# FP32 values, 40 columns: 2.5 passes of the FP32 tile (0.67 GB each) + compact
-# segment B (0.09 GB per 16 columns) against 1.29 GB; FP64 values, 30 columns:
-# two passes of the double-float tile (1.27 GB each) + pass 2 (0.12 GB per 4
-# columns) against 1.93 GB.  The index-free store reads no column indices, so
-# a ratio below 1 is possible; above 1 means the store is read once per
-# column group of the tile.
-TRAFFIC_PER_ALG_BYTE = {"bf16": 0.73, "fp32": 1.48, "fp64": 1.78}
+# over the kernels of a call: BF16 values, 48 columns: tcgen05 pass 0.523 GB +
+# segments 0.693 GB + the rest 0.012 GB against 1.06 GB algorithmic; FP32
+# values, 40 columns, digit slices: C and D segments 1.428 GB (8 bytes a value
+# once per 16 columns) + segments 0.728 GB + the rest 0.110 GB against 1.29 GB;
+# FP64 values, 30 columns, digit slices: 2.400 GB (14 bytes a value) + 1.293 GB
+# + 0.168 GB against 1.94 GB.  The index-free store reads no column indices, so
+# a ratio below 1 is possible; above 1 means digits wider than the values, and
+# vectors read and written once per segment pass.
+TRAFFIC_PER_ALG_BYTE = {"bf16": 1.16, "fp32": 1.75, "fp64": 1.99}
 TRAFFIC_SOURCE = ("ncu one-kernel captures at nocc=10/nvirt=110 (DRAM bytes of each kernel of a sigma call, summed, "
                   "per algorithmic byte, by value store), applied to this workload's calls")
 

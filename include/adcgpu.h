@@ -412,17 +412,21 @@ int adcgpu_davidson_trace(adcgpu_ctx* ctx, const adcgpu_dav_params* p, int every
  * ------------------------------------------------------------------------- */
 double adcgpu_last_sigma_ms(const adcgpu_ctx* ctx);
 
-/* Device bytes held by the context (matrix, ERI blocks, work spaces). */
+/* Device bytes held by the context (matrix, ERI blocks, work spaces; from the
+   first sigma product on also the digits its tensor-core pass reads, 14 bytes
+   per FP64 value and 8 per FP32 value, if they fit a third of the memory that
+   is free then). */
 int64_t adcgpu_device_bytes(const adcgpu_ctx* ctx);
 
 /* Arithmetic of the FP64 path's block products (no reference counterpart;
    the reference's FP64 arithmetic is MKL's): 0 (the default) FP64 fused
    multiply-adds; 1 double-float arithmetic on the FP32 pipe (hi + lo single
-   precision pairs, about 1e-14 relative per product) for sigma products of
-   16 or more columns and for the subspace GEMMs, which the GB300's FP64
-   rate (1/64 of FP32) makes several times faster.  It applies to every
-   solver that runs on the context (Davidson, Lanczos, SIL, Chebyshev); the
-   mixed ladder's FP64 refinement always uses 1. */
+   precision pairs, about 1e-14 relative per product) for the subspace GEMMs,
+   which the GB300's FP64 rate (1/64 of FP32) makes several times faster, and
+   for sigma products of 16 or more columns that do not run on the tensor
+   cores (those are as accurate as FP64 arithmetic in either mode).  It
+   applies to every solver that runs on the context (Davidson, Lanczos, SIL,
+   Chebyshev); the mixed ladder's FP64 refinement always uses 1. */
 int adcgpu_set_fp64_arith(adcgpu_ctx* ctx, int mode);
 
 /* Number of CUDA kernels this library has launched in this process, over
@@ -471,14 +475,14 @@ int adcgpu_sigma_autotune(adcgpu_ctx* ctx, int m, int* best_chunk, int* best_mc,
 /* Applies a launch shape (e.g. from the autotuner's cache).  In mc_fp64 /
    mc_fp32, bits 0-2 give the columns per pass, bit 3 selects the staged
    per-warp pass 1, bit 4 the per-warp pass 1 instead of the tiled one, bit
-   5 the CUDA-core tiled pass 1 instead of the tensor-core one (BF16 values),
-   bit 6 switches the tcgen05 sigma pass off, bit 7 runs segments A/B through
-   the per-(slab, b') pass 2 and per-run pass 3 instead of the compact
-   kernels, bit 8 makes a mixed-precision matrix's sigma product read the
+   5 the CUDA-core tiled pass 1 instead of the tensor-core ones (all value
+   types), bit 6 switches the tcgen05 sigma passes off (all value types), bit
+   7 runs segments A/B of BF16 and FP32 values through the per-(slab, b') pass
+   2 and per-run pass 3 (FP32 values then on the CUDA-core tile), bit 8 makes a mixed-precision matrix's sigma product read the
    FP32 value store instead of the BF16 one, bit 9 keeps the FP32 Gram
    products (adcgpu_gram_f32 and the solvers' V^T W) on the CUDA cores, bit
    10 runs the FP32 values on two tcgen05 passes over their BF16 slices
-   instead of the CUDA-core tile. */
+   instead of the exact digit slices. */
 int adcgpu_sigma_set_shape(adcgpu_ctx* ctx, int chunk, int mc_fp64, int mc_fp32);
 
 /* The solvers' tall-skinny Gram product on device FP32 arrays: C(p x q,
