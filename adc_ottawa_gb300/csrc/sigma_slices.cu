@@ -51,8 +51,7 @@ constexpr int OZ_THREADS = 64 + OZ_EPI;            // and the producer and MMA i
 constexpr int OZ_MAXNR = 6;                        // ring slots
 constexpr int OZ_FLUSH = 2;                        // tiles per W1 accumulation in TMEM
 constexpr int OZ_NONFINITE = 1 << 20;              // exponent of a column that holds inf or NaN
-constexpr int OZ_ZERO = -(1 << 20);                // exponent of a zero
-constexpr int OZ_EMIN = -900;                      // smaller maxima are taken as this exponent
+constexpr int OZ_EMIN = -2200;                     // below every exponent, and every sum of two
 
 __host__ __device__ constexpr int round16(int x) { return (x + 15) / 16 * 16; }
 // Vector operands: PAD zero rows, then slice j of column c at row PAD + j NP + c.
@@ -102,17 +101,18 @@ struct OzSlab {         // pair rows (a' < b') of one slab
 };
 
 // --- digits --------------------------------------------------------------
-// x = (-1)^neg m 2^(e - MB), m < 2^MB; e = OZ_ZERO for zeros and subnormals,
-// OZ_NONFINITE for inf and NaN
+// x = (-1)^neg m 2^(e - MB), m < 2^MB; zeros and subnormals have the smallest
+// exponent, inf and NaN OZ_NONFINITE
 template <typename T> struct Parts;
 template <> struct Parts<double> {
   static constexpr int MB = 53;
   __device__ __forceinline__ static int exponent(double x) {
     const int f = (int)((__double2hiint(x) >> 20) & 0x7ff);
-    return f == 0 ? OZ_ZERO : (f == 0x7ff ? OZ_NONFINITE : f - 1022);
+    return f == 0x7ff ? OZ_NONFINITE : max(f, 1) - 1022;
   }
   __device__ __forceinline__ static unsigned long long mantissa(double x) {
-    return ((unsigned long long)__double_as_longlong(x) & 0xfffffffffffffull) | 0x10000000000000ull;
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    return (u & 0xfffffffffffffull) | ((u & 0x7ff0000000000000ull) ? 0x10000000000000ull : 0ull);
   }
   __device__ __forceinline__ static bool neg(double x) { return __double2hiint(x) < 0; }
 };
@@ -120,21 +120,22 @@ template <> struct Parts<float> {
   static constexpr int MB = 24;
   __device__ __forceinline__ static int exponent(float x) {
     const int f = (int)((__float_as_uint(x) >> 23) & 0xff);
-    return f == 0 ? OZ_ZERO : (f == 0xff ? OZ_NONFINITE : f - 126);
+    return f == 0xff ? OZ_NONFINITE : max(f, 1) - 126;
   }
   __device__ __forceinline__ static unsigned long long mantissa(float x) {
-    return (__float_as_uint(x) & 0x7fffffu) | 0x800000u;
+    const uint32_t u = __float_as_uint(x);
+    return (u & 0x7fffffu) | ((u & 0x7f800000u) ? 0x800000u : 0u);
   }
   __device__ __forceinline__ static bool neg(float x) { return (int)__float_as_uint(x) < 0; }
 };
 
-// round(x 2^(8S - 1 - h)) plus the digit bias, for x of exponent e <= h: byte
-// i from the top is digit i + 128
+// round(x 2^(8S - 1 - h)) plus the digit bias, for x of exponent e <= h (for
+// zeros too: the shift stays below the word): byte i from the top is digit i + 128
 template <int S, typename T>
 __device__ __forceinline__ unsigned long long oz_fixed(T x, int shift) {   // shift = 8S - 1 - h + (scale of x)
   constexpr unsigned long long BIAS = S == 7 ? 0x80808080808080ull : 0x80808080ull;
   const int e = Parts<T>::exponent(x);
-  if (e == OZ_ZERO || e == OZ_NONFINITE) return BIAS;
+  if (e == OZ_NONFINITE) return BIAS;
   const unsigned long long m = Parts<T>::mantissa(x);
   const int sh = e - Parts<T>::MB + shift;
   unsigned long long q;
@@ -152,12 +153,22 @@ __device__ __forceinline__ uint32_t oz_digit(unsigned long long u, int i) {
 }
 // two digits as a BF16 pair (lo in the lower half)
 __device__ __forceinline__ uint32_t oz_pair(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
-// 2^e; NaN for a column that holds inf or NaN
-__device__ __forceinline__ double oz_pow2(int e) {
+// t 2^e of a group sum t (zero, or 2^-24 to 2^47 in size); NaN for a column
+// that holds inf or NaN.  A power of two outside the type's range, which a
+// result inside it can need, is taken in two factors; only the second can round.
+__device__ __forceinline__ double oz_pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+__device__ __forceinline__ double oz_scaled(double t, int e) {
+  if ((unsigned)(e + 1022) < 2046u) return t * oz_pow2(e);
   if (e > (OZ_NONFINITE >> 1)) return __longlong_as_double(0x7ff8000000000000ll);
-  if (e < -1022) return 0.0;
-  if (e > 1023) return __longlong_as_double(0x7ff0000000000000ll);
-  return __longlong_as_double((long long)(e + 1023) << 52);
+  e = min(max(e, -2044), 2046);
+  return t * oz_pow2(e >> 1) * oz_pow2(e - (e >> 1));
+}
+__device__ __forceinline__ float oz_pow2f(int e) { return __int_as_float((e + 127) << 23); }
+__device__ __forceinline__ float oz_scaled(float t, int e) {
+  if ((unsigned)(e + 126) < 254u) return t * oz_pow2f(e);
+  if (e > (OZ_NONFINITE >> 1)) return __int_as_float(0x7fc00000);
+  e = min(max(e, -252), 254);
+  return t * oz_pow2f(e >> 1) * oz_pow2f(e - (e >> 1));
 }
 
 // --- value digits of a range of storage rows ---------------------------------
@@ -200,7 +211,7 @@ __global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const T
     const int nch = (cls >= 2 ? 2 : 1) * g.nvP / 8, nbox = dst.nbox[cls];
     const TV* src = Bt + g.off[cls] + (row - g.start[cls]) * g.len[cls] + (twoa ? 2 * g.noP : g.noP);
     TV v[2][8];
-    int mx = OZ_ZERO;
+    int mx = OZ_EMIN;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int q = lane + 32 * k;
@@ -215,7 +226,7 @@ __global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const T
 #pragma unroll
       for (int u = 0; u < 8; ++u) mx = max(mx, Parts<TV>::exponent(v[k][u]));
     }
-    mx = max(__reduce_max_sync(0xffffffffu, mx), OZ_EMIN);
+    mx = __reduce_max_sync(0xffffffffu, mx);
     // a row that holds inf or NaN (integrals that do): its W2 entries and the
     // W1 sums of its tile become NaN
     if (lane == 0 && valid) rexp[row - dst.row0] = (int16_t)min(mx, 32767);
@@ -271,7 +282,7 @@ __global__ void __launch_bounds__(128) k_oz_cvs_values(OzGeom g, int npp, int64_
     __syncwarp();
     for (int x = lane; x < g.nvP + 2 * kw; x += 32) row_c[x] = 0.0;
     __syncwarp();
-    int mc = OZ_EMIN, ms = OZ_EMIN;
+    int mc = Parts<double>::exponent(0.0), ms = mc;
     if (valid) {
       int ap, bp;
       pair_decode(p, g.nv, ap, bp);
@@ -348,7 +359,7 @@ __global__ void __launch_bounds__(256) k_oz_vexp(OzGeom g, const OzItem* __restr
       if (c0 + j >= m) break;
       const int e = Parts<T>::exponent(__ldg(V + (int64_t)(c0 + j) * ldv + g.n1 + d));
       if (e == OZ_NONFINITE || rx == 32767 || sx == 32767) mx[j] = mx[4 + j] = OZ_NONFINITE;
-      else if (e != OZ_ZERO) {
+      else {
         mx[j] = max(mx[j], e + rx);
         mx[4 + j] = max(mx[4 + j], e + sx);
       }
@@ -411,8 +422,7 @@ __device__ __forceinline__ double oz_sum(const float (&d)[S]) {
     return x + __longlong_as_double(0x41B8000000000000ll + lo);
   }
 }
-// the same rounded to the vectors' type (FP32: without the FP64 pipe), and
-// powers of two of that type (those below its range are 0)
+// the same rounded to the vectors' type (FP32: without the FP64 pipe)
 template <int S, typename T> __device__ __forceinline__ T oz_round(const float (&d)[S]) {
   if constexpr (std::is_same<T, double>::value) {
     return oz_sum<S>(d);
@@ -424,14 +434,6 @@ template <int S, typename T> __device__ __forceinline__ T oz_round(const float (
     hi = mad_wide(__float2int_rn(d[0]), 1 << 24, hi);
     return __ll2float_rn(hi);
   }
-}
-template <typename T> __device__ __forceinline__ T oz_scale(int e);
-template <> __device__ __forceinline__ double oz_scale<double>(int e) { return oz_pow2(e); }
-template <> __device__ __forceinline__ float oz_scale<float>(int e) {
-  if (e > (OZ_NONFINITE >> 1)) return __int_as_float(0x7fc00000);
-  if (e < -126) return 0.f;
-  if (e > 127) return __int_as_float(0x7f800000);
-  return __int_as_float((e + 127) << 23);
 }
 // weight exponent of oz_sum's unit against scaled operands |v| < 1
 template <int S> __host__ __device__ constexpr int oz_unit() { return -14 - 8 * (S - 1) + (S == 7 ? 24 : 0); }
@@ -623,7 +625,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     auto load_v2 = [&](const OzItem& item, int row, int c0) {
       const bool valid = row < item.row1;
       const int64_t d = valid ? item.dbase + (int64_t)(row - item.row0) * item.dstr : 0;
-      rx = valid ? (int)rexp[row - g.row0] : 0;
+      rx = valid ? (int)rexp[row - g.row0] : OZ_EMIN;
 #pragma unroll
       for (int j = 0; j < NH; ++j) {
         const int c = c0 + cbeg + j;
@@ -660,13 +662,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       load_v2(item, item.row0 + r, c0);
 #pragma unroll
       for (int j = 0; j < NH; ++j)
-        vexp[j] = c0 + cbeg + j < m ? __ldg(ivexp + (int64_t)(un / ngrp) * m + c0 + cbeg + j) : OZ_EMIN;
+        vexp[j] = c0 + cbeg + j < m ? __ldg(ivexp + (int64_t)(un / ngrp) * m + c0 + cbeg + j) : 0;
       // X of this item: the previous item's products have read the old one
       // (its last D1 was waited for).  One warp per column
 #pragma unroll 1
       for (int c = ew; c < NP; c += OZ_EPI / 32) {
         T xv[4 * MS];
-        int mx = OZ_ZERO;
+        int mx = OZ_EMIN;
 #pragma unroll
         for (int u = 0; u < 4 * MS; ++u) {
           const int k = lane + 32 * u;
@@ -675,7 +677,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         }
 #pragma unroll
         for (int u = 0; u < 4 * MS; ++u) mx = max(mx, Parts<T>::exponent(xv[u]));
-        mx = max(__reduce_max_sync(0xffffffffu, mx), OZ_EMIN);
+        mx = __reduce_max_sync(0xffffffffu, mx);
         if (lane == 0) sXe[c] = mx;
 #pragma unroll
         for (int u = 0; u < 4 * MS; ++u) {
@@ -747,7 +749,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const int c = c0 + cbeg + j;
             if (c >= m) continue;
             const T x = V[(int64_t)c * ldv + n1 + d];
-            const T t = t2[j] * oz_scale<T>(sXe[cbeg + j] + re + TSH);
+            const T t = oz_scaled(t2[j], sXe[cbeg + j] + re + TSH);
             W[(int64_t)c * ldw + n1 + d] = dg * x + t;
           }
         }
@@ -765,7 +767,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 #pragma unroll
         for (int j = 0; j < NH; ++j) {
           const int c = c0 + cbeg + j;
-          const double w = acc[s][j] * oz_pow2(vexp[j] + TSH);
+          const double w = oz_scaled(acc[s][j], vexp[j] + TSH);
           if (c < m && !(w == 0.0)) atomicAdd(&W1[(int64_t)c * ld1 + single], (TA)w);
         }
       }
@@ -810,12 +812,12 @@ __global__ void __launch_bounds__(256) k_oz_seg_values(GeomDev g, int64_t row0, 
     if (!(cls == 1 || cls >= 3)) continue;
     const TV* src = Bt + g.off[cls] + (row - g.start[cls]) * g.len[cls];
     uint16_t* o = out + (row - row0) * 2 * S * kw;
-    int mx = OZ_ZERO;
+    int mx = OZ_EMIN;
     for (int x = lane; x < 2 * kw; x += 32) {
       const int seg = x >= kw ? 1 : 0, k = x - seg * kw;
       if (k < g.no) mx = max(mx, Parts<TV>::exponent(src[seg * g.noP + k]));
     }
-    mx = max(__reduce_max_sync(0xffffffffu, mx), OZ_EMIN);
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) sexp[row - row0] = (int16_t)min(mx, 32767);
     for (int x = lane; x < 2 * kw; x += 32) {
       const int seg = x >= kw ? 1 : 0, k = x - seg * kw;
@@ -931,7 +933,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, seg_blocks<KT>())
       int ev[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        int e = OZ_EMIN;
+        int e = cc[h] < m ? OZ_EMIN : 0;
         if (cc[h] < m)
           for (int i = 0; i < sl.nitem; ++i) e = max(e, __ldg(vsexp + (int64_t)(sl.item0 - item0 + i) * m + cc[h]));
         ev[h] = e;
@@ -987,7 +989,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, seg_blocks<KT>())
             float dsum[S];
 #pragma unroll
             for (int i = 0; i < S; ++i) dsum[i] = a1[n][i][2 * h + v];
-            const double w = oz_sum<S>(dsum) * oz_pow2(ev[h] + TSH);
+            const double w = oz_scaled(oz_sum<S>(dsum), ev[h] + TSH);
             if (!(w == 0.0)) atomicAdd(&W1[(int64_t)cc[h] * ld1 + (int64_t)f * no + k], (TA)w);
           }
         }
@@ -1066,7 +1068,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, seg_blocks<KT>())
 #pragma unroll
               for (int i = 0; i < S; ++i) dsum[i] = a2[i][2 * h + v];
               W[(int64_t)cc[h] * ldw + d] =
-                  wv[h][2 * hr + v] + oz_round<S, T>(dsum) * oz_scale<T>(ex[h] + ee[2 * hr + v] + TSH);
+                  wv[h][2 * hr + v] + oz_scaled(oz_round<S, T>(dsum), ex[h] + ee[2 * hr + v] + TSH);
             }
           }
         }
