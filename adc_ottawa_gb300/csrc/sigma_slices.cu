@@ -8,22 +8,32 @@
 // Exact slicing (K. Ozaki, T. Ogita, S. Oishi, S. M. Rump, "Error-free
 // transformations of matrix multiplication by using fast routines of matrix
 // multiplication and its applications", Numer. Algorithms 59, 2012).  A row
-// of values is scaled by a power of two to |v| < 1 and written as S balanced
-// base-256 digits, v = sum_i d_i 2^(-7-8i), |d_i| <= 128; so are the vector
-// entries of a slab (one exponent per column) and of a row tile.  Every digit
-// is an exact BF16 number, a product of two digits has at most 14 bits, and
-// the FP32 accumulators in TMEM add whole numbers: up to 2^24 / 2^14 = 1024
-// products without rounding.  Products of equal weight (i + j = g) share an
+// of values is scaled by a power of two to |v| < 1 and written as S base-256
+// digits, v = sum_i d_i 2^(-7-8i), |d_0| <= 128, |d_i| < 256; so are the vector
+// entries of a slab (one exponent per column) and of a row tile, all |d_i| <= 128.
+// Every digit is an exact BF16 number, and the FP32 accumulators in TMEM add
+// whole numbers.  Products of equal weight (i + j = g) share an
 // accumulator; the groups g < S are kept (the dropped ones are below the last
 // digit's weight) and combined with 64-bit integer arithmetic, so one
 // rounding per tile replaces one per multiply-add.
 //   S = 7: 55 bits below the row / column maximum (FP64 values)
 //   S = 4: 31 bits (FP32 values and vectors)
-// W1 sums cover two tiles, 256 rows: g < 4 is exact whatever the digits are.
-// W2 sums cover K <= 512 values: g < 2 (K <= 341: g < 3) likewise.  The other
-// groups are exact while their partial sums stay below 2^24, which the
-// pseudo-random lower digits do by a factor of 50 (sum of n products: about
-// 2^12 sqrt(n)).
+// Whole sums: a group of g + 1 digit pairs reaches at most (g + 1) K 2^14 over K
+// products, and FP32 adds without rounding up to 2^24.  W1 sums cover two tiles,
+// K = 256 rows: g < 4 is exact whatever the digits are, and so are W2 sums of up
+// to 256 values.  Longer rows (nvirt > 128) would leave the range in g = 2 and 3
+// if all digits had one sign and size, so their values' digits 1 to 3 are drawn
+// at random from a number's representations (d, or d - 256 and a carry), with a
+// mean of at most 32, independently along rows and columns (S = 7).  Of the group
+// sums that leaves the first digits' part, 2^23 at K = 512, 2^21 for each further
+// digit, and a random part of standard deviation 2^14 sqrt(3 K) = 2^19.3: g < 4
+// stays below 2^24 there too.  (Plain digits lost 1.2e-11 of such row sums at
+// K = 512, 5e-14 at 384; tests/test_gpu_sigma_digits.py.)
+// g >= 4 is whole while the partial sums stay below 2^24, which pseudo-random
+// digits do by a factor of 50 (sum of n products: about 2^12 sqrt(n)); digits of
+// one sign and size take it to 2^26 and lose a unit in the last of 24 bits an
+// MMA, 2^-47 of their sum at most, the size of the roundings of K FP64 adds.
+// S = 4: such sums lose 2^-30 of |values| |vectors|, below FP32's own rounding.
 //
 // What bounds it: the digit store is read once per 16 columns (S = 7), 14
 // bytes per value; the tensor cores need S (S + 1) / 2 = 28 slice products.
@@ -52,6 +62,7 @@ constexpr int OZ_MAXNR = 6;                        // ring slots
 constexpr int OZ_FLUSH = 2;                        // tiles per W1 accumulation in TMEM
 constexpr int OZ_NONFINITE = 1 << 20;              // exponent of a column that holds inf or NaN
 constexpr int OZ_EMIN = -2200;                     // below every exponent, and every sum of two
+constexpr int OZ_VALUE_EMIN = -48;                 // below that of any kept value (above 1e-12)
 
 __host__ __device__ constexpr int round16(int x) { return (x + 15) / 16 * 16; }
 // Vector operands: PAD zero rows, then slice j of column c at row PAD + j NP + c.
@@ -114,6 +125,9 @@ template <> struct Parts<double> {
     const unsigned long long u = (unsigned long long)__double_as_longlong(x);
     return (u & 0xfffffffffffffull) | ((u & 0x7ff0000000000000ull) ? 0x10000000000000ull : 0ull);
   }
+  __device__ __forceinline__ static unsigned long long normal_mantissa(double x) {
+    return ((unsigned long long)__double_as_longlong(x) & 0xfffffffffffffull) | 0x10000000000000ull;
+  }
   __device__ __forceinline__ static bool neg(double x) { return __double2hiint(x) < 0; }
 };
 template <> struct Parts<float> {
@@ -126,23 +140,37 @@ template <> struct Parts<float> {
     const uint32_t u = __float_as_uint(x);
     return (u & 0x7fffffu) | ((u & 0x7f800000u) ? 0x800000u : 0u);
   }
+  __device__ __forceinline__ static unsigned long long normal_mantissa(float x) {
+    return (__float_as_uint(x) & 0x7fffffu) | 0x800000u;
+  }
   __device__ __forceinline__ static bool neg(float x) { return (int)__float_as_uint(x) < 0; }
 };
 
+// balanced digits: byte i of the bias is 128
+template <int S> __host__ __device__ constexpr unsigned long long oz_bias() { return S == 7 ? 0x80808080808080ull : 0x80808080ull; }
 // round(x 2^(8S - 1 - h)) plus the digit bias, for x of exponent e <= h (for
-// zeros too: the shift stays below the word): byte i from the top is digit i + 128
+// zeros too: the shift stays below the word): byte i from the top is digit i
+// plus byte i of the bias
 template <int S, typename T>
-__device__ __forceinline__ unsigned long long oz_fixed(T x, int shift) {   // shift = 8S - 1 - h + (scale of x)
-  constexpr unsigned long long BIAS = S == 7 ? 0x80808080808080ull : 0x80808080ull;
+__device__ __forceinline__ unsigned long long oz_fixed_m(T x, unsigned long long m, int shift, unsigned long long BIAS) {
   const int e = Parts<T>::exponent(x);
   if (e == OZ_NONFINITE) return BIAS;
-  const unsigned long long m = Parts<T>::mantissa(x);
   const int sh = e - Parts<T>::MB + shift;
   unsigned long long q;
   if (sh >= 0) q = m << sh;
   else if (sh < -60) q = 0ull;
   else q = (m + (1ull << (-sh - 1))) >> (-sh);
   return Parts<T>::neg(x) ? BIAS - q : BIAS + q;
+}
+template <int S, typename T>
+__device__ __forceinline__ unsigned long long oz_fixed(T x, int shift) {   // shift = 8S - 1 - h + (scale of x)
+  return oz_fixed_m<S, T>(x, Parts<T>::mantissa(x), shift, oz_bias<S>());
+}
+// the same of a matrix value, never subnormal: zero is taken as the smallest
+// normal number, far below the digits of any h >= OZ_VALUE_EMIN
+template <int S, typename T>
+__device__ __forceinline__ unsigned long long oz_fixed_value(T x, int shift, unsigned long long BIAS = oz_bias<S>()) {
+  return oz_fixed_m<S, T>(x, Parts<T>::normal_mantissa(x), shift, BIAS);
 }
 // digit i as an FP32 number; its upper half is the exact BF16 one (an
 // integer of at most 8 bits)
@@ -151,24 +179,48 @@ __device__ __forceinline__ uint32_t oz_digit(unsigned long long u, int i) {
   const uint32_t f = i == 0 ? (uint32_t)(u >> (8 * (S - 1))) : (uint32_t)(u >> (8 * (S - 1 - i))) & 0xffu;
   return __float_as_uint(__uint_as_float(0x4B000000u | f) - 8388736.0f);
 }
+// random biases of digits 1 to 3 of a long row's values, 32, 96, 160 or 224 (a
+// digit of 256 - bias and more becomes 256 less): two random bits of the row and
+// two of the position in it, combined by xor, so independent along a row and
+// along a position.  Hash: splitmix64's output function (G. L. Steele, D. Lea,
+// C. H. Flood, "Fast splittable pseudorandom number generators", OOPSLA 2014).
+__device__ __forceinline__ unsigned long long oz_random_bits(unsigned long long x) {
+  x *= 0x9e3779b97f4a7c15ull;
+  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
+  x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+  return (x ^ (x >> 31)) & 0x00c0c0c0000000ull;
+}
+__device__ __forceinline__ unsigned long long oz_position_bias(int k) {
+  return 0x80202020808080ull ^ oz_random_bits(2 * (unsigned long long)k + 2);
+}
+// digit i of a value with bias b
+template <int S>
+__device__ __forceinline__ uint32_t oz_digit(unsigned long long u, unsigned long long b, int i) {
+  if (i == 0) return oz_digit<S>(u, 0);
+  const int sh = 8 * (S - 1 - i);
+  return __float_as_uint(__uint_as_float(0x4B000000u | ((uint32_t)(u >> sh) & 0xffu)) -
+                         __uint_as_float(0x4B000000u | ((uint32_t)(b >> sh) & 0xffu)));
+}
 // two digits as a BF16 pair (lo in the lower half)
 __device__ __forceinline__ uint32_t oz_pair(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
 // t 2^e of a group sum t (zero, or 2^-24 to 2^47 in size); NaN for a column
-// that holds inf or NaN.  A power of two outside the type's range, which a
-// result inside it can need, is taken in two factors; only the second can round.
+// that holds inf or NaN.  FP64: in the exponent field (the FP64 pipe takes 16
+// cycles a warp for a multiplication).  A power of two outside the type's range,
+// which a result inside it can need, and results at the ends of the range take
+// two factors; only the second can round.
 __device__ __forceinline__ double oz_pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 __device__ __forceinline__ double oz_scaled(double t, int e) {
-  if ((unsigned)(e + 1022) < 2046u) return t * oz_pow2(e);
+  const int hi = __double2hiint(t), f = (hi >> 20) & 0x7ff;
+  if (f != 0 && (unsigned)(f + e - 1) < 2046u) return __hiloint2double(hi + (int)((unsigned)e << 20), __double2loint(t));
   if (e > (OZ_NONFINITE >> 1)) return __longlong_as_double(0x7ff8000000000000ll);
+  if (f == 0) return t;
   e = min(max(e, -2044), 2046);
   return t * oz_pow2(e >> 1) * oz_pow2(e - (e >> 1));
 }
-__device__ __forceinline__ float oz_pow2f(int e) { return __int_as_float((e + 127) << 23); }
 __device__ __forceinline__ float oz_scaled(float t, int e) {
-  if ((unsigned)(e + 126) < 254u) return t * oz_pow2f(e);
-  if (e > (OZ_NONFINITE >> 1)) return __int_as_float(0x7fc00000);
-  e = min(max(e, -252), 254);
-  return t * oz_pow2f(e >> 1) * oz_pow2f(e - (e >> 1));
+  const int c = min(max(e, -252), 254), h = c >> 1;
+  const float w = t * __int_as_float((h + 127) << 23) * __int_as_float((c - h + 127) << 23);
+  return e > (OZ_NONFINITE >> 1) ? __int_as_float(0x7fc00000) : w;
 }
 
 // --- value digits of a range of storage rows ---------------------------------
@@ -192,12 +244,18 @@ template <int S> __host__ __device__ inline int64_t oz_tile_values(int nbox) { r
 
 // one warp per tile row: the exponent of the largest |C|D value|, then the
 // digits of 8 values per lane and step (16-byte stores, 128 bytes a box).
-// Bound by HBM: 8 (4) bytes read and 2 S written per value.
-template <typename TV, int S>
-__global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const TV* __restrict__ Bt,
+// Bound by HBM: 8 (4) bytes read and 2 S written per value.  LONG: geometries with
+// rows of more than 256 values, whose digits 1 to 3 have random biases.
+template <typename TV, int S, bool LONG>
+__global__ void __launch_bounds__(256, 3) k_oz_values(GeomDev g, OzDst dst, const TV* __restrict__ Bt,
                                                    uint16_t* __restrict__ out, int16_t* __restrict__ rexp) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  __shared__ unsigned long long s_pb[LONG ? 512 : 1];
+  if (LONG) {
+    for (int k = threadIdx.x; k < 2 * g.nvP; k += 256) s_pb[k] = oz_position_bias(k);
+    __syncthreads();
+  }
   for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < dst.tiles[5] * OZ_ROWS; w += nw) {
     const int64_t tile = w / OZ_ROWS;
     const int r = (int)(w % OZ_ROWS);
@@ -211,7 +269,7 @@ __global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const T
     const int nch = (cls >= 2 ? 2 : 1) * g.nvP / 8, nbox = dst.nbox[cls];
     const TV* src = Bt + g.off[cls] + (row - g.start[cls]) * g.len[cls] + (twoa ? 2 * g.noP : g.noP);
     TV v[2][8];
-    int mx = OZ_EMIN;
+    int mx = OZ_VALUE_EMIN;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int q = lane + 32 * k;
@@ -231,24 +289,29 @@ __global__ void __launch_bounds__(256) k_oz_values(GeomDev g, OzDst dst, const T
     // W1 sums of its tile become NaN
     if (lane == 0 && valid) rexp[row - dst.row0] = (int16_t)min(mx, 32767);
     uint16_t* o = out + dst.base[cls] + tc * oz_tile_values<S>(nbox);
+    unsigned long long rb = 0;
+    if (LONG) rb = oz_random_bits(2 * (unsigned long long)row + 1);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int q = lane + 32 * k;
       if (q >= 8 * nbox) continue;
-      unsigned long long u8[8];
+      unsigned long long u8[8], b8[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) u8[u] = oz_fixed<S, TV>(v[k][u], 8 * S - 1 - mx);
+      for (int u = 0; u < 8; ++u) {
+        b8[u] = LONG && q < nch ? rb ^ s_pb[8 * q + u] : oz_bias<S>();
+        u8[u] = oz_fixed_value<S, TV>(v[k][u], 8 * S - 1 - mx, b8[u]);
+      }
       // 128-value group q / 16: S slices of its (one or two) boxes
       const int grp = q >> 4, bx = (q >> 3) & 1, two = 2 * grp + 1 < nbox ? 2 : 1;
       uint16_t* og = o + ((int64_t)S * 2 * grp + bx) * (OZ_ROWS * OZ_BOX) + sw128_off(r, 8 * (q & 7)) / 2;
 #pragma unroll
       for (int i = 0; i < S; ++i) {
-        uint4 w4;
-        w4.x = oz_pair(oz_digit<S>(u8[0], i), oz_digit<S>(u8[1], i));
-        w4.y = oz_pair(oz_digit<S>(u8[2], i), oz_digit<S>(u8[3], i));
-        w4.z = oz_pair(oz_digit<S>(u8[4], i), oz_digit<S>(u8[5], i));
-        w4.w = oz_pair(oz_digit<S>(u8[6], i), oz_digit<S>(u8[7], i));
-        __stcs(reinterpret_cast<uint4*>(og + (int64_t)i * two * (OZ_ROWS * OZ_BOX)), w4);
+        auto pair = [&](int u) {
+          if (LONG && i >= 1 && i <= 3) return oz_pair(oz_digit<S>(u8[u], b8[u], i), oz_digit<S>(u8[u + 1], b8[u + 1], i));
+          return oz_pair(oz_digit<S>(u8[u], i), oz_digit<S>(u8[u + 1], i));
+        };
+        __stcs(reinterpret_cast<uint4*>(og + (int64_t)i * two * (OZ_ROWS * OZ_BOX)),
+               make_uint4(pair(0), pair(2), pair(4), pair(6)));
       }
     }
   }
@@ -282,7 +345,7 @@ __global__ void __launch_bounds__(128) k_oz_cvs_values(OzGeom g, int npp, int64_
     __syncwarp();
     for (int x = lane; x < g.nvP + 2 * kw; x += 32) row_c[x] = 0.0;
     __syncwarp();
-    int mc = Parts<double>::exponent(0.0), ms = mc;
+    int mc = OZ_VALUE_EMIN, ms = OZ_VALUE_EMIN;
     if (valid) {
       int ap, bp;
       pair_decode(p, g.nv, ap, bp);
@@ -309,7 +372,7 @@ __global__ void __launch_bounds__(128) k_oz_cvs_values(OzGeom g, int npp, int64_
     for (int q = lane; q < 8 * nbox; q += 32) {
       unsigned long long u8[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) u8[u] = oz_fixed<S, double>(8 * q < g.nvP ? row_c[8 * q + u] : 0.0, 8 * S - 1 - mc);
+      for (int u = 0; u < 8; ++u) u8[u] = oz_fixed_value<S, double>(8 * q < g.nvP ? row_c[8 * q + u] : 0.0, 8 * S - 1 - mc);
       const int grp = q >> 4, bx = (q >> 3) & 1, two = 2 * grp + 1 < nbox ? 2 : 1;
       uint16_t* og = o + ((int64_t)S * 2 * grp + bx) * (OZ_ROWS * OZ_BOX) + sw128_off(r, 8 * (q & 7)) / 2;
 #pragma unroll
@@ -324,7 +387,7 @@ __global__ void __launch_bounds__(128) k_oz_cvs_values(OzGeom g, int npp, int64_
       uint16_t* os = seg + row * 2 * S * kw;
       for (int x = lane; x < 2 * kw; x += 32) {
         const int sg = x >= kw ? 1 : 0, k = x - sg * kw;
-        const unsigned long long u = oz_fixed<S, double>(row_ab[x], 8 * S - 1 - ms);
+        const unsigned long long u = oz_fixed_value<S, double>(row_ab[x], 8 * S - 1 - ms);
 #pragma unroll
         for (int i = 0; i < S; ++i) os[(sg * S + i) * kw + k] = (uint16_t)(oz_digit<S>(u, i) >> 16);
       }
@@ -812,7 +875,7 @@ __global__ void __launch_bounds__(256) k_oz_seg_values(GeomDev g, int64_t row0, 
     if (!(cls == 1 || cls >= 3)) continue;
     const TV* src = Bt + g.off[cls] + (row - g.start[cls]) * g.len[cls];
     uint16_t* o = out + (row - row0) * 2 * S * kw;
-    int mx = OZ_EMIN;
+    int mx = OZ_VALUE_EMIN;
     for (int x = lane; x < 2 * kw; x += 32) {
       const int seg = x >= kw ? 1 : 0, k = x - seg * kw;
       if (k < g.no) mx = max(mx, Parts<TV>::exponent(src[seg * g.noP + k]));
@@ -821,7 +884,7 @@ __global__ void __launch_bounds__(256) k_oz_seg_values(GeomDev g, int64_t row0, 
     if (lane == 0) sexp[row - row0] = (int16_t)min(mx, 32767);
     for (int x = lane; x < 2 * kw; x += 32) {
       const int seg = x >= kw ? 1 : 0, k = x - seg * kw;
-      const unsigned long long u = oz_fixed<S, TV>(k < g.no ? src[seg * g.noP + k] : TV(0), 8 * S - 1 - mx);
+      const unsigned long long u = oz_fixed_value<S, TV>(k < g.no ? src[seg * g.noP + k] : TV(0), 8 * S - 1 - mx);
 #pragma unroll
       for (int i = 0; i < S; ++i) o[(seg * S + i) * kw + k] = (uint16_t)(oz_digit<S>(u, i) >> 16);
     }
@@ -1295,7 +1358,9 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
     const int grid2 = (int)std::min<int64_t>((row1 - row0 + 7) / 8, (int64_t)c->nsm * 8);
     auto make = [&](auto* v, auto s) {
       using TV = typename std::remove_const<typename std::remove_pointer<decltype(v)>::type>::type;
-      k_oz_values<TV, decltype(s)::value><<<grid, 256, 0, c->stream>>>(g, dst, v, p->dig, p->rexp);
+      constexpr bool F64 = decltype(s)::value == 7;
+      if (F64 && 2 * G.nvP > 256) k_oz_values<TV, decltype(s)::value, F64><<<grid, 256, 0, c->stream>>>(g, dst, v, p->dig, p->rexp);
+      else k_oz_values<TV, decltype(s)::value, false><<<grid, 256, 0, c->stream>>>(g, dst, v, p->dig, p->rexp);
       ADC_COUNT_LAUNCH();
       k_oz_seg_values<TV, decltype(s)::value><<<grid2, 256, 0, c->stream>>>(g, row0, row1, kw, v, p->seg, p->sexp);
       ADC_COUNT_LAUNCH();
