@@ -300,6 +300,11 @@ static int singlesubspace_block(Ctx* c, int b, std::vector<double>& q0) {
   return ADCGPU_OK;
 }
 
+static int cheb_auto_run(Ctx* c, int nvec, const double* q0, const double* bounds, int chebyord, int df,
+                         double* auto_out, double* q1h1p, int* order_out);
+static int cheb_project_run(Ctx* c, int nvec, double* q0, const double* bounds, int chebyord, double projen, int df);
+static int spectral_bounds_run(Ctx* c, const adcgpu_dav_params* fp, double* bounds);
+
 }  // namespace adcgpu
 
 extern "C" int adcgpu_chebyshev_auto(adcgpu_ctx* h, int nvec, const double* q0, const double* bounds, int chebyord,
@@ -310,6 +315,11 @@ extern "C" int adcgpu_chebyshev_auto(adcgpu_ctx* h, int nvec, const double* q0, 
   cudaSetDevice(c->device);
   ST(cheb_check(c, nvec, q0, bounds, chebyord));
   if (!auto_out) return set_err(c, ADCGPU_BAD_INPUT, "auto_out required");
+  return sigma_result(c, cheb_auto_run(c, nvec, q0, bounds, chebyord, df, auto_out, q1h1p, order_out));
+}
+
+static int adcgpu::cheb_auto_run(Ctx* c, int nvec, const double* q0, const double* bounds, int chebyord, int df,
+                                 double* auto_out, double* q1h1p, int* order_out) {
   const int ord = chebyord - chebyord % 2;   // chebyshev_initialise (:136)
   const int64_t N = mat_dim(c), n1 = mat_n1(c);
   ChebGPU G;
@@ -342,7 +352,7 @@ extern "C" int adcgpu_chebyshev_auto(adcgpu_ctx* h, int nvec, const double* q0, 
     }
   }
   if (order_out) *order_out = ord;
-  return sigma_status(c);
+  return ADCGPU_OK;
 }
 
 extern "C" int adcgpu_chebyshev_project(adcgpu_ctx* h, int nvec, double* q0, const double* bounds, int chebyord,
@@ -352,6 +362,11 @@ extern "C" int adcgpu_chebyshev_project(adcgpu_ctx* h, int nvec, double* q0, con
   if (!c) return ADCGPU_BAD_INPUT;
   cudaSetDevice(c->device);
   ST(cheb_check(c, nvec, q0, bounds, chebyord));
+  return sigma_result(c, cheb_project_run(c, nvec, q0, bounds, chebyord, projen, df));
+}
+
+static int adcgpu::cheb_project_run(Ctx* c, int nvec, double* q0, const double* bounds, int chebyord, double projen,
+                                    int df) {
   const int ord = chebyord - chebyord % 2;
   const int64_t N = mat_dim(c);
   // project_psi0 (:420-446): escale, the Jackson damping g_k and the
@@ -381,7 +396,7 @@ extern "C" int adcgpu_chebyshev_project(adcgpu_ctx* h, int nvec, double* q0, con
   ST(G.expand(a, b, &coef, 0, df));
   ADC_CUDA(c, cudaMemcpyAsync(q0, G.acc, G.blk_bytes, cudaMemcpyDeviceToHost, c->stream));
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
-  return sigma_status(c);
+  return ADCGPU_OK;
 }
 
 extern "C" int adcgpu_spectral_bounds(adcgpu_ctx* h, const adcgpu_dav_params* fp, double* bounds) {
@@ -392,6 +407,10 @@ extern "C" int adcgpu_spectral_bounds(adcgpu_ctx* h, const adcgpu_dav_params* fp
   if (!c->have_matrix) return set_err(c, ADCGPU_NO_MATRIX, "build the matrix first");
   if (!bounds) return set_err(c, ADCGPU_BAD_INPUT, "bounds required");
   if (mat_dim(c) < 200) return set_err(c, ADCGPU_BAD_INPUT, "the Lanczos estimate needs ndim >= 200 (2 x 100 vectors)");
+  return sigma_result(c, spectral_bounds_run(c, fp, bounds));
+}
+
+static int adcgpu::spectral_bounds_run(Ctx* c, const adcgpu_dav_params* fp, double* bounds) {
   // lower bound: one-root block Davidson (specbounds.f90:151-176).  The
   // reference sets davstates_f, dmain_f, maxsubdim_f, davtol_f and
   // lsubdiag_f; maxiter, precon, ldfl and guessdim stay the caller's
@@ -417,6 +436,7 @@ extern "C" int adcgpu_spectral_bounds(adcgpu_ctx* h, const adcgpu_dav_params* fp
   p.precision = ADCGPU_FP64;
   double lower = 0.0;
   adcgpu_dav_info info;
+  adcgpu_ctx* const h = reinterpret_cast<adcgpu_ctx*>(c);
   ST(adcgpu_davidson(h, &p, &lower, nullptr, &info));
   // upper bound: block Lanczos, block 2, 100 cycles, PRO, from the single
   // subspace diagonalisation (:178-199); the last Lanczos state energy
@@ -426,5 +446,5 @@ extern "C" int adcgpu_spectral_bounds(adcgpu_ctx* h, const adcgpu_dav_params* fp
   ST(adcgpu_block_lanczos(h, 2, 100, 1, q0.data(), nullptr, ev.data(), nullptr));
   bounds[0] = lower;
   bounds[1] = ev[199];
-  return sigma_status(c);
+  return ADCGPU_OK;
 }

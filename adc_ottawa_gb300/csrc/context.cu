@@ -126,6 +126,7 @@ int adcgpu_ctx_create(int device, adcgpu_ctx** out) {
   else cudaGetLastError();
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->word_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaMallocHost((void**)&c->h_word, sizeof(int)) != cudaSuccess ||
       cudaMalloc((void**)&c->d_word, sizeof(int)) != cudaSuccess ||
       cudaMemsetAsync(c->d_word, 0, sizeof(int), c->stream) != cudaSuccess) {
@@ -150,6 +151,7 @@ int adcgpu_ctx_destroy(adcgpu_ctx* h) {
   dfree(c, c->d_dpl);
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
+  cudaEventDestroy(c->word_ev);
   if (c->st_ev0) cudaEventDestroy(c->st_ev0);
   if (c->st_ev1) cudaEventDestroy(c->st_ev1);
   cudaFreeHost(c->h_word);
@@ -495,7 +497,7 @@ int adcgpu_sigma_device(adcgpu_ctx* h, int m, const void* dv, void* dw, int64_t 
   int st = c->precision == ADCGPU_MIXED
                ? sigma_fp32(c, m, (const float*)dv, ld, (float*)dw, ld)
                : sigma_fp64(c, m, (const double*)dv, ld, (double*)dw, ld);
-  if (st) return st;
+  if (st) return sigma_result(c, st);
   ADC_CUDA(c, cudaEventRecord(c->ev1, c->stream));
   ADC_CUDA(c, cudaEventSynchronize(c->ev1));
   float ms = 0.f;
@@ -555,6 +557,15 @@ int adcgpu_set_fp64_arith(adcgpu_ctx* h, int mode) {
   if (!c) return ADCGPU_BAD_INPUT;
   if (mode != 0 && mode != 1) return set_err(c, ADCGPU_BAD_INPUT, "fp64 arithmetic mode is 0 or 1");
   c->dense_df = mode;
+  return ADCGPU_OK;
+}
+
+int adcgpu_test_set_status(adcgpu_ctx* h, int code) {
+  Ctx* c = reinterpret_cast<Ctx*>(h);
+  CTX_CHECK(c);
+  if (code <= 0) return set_err(c, ADCGPU_BAD_INPUT, "stage code > 0");
+  ADC_CUDA(c, cudaMemcpyAsync(c->d_word, &code, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  ADC_CUDA(c, cudaStreamSynchronize(c->stream));
   return ADCGPU_OK;
 }
 

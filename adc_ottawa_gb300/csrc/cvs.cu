@@ -141,6 +141,7 @@ __global__ void k_cvs_export_coupling(int64_t n2, int cn1, int64_t base, const i
 
 int sigma_cvs(Ctx* c, int m, const double* dV, int64_t ldv, double* dW, int64_t ldw) {
   const int cn1 = (int)c->cvs_n1;
+  ST(sigma_status_so_far(c));
   k_cvs_singles<<<std::max(1, std::min(c->nsm * 8, (cn1 * m + 7) / 8)), 256, 0, c->stream>>>(cn1, m, c->d_Ac, dV,
                                                                                                   ldv, dW, ldw);
   ADC_COUNT_LAUNCH();

@@ -648,8 +648,7 @@ extern "C" int adcgpu_davidson(adcgpu_ctx* h, const adcgpu_dav_params* p, double
   if (!c || !p || !evals) return ADCGPU_BAD_INPUT;
   cudaSetDevice(c->device);
   if (!c->have_matrix) return set_err(c, ADCGPU_NO_MATRIX, "build the matrix first");
-  const int st = davidson_solve(c, p, evals, evecs, info, nullptr), status = sigma_status(c);
-  return status ? status : st;
+  return sigma_result(c, davidson_solve(c, p, evals, evecs, info, nullptr));
 }
 
 extern "C" int adcgpu_davidson_trace(adcgpu_ctx* h, const adcgpu_dav_params* p, int every, int max_records,
@@ -685,8 +684,7 @@ extern "C" int adcgpu_davidson_trace(adcgpu_ctx* h, const adcgpu_dav_params* p, 
   if (nrec) *nrec = D.tr_n;
   D.release();
   dfree(c, out, 0);
-  const int status = sigma_status(c);
-  return status ? status : st;
+  return sigma_result(c, st);
 }
 
 extern "C" int adcgpu_write_davidson_file(const char* path, int ndim, int nstates, const double* evals,

@@ -249,9 +249,10 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // status of the bounded waits in the tensor-core sigma kernels: they write
-  // d_word, every product queues a copy to the pinned h_word, sigma_status()
-  // reads it once the copy is done
+  // d_word, every product queues a copy to the pinned h_word and records
+  // word_ev, sigma_status() reads it once the copy is done
   int *d_word = nullptr, *h_word = nullptr;
+  cudaEvent_t word_ev = nullptr;
   bool word_pending = false;
   std::string err;
   Geometry geom;
@@ -472,9 +473,18 @@ int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t l
               double* W1, int64_t ld1);
 int sigma_queue_status(Ctx* c);
 // Waits for the products queued so far and returns ADCGPU_DEVICE_TIMEOUT when
-// a pipeline wait gave up.  Called before the next product and before results
-// leave the library, not after every product.
+// a pipeline wait gave up.  Called before results leave the library, not after
+// every product.
 int sigma_status(Ctx* c);
+// The same for the products that are known to be done, without waiting: every
+// product begins with it, so that none follows a failed one for long.
+int sigma_status_so_far(Ctx* c);
+// The return value of an entry point that ran products: a wait that gave up
+// comes before whatever its rows led to, and is not left for the next call.
+inline int sigma_result(Ctx* c, int st) {
+  const int status = sigma_status(c);
+  return status ? status : st;
+}
 
 // sigma_ab.cu : segments A and B of the mixed-precision sigma product in
 // compact form (tables copied from the BF16 or FP32 value store on first use)

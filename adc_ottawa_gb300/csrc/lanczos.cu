@@ -322,6 +322,5 @@ extern "C" int adcgpu_block_lanczos(adcgpu_ctx* h, int lmain, int ncycles, int o
   if ((int64_t)lmain * ncycles > mat_dim(c)) return set_err(c, ADCGPU_BAD_INPUT, "nvec exceeds the dimension");
   LanczosGPU L;
   L.c = c; L.N = mat_dim(c); L.b = lmain; L.ncycles = ncycles;
-  const int st = L.run(orthotype, q0, tmat, evals, ritz), status = sigma_status(c);
-  return status ? status : st;
+  return sigma_result(c, L.run(orthotype, q0, tmat, evals, ritz));
 }

@@ -1445,7 +1445,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
     ADC_CUDA(c, cudaEventCreate(&c->st_ev1));
   }
   sigma_stats_flush(c);
-  if (c->word_pending && *c->h_word) ST(sigma_status(c));   // copied before the stop event just waited for
+  ST(sigma_status_so_far(c));
   ADC_CUDA(c, cudaEventRecord(c->st_ev0, s));
   GeomDev g = to_dev(G);
   // singles block first (plain stores), then the coupling adds atomically
@@ -1901,7 +1901,7 @@ extern "C" int adcgpu_sigma_autotune(adcgpu_ctx* h, int m, int* best_chunk, int*
       if (t < best) { best = t; bc = ch; bm = mc; bs = stg; bt = 0; }
     }
   }
-  if (!st) st = sigma_status(c);
+  st = sigma_result(c, st);
   sigma_stats_flush(c);
   c->st_calls = 0; c->st_cols = 0; c->st_ms = 0.0; c->st_bytes = 0.0;
   for (auto& b : c->st_by) for (double& x : b) x = 0.0;

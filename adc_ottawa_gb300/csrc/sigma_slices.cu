@@ -1592,8 +1592,17 @@ int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t l
 
 int sigma_queue_status(Ctx* c) {
   ADC_CUDA(c, cudaMemcpyAsync(c->h_word, c->d_word, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  ADC_CUDA(c, cudaEventRecord(c->word_ev, c->stream));
   c->word_pending = true;
   return ADCGPU_OK;
+}
+
+int sigma_status_so_far(Ctx* c) {
+  if (!c->word_pending) return ADCGPU_OK;
+  const cudaError_t e = cudaEventQuery(c->word_ev);
+  if (e == cudaErrorNotReady) return ADCGPU_OK;
+  ADC_CUDA(c, e);
+  return *c->h_word ? sigma_status(c) : ADCGPU_OK;
 }
 
 int sigma_status(Ctx* c) {

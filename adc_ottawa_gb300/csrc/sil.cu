@@ -410,6 +410,11 @@ struct SilEngine {
   }
 };
 
+static int autocorr_run(Ctx* c, int nwp, const double* f, double tout, double tfinal, int kdim, double tol,
+                        double* auto_out, int* ntimes_out, int64_t* nmult_out);
+static int silstep_run(Ctx* c, double* psi, double* dtpsi, double intperiod, int intorder, double tol, int relax,
+                       double* stepsize_out, int* trueorder_out, adcgpu_sil_state* st);
+
 }  // namespace adcgpu
 
 using namespace adcgpu;
@@ -423,6 +428,11 @@ extern "C" int adcgpu_autocorr(adcgpu_ctx* h, int nwp, const double* f, double t
   if (c->precision != ADCGPU_FP64) return set_err(c, ADCGPU_BAD_INPUT, "SIL runs on the FP64 matrix");
   if (nwp <= 0 || !f || !auto_out || tout <= 0.0 || tfinal < 0.0 || kdim < 2)
     return set_err(c, ADCGPU_BAD_INPUT, "autocorr arguments");
+  return sigma_result(c, autocorr_run(c, nwp, f, tout, tfinal, kdim, tol, auto_out, ntimes_out, nmult_out));
+}
+
+static int adcgpu::autocorr_run(Ctx* c, int nwp, const double* f, double tout, double tfinal, int kdim, double tol,
+                                double* auto_out, int* ntimes_out, int64_t* nmult_out) {
   const int64_t N = mat_dim(c);
   SilEngine E;
   E.c = c; E.N = N; E.P = nwp; E.kdim = kdim;
@@ -482,7 +492,7 @@ extern "C" int adcgpu_autocorr(adcgpu_ctx* h, int nwp, const double* f, double t
   }
   if (ntimes_out) *ntimes_out = ntimes;
   if (nmult_out) *nmult_out = E.nmult / std::max(1, nwp);
-  return sigma_status(c);
+  return ADCGPU_OK;
 }
 
 extern "C" int adcgpu_silstep(adcgpu_ctx* h, double* psi, double* dtpsi, int psidim, double intperiod, int intorder,
@@ -496,6 +506,11 @@ extern "C" int adcgpu_silstep(adcgpu_ctx* h, double* psi, double* dtpsi, int psi
   if (intorder < 2) return ADCGPU_SIL_BAD_ORDER;
   if (!restart) return set_err(c, ADCGPU_UNSUPPORTED, "non-restart SILStep calls keep Krylov vectors; use restart");
   if (!stdform) return set_err(c, ADCGPU_UNSUPPORTED, "Func must be -iH (StdForm) on this path");
+  return sigma_result(c, silstep_run(c, psi, dtpsi, intperiod, intorder, tol, relax, stepsize_out, trueorder_out, st));
+}
+
+static int adcgpu::silstep_run(Ctx* c, double* psi, double* dtpsi, double intperiod, int intorder, double tol, int relax,
+                               double* stepsize_out, int* trueorder_out, adcgpu_sil_state* st) {
   const int64_t N = mat_dim(c);
   SilEngine E;
   E.c = c; E.N = N; E.P = 1; E.kdim = intorder;
@@ -518,5 +533,5 @@ extern "C" int adcgpu_silstep(adcgpu_ctx* h, double* psi, double* dtpsi, int psi
   if (stepsize_out) *stepsize_out = pk[0].Stepsize;
   if (trueorder_out) *trueorder_out = pk[0].TrueOrder;
   if (st) *st = pk[0].save;
-  return sigma_status(c);
+  return ADCGPU_OK;
 }

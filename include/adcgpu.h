@@ -429,6 +429,12 @@ int64_t adcgpu_device_bytes(const adcgpu_ctx* ctx);
    Chebyshev); the mixed ladder's FP64 refinement always uses 1. */
 int adcgpu_set_fp64_arith(adcgpu_ctx* ctx, int mode);
 
+/* For tests: puts stage 'code' into the status word that a pipeline wait of the
+   tensor-core sigma kernels writes when it gives up, so that the handling of
+   ADCGPU_DEVICE_TIMEOUT can be tested without a lost wait.  Kernels that find
+   the word set return at once; the call that reports it clears it. */
+int adcgpu_test_set_status(adcgpu_ctx* ctx, int code);
+
 /* Number of CUDA kernels this library has launched in this process, over
    all contexts (a monotonic counter; differences give the launches of a
    region). */
