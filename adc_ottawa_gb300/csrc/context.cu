@@ -32,10 +32,14 @@ int set_err(Ctx* c, int code, const std::string& msg) {
   return code;
 }
 
-int dmalloc(Ctx* c, void** p, size_t bytes) {
+int dmalloc(Ctx* c, void** p, size_t bytes, bool reclaim) {
   *p = nullptr;
   if (bytes == 0) bytes = 16;
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && reclaim && oz_reclaim(c->device) > 0) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     char buf[160];
@@ -549,7 +553,7 @@ double adcgpu_last_sigma_ms(const adcgpu_ctx* h) {
 
 int64_t adcgpu_device_bytes(const adcgpu_ctx* h) {
   const Ctx* c = reinterpret_cast<const Ctx*>(h);
-  return c ? c->dev_bytes : 0;
+  return c ? c->dev_bytes + c->oz_bytes.load() : 0;
 }
 
 int adcgpu_set_fp64_arith(adcgpu_ctx* h, int mode) {

@@ -151,10 +151,13 @@ int sigma_cvs(Ctx* c, int m, const double* dV, int64_t ldv, double* dW, int64_t 
   // atomics: 1.85 ms for 7 columns at nocc=9, nvirt=107, 3 core orbitals)
   // takes the rows with a' = b', and all rows when the digits do not fit
   bool usable = false;
-  ST(oz_prepare_cvs(c, c->cvs_oz, m, &usable));
   int64_t n2 = c->cvs_N - cn1;
+  {
+    const std::unique_lock<std::mutex> lock = oz_lock(c, c->cvs_oz);
+    ST(oz_prepare_cvs(c, c->cvs_oz, m, &usable));
+    if (usable) ST(oz_launch(c, c->cvs_oz, c->d_diag, dV, ldv, m, dW, ldw, dW, ldw));
+  }
   if (usable) {
-    ST(oz_launch(c, c->cvs_oz, c->d_diag, dV, ldv, m, dW, ldw, dW, ldw));
     const int64_t nc = cn1 / c->geom.nv;
     n2 = nc * (c->geom.no - nc) * c->geom.nv;
   }

@@ -45,6 +45,7 @@
 #include <thread>
 #include <string>
 #include <unordered_map>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -307,6 +308,7 @@ struct Ctx {
   int st_pending_kind = 0;        // value store of the pending call: 0 BF16, 1 FP32, 2 FP64
   double st_by[3][4] = {};        // per value store: calls, ms, algorithmic bytes, columns
   int64_t dev_bytes = 0;          // sum of the live dmalloc sizes
+  std::atomic<int64_t> oz_bytes{0};   // digits of the sliced sigma products (another thread may give them back)
   std::unordered_map<void*, size_t> dev_allocs;   // dmalloc pointer -> size
   // learned preconditioner (MlpState, mlp.cu); DPR is used when absent
   void* mlp = nullptr;
@@ -374,7 +376,9 @@ inline cudaError_t d2h(Ctx* c, void* dst, const void* src, size_t bytes) {
   return e != cudaSuccess ? e : cudaStreamSynchronize(c->stream);
 }
 
-int dmalloc(Ctx* c, void** p, size_t bytes);
+// reclaim: when the device has no room, the digit stores of all contexts are
+// given back and the allocation is tried once more
+int dmalloc(Ctx* c, void** p, size_t bytes, bool reclaim = true);
 void dfree(Ctx* c, void* p, size_t bytes = 0);
 
 // ---------------------------------------------------------------------------
@@ -462,6 +466,11 @@ int umma3_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float
 // sigma_slices.cu : tensor-core pass by exact digit slices (FP64 and FP32 values)
 bool oz_geometry_ok(const Geometry& G);
 std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, int64_t row1, int64_t* reserve);
+// The digit stores are a cache: a dmalloc that fails gives back those of every
+// context on the device (oz_reclaim, from any thread) and tries once more.  So a
+// product prepares and uses its digits under the plan's lock (made on first use).
+std::unique_lock<std::mutex> oz_lock(Ctx* c, void*& handle);
+int64_t oz_reclaim(int device);
 int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int64_t reserve, int m,
                bool* usable);
 int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable);

@@ -1479,6 +1479,7 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
       // FP64 and FP32 values on the tensor cores by exact digit slices
       if (P->tiled == 1 && !P->umma_off && !(sizeof(T) == 4 && (P->umma3_on || P->ab_off))) {
         void*& oz = plan->oz[sizeof(T) == 8 ? 0 : 1];
+        const std::unique_lock<std::mutex> lock = oz_lock(c, oz);
         // the digits of a range are made and used before those of the next
         int64_t reserve = 0;
         bool usable = true;
@@ -1486,6 +1487,8 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
         const int64_t ld1 = sizeof(T) == 8 ? ldw : (int64_t)n1;
         for (const auto& rg : oz_ranges(c, row0, row1, &reserve)) {
           ST(oz_prepare(c, oz, BtP, sizeof(T) == 8, rg.first, rg.second, reserve, m, &usable));
+          // (the memory and the lists of the first range serve all of them)
+          if (!usable && rg.first != row0) return set_err(c, ADCGPU_OUT_OF_MEMORY, "digits of a range");
           if (!usable) break;
           ST(oz_launch(c, oz, diag, dV, ldv, m, dW, ldw, W1, ld1));
           oz_used = true;

@@ -1145,8 +1145,11 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, seg_blocks<KT>())
 
 // Digit store of the rows [row0, row1) of B^T and the work lists of the pass.
 struct OzPlan {
+  Ctx* ctx = nullptr;
+  std::mutex mu;                      // held while a product is prepared and queued
   unsigned char* d_mem = nullptr;     // C|D digits, segment digits, their row exponents
   size_t mem_bytes = 0;
+  bool refused = false;               // the digits did not fit when this matrix first asked
   uint16_t *dig = nullptr, *seg = nullptr;
   int16_t *rexp = nullptr, *sexp = nullptr;
   const void* values_for = nullptr;   // value store the digits were made of
@@ -1165,13 +1168,101 @@ struct OzPlan {
   int item_rows = 0, lists_m = 0;
 };
 
+// All plans of the process, for oz_reclaim.  Lock order: the registry, then one
+// plan at a time; a thread that holds a plan's lock takes no other.
+static std::mutex g_oz_mu;
+static std::vector<OzPlan*> g_oz_plans;
+
+std::unique_lock<std::mutex> oz_lock(Ctx* c, void*& handle) {
+  OzPlan* p = reinterpret_cast<OzPlan*>(handle);
+  if (!p) {
+    p = new OzPlan;
+    p->ctx = c;
+    const std::lock_guard<std::mutex> lock(g_oz_mu);
+    g_oz_plans.push_back(p);
+    handle = p;
+  }
+  return std::unique_lock<std::mutex>(p->mu);
+}
+
+// the digits (the plan's lock is held, and nothing queued reads them)
+static void oz_drop_digits(OzPlan* p) {
+  if (!p->d_mem) return;
+  cudaFree(p->d_mem);
+  p->ctx->oz_bytes -= (int64_t)p->mem_bytes;
+  p->d_mem = nullptr;
+  p->mem_bytes = 0;
+  p->values_for = nullptr;
+}
+
+int64_t oz_reclaim(int device) {
+  const std::lock_guard<std::mutex> registry(g_oz_mu);
+  int64_t n = 0;
+  for (OzPlan* p : g_oz_plans) {
+    if (p->ctx->device != device) continue;
+    const std::lock_guard<std::mutex> lock(p->mu);
+    if (!p->d_mem) continue;
+    n += (int64_t)p->mem_bytes;
+    cudaStreamSynchronize(p->ctx->stream);   // its queued products
+    oz_drop_digits(p);
+  }
+  return n;
+}
+
 void oz_free(Ctx* c, void*& handle) {
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
   if (!p) return;
-  dfree(c, p->d_mem);
+  {
+    const std::lock_guard<std::mutex> registry(g_oz_mu);
+    g_oz_plans.erase(std::find(g_oz_plans.begin(), g_oz_plans.end(), p));
+  }
+  oz_drop_digits(p);
   dfree(c, p->d_lists);
   delete p;
   handle = nullptr;
+}
+
+// no room for the work lists beside the digits
+static int oz_give_up(Ctx* c, OzPlan* p) {
+  ADC_CUDA(c, cudaStreamSynchronize(c->stream));
+  oz_drop_digits(p);
+  p->item_rows = 0;
+  p->refused = true;
+  return ADCGPU_OK;
+}
+
+// Room for the digits: a third of the device memory that is free now at most.
+// The answer is kept for the matrix (until its digits are given back), so that
+// its products do not change kernels with what else comes and goes on the device.
+static int oz_room(Ctx* c, OzPlan* p, size_t bytes, bool* ok) {
+  *ok = false;
+  if (p->refused) return ADCGPU_OK;
+  if (p->mem_bytes >= bytes) {
+    *ok = true;
+    return ADCGPU_OK;
+  }
+  // below 64 MB the question costs more than the answer is worth (40 us)
+  if (bytes > (64u << 20)) {
+    size_t free_b = 0, total_b = 0;
+    ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
+    if (bytes > (free_b + p->mem_bytes) / 3) {
+      p->refused = true;
+      return ADCGPU_OK;
+    }
+  }
+  oz_drop_digits(p);
+  const cudaError_t e = cudaMalloc((void**)&p->d_mem, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    p->d_mem = nullptr;
+    p->refused = true;
+    return ADCGPU_OK;
+  }
+  ADC_CUDA(c, e);
+  p->mem_bytes = bytes;
+  c->oz_bytes += (int64_t)bytes;
+  *ok = true;
+  return ADCGPU_OK;
 }
 
 void oz_invalidate(void* handle) {
@@ -1290,7 +1381,7 @@ int oz_upload_lists(Ctx* c, OzPlan* p, int item_rows, int m) {
     dfree(c, p->d_lists);
     p->d_lists = nullptr;
     p->list_bytes = 0;
-    ST(dmalloc(c, (void**)&p->d_lists, need));
+    ST(dmalloc(c, (void**)&p->d_lists, need, false));   // (the plan is locked)
     p->list_bytes = need;
   }
   p->items = reinterpret_cast<OzItem*>(p->d_lists);
@@ -1313,8 +1404,8 @@ int oz_upload_lists(Ctx* c, OzPlan* p, int item_rows, int m) {
 // the direct path's chunk buffer is rewritten for every chunk) and the work
 // lists of an m-column product.  reserve: bytes the digits of any range of
 // this matrix may take.  *usable stays false, and the CUDA-core tile takes the
-// product, for shapes the pass does not take and when the digits would fill
-// more than a third of the device memory that is free now.
+// product, for shapes the pass does not take and when there is no room for the
+// digits.  The plan is locked (oz_lock).
 int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0, int64_t row1, int64_t reserve, int m,
                bool* usable) {
   *usable = false;
@@ -1322,30 +1413,12 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
   if (!oz_geometry_ok(G)) return ADCGPU_OK;
   const int S = f64 ? 7 : 4;
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
-  if (!p) {
-    p = new OzPlan;
-    handle = p;
-  }
   OzDst dst;
   const int kw = (G.no + 15) / 16 * 16;
   const OzBytes need = oz_bytes(G, row0, row1, S, &dst);
-  const size_t bytes = std::max(need.all, (size_t)reserve);
-  if (p->mem_bytes < bytes) {
-    // below 64 MB the question costs more than the answer is worth (40 us)
-    if (bytes > (64u << 20)) {
-      size_t free_b = 0, total_b = 0;
-      ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
-      if (bytes > (free_b + p->mem_bytes) / 3) return ADCGPU_OK;
-    }
-    dfree(c, p->d_mem);
-    p->d_mem = nullptr;
-    p->mem_bytes = 0;
-    p->values_for = nullptr;
-    const int st = dmalloc(c, (void**)&p->d_mem, bytes);
-    if (st == ADCGPU_OUT_OF_MEMORY) return ADCGPU_OK;
-    ST(st);
-    p->mem_bytes = bytes;
-  }
+  bool room = false;
+  ST(oz_room(c, p, std::max(need.all, (size_t)reserve), &room));
+  if (!room) return ADCGPU_OK;
   if (!(p->values_for && p->values_for == values && p->S == S && p->dst.row0 == row0 && p->dst.row1 == row1)) {
     p->dst = dst;
     p->S = S;
@@ -1398,7 +1471,9 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
     }
     if (!c->direct)
       for (OzItem& it : p->h_items) set_tile(it);
-    ST(oz_upload_lists(c, p, item_rows, m));
+    const int st = oz_upload_lists(c, p, item_rows, m);
+    if (st == ADCGPU_OUT_OF_MEMORY) return oz_give_up(c, p);
+    ST(st);
   }
   // the prepared rows' items
   auto first = [](const auto& v, int64_t row) {
@@ -1421,7 +1496,7 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
 
 // Digits and work lists of the CVS matrix's pair rows (spins I and II); the
 // rows with a' = b' stay with the compressed-row kernel.
-int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable) {
+int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable) {   // (the plan is locked)
   *usable = false;
   const Geometry& G = c->geom;
   constexpr int S = 7;
@@ -1439,20 +1514,11 @@ int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable) {
   const int64_t tps = (npair + OZ_ROWS - 1) / OZ_ROWS;
   if (nrows == 0 || c->cvs_N != c->cvs_n1 + c3 + nrows) return ADCGPU_OK;
   OzPlan* p = reinterpret_cast<OzPlan*>(handle);
-  if (!p) {
-    p = new OzPlan;
-    handle = p;
-  }
   const size_t dig_b = align256(sizeof(uint16_t) * (size_t)(2 * npp * tps) * S * nbox * OZ_ROWS * OZ_BOX);
   const size_t seg_b = align256(sizeof(uint16_t) * (size_t)nrows * 2 * S * kw), exp_b = align256(sizeof(int16_t) * (size_t)nrows);
-  if (!p->d_mem) {
-    const size_t bytes = dig_b + seg_b + 2 * exp_b;
-    size_t free_b = 0, total_b = 0;
-    ADC_CUDA(c, cudaMemGetInfo(&free_b, &total_b));
-    if (bytes > free_b / 3) return ADCGPU_OK;
-    ST(dmalloc(c, (void**)&p->d_mem, bytes));
-    p->mem_bytes = bytes;
-  }
+  bool room = false;
+  ST(oz_room(c, p, dig_b + seg_b + 2 * exp_b, &room));
+  if (!room) return ADCGPU_OK;
   p->geom = OzGeom{nc, G.nv, G.nvP, c->cvs_n1, 0};
   if (p->values_for != c->d_cval) {
     p->S = S;
@@ -1477,7 +1543,9 @@ int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable) {
       for (int i = first; i < (int)p->h_items.size(); ++i)
         p->h_items[i].tile = (int)((s * tps + (p->h_items[i].row0 - s * npair) / OZ_ROWS) * nbox);
     }
-    ST(oz_upload_lists(c, p, item_rows, m));
+    const int st = oz_upload_lists(c, p, item_rows, m);
+    if (st == ADCGPU_OUT_OF_MEMORY) return oz_give_up(c, p);
+    ST(st);
   }
   p->item0 = p->slab0 = 0;
   p->nitems = (int)p->h_items.size();

@@ -413,9 +413,12 @@ int adcgpu_davidson_trace(adcgpu_ctx* ctx, const adcgpu_dav_params* p, int every
 double adcgpu_last_sigma_ms(const adcgpu_ctx* ctx);
 
 /* Device bytes held by the context (matrix, ERI blocks, work spaces; from the
-   first sigma product on also the digits its tensor-core pass reads, 14 bytes
-   per FP64 value and 8 per FP32 value, if they fit a third of the memory that
-   is free then). */
+   first sigma product on also the digits its tensor-core pass reads: 14 bytes
+   per FP64 value and 8 per FP32 value, with rows padded to 64 values and slabs to
+   128 rows, which multiplies them for small systems).  A matrix whose digits do
+   not fit a third of the memory that is free at its first product keeps its other
+   kernels.  The digits are given back when an allocation of any context of the
+   process on the device finds no room (the next product then asks again). */
 int64_t adcgpu_device_bytes(const adcgpu_ctx* ctx);
 
 /* Arithmetic of the FP64 path's block products (no reference counterpart;
