@@ -57,7 +57,7 @@ __host__ __device__ inline void untri(int64_t t, int64_t& P, int64_t& Q) {
 // kind 0: (a i|b j) 1: (a b|i j) 2: (i j|k a) 3: (a b|i c) 4: (i j|k l)
 // 5: (a c|b d) packed over virtual pairs, index tri(pair(a,c), pair(b,d))
 __global__ void k_gather_block(const double* __restrict__ packed, double* __restrict__ out, int kind,
-                               int no, int nv, int64_t total) {
+                               int no, int nv, int64_t total, int b0 = 0, int nb = 0) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
     int64_t x = t;
@@ -74,24 +74,24 @@ __global__ void k_gather_block(const double* __restrict__ packed, double* __rest
                 p = no + a; q = no + b; r = i; s = j; } break;
       case 2: { int a = x % nv; x /= nv; int k = x % no; x /= no; int j = x % no; int i = (int)(x / no);
                 p = i; q = j; r = k; s = no + a; } break;
-      default: { int c = x % nv; x /= nv; int i = x % no; x /= no; int b = x % nv; int a = (int)(x / nv);
+      default: { int c = x % nv; x /= nv; int i = x % no; x /= no; int b = b0 + x % nb; int a = (int)(x / nb);
                  p = no + a; q = no + b; r = i; s = no + c; } break;
     }
     out[t] = packed[canon(p, q, r, s)];
   }
 }
 
-// (a b|i c) from [a][b][i][c] to the stored [b][i][c][a]: per b a transposition
-// of nv x (no nv) through 32 x 32 tiles.
+// (a b|i c) of nb values of b (gridDim.z) from [a][b][i][c] to the stored
+// [b][i][c][a]: per b a transposition of nv x (no nv) through 32 x 32 tiles.
 __global__ void __launch_bounds__(256) k_vvov_layout(const double* __restrict__ in, double* __restrict__ out, int no,
                                                      int nv) {
   __shared__ double t[32][33];
   const int64_t w = (int64_t)no * nv;
-  const int b = blockIdx.z, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int b = blockIdx.z, nb = gridDim.z, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int y = ty; y < 32; y += 8) {
     const int a = blockIdx.y * 32 + y;
     const int64_t x = blockIdx.x * 32ll + tx;
-    if (a < nv && x < w) t[y][tx] = in[((int64_t)a * nv + b) * w + x];
+    if (a < nv && x < w) t[y][tx] = in[((int64_t)a * nb + b) * w + x];
   }
   __syncthreads();
   for (int y = ty; y < 32; y += 8) {
@@ -672,19 +672,27 @@ int build_eri_blocks_from_packed(Ctx* c, const double* d_packed) {
     if (*dst[k]) { dfree(c, *dst[k], 0); *dst[k] = nullptr; }
     int st = dmalloc(c, (void**)dst[k], sizeof(double) * sz[k]);
     if (st) return st;
-    // (vv|ov): gathered as [a][b][i][c], then brought into the stored order
-    double* to = *dst[k];
-    if (k == 3 && (st = dmalloc(c, (void**)&to, sizeof(double) * sz[k]))) return st;
-    k_gather_block<<<grid_for(c, sz[k], 256), 256, 0, c->stream>>>(d_packed, to, k, no, nv, sz[k]); ADC_COUNT_LAUNCH();
-    ADC_CUDA(c, cudaGetLastError());
-    if (k == 3) {
-      k_vvov_layout<<<dim3((no * nv + 31) / 32, (nv + 31) / 32, nv), 256, 0, c->stream>>>(to, *dst[k], no, nv);
-      ADC_COUNT_LAUNCH();
-      ADC_CUDA(c, cudaGetLastError());
-      ADC_CUDA(c, cudaStreamSynchronize(c->stream));
-      dfree(c, to);
-    }
   }
+  // (vv|ov): as many b at a time as the (vv|vv) block, filled last, has room for
+  // are gathered there as [a][b][i][c], then brought into the stored order
+  const int64_t slab = (int64_t)nv * no * nv;
+  double* stage = c->d_vvvv;
+  if (sz[5] < slab) ST(dmalloc(c, (void**)&stage, sizeof(double) * slab));   // (nvirt^2 < about 8 nocc)
+  const int per = (int)std::max<int64_t>(1, std::min<int64_t>(nv, sz[5] / slab));
+  for (int b0 = 0; b0 < nv; b0 += per) {
+    const int nb = std::min(per, nv - b0);
+    k_gather_block<<<grid_for(c, nb * slab, 256), 256, 0, c->stream>>>(d_packed, stage, 3, no, nv, nb * slab, b0, nb);
+    ADC_COUNT_LAUNCH();
+    k_vvov_layout<<<dim3((no * nv + 31) / 32, (nv + 31) / 32, nb), 256, 0, c->stream>>>(
+        stage, c->d_vvov + b0 * slab, no, nv);
+    ADC_COUNT_LAUNCH();
+  }
+  for (int k : {0, 1, 2, 4, 5}) {
+    k_gather_block<<<grid_for(c, sz[k], 256), 256, 0, c->stream>>>(d_packed, *dst[k], k, no, nv, sz[k]); ADC_COUNT_LAUNCH();
+  }
+  const cudaError_t e = cudaGetLastError();
+  if (stage != c->d_vvvv) dfree(c, stage);
+  ADC_CUDA(c, e);
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
   return ADCGPU_OK;
 }
@@ -712,7 +720,7 @@ namespace {
 // and whatever the caller queues on the context's stream before join().
 struct SecondOrder {
   Ctx* c;
-  double *d_terms_a = nullptr, *d_terms_b = nullptr;
+  double* d_terms_a = nullptr;    // terms of CA, then those of CB
   int2* d_pairs = nullptr;
   cudaStream_t side = nullptr;
   cudaEvent_t ready = nullptr, done = nullptr;
@@ -726,7 +734,6 @@ struct SecondOrder {
     if (ready) cudaEventDestroy(ready);
     if (done) cudaEventDestroy(done);
     dfree(c, d_terms_a);
-    dfree(c, d_terms_b);
     dfree(c, d_pairs);
   }
   // d_ca (nv x nv) is complete on the context's stream, d_cb (no x no) after join()
@@ -740,13 +747,19 @@ struct SecondOrder {
     for (int k = 0; k < no; ++k)
       for (int k1 = k; k1 < no; ++k1) pairs.push_back(make_int2(k, k1));
     const int nb = (int)pairs.size() - na;
-    // batches of sums: term buffers near 1 GiB (a quarter on the direct path)
-    const int64_t budget = (int64_t)1 << (c->direct ? 25 : 27);
-    const int ba = (int)std::max<int64_t>(1, std::min<int64_t>(na, budget / nta));
-    const int bb = (int)std::max<int64_t>(1, std::min<int64_t>(nb, budget / ntb));
     ST(dmalloc(c, (void**)&d_pairs, sizeof(int2) * pairs.size()));
-    ST(dmalloc(c, (void**)&d_terms_a, sizeof(double) * (size_t)ba * nta));
-    ST(dmalloc(c, (void**)&d_terms_b, sizeof(double) * (size_t)bb * ntb));
+    // batches of sums: term buffers near 1 GiB each (a quarter on the direct
+    // path), smaller ones where the matrix leaves less room, one sum at least
+    int ba = 0, bb = 0;
+    for (int64_t budget = (int64_t)1 << (c->direct ? 25 : 27);; budget /= 2) {
+      ba = (int)std::max<int64_t>(1, std::min<int64_t>(na, budget / nta));
+      bb = (int)std::max<int64_t>(1, std::min<int64_t>(nb, budget / ntb));
+      const int st = dmalloc(c, (void**)&d_terms_a, sizeof(double) * (size_t)(ba * nta + bb * ntb));
+      if (st == ADCGPU_OUT_OF_MEMORY && (ba > 1 || bb > 1)) continue;
+      ST(st);
+      break;
+    }
+    double* const d_terms_b = d_terms_a + ba * nta;
     ADC_CUDA(c, cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     ADC_CUDA(c, cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
     ADC_CUDA(c, cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
