@@ -568,6 +568,7 @@ int adcgpu_test_set_status(adcgpu_ctx* h, int code) {
   Ctx* c = reinterpret_cast<Ctx*>(h);
   CTX_CHECK(c);
   if (code <= 0) return set_err(c, ADCGPU_BAD_INPUT, "stage code > 0");
+  c->oz_always = true;
   ADC_CUDA(c, cudaMemcpyAsync(c->d_word, &code, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   ADC_CUDA(c, cudaStreamSynchronize(c->stream));
   return ADCGPU_OK;

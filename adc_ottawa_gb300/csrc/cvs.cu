@@ -149,10 +149,11 @@ int sigma_cvs(Ctx* c, int m, const double* dV, int64_t ldv, double* dW, int64_t 
   // the pair rows (all but the first npp nvirt) on the tensor cores by exact
   // digit slices; the compressed-row kernel (FP64 multiply-adds and shared
   // atomics: 1.85 ms for 7 columns at nocc=9, nvirt=107, 3 core orbitals)
-  // takes the rows with a' = b', and all rows when the digits do not fit
+  // takes the rows with a' = b', and all rows of small products and when the
+  // digits do not fit
   bool usable = false;
   int64_t n2 = c->cvs_N - cn1;
-  {
+  if (oz_faster_cvs(c, m)) {
     const std::unique_lock<std::mutex> lock = oz_lock(c, c->cvs_oz);
     ST(oz_prepare_cvs(c, c->cvs_oz, m, &usable));
     if (usable) ST(oz_launch(c, c->cvs_oz, c->d_diag, dV, ldv, m, dW, ldw, dW, ldw));

@@ -255,6 +255,7 @@ struct Ctx {
   int *d_word = nullptr, *h_word = nullptr;
   cudaEvent_t word_ev = nullptr;
   bool word_pending = false;
+  bool oz_always = false;         // tests: the sliced pass whatever the column count
   std::string err;
   Geometry geom;
   bool have_orb = false, have_eri = false, have_matrix = false;
@@ -465,6 +466,8 @@ int umma3_launch(Ctx* c, void* handle, const float* V, int64_t ldv, int m, float
 
 // sigma_slices.cu : tensor-core pass by exact digit slices (FP64 and FP32 values)
 bool oz_geometry_ok(const Geometry& G);
+bool oz_faster(const Ctx* c, bool f64, int m);
+bool oz_faster_cvs(const Ctx* c, int m);
 std::vector<std::pair<int64_t, int64_t>> oz_ranges(const Ctx* c, int64_t row0, int64_t row1, int64_t* reserve);
 // The digit stores are a cache: a dmalloc that fails gives back those of every
 // context on the device (oz_reclaim, from any thread) and tries once more.  So a

@@ -13,8 +13,8 @@
 //   FP64 and FP32 values: exact digit slices on the tensor cores
 //     (sigma_slices.cu), segment A of the rows with a' = b' by k_sigma_rows_a
 //   BF16 values: sigma_umma.cu, segments in sigma_ab.cu
-//   otherwise (no room for the digits, nocc > 32 or nvirt > 256, or a launch
-//     shape that asks for it): the tiles k_sigma_tile / k_sigma_tile_mma from
+//   otherwise (few columns: oz_faster; no room for the digits, nocc > 32 or
+//     nvirt > 256, or a launch shape that asks for it): the tiles k_sigma_tile / k_sigma_tile_mma from
 //     16 columns, the per-warp pass 1 below, segment B in k_sigma_p2
 #include <cuda_bf16.h>
 
@@ -1477,7 +1477,8 @@ int sigma_impl(Ctx* c, int m, const T* dV, int64_t ldv, T* dW, int64_t ldw, cons
     int c0 = 0;
     if constexpr (!std::is_same<TV, __nv_bfloat16>::value) {
       // FP64 and FP32 values on the tensor cores by exact digit slices
-      if (P->tiled == 1 && !P->umma_off && !(sizeof(T) == 4 && (P->umma3_on || P->ab_off))) {
+      if (P->tiled == 1 && !P->umma_off && !(sizeof(T) == 4 && (P->umma3_on || P->ab_off)) &&
+          oz_faster(c, sizeof(T) == 8, m)) {
         void*& oz = plan->oz[sizeof(T) == 8 ? 0 : 1];
         const std::unique_lock<std::mutex> lock = oz_lock(c, oz);
         // the digits of a range are made and used before those of the next

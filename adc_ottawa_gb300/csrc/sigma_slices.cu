@@ -1273,6 +1273,36 @@ void oz_invalidate(void* handle) {
 // system the library takes
 bool oz_geometry_ok(const Geometry& G) { return G.no <= 32 && G.nv >= 2 && 2 * G.nvP <= 512; }
 
+// Column counts from which the sliced pass is the faster one.  It reads 14 (8)
+// bytes a value instead of 8 (4), pads segments A and B to 16 or 32 holes and
+// computes 8 or 16 columns whatever m is; the per-warp passes below 16 columns
+// take 4, 2 and 1 FP32 or 2 and 1 FP64 columns at a time.  Microseconds, per-warp
+// / sliced, at nocc/nvirt:
+//   FP64     10/110 m=1 1494/915; 5/19 m=1 166/89; 20/40 m=1 954/1150, m=2
+//            1773/1164; 32/32 m=1 1472/2049; 18/90 m=1 3406/3324; 3/6 m=1 77/86, m=2 102/87
+//   FP32     10/110 m=1 353/619, m=2 495/635, m=3 810/658, m=4 785/673; 8/40 m=2
+//            110/145, m=3 171/152; 5/130 m=3 394/379, m=4 326/388; 18/90 m=4
+//            1713/2188, m=8 3378/2246; 32/32 m=5 1113/1409, m=8 1531/1414; 2/6 m=4 61/87
+//   direct   (digits made in every product) 10/110 m=1 3805/4501, m=2 5357/4539;
+//            18/90 m=1 8015/10246, m=2 11223/10286; 5/19 m=1 737/1367, m=4 2292/1405
+bool oz_faster(const Ctx* c, bool f64, int m) {
+  const Geometry& G = c->geom;
+  if (c->oz_always) return true;
+  if (f64) return m > (c->direct || G.no > 16 ? 1 : 0) && m * G.nv >= 8;
+  // (tiny systems: the fixed time of the launches decides)
+  const int passes = m < 16 ? m / 4 + (m >> 1 & 1) + (m & 1) : (m + 15) / 16;
+  return m >= (G.no > 16 ? 6 : 3) && passes * G.nv > 12;
+}
+
+// The same for the CVS matrix against its compressed rows: an entry costs the row
+// kernel 11.5 ps a column, a row the sliced pass 0.85 ns more, and its launches
+// 25 us more.  (8/40, 1 core orbital: 4 columns 61/80 us, 8 100/89; 9/107: one
+// column 225/167; 14/60, 3 core orbitals: one column 158/200, two 239/201; 5/19,
+// 3: 32 columns 92/107.)
+bool oz_faster_cvs(const Ctx* c, int m) {
+  return c->oz_always || c->cvs_nnz * m - 74 * (c->cvs_N - c->cvs_n1) >= 2200000;
+}
+
 namespace {
 
 // rows of a typical range of the direct path: the digits of a range take about

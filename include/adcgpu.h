@@ -435,7 +435,9 @@ int adcgpu_set_fp64_arith(adcgpu_ctx* ctx, int mode);
 /* For tests: puts stage 'code' into the status word that a pipeline wait of the
    tensor-core sigma kernels writes when it gives up, so that the handling of
    ADCGPU_DEVICE_TIMEOUT can be tested without a lost wait.  Kernels that find
-   the word set return at once; the call that reports it clears it. */
+   the word set return at once; the call that reports it clears it.  From then on
+   all FP64 and FP32-value products of the context take the tensor-core pass by
+   digit slices, also those of few columns that other kernels are faster for. */
 int adcgpu_test_set_status(adcgpu_ctx* ctx, int code);
 
 /* Number of CUDA kernels this library has launched in this process, over
