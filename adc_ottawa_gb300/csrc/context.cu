@@ -147,6 +147,7 @@ int adcgpu_ctx_destroy(adcgpu_ctx* h) {
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
   free_matrix(c);
+  oz_free(c, c->oz_spare, false);
   free_eri(c);
   free_mlp(c);
   gram_free(c);

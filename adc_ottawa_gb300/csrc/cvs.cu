@@ -215,7 +215,7 @@ void free_cvs(Ctx* c) {
   dfree(c, c->d_crow); c->d_crow = nullptr;
   dfree(c, c->d_ccol); c->d_ccol = nullptr;
   dfree(c, c->d_cval); c->d_cval = nullptr;
-  oz_free(c, c->cvs_oz);
+  oz_free(c, c->cvs_oz, true);
   c->cvs = 0;
   c->cvs_n1 = c->cvs_N = c->cvs_nnz = 0;
   c->cvs_kpq.clear();

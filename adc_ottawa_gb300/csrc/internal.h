@@ -255,6 +255,7 @@ struct Ctx {
   int *d_word = nullptr, *h_word = nullptr;
   cudaEvent_t word_ev = nullptr;
   bool word_pending = false;
+  void* oz_spare = nullptr;       // plan and digits of a small matrix that is gone (sigma_slices.cu)
   bool oz_always = false;         // tests: the sliced pass whatever the column count
   std::string err;
   Geometry geom;
@@ -478,7 +479,7 @@ int oz_prepare(Ctx* c, void*& handle, const void* values, bool f64, int64_t row0
                bool* usable);
 int oz_prepare_cvs(Ctx* c, void*& handle, int m, bool* usable);
 void oz_invalidate(void* handle);
-void oz_free(Ctx* c, void*& handle);
+void oz_free(Ctx* c, void*& handle, bool keep);   // keep: small digits, for the context's next matrix
 int oz_launch(Ctx* c, void* handle, const double* diag, const double* V, int64_t ldv, int m, double* W, int64_t ldw,
               double* W1, int64_t ld1);
 int oz_launch(Ctx* c, void* handle, const float* diag, const float* V, int64_t ldv, int m, float* W, int64_t ldw,

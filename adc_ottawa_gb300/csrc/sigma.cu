@@ -1789,8 +1789,8 @@ void free_sigma_plan(Ctx* c) {
   dfree(c, plan->d_acc);
   dfree(c, plan->d_sk);
   umma_free(c, plan->umma);
-  oz_free(c, plan->oz[0]);
-  oz_free(c, plan->oz[1]);
+  oz_free(c, plan->oz[0], true);
+  oz_free(c, plan->oz[1], true);
   ab_free(c, plan->ab);
   delete plan;
   c->sigma_plan = nullptr;
