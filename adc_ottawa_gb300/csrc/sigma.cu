@@ -1861,6 +1861,7 @@ extern "C" int adcgpu_sigma_autotune(adcgpu_ctx* h, int m, int* best_chunk, int*
   cudaSetDevice(c->device);
   if (!c->have_matrix) return set_err(c, ADCGPU_NO_MATRIX, "build the matrix first");
   SigmaPlan* plan = reinterpret_cast<SigmaPlan*>(c->sigma_plan);
+  if (!plan) return set_err(c, ADCGPU_UNSUPPORTED, "the CVS sigma product has no launch shapes");
   const int64_t N = c->geom.N;
   const bool mixed = c->precision == ADCGPU_MIXED;
   const size_t esz = mixed ? sizeof(float) : sizeof(double);
@@ -1929,6 +1930,7 @@ extern "C" int adcgpu_sigma_set_shape(adcgpu_ctx* h, int chunk, int mc_fp64, int
   cudaSetDevice(c->device);
   if (!c->have_matrix) return set_err(c, ADCGPU_NO_MATRIX, "build the matrix first");
   SigmaPlan* plan = reinterpret_cast<SigmaPlan*>(c->sigma_plan);
+  if (!plan) return set_err(c, ADCGPU_UNSUPPORTED, "the CVS sigma product has no launch shapes");
   plan->staged = ((mc_fp64 | mc_fp32) & 8) ? 1 : 0;
   plan->tiled = ((mc_fp64 | mc_fp32) & 16) ? 0 : (((mc_fp64 | mc_fp32) & 32) ? 2 : 1);
   plan->umma_off = ((mc_fp64 | mc_fp32) & 64) ? 1 : 0;
