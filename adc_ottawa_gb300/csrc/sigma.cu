@@ -1906,6 +1906,9 @@ extern "C" int adcgpu_sigma_autotune(adcgpu_ctx* h, int m, int* best_chunk, int*
       if (t < best) { best = t; bc = ch; bm = mc; bs = stg; bt = 0; }
     }
   }
+  // where the product takes the per-warp pass at m columns in any case, the flag
+  // says nothing about other column counts: it stays, the shape is kept
+  if (m < 16 && !(mixed ? umma_supported(c) : oz_faster(c, true, m))) bt = 1;
   st = sigma_result(c, st);
   sigma_stats_flush(c);
   c->st_calls = 0; c->st_cols = 0; c->st_ms = 0.0; c->st_bytes = 0.0;

@@ -56,3 +56,20 @@ def test_the_kernel_follows_the_columns(gpu, kind, no, nv, m, sliced):
     digits = product() - first          # those that were not there
     assert (digits == 0) == sliced
     g.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_tuning_few_columns_leaves_the_others_alone(gpu, tmp_path, prec):
+    """One column takes the per-warp pass at nocc=17 whatever the flag for it
+    (bit 4) says; set, the flag would take it for every later product."""
+    from adc_ottawa_gb300 import AdcGpu, autotune
+
+    e, eri = system(17, 9, 94)
+    g = AdcGpu(0)
+    g.set_orbitals(17, 9, e)
+    g.set_eri_packed(eri)
+    g.write_fspace_adc2_1(None, precision=prec)
+    for i in range(4):
+        r = autotune.tune(g, 1, prec, cache=str(tmp_path / f"{i}.json"))
+        assert r["mc"] & 16 == 0
+    g.close()
