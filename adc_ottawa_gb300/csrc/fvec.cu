@@ -302,7 +302,7 @@ __global__ void k_fv_taub(int no, int nv, const double* __restrict__ T, const do
 // One block per virtual v, accumulating over items (l,b,c) for all holes:
 //   mode 0 (tau21): out(v,m) = -1/(e_m - e_v) sum_{lbc} A1[(b,l),(c,m)] (2(vc|lb) - (vb|lc))
 //   mode 1 (tau24): out(v,k) =  1/(e_k - e_v) sum_{lbc} A1[(c,l),(b,k)] (2(vb|lc) - (vc|lb))
-// (A1 is symmetric, so A1[(c,l),(b,k)] = A1[(b,k),(c,l)]); vvov = (ab|ic) [a][b][i][c].
+// (A1 is symmetric, so A1[(c,l),(b,k)] = A1[(b,k),(c,l)]); vvov = (ab|ic) [b][i][c][a].
 __global__ void __launch_bounds__(256) k_fv_tau_vo(int mode, int no, int nv, const double* __restrict__ e,
                                                    const double* __restrict__ A1, const double* __restrict__ vvov,
                                                    double* __restrict__ out) {

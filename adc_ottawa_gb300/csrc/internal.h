@@ -427,7 +427,7 @@ struct SigmaPlan {
   int ntitems = 0;
   void* d_acc = nullptr;      // FP64 accumulator of the singles rows (FP32 path)
   size_t acc_bytes = 0;
-  void* d_sk = nullptr;       // split-K partials of the FP32 singles block
+  void* d_sk = nullptr;       // split-K partials of the singles block (FP64 or FP32)
   size_t sk_bytes = 0;
   void* umma = nullptr;       // tensor-core pass plan (sigma_umma.cu), built on first use
   int umma_off = 0;           // 1: the tensor-core pass is not used

@@ -62,7 +62,9 @@ constexpr int UMMA_THREADS = 320;             // producer, MMA issuer, 8 epilogu
 constexpr int UMMA_NOP = 16;                  // segment A lengths (noP) up to 16 (nocc <= 16)
 // an item's X operand and W1 atomics in tiles (nocc=9/nvirt=101, 5 columns:
 // 4,096 rows make two rounds, 86 us for the pass, 512 rows six rounds, 81 us;
-// the rule's choice takes 70 us)
+// the rule's choice takes 70 us).  The product is not sensitive to it: with 1, 5
+// and 15 tiles, 40 columns, 428, 440, 441 us there, 612, 613, 614 at 10/110, 1535,
+// 1600, 1598 at 16/120, 3207, 3319, 3331 at 16/180.
 constexpr double UMMA_ITEM_OVERHEAD = 5.0;
 // rows per work item of the FP32-value main pass: the W1 sums of an item run
 // in one TMEM chain (8 MMA steps per 128-row tile), and shorter chains keep

@@ -343,10 +343,10 @@ int adcgpu_autocorr(adcgpu_ctx* ctx, int nwp, const double* f, double tout,
    [vector][k], C_k = <q_0|q_k> for k <= ord and the doubling formulas above.
    q1h1p (may be NULL, the save1h1p output): the first nocc*nvirt elements of
    q_0..q_ord, layout [vector][k][n1].
-   df != 0: for nvec >= 16 the sigma product's tiled pass runs in double-float
-   arithmetic on the FP32 pipe (a 48-bit significand, about 1e-14 relative
-   per product) instead of native FP64, whose pipe GB300 runs at 1/64 of the
-   FP32 rate; df = 0 is the plain FP64 path. */
+   df != 0: sigma products of 16 or more columns that do not run on the tensor
+   cores (adcgpu_set_fp64_arith) use double-float arithmetic on the FP32 pipe (a
+   48-bit significand, about 1e-14 relative per product) instead of native FP64,
+   whose pipe GB300 runs at 1/64 of the FP32 rate; df = 0 is the plain FP64 path. */
 int adcgpu_chebyshev_auto(adcgpu_ctx* ctx, int nvec, const double* q0,
                           const double* bounds, int chebyord, int df,
                           double* auto_out, double* q1h1p, int* order_out);
@@ -417,7 +417,8 @@ double adcgpu_last_sigma_ms(const adcgpu_ctx* ctx);
    per FP64 value and 8 per FP32 value, with rows padded to 64 values and slabs to
    128 rows, which multiplies them for small systems).  A matrix whose digits do
    not fit a third of the memory that is free at its first product keeps its other
-   kernels.  The digits are given back when an allocation of any context of the
+   kernels, and products of few columns, which those are faster for, make none.  Digits
+   of up to 128 MB stay with the context when their matrix goes, for the next one.  The digits are given back when an allocation of any context of the
    process on the device finds no room (the next product then asks again). */
 int64_t adcgpu_device_bytes(const adcgpu_ctx* ctx);
 
@@ -427,7 +428,10 @@ int64_t adcgpu_device_bytes(const adcgpu_ctx* ctx);
    precision pairs, about 1e-14 relative per product) for the subspace GEMMs,
    which the GB300's FP64 rate (1/64 of FP32) makes several times faster, and
    for sigma products of 16 or more columns that do not run on the tensor
-   cores (those are as accurate as FP64 arithmetic in either mode).  It
+   cores.  (Those that do are as accurate as FP64 multiply-adds in either mode,
+   normwise: an element's error is a few 2^-55 of the largest coupling of its
+   row times the largest entry of the column that it meets, also where its own
+   couplings or entries are much smaller.  FP32 values likewise at 2^-31.)  It
    applies to every solver that runs on the context (Davidson, Lanczos, SIL,
    Chebyshev); the mixed ladder's FP64 refinement always uses 1. */
 int adcgpu_set_fp64_arith(adcgpu_ctx* ctx, int mode);
@@ -493,7 +497,8 @@ int adcgpu_sigma_autotune(adcgpu_ctx* ctx, int m, int* best_chunk, int* best_mc,
    FP32 value store instead of the BF16 one, bit 9 keeps the FP32 Gram
    products (adcgpu_gram_f32 and the solvers' V^T W) on the CUDA cores, bit
    10 runs the FP32 values on two tcgen05 passes over their BF16 slices
-   instead of the exact digit slices. */
+   instead of the exact digit slices.  A CVS matrix has no launch shapes: status
+   16 (ADCGPU_UNSUPPORTED). */
 int adcgpu_sigma_set_shape(adcgpu_ctx* ctx, int chunk, int mc_fp64, int mc_fp32);
 
 /* The solvers' tall-skinny Gram product on device FP32 arrays: C(p x q,
