@@ -69,8 +69,7 @@ template <> __device__ inline float to_f<__nv_bfloat16>(__nv_bfloat16 x) { retur
 template <> __device__ inline float to_f<float>(float x) { return x; }
 
 // Copies Y, Z and the coincident entries out of the value store.
-template <typename TV>
-__global__ void k_ab_extract(GeomDev g, const TV* __restrict__ Bt, int nslab, float* __restrict__ Y,
+__global__ void k_ab_extract(GeomDev g, const float* __restrict__ Bt, int nslab, float* __restrict__ Y,
                              float* __restrict__ Z, float4* __restrict__ coin) {
   const int nv = g.nv, no = g.no, noP = g.noP;
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
@@ -86,11 +85,11 @@ __global__ void k_ab_extract(GeomDev g, const TV* __restrict__ Bt, int nslab, fl
     float y = 0.f, z = 0.f;
     if (kin && x >= 1) {           // row (0, x): segment A at k
       const int64_t row = ps.row0 + pair_index(0, x, nv);
-      y = to_f(Bt[g.off[ps.cls] + (row - g.start[ps.cls]) * L + k]);
+      y = Bt[g.off[ps.cls] + (row - g.start[ps.cls]) * L + k];
     }
     if (kin && x <= nv - 2) {      // row (x, nv - 1): segment B at k
       const int64_t row = ps.row0 + pair_index(x, nv - 1, nv);
-      z = to_f(Bt[g.off[ps.cls] + (row - g.start[ps.cls]) * L + noP + k]);
+      z = Bt[g.off[ps.cls] + (row - g.start[ps.cls]) * L + noP + k];
     }
     Y[i] = y;
     Z[i] = z;
@@ -108,12 +107,12 @@ __global__ void k_ab_extract(GeomDev g, const TV* __restrict__ Bt, int nslab, fl
     } else {
       pair_decode(rl / g.npair_v, no, kp, lp);
     }
-    const TV* rp = Bt + g.off[cls] + rl * L;
+    const float* rp = Bt + g.off[cls] + rl * L;
     float4 q;
-    q.x = to_f(rp[kp]);
-    q.y = kp != lp ? to_f(rp[lp]) : 0.f;
-    q.z = to_f(rp[noP + kp]);
-    q.w = kp != lp ? to_f(rp[noP + lp]) : 0.f;
+    q.x = rp[kp];
+    q.y = kp != lp ? rp[lp] : 0.f;
+    q.z = rp[noP + kp];
+    q.w = kp != lp ? rp[noP + lp] : 0.f;
     coin[t] = q;
   }
 }
@@ -345,10 +344,11 @@ __device__ __forceinline__ void seg_frag(const float (&x)[2][4], uint32_t (&f)[3
 }
 
 constexpr int SEG_F = 8;
-template <int KT, bool SEGB>
+template <bool SEGB>
 __global__ void __launch_bounds__(32 * SEG_F)
     k_seg_bf16(GeomDev g, int nslab, int ngrp, const __nv_bfloat16* __restrict__ seg, const float* __restrict__ V,
                  int64_t ldv, int m, float* __restrict__ W, int64_t ldw, double* __restrict__ W1, int64_t ld1) {
+  constexpr int KT = 1;   // k tiles of 16 holes: the pass takes nocc <= 16
   constexpr int PITCH = KT * 32 + 16, KW = 16 * KT, NPIECE = 32 * KT;
   constexpr int PA = SEG_F + 1, PC = 16 * PA + 1;        // pitches of a' and c in the tiles
   __shared__ __align__(16) unsigned char smem_seg[SEG_F * 2 * 16 * PITCH];
@@ -621,7 +621,7 @@ static int ab_tables(Ctx* c, void*& handle, int which, const void* Bt) {
   if (!t.Y && (st = dmalloc(c, (void**)&t.Y, sizeof(float) * ntab))) return st;
   if (!t.Z && (st = dmalloc(c, (void**)&t.Z, sizeof(float) * ntab))) return st;
   if (!t.coin && (st = dmalloc(c, (void**)&t.coin, sizeof(float4) * std::max<size_t>(nrow, 1)))) return st;
-  k_ab_extract<float><<<c->nsm * 8, 256, 0, c->stream>>>(g, (const float*)Bt, nslab, t.Y, t.Z, t.coin);
+  k_ab_extract<<<c->nsm * 8, 256, 0, c->stream>>>(g, (const float*)Bt, nslab, t.Y, t.Z, t.coin);
   ADC_COUNT_LAUNCH();
   ADC_CUDA(c, cudaGetLastError());
   t.made_from = Bt;
@@ -665,9 +665,9 @@ int ab_launch(Ctx* c, void*& handle, const TV* Bt, bool do_a, const float* V, in
       ADC_CUDA(c, cudaGetLastError());
       return ADCGPU_OK;
     };
-    // BF16 values are stored for nocc <= 16 only (umma_supported): one k tile
-    if (do_a) ST(seg(k_seg_bf16<1, false>));
-    ST(seg(k_seg_bf16<1, true>));
+    // (the pass takes nocc <= 16 only, umma_supported)
+    if (do_a) ST(seg(k_seg_bf16<false>));
+    ST(seg(k_seg_bf16<true>));
   } else if (nslab > 0) {
     switch (G.noP) {
       case 8: ST(do_a ? pairs(k_ab_pairs<8, true>) : pairs(k_ab_pairs<8, false>)); break;

@@ -588,7 +588,7 @@ bool umma_supported(const Ctx* c) {
     cudaGetLastError();
     return false;
   }
-  // segment A in registers (noP <= 24), C|D of at most six 64-value boxes
+  // segment A in registers (noP <= 16), C|D of at most six 64-value boxes
   return major >= 10 && umma_geometry_ok(G) && c->d_Bt16 != nullptr && encode_fn() != nullptr;
 }
 
